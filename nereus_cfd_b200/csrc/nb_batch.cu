@@ -610,7 +610,7 @@ struct Batch
             tailStart = A.tailStart;
             views.clear();
             for (auto &Lv : A.L) views.push_back(Lv.view());
-            PrepareSplitKernels();
+            PrepareSplitKernels(sizeof(float));
             PrepareTail<float>(kTailMaxSmem);
             dirty = true;
             tuning.clear();

@@ -41,13 +41,13 @@ struct LevelView
     // the mid axis and marches `slowChunk` steps along the slow axis. 3D: (fast, mid, slow) = (k, j, i);
     // 2D: (j, i, -) with slowLen = 1.
     int fastLen, midLen, slowLen, slowChunk;
-    // Colour-split layout of the level's FP32 vectors (sRS = 0: the grid layout). Cell (i, j, k) of colour
+    // Colour-split layout of the level's solver vectors (sRS = 0: the grid layout). Cell (i, j, k) of colour
     // c = (i+j+k) & 1 sits at c*sHalf + i*sPS + j*sRS + (k >> 1): each colour is an Ny x Nx x sRS array whose rows
     // hold the Nz/2 cells of that colour, padded with zeros to a multiple of 4.
     int sRS, sPS;
     long long sHalf;
-    // Colour-split level: act[i * actTiles + t] != 0 when tile t of plane i (elements 1024 t .. 1024 t + 1023 of
-    // either colour's plane, the cells one block of a quad kernel owns on that plane) holds an unknown; null: every
+    // Colour-split level: act[i * actTiles + t] != 0 when tile t of plane i (1024 FP32 or 512 FP64 elements of either
+    // colour's plane, the cells one block of a quad kernel owns on that plane) holds an unknown; null: every
     // tile counts as holding one. A block whose planes' tiles hold none skips its work: its cells stay zero.
     const uint8_t *act;
     int actTiles;

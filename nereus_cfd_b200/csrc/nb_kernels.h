@@ -99,43 +99,55 @@ void LaunchPairRefine64(const LevelView &v, const uint8_t *du, const double *b, 
 void LaunchLinDot(long long cells, const float *r, const float *z, const Reducer &R, const int *it, int baseEven,
                   int baseOdd, cudaStream_t st);
 // the same on a colour-split level 0 (v), skipping the tiles its activity marks empty (all tiles without one)
-void LaunchSplitLinXR(const LevelView &v, long long vecLen, float *x, float *r, const float *p0, const float *p1,
-                      const float *q, const Reducer &R, const double *S, int *it, int baseEven, int baseOdd, int slotN,
+template <typename T>
+void LaunchSplitLinXR(const LevelView &v, long long vecLen, T *x, T *r, const T *p0, const T *p1, const T *q,
+                      const Reducer &R, const double *S, int *it, int baseEven, int baseOdd, int slotN,
                       int singular, int slotPQ, int slotRR, cudaStream_t st);
 void LaunchBatchLinXR(const BatchLevel *lv, int ls, const BatchReq *rq, BatchList a, int cap, int baseEven,
                       int baseOdd, int slotN, int slotPQ, int slotRR, cudaStream_t st);
-void LaunchLinXR(long long cells, float *x, float *r, const float *p0, const float *p1, const float *q,
-                 const Reducer &R, const double *S, int *it, int baseEven, int baseOdd, int slotN, int singular,
-                 int slotPQ, int slotRR, cudaStream_t st);
+template <typename T>
+void LaunchLinXR(long long cells, T *x, T *r, const T *p0, const T *p1, const T *q, const Reducer &R,
+                 const double *S, int *it, int baseEven, int baseOdd, int slotN, int singular, int slotPQ, int slotRR,
+                 cudaStream_t st);
 
-// ---- nb_split.cu: FP32 kernels for 3D levels with Nz even in the colour-split layout (LevelView::sRS) ----
+// ---- nb_split.cu: kernels for 3D levels with Nz even in the colour-split layout (LevelView::sRS), T = float (the
+//      mixed form's inner solve) or double (the plain FP64 form) ----
 // uniform levels only; du: the level's diagonal units in that layout; pext: the red cells' bytes
 // reads the kernels' occupancy (their grids follow it); call before capturing launches into a graph
-void PrepareSplitKernels();
+void PrepareSplitKernels(int elemBytes);
 // the first red-black sweep from a zero iterate
-void LaunchSplitFirst(const LevelView &v, const uint8_t *du, const float *r, float *e, cudaStream_t st);
-void LaunchSplitHalf(const LevelView &v, const uint8_t *du, const float *r, float *e, int colour, cudaStream_t st);
+template <typename T>
+void LaunchSplitFirst(const LevelView &v, const uint8_t *du, const T *r, T *e, cudaStream_t st);
+template <typename T>
+void LaunchSplitHalf(const LevelView &v, const uint8_t *du, const T *r, T *e, int colour, cudaStream_t st);
 // the post-smoothing's last sweep on level 0: the black half (last = false) sums its (r.z, z, r) into
 // out[partSlot..], the red half (last = true) adds its own into the scalar block of the iteration's parity
-void LaunchSplitHalfDot(const LevelView &v, const uint8_t *du, const float *r, float *e, int colour, bool last,
+template <typename T>
+void LaunchSplitHalfDot(const LevelView &v, const uint8_t *du, const T *r, T *e, int colour, bool last,
                         const Reducer &R, const int *it, int baseEven, int baseOdd, int partSlot, cudaStream_t st);
 // the red residual after a sweep that ended black (into the first half of res)
-void LaunchSplitResidual(const LevelView &v, const uint8_t *du, const float *r, const float *e, float *res,
-                         cudaStream_t st);
-void LaunchSplitProlong(const LevelView &fine, const LevelView &coarse, const uint8_t *pext, const float *eCoarse,
-                        float *eFine, cudaStream_t st);
-// mode: 0 by the coarse level's size, 1 one thread per coarse cell, 2 one thread per 4 coarse cells (same result)
-void LaunchSplitRestrict(const LevelView &fine, const LevelView &coarse, const uint8_t *pext, const float *resFine,
-                         float *rCoarse, int mode, cudaStream_t st);
-void LaunchSplitPApply(const LevelView &v, const uint8_t *du, const float *z, float *p0, float *p1, float *q,
+template <typename T>
+void LaunchSplitResidual(const LevelView &v, const uint8_t *du, const T *r, const T *e, T *res, cudaStream_t st);
+template <typename T>
+void LaunchSplitProlong(const LevelView &fine, const LevelView &coarse, const uint8_t *pext, const T *eCoarse,
+                        T *eFine, cudaStream_t st);
+// mode: 0 by the coarse level's size, 1 one thread per coarse cell, 2 one thread per quad of them (same result)
+template <typename T>
+void LaunchSplitRestrict(const LevelView &fine, const LevelView &coarse, const uint8_t *pext, const T *resFine,
+                         T *rCoarse, int mode, cudaStream_t st);
+template <typename T>
+void LaunchSplitPApply(const LevelView &v, const uint8_t *du, const T *z, T *p0, T *p1, T *q,
                        const Reducer &R, const double *S, const int *it, int baseEven, int baseOdd, int slotN,
                        int singular, int slotPQ, cudaStream_t st);
-void LaunchSplitScaleSum(const LevelView &v, const double *b, float *r, double sfac, const Reducer &R, int slot,
+template <typename T>
+void LaunchSplitScaleSum(const LevelView &v, const double *b, T *r, double sfac, const Reducer &R, int slot,
                          cudaStream_t st);
-// the tiles of a plane of a colour-split level (1024 elements each, the cells one quad-kernel block owns), and the
-// activity bytes of every (plane, tile): nonzero where a tile holds an unknown of either colour (LevelView::act)
-int SplitActivityTiles(const LevelView &v);
-void LaunchSplitActivity(const LevelView &v, const uint8_t *du, uint8_t *act, int tiles, cudaStream_t st);
+// the tiles of a plane of a colour-split level (the elements one quad-kernel block owns: 1024 floats or 512 doubles),
+// and the activity bytes of every (plane, tile): nonzero where a tile holds an unknown of either colour
+// (LevelView::act)
+int SplitActivityTiles(const LevelView &v, int elemBytes);
+void LaunchSplitActivity(const LevelView &v, const uint8_t *du, uint8_t *act, int tiles, int elemBytes,
+                         cudaStream_t st);
 // the batched forms (nb_batch.cu): kind NB_BK_*; S the march length of the non-reducing kernels; coarse: the next
 // coarser level (restriction, prolongation); mode: the restriction's kernel (1 per coarse cell, else per 4)
 enum : int { NB_BK_FIRST = 0, NB_BK_HALF, NB_BK_RESIDUAL, NB_BK_RESTRICT, NB_BK_PROLONG, NB_BK_COUNT };
@@ -150,8 +162,9 @@ void LaunchBatchSplitScaleSum(const BatchLevel *lv, int ls, const BatchReq *rq, 
                               cudaStream_t st);
 void LaunchBatchSplitRefine64(const LevelView &v, const BatchLevel *lv, int ls, const BatchReq *rq, BatchList a,
                               int cap, const int *parity, int slot, cudaStream_t st);
-void LaunchSplitRefine64(const LevelView &v, const uint8_t *du, const double *b, const double *xin, const float *e,
-                         double *xout, float *r, double scale, double sfac, const Reducer &R, int slot,
+template <typename T>
+void LaunchSplitRefine64(const LevelView &v, const uint8_t *du, const double *b, const double *xin, const T *e,
+                         double *xout, T *r, double scale, double sfac, const Reducer &R, int slot,
                          cudaStream_t st, const int *swap = nullptr);
 
 // ---- nb_kernels.cu: multigrid and PCG kernels, T = float (inner solve) or double (plain FP64) ----

@@ -947,35 +947,61 @@ __global__ void __launch_bounds__(256) k_lin_dot(long long cells, const float *_
     GridReduce<3>(R, acc, base);
 }
 
+// 16 bytes of a vector: four floats or two doubles
+template <typename T> struct Vec16;
+template <> struct Vec16<float>
+{
+    using V = float4;
+};
+template <> struct Vec16<double>
+{
+    using V = double2;
+};
+// x += a p, r -= a q on 16 bytes; returns the sum of r^2
+__device__ __forceinline__ double XR16(float a, const float4 &pv, const float4 &qv, float4 &xv, float4 &rv)
+{
+    xv.x += a * pv.x; xv.y += a * pv.y; xv.z += a * pv.z; xv.w += a * pv.w;
+    rv.x -= a * qv.x; rv.y -= a * qv.y; rv.z -= a * qv.z; rv.w -= a * qv.w;
+    return ((double)rv.x * rv.x + (double)rv.y * rv.y) + ((double)rv.z * rv.z + (double)rv.w * rv.w);
+}
+__device__ __forceinline__ double XR16(double a, const double2 &pv, const double2 &qv, double2 &xv, double2 &rv)
+{
+    xv.x += a * pv.x; xv.y += a * pv.y;
+    rv.x -= a * qv.x; rv.y -= a * qv.y;
+    return rv.x * rv.x + rv.y * rv.y;
+}
+
 // alpha = rz / pq; x += alpha p; r -= alpha q; sum r.r; the last block advances the iteration counter
 // bx of gx: this block among the launch's blocks (a grid-stride loop)
-__device__ __forceinline__ void LinXR(long long cells, float *__restrict__ x, float *__restrict__ r, const float *p0,
-                                      const float *p1, const float *__restrict__ q, const Reducer &R, const double *S,
+template <typename T>
+__device__ __forceinline__ void LinXR(long long cells, T *__restrict__ x, T *__restrict__ r, const T *p0,
+                                      const T *p1, const T *__restrict__ q, const Reducer &R, const double *S,
                                       int *it, int baseEven, int baseOdd, int slotN, int singular, int slotPQ,
                                       int slotRR, int bx, int gx)
 {
+    using V = typename Vec16<T>::V;
+    constexpr int N = 16 / (int)sizeof(T);
     const int par = *it & 1;
-    const float *__restrict__ p = par ? p0 : p1;
+    const T *__restrict__ p = par ? p0 : p1;
     const int base = par ? baseOdd : baseEven;
-    const float a = (float)(RzEffP(S, base, S[slotN], singular) / S[slotPQ]);
+    const T a = (T)(RzEffP(S, base, S[slotN], singular) / S[slotPQ]);
     double acc[1] = {0.0};
-    const long long n4 = cells >> 2, stride = (long long)gx * blockDim.x;
-    float4 *x4 = reinterpret_cast<float4 *>(x), *r4 = reinterpret_cast<float4 *>(r);
-    const float4 *p4 = reinterpret_cast<const float4 *>(p), *q4 = reinterpret_cast<const float4 *>(q);
-    for (long long t = bx * (long long)blockDim.x + threadIdx.x; t < n4; t += stride)
+    const long long nv = cells / N, stride = (long long)gx * blockDim.x;
+    V *x4 = reinterpret_cast<V *>(x), *r4 = reinterpret_cast<V *>(r);
+    const V *p4 = reinterpret_cast<const V *>(p), *q4 = reinterpret_cast<const V *>(q);
+    for (long long t = bx * (long long)blockDim.x + threadIdx.x; t < nv; t += stride)
     {
-        const float4 pv = p4[t], qv = q4[t];
-        float4 xv = x4[t], rv = r4[t];
-        xv.x += a * pv.x; xv.y += a * pv.y; xv.z += a * pv.z; xv.w += a * pv.w;
-        rv.x -= a * qv.x; rv.y -= a * qv.y; rv.z -= a * qv.z; rv.w -= a * qv.w;
+        const V pv = p4[t], qv = q4[t];
+        V xv = x4[t], rv = r4[t];
+        const double rr = XR16(a, pv, qv, xv, rv);
         x4[t] = xv;
         r4[t] = rv;
-        acc[0] += ((double)rv.x * rv.x + (double)rv.y * rv.y) + ((double)rv.z * rv.z + (double)rv.w * rv.w);
+        acc[0] += rr;
     }
-    for (long long t = 4 * n4 + bx * (long long)blockDim.x + threadIdx.x; t < cells; t += stride)
+    for (long long t = N * nv + bx * (long long)blockDim.x + threadIdx.x; t < cells; t += stride)
     {
         x[t] += a * p[t];
-        const float rn = r[t] - a * q[t];
+        const T rn = r[t] - a * q[t];
         r[t] = rn;
         acc[0] += (double)rn * rn;
     }
@@ -983,60 +1009,64 @@ __device__ __forceinline__ void LinXR(long long cells, float *__restrict__ x, fl
 }
 
 // The same update on a colour-split level 0 with its tile activity (LevelView::act): the vector walked tile by tile
-// (1024 elements of one colour's plane), the tiles that hold no unknown skipped (p and q are zero there, so x and r
-// stay as they are and add nothing to r.r).
-__device__ __forceinline__ void LinXRTiles(const LevelView &v, float *__restrict__ x, float *__restrict__ r,
-                                           const float *p0, const float *p1, const float *__restrict__ q,
+// (a quad-kernel block's elements of one colour's plane), the tiles that hold no unknown skipped (p and q are zero
+// there, so x and r stay as they are and add nothing to r.r).
+template <typename T>
+__device__ __forceinline__ void LinXRTiles(const LevelView &v, T *__restrict__ x, T *__restrict__ r,
+                                           const T *p0, const T *p1, const T *__restrict__ q,
                                            const Reducer &R, const double *S, int *it, int baseEven, int baseOdd,
                                            int slotN, int singular, int slotPQ, int slotRR, int bx, int gx)
 {
+    using V = typename Vec16<T>::V;
+    constexpr int N = 16 / (int)sizeof(T);
     const int par = *it & 1;
-    const float *__restrict__ p = par ? p0 : p1;
+    const T *__restrict__ p = par ? p0 : p1;
     const int base = par ? baseOdd : baseEven;
-    const float a = (float)(RzEffP(S, base, S[slotN], singular) / S[slotPQ]);
+    const T a = (T)(RzEffP(S, base, S[slotN], singular) / S[slotPQ]);
     double acc[1] = {0.0};
     const int tiles = v.actTiles, perColour = v.Ny * tiles, units = 2 * perColour;
     for (int u = bx; u < units; u += gx)
     {
         const int c = u / perColour, rem = u - c * perColour, i = rem / tiles, t = rem - i * tiles;
         if (!v.act[(long long)i * tiles + t]) continue;
-        const long long e0 = (long long)c * v.sHalf + (long long)i * v.sPS + 4LL * kPairThreads * t;
-        const int n4 = min(kPairThreads, (v.sPS - 4 * kPairThreads * t) >> 2);
-        for (int k = threadIdx.x; k < n4; k += blockDim.x)
+        const long long e0 = (long long)c * v.sHalf + (long long)i * v.sPS + (long long)N * kPairThreads * t;
+        const int nv = min(kPairThreads, (v.sPS - N * kPairThreads * t) / N);
+        for (int k = threadIdx.x; k < nv; k += blockDim.x)
         {
-            const long long o = e0 + 4LL * k;
-            const float4 pv = *reinterpret_cast<const float4 *>(p + o), qv = *reinterpret_cast<const float4 *>(q + o);
-            float4 xv = *reinterpret_cast<float4 *>(x + o), rv = *reinterpret_cast<float4 *>(r + o);
-            xv.x += a * pv.x; xv.y += a * pv.y; xv.z += a * pv.z; xv.w += a * pv.w;
-            rv.x -= a * qv.x; rv.y -= a * qv.y; rv.z -= a * qv.z; rv.w -= a * qv.w;
-            *reinterpret_cast<float4 *>(x + o) = xv;
-            *reinterpret_cast<float4 *>(r + o) = rv;
-            acc[0] += ((double)rv.x * rv.x + (double)rv.y * rv.y) + ((double)rv.z * rv.z + (double)rv.w * rv.w);
+            const long long o = e0 + (long long)N * k;
+            const V pv = *reinterpret_cast<const V *>(p + o), qv = *reinterpret_cast<const V *>(q + o);
+            V xv = *reinterpret_cast<V *>(x + o), rv = *reinterpret_cast<V *>(r + o);
+            const double rr = XR16(a, pv, qv, xv, rv);
+            *reinterpret_cast<V *>(x + o) = xv;
+            *reinterpret_cast<V *>(r + o) = rv;
+            acc[0] += rr;
         }
     }
     GridReduceB<1>(R, acc, slotRR, (unsigned)bx, (unsigned)gx, 0, it);
 }
 
-__global__ void __launch_bounds__(256) k_lin_xr_tiles(LevelView v, float *__restrict__ x, float *__restrict__ r,
-                                                      const float *p0, const float *p1, const float *__restrict__ q,
+template <typename T>
+__global__ void __launch_bounds__(256) k_lin_xr_tiles(LevelView v, T *__restrict__ x, T *__restrict__ r,
+                                                      const T *p0, const T *p1, const T *__restrict__ q,
                                                       Reducer R, const double *S, int *it, int baseEven, int baseOdd,
                                                       int slotN, int singular, int slotPQ, int slotRR)
 {
     PdlWait();
     PdlTrigger();
-    LinXRTiles(v, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, (int)blockIdx.x,
-               (int)gridDim.x);
+    LinXRTiles<T>(v, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, (int)blockIdx.x,
+                  (int)gridDim.x);
 }
 
-__global__ void __launch_bounds__(256) k_lin_xr(long long cells, float *__restrict__ x, float *__restrict__ r,
-                                                const float *p0, const float *p1, const float *__restrict__ q,
+template <typename T>
+__global__ void __launch_bounds__(256) k_lin_xr(long long cells, T *__restrict__ x, T *__restrict__ r,
+                                                const T *p0, const T *p1, const T *__restrict__ q,
                                                 Reducer R, const double *S, int *it, int baseEven, int baseOdd, int slotN,
                                                 int singular, int slotPQ, int slotRR)
 {
     PdlWait();
     PdlTrigger();
-    LinXR(cells, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, (int)blockIdx.x,
-          (int)gridDim.x);
+    LinXR<T>(cells, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, (int)blockIdx.x,
+             (int)gridDim.x);
 }
 
 // batched (nb_batch.cu): block z runs the request at list[z]; r is its level 0's r
@@ -1051,10 +1081,10 @@ __global__ void __launch_bounds__(256) kb_lin_xr(const BatchLevel *__restrict__ 
     const BatchReq &Q = rq[q];
     const BatchLevel &L = lv[q * ls];
     if (L.v.act)
-        LinXRTiles(L.v, Q.x, L.r, Q.p0, Q.p1, Q.q, Q.red, Q.red.out, Q.it, baseEven, baseOdd, slotN, Q.singular,
+        LinXRTiles<float>(L.v, Q.x, L.r, Q.p0, Q.p1, Q.q, Q.red, Q.red.out, Q.it, baseEven, baseOdd, slotN, Q.singular,
                    slotPQ, slotRR, (int)blockIdx.x, (int)gridDim.x);
     else
-        LinXR(Q.vecLen, Q.x, L.r, Q.p0, Q.p1, Q.q, Q.red, Q.red.out, Q.it, baseEven, baseOdd, slotN, Q.singular,
+        LinXR<float>(Q.vecLen, Q.x, L.r, Q.p0, Q.p1, Q.q, Q.red, Q.red.out, Q.it, baseEven, baseOdd, slotN, Q.singular,
               slotPQ, slotRR, (int)blockIdx.x, (int)gridDim.x);
 }
 
@@ -1073,27 +1103,38 @@ void LaunchBatchLinXR(const BatchLevel *lv, int ls, const BatchReq *rq, BatchLis
               slotRR);
 }
 
-void LaunchSplitLinXR(const LevelView &v, long long vecLen, float *x, float *r, const float *p0, const float *p1,
-                      const float *q, const Reducer &R, const double *S, int *it, int baseEven, int baseOdd, int slotN,
-                      int singular, int slotPQ, int slotRR, cudaStream_t st)
+template <typename T>
+void LaunchLinXR(long long cells, T *x, T *r, const T *p0, const T *p1, const T *q, const Reducer &R,
+                 const double *S, int *it, int baseEven, int baseOdd, int slotN, int singular, int slotPQ, int slotRR,
+                 cudaStream_t st)
 {
-    if (!v.act)
-    {
-        LaunchLinXR(vecLen, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, st);
-        return;
-    }
     NB_COUNT_LAUNCH();
-    LaunchPdl(k_lin_xr_tiles, dim3(kLinBlocks), dim3(256), 0, st, v, x, r, p0, p1, q, R, S, it, baseEven, baseOdd,
+    LaunchPdl(k_lin_xr<T>, dim3(kLinBlocks), dim3(256), 0, st, cells, x, r, p0, p1, q, R, S, it, baseEven, baseOdd,
               slotN, singular, slotPQ, slotRR);
 }
 
-void LaunchLinXR(long long cells, float *x, float *r, const float *p0, const float *p1, const float *q,
-                 const Reducer &R, const double *S, int *it, int baseEven, int baseOdd, int slotN, int singular,
-                 int slotPQ, int slotRR, cudaStream_t st)
+template <typename T>
+void LaunchSplitLinXR(const LevelView &v, long long vecLen, T *x, T *r, const T *p0, const T *p1, const T *q,
+                      const Reducer &R, const double *S, int *it, int baseEven, int baseOdd, int slotN, int singular,
+                      int slotPQ, int slotRR, cudaStream_t st)
 {
+    if (!v.act)
+    {
+        LaunchLinXR<T>(vecLen, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, st);
+        return;
+    }
     NB_COUNT_LAUNCH();
-    LaunchPdl(k_lin_xr, dim3(kLinBlocks), dim3(256), 0, st, cells, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN,
-              singular, slotPQ, slotRR);
+    LaunchPdl(k_lin_xr_tiles<T>, dim3(kLinBlocks), dim3(256), 0, st, v, x, r, p0, p1, q, R, S, it, baseEven, baseOdd,
+              slotN, singular, slotPQ, slotRR);
 }
+
+template void LaunchLinXR<float>(long long, float *, float *, const float *, const float *, const float *,
+                                 const Reducer &, const double *, int *, int, int, int, int, int, int, cudaStream_t);
+template void LaunchSplitLinXR<float>(const LevelView &, long long, float *, float *, const float *, const float *,
+                                      const float *, const Reducer &, const double *, int *, int, int, int, int, int,
+                                      int, cudaStream_t);
+template void LaunchSplitLinXR<double>(const LevelView &, long long, double *, double *, const double *,
+                                       const double *, const double *, const Reducer &, const double *, int *, int,
+                                       int, int, int, int, int, cudaStream_t);
 
 } // namespace nb

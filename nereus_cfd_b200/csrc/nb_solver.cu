@@ -352,13 +352,13 @@ void Context::BuildHierarchy()
     NB_CK(cudaGetLastError());
 }
 
-// The colour-split levels (pair_kernels = 2, mixed precision): the uniform 3D levels with Nz even above the coarse
+// The colour-split levels (pair_kernels = 2): the uniform 3D levels with Nz even above the coarse
 // end, as long as every finer level is one too (a level's transfers read and write the next coarser level in either
 // layout, the grid-layout kernels only the grid layout). A stretched grid keeps the cell-pair kernels: its
 // per-cell coefficients make the split kernels compute-bound (measured slower on the stretched cylinder).
 void Context::AssignSplit()
 {
-    const bool on = opt.precision == NB_PRECISION_MIXED && opt.pair_kernels == 2 && !nonuniform;
+    const bool on = opt.pair_kernels == 2 && !nonuniform;
     bool finer = true;
     for (size_t l = 0; l < L.size(); l++)
     {
@@ -380,23 +380,26 @@ void Context::AssignSplit()
 // and the prolongation's moved weights.
 void Context::BuildPairData()
 {
-    // the FP32 kernels' diagonal units (mixed precision: the inner solve runs in FP32)
+    // the diagonal units: of the colour-split levels in either precision, and of the cell-pair levels, whose kernels
+    // are FP32 (the mixed form's inner solve)
+    const bool mixed = opt.precision == NB_PRECISION_MIXED;
+    const int elem = mixed ? (int)sizeof(float) : (int)sizeof(double);
     for (auto &Lv : L)
     {
         const LevelView v = Lv.view();
-        if (opt.precision == NB_PRECISION_MIXED && opt.pair_kernels && PairLevelShape(v))
+        if (Lv.sRS || (mixed && opt.pair_kernels && PairLevelShape(v)))
         {
             if (Lv.sRS)
             {
-                PrepareSplitKernels();
+                PrepareSplitKernels(elem);
                 Lv.du.alloc((size_t)(2 * Lv.sHalf));
                 Lv.du.zero(st); // the padding
                 LaunchBuildDu(v, Lv.du.p, st);
                 if (opt.skip_idle_tiles)
                 {
-                    Lv.actTiles = SplitActivityTiles(v);
+                    Lv.actTiles = SplitActivityTiles(v, elem);
                     Lv.act.alloc((size_t)Lv.Ny * Lv.actTiles);
-                    LaunchSplitActivity(v, Lv.du.p, Lv.act.p, Lv.actTiles, st);
+                    LaunchSplitActivity(v, Lv.du.p, Lv.act.p, Lv.actTiles, elem, st);
                 }
                 else
                 {
@@ -466,14 +469,13 @@ void Context::AllocVectors()
     for (size_t l = 0; l < L.size(); l++)
     {
         LevelData &Lv = L[l];
-        const size_t c = (size_t)Lv.cells;
+        const size_t c = Lv.VecLen(); // zeroed whole: the split layout's padding stays zero
         const bool last = l + 1 == L.size();
         if (mixed)
         {
-            const size_t c32 = Lv.VecLen(); // zeroed whole: the split layout's padding stays zero
-            Lv.r32.alloc(c32); Lv.r32.zero(st);
-            Lv.e32.alloc(c32); Lv.e32.zero(st);
-            if (!last) { Lv.res32.alloc(c32); Lv.res32.zero(st); }
+            Lv.r32.alloc(c); Lv.r32.zero(st);
+            Lv.e32.alloc(c); Lv.e32.zero(st);
+            if (!last) { Lv.res32.alloc(c); Lv.res32.zero(st); }
             Lv.r64.release(); Lv.e64.release(); Lv.res64.release();
         }
         else
@@ -488,19 +490,22 @@ void Context::AllocVectors()
     b.alloc(c); b.zero(st);
     xa.alloc(c); xa.zero(st);
     xb.alloc(c); xb.zero(st);
+    const size_t c0 = VecLen0();
     if (mixed)
     {
-        const size_t c32 = VecLen0();
-        for (auto &a : p32) { a.alloc(c32); a.zero(st); }
-        q32.alloc(c32); q32.zero(st);
-        x32.alloc(c32); x32.zero(st);
+        for (auto &a : p32) { a.alloc(c0); a.zero(st); }
+        q32.alloc(c0); q32.zero(st);
+        x32.alloc(c0); x32.zero(st);
         for (auto &a : p64) a.release();
         q64.release();
+        x64.release();
     }
     else
     {
-        for (auto &a : p64) { a.alloc(c); a.zero(st); }
-        q64.alloc(c); q64.zero(st);
+        for (auto &a : p64) { a.alloc(c0); a.zero(st); }
+        q64.alloc(c0); q64.zero(st);
+        if (Split(0)) { x64.alloc(c0); x64.zero(st); }
+        else x64.release();
         for (auto &a : p32) a.release();
         q32.release();
         x32.release();
@@ -859,13 +864,13 @@ template <typename T> void Context::VCycle(int l, T *r, T *e)
         ProfEnd();
         return;
     }
+    if (Split(l))
+    {
+        VCycleSplit<T>(l, r, e);
+        return;
+    }
     if constexpr (std::is_same<T, float>::value)
     {
-        if (Split(l))
-        {
-            VCycleSplit(l, r, e);
-            return;
-        }
         if (PairLevel(l))
         {
             VCyclePairs(l, r, e);
@@ -989,11 +994,11 @@ void Context::VCyclePairs(int l, float *r, float *e)
 // colour per launch, the residual and the transfers on the
 // red cells (the black residual after a black half-sweep is zero; the post-smoothing's black half replaces the black
 // values without reading them), and on level 0 the (r.z, z, r) sums of the last sweep, black then red.
-void Context::VCycleSplit(int l, float *r, float *e)
+template <typename T> void Context::VCycleSplit(int l, T *r, T *e)
 {
     LevelData &Lv = L[l];
     const LevelView v = Lv.view();
-    const double s = sizeof(float), cells = (double)Lv.cells;
+    const double s = sizeof(T), cells = (double)Lv.cells;
     auto prof = [&](int id, double bytesPerCell) {
         ProfBegin(l == 0 ? id : NB_K_COARSE, l == 0 ? bytesPerCell * cells : 0.0);
     };
@@ -1011,19 +1016,19 @@ void Context::VCycleSplit(int l, float *r, float *e)
             LaunchSplitHalf(v, du, r, e, c, st);
             ProfEnd();
         }
-    float *res = Lv.res<float>();
+    T *res = Lv.res<T>();
     prof(NB_K_RESIDUAL0, (4.0 * s + 1.0) / 2.0); // reads e, and r and the bytes of red; writes red
     LaunchSplitResidual(v, du, r, e, res, st);
     ProfEnd();
     LevelData &Lc = L[l + 1];
     const LevelView vc = Lc.view();
     prof(NB_K_RESTRICT0, (s + 1.0) / 2.0 + s / 8.0);
-    LaunchSplitRestrict(v, vc, Lv.pext.p, res, Lc.r<float>(), opt.transfer_kernels, st);
+    LaunchSplitRestrict<T>(v, vc, Lv.pext.p, res, Lc.r<T>(), opt.transfer_kernels, st);
     ProfEnd();
-    if (l == 0) CoarseBracket<float>(l + 1, Lc.r<float>(), Lc.e<float>());
-    else VCycle<float>(l + 1, Lc.r<float>(), Lc.e<float>());
+    if (l == 0) CoarseBracket<T>(l + 1, Lc.r<T>(), Lc.e<T>());
+    else VCycle<T>(l + 1, Lc.r<T>(), Lc.e<T>());
     prof(NB_K_PROLONG0, s + 0.5 + s / 8.0); // reads and writes red e, reads the red bytes and the coarse e
-    LaunchSplitProlong(v, vc, Lv.pext.p, Lc.e<float>(), e, st);
+    LaunchSplitProlong<T>(v, vc, Lv.pext.p, Lc.e<T>(), e, st);
     ProfEnd();
     for (int q = 0; q < post; q++)
     {
@@ -1048,21 +1053,20 @@ template <typename T> void Context::IterBody(T *x, T *r, T *z, T *p0, T *p1, T *
     const double s = sizeof(T), cells = (double)Cells();
     const int sing = singular ? 1 : 0;
     VCycle<T>(0, r, z);
+    if (Split(0)) // r.z came with the V-cycle's last sweep
+    {
+        ProfBegin(NB_K_PAPPLY, (4.0 * s + 1.0) * cells);
+        LaunchSplitPApply<T>(v0, L[0].du.p, z, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, st);
+        ProfEnd();
+        ProfBegin(NB_K_XR, 6.0 * s * cells);
+        LaunchSplitLinXR<T>(v0, (long long)VecLen0(), x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing,
+                            S_PQ, S_RR, st);
+        ProfEnd();
+        if (copyRR) NB_CK(cudaMemcpyAsync(hostSlots + S_RR, slots.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, st));
+        return;
+    }
     if constexpr (std::is_same<T, float>::value)
     {
-        if (Split(0)) // r.z came with the V-cycle's last sweep
-        {
-            ProfBegin(NB_K_PAPPLY, (4.0 * s + 1.0) * cells);
-            LaunchSplitPApply(v0, L[0].du.p, z, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, st);
-            ProfEnd();
-            ProfBegin(NB_K_XR, 6.0 * s * cells);
-            LaunchSplitLinXR(v0, (long long)VecLen0(), x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK,
-                             sing, S_PQ, S_RR, st);
-            ProfEnd();
-            if (copyRR)
-                NB_CK(cudaMemcpyAsync(hostSlots + S_RR, slots.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, st));
-            return;
-        }
         if (PairLevel(0))
         {
             // r.z came with the V-cycle's last sweep unless level 0 is itself the coarse end (tail or single level)
@@ -1076,7 +1080,7 @@ template <typename T> void Context::IterBody(T *x, T *r, T *z, T *p0, T *p1, T *
             LaunchPairPApply(v0, L[0].du.p, z, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, st);
             ProfEnd();
             ProfBegin(NB_K_XR, 6.0 * s * cells);
-            LaunchLinXR(L[0].cells, x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, S_RR, st);
+            LaunchLinXR<float>(L[0].cells, x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, S_RR, st);
             ProfEnd();
             if (copyRR)
                 NB_CK(cudaMemcpyAsync(hostSlots + S_RR, slots.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -1355,7 +1359,7 @@ void Context::BuildSolveGraph()
     try
     {
         NB_CK(cudaMemsetAsync(xa.p, 0, xa.bytes(), st));
-        if (Split(0)) LaunchSplitScaleSum(v0, b.p, r32, sfac, red, S_RES, st);
+        if (Split(0)) LaunchSplitScaleSum<float>(v0, b.p, r32, sfac, red, S_RES, st);
         else LaunchScaleSum<float>(L[0].cells, b.p, r32, sfac, red, S_RES, st);
         NB_COUNT_LAUNCH();
         k_mixed_init<<<1, 1, 0, st>>>(hOuter, slots.p, passes.p, maxOuter);
@@ -1417,7 +1421,7 @@ void Context::BuildSolveGraph()
     try
     {
         if (Split(0) && !nonuniform)
-            LaunchSplitRefine64(v0, L[0].du.p, b.p, xa.p, x32.p, xb.p, r32, scale, sfac, red, S_RES, st, passes.p);
+            LaunchSplitRefine64<float>(v0, L[0].du.p, b.p, xa.p, x32.p, xb.p, r32, scale, sfac, red, S_RES, st, passes.p);
         else if (PairLevel(0) && !nonuniform && dim == 3)
             LaunchPairRefine64(v0, L[0].du.p, b.p, xa.p, x32.p, xb.p, r32, scale, sfac, red, S_RES, st, passes.p);
         else
@@ -1476,7 +1480,7 @@ int Context::SolveMixed(double tol, double **xOut, nb_result *out, const double 
     xa.zero(st);
     float *r32 = L[0].r32.p, *z32 = L[0].e32.p;
     ProfBegin(NB_K_REFINE, (8.0 + 4.0) * (double)Cells());
-    if (Split(0)) LaunchSplitScaleSum(v0, b.p, r32, sfac, red, S_RES, st); // the residual of x = 0
+    if (Split(0)) LaunchSplitScaleSum<float>(v0, b.p, r32, sfac, red, S_RES, st); // the residual of x = 0
     else LaunchScaleSum<float>(L[0].cells, b.p, r32, sfac, red, S_RES, st);
     ProfEnd();
     const double bn2 = ReadSlot(S_RES);
@@ -1508,7 +1512,7 @@ int Context::SolveMixed(double tol, double **xOut, nb_result *out, const double 
                                    std::max(1, opt.max_iters), false, &rrEnd);
             ProfBegin(NB_K_REFINE, (8.0 + 4.0 + 8.0 + 1.0 + 8.0 + 4.0) * (double)Cells());
             if (Split(0) && !nonuniform)
-                LaunchSplitRefine64(v0, L[0].du.p, b.p, x, x32.p, xo, r32, scale, sfac, red, S_RES, st);
+                LaunchSplitRefine64<float>(v0, L[0].du.p, b.p, x, x32.p, xo, r32, scale, sfac, red, S_RES, st);
             else if (PairLevel(0) && !nonuniform && dim == 3)
                 LaunchPairRefine64(v0, L[0].du.p, b.p, x, x32.p, xo, r32, scale, sfac, red, S_RES, st);
             else
@@ -1530,11 +1534,14 @@ int Context::SolveFP64(double tol, double **xOut, nb_result *out, const double *
 {
     const LevelView v0 = L[0].view();
     const double sfac = -1.0 / scale;
-    double *x = xa.p;
+    // on a colour-split level 0 CG runs on a correction in that layout, added to x (grid layout) with the true residual
+    const bool split = Split(0);
+    double *x = xa.p, *xo = xb.p;
     xa.zero(st);
     double *r = L[0].r64.p, *z = L[0].e64.p;
     ProfBegin(NB_K_REFINE, (8.0 + 8.0) * (double)Cells());
-    LaunchScaleSum<double>(L[0].cells, b.p, r, sfac, red, S_RES, st); // the residual of x = 0
+    if (split) LaunchSplitScaleSum<double>(v0, b.p, r, sfac, red, S_RES, st); // the residual of x = 0
+    else LaunchScaleSum<double>(L[0].cells, b.p, r, sfac, red, S_RES, st);
     ProfEnd();
     const double bn2 = ReadSlot(S_RES);
     out->b_norm = std::sqrt(bn2);
@@ -1560,10 +1567,16 @@ int Context::SolveFP64(double tol, double **xOut, nb_result *out, const double *
             double rrEnd = 0.0;
             // the recursive residual is driven a little below the target, then checked against the true one
             const double target = 0.25 * tolEff * tolEff * bn2 * sfac * sfac;
-            its += RunPCG<double>(x, r, z, p64[0].p, p64[1].p, q64.p, rr * sfac * sfac, target, maxIt - its, true,
-                                  &rrEnd);
+            if (split) x64.zero(st);
+            its += RunPCG<double>(split ? x64.p : x, r, z, p64[0].p, p64[1].p, q64.p, rr * sfac * sfac, target,
+                                  maxIt - its, true, &rrEnd);
             ProfBegin(NB_K_REFINE, (8.0 + 8.0 + 1.0 + 8.0) * (double)Cells());
-            LaunchResidual64<double>(v0, b.p, x, r, scale, sfac, red, S_RES, st);
+            if (split)
+            {
+                LaunchSplitRefine64<double>(v0, L[0].du.p, b.p, x, x64.p, xo, r, scale, sfac, red, S_RES, st);
+                std::swap(x, xo);
+            }
+            else LaunchResidual64<double>(v0, b.p, x, r, scale, sfac, red, S_RES, st);
             ProfEnd();
             rr = ReadSlot(S_RES);
             restarts++;

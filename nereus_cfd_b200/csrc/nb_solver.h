@@ -201,7 +201,7 @@ struct LevelData
                                           // (colour-split level: the red cells only)
     DevArray<uint8_t> act;                // colour-split level: which (plane, tile) holds an unknown (LevelView::act)
     int actTiles = 0;
-    // the colour-split layout of the FP32 vectors (nb_split.cu); sRS = 0: the grid layout
+    // the colour-split layout of the solver's vectors (nb_split.cu); sRS = 0: the grid layout
     int sRS = 0, sPS = 0;
     long long sHalf = 0;
     size_t VecLen() const { return sRS ? (size_t)(2 * sHalf) : (size_t)cells; }
@@ -246,7 +246,7 @@ struct Context
     // solver vectors on level 0 (grid layout)
     DevArray<double> b, xa, xb;
     DevArray<float> p32[2], q32, x32;
-    DevArray<double> p64[2], q64;
+    DevArray<double> p64[2], q64, x64; // x64: a pass's correction, on a colour-split level 0
 
     // fields for the host-buffer entry points
     DevArray<double> du, dv, dw, dp, dpPrev;
@@ -407,12 +407,12 @@ struct Context
     int PostSweeps(int l) const { return std::max(1, L[l].stretched ? opt.stretched_sweeps : opt.post_sweeps); }
     // the FP32 cell-pair kernels serve this level (its du is built)
     bool PairLevel(int l) const { return opt.pair_kernels && L[l].du.p != nullptr; }
-    // the FP32 vectors of this level are colour-split and its V-cycle runs the split kernels
+    // the solver's vectors of this level are colour-split and its V-cycle runs the split kernels
     bool Split(int l) const { return L[l].sRS != 0; }
-    // FP32 elements of a level-0 vector (the split layout pads its rows)
+    // elements of a level-0 solver vector (the split layout pads its rows)
     size_t VecLen0() const { return L[0].VecLen(); }
     void VCyclePairs(int l, float *r, float *e);
-    void VCycleSplit(int l, float *r, float *e);
+    template <typename T> void VCycleSplit(int l, T *r, T *e);
     void UploadTables();
     void AssignSplit();
     void BuildTailLists();

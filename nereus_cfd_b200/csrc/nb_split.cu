@@ -1,5 +1,6 @@
-// Multigrid and PCG kernels for 3D FP32 levels in the colour-split layout (the inner solve of the mixed-precision
-// form), built so that each red-black half-sweep moves only the bytes the algorithm needs.
+// Multigrid and PCG kernels for uniform 3D levels in the colour-split layout, built so that each red-black half-sweep
+// moves only the bytes the algorithm needs: T = float for the inner solve of the mixed-precision form, double for the
+// plain FP64 form.
 //
 // Colour-split layout. Cell (i, j, k) has colour c = (i + j + k) & 1 and sits at c*H + i*PS + j*RS + (k >> 1) of a
 // level vector: each colour is an Ny x Nx x RS array whose rows hold the Nz/2 cells of that colour (RS = Nz/2
@@ -9,10 +10,13 @@
 // A half-sweep of colour c therefore reads the other colour, r and the diagonal bytes of colour c, and writes
 // colour c: half of every array, where a cell-pair sweep reads and writes both colours.
 //
-// Quads. Thread t of a launch takes the four elements 4t .. 4t+3 of a plane of one colour (RS is a multiple of 4, so
-// a quad never crosses a row) and marches along i over up to kPairS planes, keeping planes i-1, i, i+1 in
-// registers. The j neighbours are the quads RS elements away; the element across the quad's edge comes from the
-// neighbouring lane (a shuffle; lanes 0 and 31 load it).
+// Quads. Thread t of a launch takes the 16 bytes of elements N t .. N t + N - 1 of a plane of one colour (N = 4 floats
+// or 2 doubles; RS is a multiple of 4, so a quad never crosses a row) and marches along i over up to kQuadMaxS planes,
+// keeping planes i-1, i, i+1 in registers. The j neighbours are the quads RS elements away; the element across the
+// quad's edge comes from the neighbouring lane (a shuffle; lanes 0 and 31 load it). Two doubles a thread keep the FP64
+// kernels at the FP32 ones' register counts and loads in flight. FP64 at 256^3 (B200): these kernels took the plain
+// form's step from 25.0 ms (one thread per cell, a code and a neighbour mask per cell; the bytes of its 12 iterations at
+// 0.24 of the measured copy bandwidth) to 9.8 ms (0.62).
 //
 // Every vector is zero off the unknowns (and on the padding), so the neighbour sum runs over all six neighbours. The
 // levels are uniform (a stretched grid keeps the cell-pair kernels of nb_pairs.cu): the coefficient is gamma
@@ -32,35 +36,62 @@ namespace nb
 namespace
 {
 
-struct F4
+// the 16 bytes a thread moves at a time
+template <typename T> struct Quad
 {
-    float v[4];
+    static constexpr int N = 16 / (int)sizeof(T);
+    T v[N];
 };
+template <typename T> constexpr int kQ = Quad<T>::N;
 
-__device__ __forceinline__ F4 L4(const float *p)
+__device__ __forceinline__ Quad<float> LQ(const float *p)
 {
     const float4 a = *reinterpret_cast<const float4 *>(p);
-    return F4{{a.x, a.y, a.z, a.w}};
+    return Quad<float>{{a.x, a.y, a.z, a.w}};
 }
-__device__ __forceinline__ void S4(float *p, const F4 &a)
+__device__ __forceinline__ Quad<double> LQ(const double *p)
+{
+    const double2 a = *reinterpret_cast<const double2 *>(p);
+    return Quad<double>{{a.x, a.y}};
+}
+__device__ __forceinline__ void SQ(float *p, const Quad<float> &a)
 {
     *reinterpret_cast<float4 *>(p) = make_float4(a.v[0], a.v[1], a.v[2], a.v[3]);
 }
-__device__ __forceinline__ unsigned LdU4(const uint8_t *p) { return *reinterpret_cast<const unsigned *>(p); }
+__device__ __forceinline__ void SQ(double *p, const Quad<double> &a)
+{
+    *reinterpret_cast<double2 *>(p) = make_double2(a.v[0], a.v[1]);
+}
 // loads of values a kernel reads once (evict-first): measured to keep the half-sweep's j-row loads in L1 longer
-__device__ __forceinline__ F4 L4Once(const float *p)
+__device__ __forceinline__ Quad<float> LQOnce(const float *p)
 {
     const float4 a = __ldcs(reinterpret_cast<const float4 *>(p));
-    return F4{{a.x, a.y, a.z, a.w}};
+    return Quad<float>{{a.x, a.y, a.z, a.w}};
 }
-__device__ __forceinline__ unsigned LdU4Once(const uint8_t *p) { return __ldcs(reinterpret_cast<const unsigned *>(p)); }
+__device__ __forceinline__ Quad<double> LQOnce(const double *p)
+{
+    const double2 a = __ldcs(reinterpret_cast<const double2 *>(p));
+    return Quad<double>{{a.x, a.y}};
+}
+// a quad's N bytes of a byte array
+template <int N> __device__ __forceinline__ unsigned LdB(const uint8_t *p)
+{
+    static_assert(N == 4 || N == 2, "four or two bytes");
+    if constexpr (N == 4) return *reinterpret_cast<const unsigned *>(p);
+    else return *reinterpret_cast<const unsigned short *>(p);
+}
+template <int N> __device__ __forceinline__ unsigned LdBOnce(const uint8_t *p)
+{
+    if constexpr (N == 4) return __ldcs(reinterpret_cast<const unsigned *>(p));
+    else return __ldcs(reinterpret_cast<const unsigned short *>(p));
+}
 __device__ __forceinline__ unsigned Byte(unsigned d, int x) { return (d >> (8 * x)) & 0xFFu; }
-__device__ __forceinline__ float Unk(unsigned b) { return (b & 0x80u) ? 1.0f : 0.0f; }
+template <typename T> __device__ __forceinline__ T Unk(unsigned b) { return (b & 0x80u) ? (T)1 : (T)0; }
 
 // 1 / (gamma/2 * units), entry 0 = 0
-__device__ __forceinline__ void FillInv(float *inv, double gamma)
+template <typename T> __device__ __forceinline__ void FillInv(T *inv, double gamma)
 {
-    if (threadIdx.x < 32) inv[threadIdx.x] = threadIdx.x ? 1.0f / (0.5f * (float)gamma * (float)threadIdx.x) : 0.0f;
+    if (threadIdx.x < 32) inv[threadIdx.x] = threadIdx.x ? (T)1 / ((T)0.5 * (T)gamma * (T)threadIdx.x) : (T)0;
     __syncthreads();
 }
 
@@ -75,10 +106,10 @@ struct QuadPos
     long long off; // element of the quad on plane i0, within one colour
 };
 
-__device__ __forceinline__ QuadPos QuadStart(const LevelView &v, const Blk &b)
+template <int N> __device__ __forceinline__ QuadPos QuadStart(const LevelView &v, const Blk &b)
 {
     QuadPos p;
-    const int Q = v.sRS >> 2, nq = v.Nx * Q;
+    const int Q = v.sRS / N, nq = v.Nx * Q;
     p.lane = threadIdx.x & 31;
     int t = b.x * kPairThreads + threadIdx.x;
     p.valid = t < nq;
@@ -91,8 +122,8 @@ __device__ __forceinline__ QuadPos QuadStart(const LevelView &v, const Blk &b)
     p.RS = v.sRS;
     p.PS = v.sPS;
     p.j = t / Q;
-    p.m0 = 4 * (t - p.j * Q);
-    p.off = (long long)p.i0 * v.sPS + 4LL * t;
+    p.m0 = N * (t - p.j * Q);
+    p.off = (long long)p.i0 * v.sPS + (long long)N * t;
     return p;
 }
 
@@ -107,12 +138,12 @@ __device__ __forceinline__ bool TileIdle(const LevelView &v, int bx, int i0, int
 }
 
 // The same for a block of a grid-layout pair kernel (PairStart): its rows j0 .. j1 of planes [i0, i1), checked
-// through the split tiles that hold those rows' cells in either colour.
-__device__ __forceinline__ bool RowsIdle(const LevelView &v, int j0, int j1, int i0, int i1)
+// through the split tiles (of kTile elements) that hold those rows' cells in either colour.
+template <int kTile> __device__ __forceinline__ bool RowsIdle(const LevelView &v, int j0, int j1, int i0, int i1)
 {
     if (!v.act) return false;
-    const int t0 = (int)(((long long)j0 * v.sRS) / (4 * kPairThreads));
-    const int t1 = min(v.actTiles - 1, (int)(((long long)(j1 + 1) * v.sRS - 1) / (4 * kPairThreads)));
+    const int t0 = (int)(((long long)j0 * v.sRS) / kTile);
+    const int t1 = min(v.actTiles - 1, (int)(((long long)(j1 + 1) * v.sRS - 1) / kTile));
     for (int i = i0; i < i1; i++)
         for (int t = t0; t <= t1; t++)
             if (v.act[(long long)i * v.actTiles + t]) return false;
@@ -171,36 +202,42 @@ inline long long BestMarch(long long perPlane, long long planes, long long slots
     return bestS;
 }
 
-// A quad kernel's grid with a march of S planes (S > 0), or sized as above (S = 0).
-inline dim3 QuadGridS(const LevelView &v, int S)
+// A quad kernel's grid with a march of S planes (S > 0), or sized as above (S = 0); N elements a thread.
+template <int N = 4> inline dim3 QuadGridS(const LevelView &v, int S)
 {
-    const long long nq = (long long)v.Nx * (v.sRS / 4), perPlane = (nq + kPairThreads - 1) / kPairThreads;
+    const long long nq = (long long)v.Nx * (v.sRS / N), perPlane = (nq + kPairThreads - 1) / kPairThreads;
     const long long planes = v.Ny - 2 > 0 ? v.Ny - 2 : 1;
     return dim3((unsigned)perPlane, (unsigned)((planes + S - 1) / S));
 }
 
-inline dim3 QuadGrid(const LevelView &v, int resident)
+template <int N> inline dim3 QuadGrid(const LevelView &v, int resident)
 {
-    const long long nq = (long long)v.Nx * (v.sRS / 4), perPlane = (nq + kPairThreads - 1) / kPairThreads;
+    const long long nq = (long long)v.Nx * (v.sRS / N), perPlane = (nq + kPairThreads - 1) / kPairThreads;
     const long long planes = v.Ny - 2 > 0 ? v.Ny - 2 : 1;
     const long long bestS = BestMarch(perPlane, planes, (long long)SmCount() * (resident > 0 ? resident : 1));
     return dim3((unsigned)perPlane, (unsigned)((planes + bestS - 1) / bestS));
 }
 
 // The other colour's k neighbours of a quad: the element at m (c) and the one at m + (q ? 1 : -1) (returned).
-__device__ __forceinline__ F4 KShift(const F4 &c, float prevW, float nextX, int q)
+__device__ __forceinline__ Quad<float> KShift(const Quad<float> &c, float prevW, float nextX, int q)
 {
-    return q ? F4{{c.v[1], c.v[2], c.v[3], nextX}} : F4{{prevW, c.v[0], c.v[1], c.v[2]}};
+    return q ? Quad<float>{{c.v[1], c.v[2], c.v[3], nextX}} : Quad<float>{{prevW, c.v[0], c.v[1], c.v[2]}};
+}
+__device__ __forceinline__ Quad<double> KShift(const Quad<double> &c, double prevW, double nextX, int q)
+{
+    return q ? Quad<double>{{c.v[1], nextX}} : Quad<double>{{prevW, c.v[0]}};
 }
 
 // The elements just before and after this lane's quad in its row (0 past the row's ends; the values a lane takes
 // from a neighbouring row only reach ring or padding cells, whose results are masked).
-__device__ __forceinline__ void Edges(const QuadPos &P, const F4 &c, const float *row, float &prevW, float &nextX)
+template <typename T>
+__device__ __forceinline__ void Edges(const QuadPos &P, const Quad<T> &c, const T *row, T &prevW, T &nextX)
 {
-    prevW = __shfl_up_sync(0xffffffffu, c.v[3], 1);
+    constexpr int N = kQ<T>;
+    prevW = __shfl_up_sync(0xffffffffu, c.v[N - 1], 1);
     nextX = __shfl_down_sync(0xffffffffu, c.v[0], 1);
-    if (P.lane == 0) prevW = P.m0 > 0 ? row[-1] : 0.f;
-    if (P.lane == 31) nextX = P.m0 + 4 < P.RS ? row[4] : 0.f;
+    if (P.lane == 0) prevW = P.m0 > 0 ? row[-1] : (T)0;
+    if (P.lane == 31) nextX = P.m0 + N < P.RS ? row[N] : (T)0;
 }
 
 } // namespace
@@ -215,106 +252,110 @@ constexpr int kSplitReduceS = 16;
 // The first red-black sweep from a zero iterate on a uniform level, one launch: red e = r / diag, then black
 // e = (r + gamma * sum of the red neighbours) / diag with the red neighbours formed from r and the bytes. A thread
 // owns one quad position and writes the red and the black quad there.
+template <typename T>
 __device__ __forceinline__ void SplitFirst(const LevelView &v, const uint8_t *__restrict__ du,
-                                           const float *__restrict__ r, float *__restrict__ e, const Blk &blk)
+                                           const T *__restrict__ r, T *__restrict__ e, const Blk &blk)
 {
-    __shared__ float inv[32];
-    FillInv(inv, v.gamma);
-    const QuadPos P = QuadStart(v, blk);
+    constexpr int N = kQ<T>;
+    __shared__ T inv[32];
+    FillInv<T>(inv, v.gamma);
+    const QuadPos P = QuadStart<N>(v, blk);
     if (TileIdle(v, blk.x, P.i0, P.i1)) return;
-    const float g = (float)v.gamma;
+    const T g = (T)v.gamma;
     const long long hb = v.sHalf;
-    const float *R0 = r + P.off, *R1 = r + hb + P.off;
+    const T *R0 = r + P.off, *R1 = r + hb + P.off;
     const uint8_t *D0 = du + P.off, *D1 = du + hb + P.off;
-    float *X0 = e + P.off, *X1 = e + hb + P.off;
+    T *X0 = e + P.off, *X1 = e + hb + P.off;
     auto red = [&](long long o) {
-        F4 a = L4(R0 + o);
-        const unsigned d = LdU4(D0 + o);
+        Quad<T> a = LQ(R0 + o);
+        const unsigned d = LdB<N>(D0 + o);
 #pragma unroll
         for (int x = 0; x < 4; x++) a.v[x] *= inv[Byte(d, x) & 0x7Fu];
         return a;
     };
     auto red1 = [&](long long o) { return R0[o] * inv[D0[o] & 0x7Fu]; };
-    F4 RM = red(-P.PS), RC = red(0);
+    Quad<T> RM = red(-P.PS), RC = red(0);
     long long o = 0;
     for (int i = P.i0; i < P.i1; i++, o += P.PS)
     {
-        const F4 RP = red(o + P.PS), RJp = red(o + P.RS), RJm = red(o - P.RS);
-        const F4 rb = L4Once(R1 + o);
-        const unsigned db = LdU4Once(D1 + o);
-        float prevW = __shfl_up_sync(0xffffffffu, RC.v[3], 1), nextX = __shfl_down_sync(0xffffffffu, RC.v[0], 1);
-        if (P.lane == 0) prevW = P.m0 > 0 ? red1(o - 1) : 0.f;
-        if (P.lane == 31) nextX = P.m0 + 4 < P.RS ? red1(o + 4) : 0.f;
-        const F4 sh = KShift(RC, prevW, nextX, (i + P.j + 1) & 1);
-        F4 nb;
+        const Quad<T> RP = red(o + P.PS), RJp = red(o + P.RS), RJm = red(o - P.RS);
+        const Quad<T> rb = LQOnce(R1 + o);
+        const unsigned db = LdBOnce<N>(D1 + o);
+        T prevW = __shfl_up_sync(0xffffffffu, RC.v[N - 1], 1), nextX = __shfl_down_sync(0xffffffffu, RC.v[0], 1);
+        if (P.lane == 0) prevW = P.m0 > 0 ? red1(o - 1) : (T)0;
+        if (P.lane == 31) nextX = P.m0 + N < P.RS ? red1(o + N) : (T)0;
+        const Quad<T> sh = KShift(RC, prevW, nextX, (i + P.j + 1) & 1);
+        Quad<T> nb;
 #pragma unroll
-        for (int x = 0; x < 4; x++)
+        for (int x = 0; x < N; x++)
         {
-            const float s = ((RP.v[x] + RM.v[x]) + (RJp.v[x] + RJm.v[x])) + (RC.v[x] + sh.v[x]);
+            const T s = ((RP.v[x] + RM.v[x]) + (RJp.v[x] + RJm.v[x])) + (RC.v[x] + sh.v[x]);
             nb.v[x] = (rb.v[x] + g * s) * inv[Byte(db, x) & 0x7Fu];
         }
         if (P.valid)
         {
-            S4(X0 + o, RC);
-            S4(X1 + o, nb);
+            SQ(X0 + o, RC);
+            SQ(X1 + o, nb);
         }
         RM = RC;
         RC = RP;
     }
 }
 
+template <typename T>
 __global__ void __launch_bounds__(kPairThreads) k_split_first(LevelView v, const uint8_t *__restrict__ du,
-                                                              const float *__restrict__ r, float *__restrict__ e)
+                                                              const T *__restrict__ r, T *__restrict__ e)
 {
     PdlWait();
     PdlTrigger();
-    SplitFirst(v, du, r, e, ThisBlk());
+    SplitFirst<T>(v, du, r, e, ThisBlk());
 }
 
 // One colour of a red-black sweep: e_c = (r_c + gamma * sum of the other colour's six neighbours) / diag_c.
 // kDot 1: (sum r.e, sum e, sum r) of this colour into out[partSlot..]; kDot 2: the same plus the totals already in
 // out[partSlot..], into the scalar block of the iteration's parity (the CG's r.z, sum z, sum r of the V-cycle's z).
 // du, r: this colour's halves; eo, ec: the other colour's and this colour's halves of e (disjoint).
-template <int kDot>
+template <typename T, int kDot>
 __device__ __forceinline__ void SplitHalf(const LevelView &v, const uint8_t *__restrict__ du,
-                                          const float *__restrict__ r, const float *__restrict__ eo,
-                                          float *__restrict__ ec, int colour, const Reducer &R, const int *it,
+                                          const T *__restrict__ r, const T *__restrict__ eo,
+                                          T *__restrict__ ec, int colour, const Reducer &R, const int *it,
                                           int baseEven, int baseOdd, int partSlot, const Blk &blk)
 {
-    float facc[3] = {0.f, 0.f, 0.f}; // a thread's terms in FP32, the block and grid sums in FP64
-    __shared__ float inv[32];
-    FillInv(inv, v.gamma);
-    QuadPos P = QuadStart(v, blk);
+    constexpr int N = kQ<T>;
+    T facc[3] = {(T)0, (T)0, (T)0}; // a thread's terms in T, the block and grid sums in FP64
+    __shared__ T inv[32];
+    FillInv<T>(inv, v.gamma);
+    QuadPos P = QuadStart<N>(v, blk);
     if (TileIdle(v, blk.x, P.i0, P.i1))
     {
         if (!kDot) return;
         P.i1 = P.i0; // nothing to sweep; the block still adds its zero terms to the sums
     }
-    const float g = (float)v.gamma;
-    const float *O = eo + P.off;
-    const float *Rr = r + P.off;
+    const T g = (T)v.gamma;
+    const T *O = eo + P.off;
+    const T *Rr = r + P.off;
     const uint8_t *D = du + P.off;
-    float *C = ec + P.off;
+    T *C = ec + P.off;
     // one plane: the six other-colour neighbours, r and the bytes given, the new values stored (and summed)
-    auto plane = [&](int i, long long o, const F4 &oM, const F4 &oC, const F4 &oP, const F4 &jp, const F4 &jm,
-                     const F4 &rr, unsigned d) {
-        float prevW, nextX;
+    auto plane = [&](int i, long long o, const Quad<T> &oM, const Quad<T> &oC, const Quad<T> &oP, const Quad<T> &jp,
+                     const Quad<T> &jm, const Quad<T> &rr, unsigned d) {
+        T prevW, nextX;
         Edges(P, oC, O + o, prevW, nextX);
-        const F4 sh = KShift(oC, prevW, nextX, (i + P.j + colour) & 1);
-        F4 nv;
+        const Quad<T> sh = KShift(oC, prevW, nextX, (i + P.j + colour) & 1);
+        Quad<T> nv;
 #pragma unroll
-        for (int x = 0; x < 4; x++)
+        for (int x = 0; x < N; x++)
         {
-            const float s = ((oP.v[x] + oM.v[x]) + (jp.v[x] + jm.v[x])) + (oC.v[x] + sh.v[x]);
+            const T s = ((oP.v[x] + oM.v[x]) + (jp.v[x] + jm.v[x])) + (oC.v[x] + sh.v[x]);
             nv.v[x] = (rr.v[x] + g * s) * inv[Byte(d, x) & 0x7Fu];
         }
         if (P.valid)
         {
-            S4(C + o, nv);
+            SQ(C + o, nv);
             if (kDot)
             {
 #pragma unroll
-                for (int x = 0; x < 4; x++)
+                for (int x = 0; x < N; x++)
                 {
                     facc[0] += rr.v[x] * nv.v[x];
                     facc[1] += nv.v[x];
@@ -325,22 +366,22 @@ __device__ __forceinline__ void SplitHalf(const LevelView &v, const uint8_t *__r
     };
     // two planes per trip: all the streamed values of both (the other colour up to two planes ahead, the j rows,
     // r and the bytes) are loaded before either is computed, twice the loads in flight of a plane-by-plane march
-    F4 oM{}, oC{};
+    Quad<T> oM{}, oC{};
     if (P.i0 < P.i1)
     {
-        oM = L4(O - P.PS);
-        oC = L4(O);
+        oM = LQ(O - P.PS);
+        oC = LQ(O);
     }
     long long o = 0;
     for (int i = P.i0; i < P.i1; i += 2, o += 2 * P.PS)
     {
         const bool two = i + 1 < P.i1;
-        const F4 oP = L4(O + o + P.PS);
-        const F4 oPP = two ? L4(O + o + 2 * P.PS) : F4{};
-        const F4 r0 = L4Once(Rr + o), r1 = two ? L4Once(Rr + o + P.PS) : F4{};
-        const unsigned d0 = LdU4Once(D + o), d1 = two ? LdU4Once(D + o + P.PS) : 0u;
-        const F4 jp0 = L4(O + o + P.RS), jm0 = L4(O + o - P.RS);
-        const F4 jp1 = two ? L4(O + o + P.PS + P.RS) : F4{}, jm1 = two ? L4(O + o + P.PS - P.RS) : F4{};
+        const Quad<T> oP = LQ(O + o + P.PS);
+        const Quad<T> oPP = two ? LQ(O + o + 2 * P.PS) : Quad<T>{};
+        const Quad<T> r0 = LQOnce(Rr + o), r1 = two ? LQOnce(Rr + o + P.PS) : Quad<T>{};
+        const unsigned d0 = LdBOnce<N>(D + o), d1 = two ? LdBOnce<N>(D + o + P.PS) : 0u;
+        const Quad<T> jp0 = LQ(O + o + P.RS), jm0 = LQ(O + o - P.RS);
+        const Quad<T> jp1 = two ? LQ(O + o + P.PS + P.RS) : Quad<T>{}, jm1 = two ? LQ(O + o + P.PS - P.RS) : Quad<T>{};
         plane(i, o, oM, oC, oP, jp0, jm0, r0, d0);
         if (two) plane(i + 1, o + P.PS, oC, oP, oPP, jp1, jm1, r1, d1);
         oM = oP;
@@ -359,15 +400,15 @@ __device__ __forceinline__ void SplitHalf(const LevelView &v, const uint8_t *__r
 }
 
 // 4 resident blocks (64 registers): the two-plane march measured 12% faster there than at 3 (73 registers)
-template <int kDot>
+template <typename T, int kDot>
 __global__ void __launch_bounds__(kPairThreads, 4)
-    k_split_half(LevelView v, const uint8_t *__restrict__ du, const float *__restrict__ r,
-                 const float *__restrict__ eo, float *__restrict__ ec, int colour, Reducer R, const int *it,
+    k_split_half(LevelView v, const uint8_t *__restrict__ du, const T *__restrict__ r,
+                 const T *__restrict__ eo, T *__restrict__ ec, int colour, Reducer R, const int *it,
                  int baseEven, int baseOdd, int partSlot)
 {
     PdlWait();
     PdlTrigger();
-    SplitHalf<kDot>(v, du, r, eo, ec, colour, R, it, baseEven, baseOdd, partSlot, ThisBlk());
+    SplitHalf<T, kDot>(v, du, r, eo, ec, colour, R, it, baseEven, baseOdd, partSlot, ThisBlk());
 }
 
 // the arguments of k_split_half for colour c: its halves of du and r, the other colour's and its own halves of e
@@ -375,73 +416,78 @@ __global__ void __launch_bounds__(kPairThreads, 4)
     v, du + (long long)(c) * v.sHalf, r + (long long)(c) * v.sHalf, e + (long long)((c) ^ 1) * v.sHalf,               \
         e + (long long)(c) * v.sHalf, (c)
 
-void LaunchSplitFirst(const LevelView &v, const uint8_t *du, const float *r, float *e, cudaStream_t st)
+template <typename T>
+void LaunchSplitFirst(const LevelView &v, const uint8_t *du, const T *r, T *e, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    LaunchPdl(k_split_first, QuadGrid(v, Occ<k_split_first>()), kPairThreads, 0, st, v, du, r, e);
+    LaunchPdl(k_split_first<T>, QuadGrid<kQ<T>>(v, Occ<k_split_first<T>>()), kPairThreads, 0, st, v, du, r, e);
 }
 
-void LaunchSplitHalf(const LevelView &v, const uint8_t *du, const float *r, float *e, int colour, cudaStream_t st)
+template <typename T>
+void LaunchSplitHalf(const LevelView &v, const uint8_t *du, const T *r, T *e, int colour, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    LaunchPdl(k_split_half<0>, QuadGrid(v, Occ<k_split_half<0>>()), kPairThreads, 0, st, NB_SPLIT_HALF_ARGS(colour),
-              Reducer{}, (const int *)nullptr, 0, 0, 0);
+    LaunchPdl(k_split_half<T, 0>, QuadGrid<kQ<T>>(v, Occ<k_split_half<T, 0>>()), kPairThreads, 0, st,
+              NB_SPLIT_HALF_ARGS(colour), Reducer{}, (const int *)nullptr, 0, 0, 0);
 }
 
-void LaunchSplitHalfDot(const LevelView &v, const uint8_t *du, const float *r, float *e, int colour, bool last,
+template <typename T>
+void LaunchSplitHalfDot(const LevelView &v, const uint8_t *du, const T *r, T *e, int colour, bool last,
                         const Reducer &R, const int *it, int baseEven, int baseOdd, int partSlot, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
     if (last)
-        LaunchPdl(k_split_half<2>, QuadGrid(v, Occ<k_split_half<2>>()), kPairThreads, 0, st,
+        LaunchPdl(k_split_half<T, 2>, QuadGrid<kQ<T>>(v, Occ<k_split_half<T, 2>>()), kPairThreads, 0, st,
                   NB_SPLIT_HALF_ARGS(colour), R, it, baseEven, baseOdd, partSlot);
     else
-        LaunchPdl(k_split_half<1>, QuadGrid(v, Occ<k_split_half<1>>()), kPairThreads, 0, st,
+        LaunchPdl(k_split_half<T, 1>, QuadGrid<kQ<T>>(v, Occ<k_split_half<T, 1>>()), kPairThreads, 0, st,
                   NB_SPLIT_HALF_ARGS(colour), R, it, baseEven, baseOdd, partSlot);
 }
 #undef NB_SPLIT_HALF_ARGS
 
 // res = r - M e on the red cells (colour 0), into the first half of `res`; the black residual after a black
 // half-sweep is zero.
+template <typename T>
 __device__ __forceinline__ void SplitResidual(const LevelView &v, const uint8_t *__restrict__ du,
-                                              const float *__restrict__ r, const float *__restrict__ e,
-                                              float *__restrict__ res, const Blk &blk)
+                                              const T *__restrict__ r, const T *__restrict__ e,
+                                              T *__restrict__ res, const Blk &blk)
 {
-    const QuadPos P = QuadStart(v, blk);
+    constexpr int N = kQ<T>;
+    const QuadPos P = QuadStart<N>(v, blk);
     if (TileIdle(v, blk.x, P.i0, P.i1)) return;
-    const float g = (float)v.gamma, hg = 0.5f * (float)v.gamma;
-    const float *O = e + v.sHalf + P.off;
-    const float *Xr = e + P.off;
-    const float *Rr = r + P.off;
+    const T g = (T)v.gamma, hg = (T)0.5 * (T)v.gamma;
+    const T *O = e + v.sHalf + P.off;
+    const T *Xr = e + P.off;
+    const T *Rr = r + P.off;
     const uint8_t *D = du + P.off;
-    float *Out = res + P.off;
-    auto plane = [&](int i, long long o, const F4 &oM, const F4 &oC, const F4 &oP, const F4 &jp, const F4 &jm,
-                     const F4 &xc, const F4 &rr, unsigned d) {
-        float prevW, nextX;
+    T *Out = res + P.off;
+    auto plane = [&](int i, long long o, const Quad<T> &oM, const Quad<T> &oC, const Quad<T> &oP, const Quad<T> &jp,
+                     const Quad<T> &jm, const Quad<T> &xc, const Quad<T> &rr, unsigned d) {
+        T prevW, nextX;
         Edges(P, oC, O + o, prevW, nextX);
-        const F4 sh = KShift(oC, prevW, nextX, (i + P.j) & 1);
-        F4 out;
+        const Quad<T> sh = KShift(oC, prevW, nextX, (i + P.j) & 1);
+        Quad<T> out;
 #pragma unroll
-        for (int x = 0; x < 4; x++)
+        for (int x = 0; x < N; x++)
         {
             const unsigned b = Byte(d, x);
-            const float s = ((oP.v[x] + oM.v[x]) + (jp.v[x] + jm.v[x])) + (oC.v[x] + sh.v[x]);
-            out.v[x] = (b & 0x80u) ? rr.v[x] - (hg * (float)(b & 0x7Fu) * xc.v[x] - g * s) : 0.f;
+            const T s = ((oP.v[x] + oM.v[x]) + (jp.v[x] + jm.v[x])) + (oC.v[x] + sh.v[x]);
+            out.v[x] = (b & 0x80u) ? rr.v[x] - (hg * (T)(b & 0x7Fu) * xc.v[x] - g * s) : (T)0;
         }
-        if (P.valid) S4(Out + o, out);
+        if (P.valid) SQ(Out + o, out);
     };
     // two planes per trip, all their streamed values loaded first (as in the half-sweep)
-    F4 oM = L4(O - P.PS), oC = L4(O);
+    Quad<T> oM = LQ(O - P.PS), oC = LQ(O);
     long long o = 0;
     for (int i = P.i0; i < P.i1; i += 2, o += 2 * P.PS)
     {
         const bool two = i + 1 < P.i1;
-        const F4 oP = L4(O + o + P.PS), oPP = two ? L4(O + o + 2 * P.PS) : F4{};
-        const F4 jp0 = L4(O + o + P.RS), jm0 = L4(O + o - P.RS);
-        const F4 jp1 = two ? L4(O + o + P.PS + P.RS) : F4{}, jm1 = two ? L4(O + o + P.PS - P.RS) : F4{};
-        const F4 x0 = L4(Xr + o), r0 = L4Once(Rr + o), x1 = two ? L4(Xr + o + P.PS) : F4{},
-                 r1 = two ? L4Once(Rr + o + P.PS) : F4{};
-        const unsigned d0 = LdU4Once(D + o), d1 = two ? LdU4Once(D + o + P.PS) : 0u;
+        const Quad<T> oP = LQ(O + o + P.PS), oPP = two ? LQ(O + o + 2 * P.PS) : Quad<T>{};
+        const Quad<T> jp0 = LQ(O + o + P.RS), jm0 = LQ(O + o - P.RS);
+        const Quad<T> jp1 = two ? LQ(O + o + P.PS + P.RS) : Quad<T>{}, jm1 = two ? LQ(O + o + P.PS - P.RS) : Quad<T>{};
+        const Quad<T> x0 = LQ(Xr + o), r0 = LQOnce(Rr + o), x1 = two ? LQ(Xr + o + P.PS) : Quad<T>{},
+                      r1 = two ? LQOnce(Rr + o + P.PS) : Quad<T>{};
+        const unsigned d0 = LdBOnce<N>(D + o), d1 = two ? LdBOnce<N>(D + o + P.PS) : 0u;
         plane(i, o, oM, oC, oP, jp0, jm0, x0, r0, d0);
         if (two) plane(i + 1, o + P.PS, oC, oP, oPP, jp1, jm1, x1, r1, d1);
         oM = oP;
@@ -449,20 +495,22 @@ __device__ __forceinline__ void SplitResidual(const LevelView &v, const uint8_t 
     }
 }
 
-__global__ void __launch_bounds__(kPairThreads, 4) k_split_residual(LevelView v, const uint8_t *__restrict__ du,
-                                                                 const float *__restrict__ r,
-                                                                 const float *__restrict__ e, float *__restrict__ res)
+template <typename T>
+__global__ void __launch_bounds__(kPairThreads, sizeof(T) == 8 ? 3 : 4) k_split_residual(LevelView v, const uint8_t *__restrict__ du,
+                                                                 const T *__restrict__ r,
+                                                                 const T *__restrict__ e, T *__restrict__ res)
 {
     PdlWait();
     PdlTrigger();
-    SplitResidual(v, du, r, e, res, ThisBlk());
+    SplitResidual<T>(v, du, r, e, res, ThisBlk());
 }
 
-void LaunchSplitResidual(const LevelView &v, const uint8_t *du, const float *r, const float *e, float *res,
-                         cudaStream_t st)
+template <typename T>
+void LaunchSplitResidual(const LevelView &v, const uint8_t *du, const T *r, const T *e, T *res, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    LaunchPdl(k_split_residual, QuadGrid(v, Occ<k_split_residual>()), kPairThreads, 0, st, v, du, r, e, res);
+    LaunchPdl(k_split_residual<T>, QuadGrid<kQ<T>>(v, Occ<k_split_residual<T>>()), kPairThreads, 0, st, v, du, r, e,
+              res);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -481,99 +529,114 @@ void LaunchSplitResidual(const LevelView &v, const uint8_t *du, const float *r, 
 // neighbouring planes' rows (kept in registers) serves the four fine quads of fine planes 2A-1, 2A and rows 2B-1,
 // 2B, whose red values and bytes it loads together.
 
-// coarse k-cells m0 .. m0+4 of coarse row (A, B)
-__device__ __forceinline__ void CoarseRow5(const LevelView &cv, const float *__restrict__ ec, int A, int B, int m0,
-                                           float c[5])
+// coarse k-cells m0 .. m0+N of coarse row (A, B), N = kQ<T>
+template <typename T>
+__device__ __forceinline__ void CoarseRowK(const LevelView &cv, const T *__restrict__ ec, int A, int B, int m0,
+                                           T c[kQ<T> + 1])
 {
+    constexpr int N = kQ<T>;
     const int Dmax = cv.Nz - 1;
-    if (cv.sRS && m0 + 4 <= Dmax)
+    if (cv.sRS && m0 + N <= Dmax)
     {
-        // a colour-split coarse level: k-cells m0, m0+2, m0+4 are elements m0/2 .. m0/2+2 of colour (A+B) & 1, and
-        // m0+1, m0+3 elements m0/2, m0/2+1 of the other (m0 is a multiple of 4)
+        // a colour-split coarse level: the even k-cells m0, m0+2, .. are elements m0/2, m0/2+1, .. of colour
+        // (A+B) & 1, the odd ones the same elements of the other (m0 is a multiple of N)
         const int ce = (A + B) & 1;
-        const float *rb = ec + (long long)A * cv.sPS + (long long)B * cv.sRS + (m0 >> 1);
-        const float2 ev = *reinterpret_cast<const float2 *>(rb + ce * cv.sHalf);
-        const float2 od = *reinterpret_cast<const float2 *>(rb + (ce ^ 1) * cv.sHalf);
-        c[0] = ev.x;
-        c[1] = od.x;
-        c[2] = ev.y;
-        c[3] = od.y;
-        c[4] = rb[ce * cv.sHalf + 2];
+        const T *rb = ec + (long long)A * cv.sPS + (long long)B * cv.sRS + (m0 >> 1);
+        if constexpr (N == 4)
+        {
+            const float2 ev = *reinterpret_cast<const float2 *>(rb + ce * cv.sHalf);
+            const float2 od = *reinterpret_cast<const float2 *>(rb + (ce ^ 1) * cv.sHalf);
+            c[0] = ev.x;
+            c[1] = od.x;
+            c[2] = ev.y;
+            c[3] = od.y;
+            c[4] = rb[ce * cv.sHalf + 2];
+        }
+        else
+        {
+            c[0] = rb[ce * cv.sHalf];
+            c[1] = rb[(ce ^ 1) * cv.sHalf];
+            c[2] = rb[ce * cv.sHalf + 1];
+        }
         return;
     }
 #pragma unroll
-    for (int t = 0; t < 5; t++) c[t] = ec[VecIdx(cv, A, B, min(m0 + t, Dmax))]; // past the row: masked cells only
+    for (int t = 0; t <= N; t++) c[t] = ec[VecIdx(cv, A, B, min(m0 + t, Dmax))]; // past the row: masked cells only
 }
 
 // the coarse plane's rows interpolated across j for fine rows 2B-1 (y0) and 2B (y1), and row B itself (par)
-__device__ __forceinline__ void CoarsePlaneRows(const LevelView &cv, const float *__restrict__ ec, int A, int B,
-                                                int m0, float y0[5], float y1[5], float par[5])
+template <typename T>
+__device__ __forceinline__ void CoarsePlaneRows(const LevelView &cv, const T *__restrict__ ec, int A, int B, int m0,
+                                                T y0[kQ<T> + 1], T y1[kQ<T> + 1], T par[kQ<T> + 1])
 {
-    float cm[5], cp[5];
-    CoarseRow5(cv, ec, A, B, m0, par);
-    CoarseRow5(cv, ec, A, B - 1, m0, cm);
-    CoarseRow5(cv, ec, A, B + 1, m0, cp);
+    T cm[kQ<T> + 1], cp[kQ<T> + 1];
+    CoarseRowK<T>(cv, ec, A, B, m0, par);
+    CoarseRowK<T>(cv, ec, A, B - 1, m0, cm);
+    CoarseRowK<T>(cv, ec, A, B + 1, m0, cp);
 #pragma unroll
-    for (int t = 0; t < 5; t++)
+    for (int t = 0; t <= kQ<T>; t++)
     {
-        y0[t] = 0.75f * par[t] + 0.25f * cm[t];
-        y1[t] = 0.75f * par[t] + 0.25f * cp[t];
+        y0[t] = (T)0.75 * par[t] + (T)0.25 * cm[t];
+        y1[t] = (T)0.75 * par[t] + (T)0.25 * cp[t];
     }
 }
 
+template <typename T>
 __device__ __forceinline__ void SplitProlong(const LevelView &fv, const LevelView &cv,
-                                             const uint8_t *__restrict__ pext, const float *__restrict__ ec,
-                                             float *__restrict__ ef, const Blk &blk)
+                                             const uint8_t *__restrict__ pext, const T *__restrict__ ec,
+                                             T *__restrict__ ef, const Blk &blk)
 {
-    const int Q = fv.sRS >> 2, nrow = cv.Nx - 2, nq = nrow * Q;
+    constexpr int N = kQ<T>;
+    constexpr unsigned kUnkMask = N == 4 ? 0x80808080u : 0x8080u;
+    const int Q = fv.sRS / N, nrow = cv.Nx - 2, nq = nrow * Q;
     int t = blk.x * kPairThreads + threadIdx.x;
     const bool valid = t < nq;
     if (!valid) t = nq - 1;
-    const int B = 1 + t / Q, m0 = 4 * (t - (B - 1) * Q);
+    const int B = 1 + t / Q, m0 = N * (t - (B - 1) * Q);
     const int S = (cv.Ny - 2 + blk.gy - 1) / blk.gy;
     const int A0 = min(1 + blk.y * S, cv.Ny - 1), A1 = min(A0 + S, cv.Ny - 1);
     if (!valid || A0 >= A1) return;
-    float yM0[5], yM1[5], yC0[5], yC1[5], pC[5], pD[5];
-    CoarsePlaneRows(cv, ec, A0 - 1, B, m0, yM0, yM1, pD);
-    CoarsePlaneRows(cv, ec, A0, B, m0, yC0, yC1, pC);
+    T yM0[N + 1], yM1[N + 1], yC0[N + 1], yC1[N + 1], pC[N + 1], pD[N + 1];
+    CoarsePlaneRows<T>(cv, ec, A0 - 1, B, m0, yM0, yM1, pD);
+    CoarsePlaneRows<T>(cv, ec, A0, B, m0, yC0, yC1, pC);
     const int fb0 = 2 * B - 1, fb1 = 2 * B;
     for (int A = A0; A < A1; A++)
     {
-        float yP0[5], yP1[5], pP[5];
-        CoarsePlaneRows(cv, ec, A + 1, B, m0, yP0, yP1, pP);
+        T yP0[N + 1], yP1[N + 1], pP[N + 1];
+        CoarsePlaneRows<T>(cv, ec, A + 1, B, m0, yP0, yP1, pP);
         // fine planes 2A-1 (with coarse plane A-1) and 2A (with A+1), rows 2B-1 and 2B
 #pragma unroll
         for (int h = 0; h < 2; h++)
         {
             const int fa = 2 * A - 1 + h;
             const long long o0 = (long long)fa * fv.sPS + (long long)fb0 * fv.sRS + m0, o1 = o0 + fv.sRS;
-            const unsigned w0 = LdU4(pext + o0), w1 = LdU4(pext + o1);
-            F4 e0 = L4(ef + o0), e1 = L4(ef + o1);
-            const float *yo0 = h ? yP0 : yM0, *yo1 = h ? yP1 : yM1;
+            const unsigned w0 = LdB<N>(pext + o0), w1 = LdB<N>(pext + o1);
+            Quad<T> e0 = LQ(ef + o0), e1 = LQ(ef + o1);
+            const T *yo0 = h ? yP0 : yM0, *yo1 = h ? yP1 : yM1;
 #pragma unroll
             for (int rI = 0; rI < 2; rI++)
             {
                 const unsigned w = rI ? w1 : w0;
-                if (!(w & 0x80808080u)) continue;
+                if (!(w & kUnkMask)) continue;
                 const int q = (fa + (rI ? fb1 : fb0)) & 1;
-                float z[5];
+                T z[N + 1];
 #pragma unroll
-                for (int k = 0; k < 5; k++)
-                    z[k] = rI ? 0.75f * yC1[k] + 0.25f * yo1[k] : 0.75f * yC0[k] + 0.25f * yo0[k];
-                F4 &ev = rI ? e1 : e0;
+                for (int k = 0; k <= N; k++)
+                    z[k] = rI ? (T)0.75 * yC1[k] + (T)0.25 * yo1[k] : (T)0.75 * yC0[k] + (T)0.25 * yo0[k];
+                Quad<T> &ev = rI ? e1 : e0;
 #pragma unroll
-                for (int x = 0; x < 4; x++)
+                for (int x = 0; x < N; x++)
                 {
                     const unsigned px = Byte(w, x);
                     if (!(px & 0x80u)) continue;
-                    const float lohi = q ? 0.25f * z[x] + 0.75f * z[x + 1] : 0.75f * z[x] + 0.25f * z[x + 1];
-                    ev.v[x] += lohi + (float)(px & 0x3Fu) * (1.0f / 64.0f) * (q ? pC[x + 1] : pC[x]);
+                    const T lohi = q ? (T)0.25 * z[x] + (T)0.75 * z[x + 1] : (T)0.75 * z[x] + (T)0.25 * z[x + 1];
+                    ev.v[x] += lohi + (T)(px & 0x3Fu) * (T)(1.0 / 64.0) * (q ? pC[x + 1] : pC[x]);
                 }
-                S4(ef + (rI ? o1 : o0), ev);
+                SQ(ef + (rI ? o1 : o0), ev);
             }
         }
 #pragma unroll
-        for (int k = 0; k < 5; k++)
+        for (int k = 0; k <= N; k++)
         {
             yM0[k] = yC0[k];
             yM1[k] = yC1[k];
@@ -586,55 +649,59 @@ __device__ __forceinline__ void SplitProlong(const LevelView &fv, const LevelVie
 
 // 3 resident blocks (80 registers, 40 bytes spilled) where the kernel would take 88: measured 14% faster on the 258^3
 // level (its grid of one block per SM or so is latency-bound)
+template <typename T>
 __global__ void __launch_bounds__(kPairThreads, 3) k_split_prolong(LevelView fv, LevelView cv,
                                                                 const uint8_t *__restrict__ pext,
-                                                                const float *__restrict__ ec, float *__restrict__ ef)
+                                                                const T *__restrict__ ec, T *__restrict__ ef)
 {
     PdlWait();
     PdlTrigger();
-    SplitProlong(fv, cv, pext, ec, ef, ThisBlk());
+    SplitProlong<T>(fv, cv, pext, ec, ef, ThisBlk());
 }
 
 // The grid of k_split_prolong: threads over (coarse row, fine quad), grid.y chunks of coarse planes sized like
 // QuadGrid's (the longest march with a full last wave).
-inline dim3 ProlongGridS(const LevelView &fine, const LevelView &coarse, int S)
+template <int N = 4> inline dim3 ProlongGridS(const LevelView &fine, const LevelView &coarse, int S)
 {
-    const long long nq = (long long)(coarse.Nx - 2) * (fine.sRS / 4), perPlane = (nq + kPairThreads - 1) / kPairThreads;
+    const long long nq = (long long)(coarse.Nx - 2) * (fine.sRS / N), perPlane = (nq + kPairThreads - 1) / kPairThreads;
     const long long planes = coarse.Ny - 2 > 0 ? coarse.Ny - 2 : 1;
     return dim3((unsigned)perPlane, (unsigned)((planes + S - 1) / S));
 }
 
-inline dim3 ProlongGrid(const LevelView &fine, const LevelView &coarse, int resident)
+template <int N> inline dim3 ProlongGrid(const LevelView &fine, const LevelView &coarse, int resident)
 {
-    const long long nq = (long long)(coarse.Nx - 2) * (fine.sRS / 4), perPlane = (nq + kPairThreads - 1) / kPairThreads;
+    const long long nq = (long long)(coarse.Nx - 2) * (fine.sRS / N), perPlane = (nq + kPairThreads - 1) / kPairThreads;
     const long long planes = coarse.Ny - 2 > 0 ? coarse.Ny - 2 : 1;
     const long long bestS = BestMarch(perPlane, planes, (long long)SmCount() * (resident > 0 ? resident : 1));
     return dim3((unsigned)perPlane, (unsigned)((planes + bestS - 1) / bestS));
 }
 
-void LaunchSplitProlong(const LevelView &fine, const LevelView &coarse, const uint8_t *pext, const float *eCoarse,
-                        float *eFine, cudaStream_t st)
+template <typename T>
+void LaunchSplitProlong(const LevelView &fine, const LevelView &coarse, const uint8_t *pext, const T *eCoarse,
+                        T *eFine, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    const int occ = Occ<k_split_prolong>();
-    LaunchPdl(k_split_prolong, ProlongGrid(fine, coarse, occ), kPairThreads, 0, st, fine, coarse, pext, eCoarse,
+    const int occ = Occ<k_split_prolong<T>>();
+    LaunchPdl(k_split_prolong<T>, ProlongGrid<kQ<T>>(fine, coarse, occ), kPairThreads, 0, st, fine, coarse, pext, eCoarse,
               eFine);
 }
 
-// r_c = R res_f = P^T res_f at the coarse unknowns, from the red fine residual. A thread owns four consecutive coarse
-// cells K0 .. K0+3 (K0 = 1 + 4 t) of coarse row J (one flat index over (J, t)) and marches along I: fine planes
+// r_c = R res_f = P^T res_f at the coarse unknowns, from the red fine residual. A thread owns N = 4 (FP64: 2) consecutive
+// coarse cells K0 .. K0+N-1 (K0 = 1 + N t) of coarse row J (one flat index over (J, t)) and marches along I: fine planes
 // 2I-2 .. 2I+1 enter as their (j, k)-weighted 4x4 sums T(a), each kept for the next coarse plane; the red children's
 // moved weights enter as X(a). In fine row (a, b) the red cells among k = 2K-2 .. 2K+1 are elements K-1 and K, at
-// k = 2K-2+q and 2K+q (q = (a + b) & 1), and the red child of coarse K is element K - q; the five elements
-// K0-1 .. K0+3 of a row are one aligned float4 and one more.
+// k = 2K-2+q and 2K+q (q = (a + b) & 1), and the red child of coarse K is element K - q; the N + 1 elements
+// K0-1 .. K0+N-1 of a row are one aligned quad and one more.
+template <typename T>
 __device__ __forceinline__ void SplitRestrictPlane(const LevelView &fv, const uint8_t *__restrict__ pext,
-                                                   const float *__restrict__ res, int a, int J, int K0, bool five,
-                                                   float T[4], float X[4])
+                                                   const T *__restrict__ res, int a, int J, int K0, bool more,
+                                                   T (&Tw)[kQ<T>], T (&X)[kQ<T>])
 {
+    constexpr int N = kQ<T>;
 #pragma unroll
-    for (int x = 0; x < 4; x++) T[x] = X[x] = 0.f;
+    for (int x = 0; x < N; x++) Tw[x] = X[x] = (T)0;
     if (a > fv.Ny - 1) return;
-    const float wt[4] = {0.25f, 0.75f, 0.75f, 0.25f};
+    const T wt[4] = {(T)0.25, (T)0.75, (T)0.75, (T)0.25};
 #pragma unroll
     for (int dj = 0; dj < 4; dj++)
     {
@@ -642,55 +709,60 @@ __device__ __forceinline__ void SplitRestrictPlane(const LevelView &fv, const ui
         if (b > fv.Nx - 1) continue;
         const int q = (a + b) & 1;
         const long long row = (long long)a * fv.sPS + (long long)b * fv.sRS + (K0 - 1);
-        const F4 r4 = L4(res + row);
-        const float R[5] = {r4.v[0], r4.v[1], r4.v[2], r4.v[3], five ? res[row + 4] : 0.f};
+        const Quad<T> r4 = LQ(res + row);
+        T R[N + 1];
 #pragma unroll
-        for (int x = 0; x < 4; x++)
-            T[x] += wt[dj] * (q ? 0.75f * R[x] + 0.25f * R[x + 1] : 0.25f * R[x] + 0.75f * R[x + 1]);
+        for (int x = 0; x < N; x++) R[x] = r4.v[x];
+        R[N] = more ? res[row + N] : (T)0;
+#pragma unroll
+        for (int x = 0; x < N; x++)
+            Tw[x] += wt[dj] * (q ? (T)0.75 * R[x] + (T)0.25 * R[x + 1] : (T)0.25 * R[x] + (T)0.75 * R[x + 1]);
         if (dj == 1 || dj == 2)
         {
-            const unsigned w = LdU4(pext + row);
-            const unsigned w4 = five ? pext[row + 4] : 0u;
+            const unsigned w = LdB<N>(pext + row);
+            const unsigned wN = more ? pext[row + N] : 0u;
 #pragma unroll
-            for (int x = 0; x < 4; x++)
+            for (int x = 0; x < N; x++)
             {
-                // the red child of coarse K0 + x is element K0 + x - q: index x + 1 - q of the five
-                const unsigned pw = q ? Byte(w, x) : (x < 3 ? Byte(w, x + 1) : w4);
-                X[x] += (float)(pw & 0x3Fu) * R[x + 1 - q];
+                // the red child of coarse K0 + x is element K0 + x - q: index x + 1 - q of the N + 1
+                const unsigned pw = q ? Byte(w, x) : (x < N - 1 ? Byte(w, x + 1) : wN);
+                X[x] += (T)(pw & 0x3Fu) * R[x + 1 - q];
             }
         }
     }
 #pragma unroll
-    for (int x = 0; x < 4; x++) X[x] *= 1.0f / 64.0f;
+    for (int x = 0; x < N; x++) X[x] *= (T)(1.0 / 64.0);
 }
 
+template <typename T>
 __device__ __forceinline__ void SplitRestrictQ(const LevelView &fv, const LevelView &cv,
-                                               const uint8_t *__restrict__ pext, const float *__restrict__ res,
-                                               float *__restrict__ rc, const Blk &blk)
+                                               const uint8_t *__restrict__ pext, const T *__restrict__ res,
+                                               T *__restrict__ rc, const Blk &blk)
 {
-    const int nq = (cv.Nz - 2 + 3) / 4, nt = (cv.Nx - 2) * nq;
+    constexpr int N = kQ<T>;
+    const int nq = (cv.Nz - 2 + N - 1) / N, nt = (cv.Nx - 2) * nq;
     const int t = blk.x * kPairThreads + threadIdx.x;
     if (t >= nt) return;
-    const int J = 1 + t / nq, K0 = 1 + 4 * (t - (J - 1) * nq);
+    const int J = 1 + t / nq, K0 = 1 + N * (t - (J - 1) * nq);
     const int S = (cv.Ny - 2 + blk.gy - 1) / blk.gy;
     const int I0 = 1 + blk.y * S, I1 = min(I0 + S, cv.Ny - 1);
     if (I0 >= I1) return;
-    const bool five = K0 + 3 <= cv.Nz - 2; // element K0+3 is read only for coarse cell K0+3
-    float Tm2[4], Tm1[4], Xm1[4], Xd[4];
-    SplitRestrictPlane(fv, pext, res, 2 * I0 - 2, J, K0, five, Tm2, Xd);
-    SplitRestrictPlane(fv, pext, res, 2 * I0 - 1, J, K0, five, Tm1, Xm1);
+    const bool more = K0 + N - 1 <= cv.Nz - 2; // element K0+N-1 is read only for coarse cell K0+N-1
+    T Tm2[N], Tm1[N], Xm1[N], Xd[N];
+    SplitRestrictPlane<T>(fv, pext, res, 2 * I0 - 2, J, K0, more, Tm2, Xd);
+    SplitRestrictPlane<T>(fv, pext, res, 2 * I0 - 1, J, K0, more, Tm1, Xm1);
     for (int I = I0; I < I1; I++)
     {
-        float T0[4], X0[4], T1[4], X1[4];
-        SplitRestrictPlane(fv, pext, res, 2 * I, J, K0, five, T0, X0);
-        SplitRestrictPlane(fv, pext, res, 2 * I + 1, J, K0, five, T1, X1);
+        T T0[N], X0[N], T1[N], X1[N];
+        SplitRestrictPlane<T>(fv, pext, res, 2 * I, J, K0, more, T0, X0);
+        SplitRestrictPlane<T>(fv, pext, res, 2 * I + 1, J, K0, more, T1, X1);
         const long long c = (long long)I * cv.sI + (long long)J * cv.sJ + K0;
 #pragma unroll
-        for (int x = 0; x < 4; x++)
+        for (int x = 0; x < N; x++)
         {
             if (K0 + x <= cv.Nz - 2 && (cv.code[c + x] & CODE_UNKNOWN))
                 rc[VecIdx(cv, I, J, K0 + x)] =
-                    ((0.25f * Tm2[x] + 0.75f * Tm1[x]) + (0.75f * T0[x] + 0.25f * T1[x])) + (Xm1[x] + X0[x]);
+                    (((T)0.25 * Tm2[x] + (T)0.75 * Tm1[x]) + ((T)0.75 * T0[x] + (T)0.25 * T1[x])) + (Xm1[x] + X0[x]);
             Tm2[x] = T0[x];
             Tm1[x] = T1[x];
             Xm1[x] = X1[x];
@@ -698,24 +770,26 @@ __device__ __forceinline__ void SplitRestrictQ(const LevelView &fv, const LevelV
     }
 }
 
+template <typename T>
 __global__ void __launch_bounds__(kPairThreads) k_split_restrict(LevelView fv, LevelView cv,
                                                                  const uint8_t *__restrict__ pext,
-                                                                 const float *__restrict__ res, float *__restrict__ rc)
+                                                                 const T *__restrict__ res, T *__restrict__ rc)
 {
     PdlWait();
     PdlTrigger();
-    SplitRestrictQ(fv, cv, pext, res, rc, ThisBlk());
+    SplitRestrictQ<T>(fv, cv, pext, res, rc, ThisBlk());
 }
 
 // The same restriction with one thread per coarse cell (K along the 32 lanes, J across the 8 warps), for the smaller
 // coarse levels: more threads, and their launches are latency-bound.
-__device__ __forceinline__ void SplitRestrictPlane1(const LevelView &fv, const uint8_t *pext, const float *res, int a,
-                                                   int J, int K, float &T, float &X)
+template <typename T>
+__device__ __forceinline__ void SplitRestrictPlane1(const LevelView &fv, const uint8_t *pext, const T *res, int a,
+                                                   int J, int K, T &Tw, T &X)
 {
-    T = 0.f;
-    X = 0.f;
+    Tw = (T)0;
+    X = (T)0;
     if (a > fv.Ny - 1) return;
-    const float wt[4] = {0.25f, 0.75f, 0.75f, 0.25f};
+    const T wt[4] = {(T)0.25, (T)0.75, (T)0.75, (T)0.25};
 #pragma unroll
     for (int dj = 0; dj < 4; dj++)
     {
@@ -723,46 +797,48 @@ __device__ __forceinline__ void SplitRestrictPlane1(const LevelView &fv, const u
         if (b > fv.Nx - 1) continue;
         const int q = (a + b) & 1;
         const long long row = (long long)a * fv.sPS + (long long)b * fv.sRS;
-        const float lo = res[row + K - 1], hi = res[row + K];
-        T += wt[dj] * (q ? 0.75f * lo + 0.25f * hi : 0.25f * lo + 0.75f * hi);
-        if (dj == 1 || dj == 2) X += (float)(pext[row + K - q] & 0x3Fu) * (q ? lo : hi);
+        const T lo = res[row + K - 1], hi = res[row + K];
+        Tw += wt[dj] * (q ? (T)0.75 * lo + (T)0.25 * hi : (T)0.25 * lo + (T)0.75 * hi);
+        if (dj == 1 || dj == 2) X += (T)(pext[row + K - q] & 0x3Fu) * (q ? lo : hi);
     }
-    X *= 1.0f / 64.0f;
+    X *= (T)(1.0 / 64.0);
 }
 
 // bx, by: the K and J tiles; bz of gz: the chunk of coarse planes
+template <typename T>
 __device__ __forceinline__ void SplitRestrict1(const LevelView &fv, const LevelView &cv,
-                                               const uint8_t *__restrict__ pext, const float *__restrict__ res,
-                                               float *__restrict__ rc, int bx, int by, int bz, int gz)
+                                               const uint8_t *__restrict__ pext, const T *__restrict__ res,
+                                               T *__restrict__ rc, int bx, int by, int bz, int gz)
 {
     const int K = 1 + bx * 32 + threadIdx.x, J = 1 + by * 8 + threadIdx.y;
     if (K > cv.Nz - 2 || J > cv.Nx - 2) return;
     const int S = (cv.Ny - 2 + gz - 1) / gz;
     const int I0 = 1 + bz * S, I1 = min(I0 + S, cv.Ny - 1);
     if (I0 >= I1) return;
-    float Tm2, Tm1, Xm1, Xdummy;
-    SplitRestrictPlane1(fv, pext, res, 2 * I0 - 2, J, K, Tm2, Xdummy);
-    SplitRestrictPlane1(fv, pext, res, 2 * I0 - 1, J, K, Tm1, Xm1);
+    T Tm2, Tm1, Xm1, Xdummy;
+    SplitRestrictPlane1<T>(fv, pext, res, 2 * I0 - 2, J, K, Tm2, Xdummy);
+    SplitRestrictPlane1<T>(fv, pext, res, 2 * I0 - 1, J, K, Tm1, Xm1);
     for (int I = I0; I < I1; I++)
     {
-        float T0, X0, T1, X1;
-        SplitRestrictPlane1(fv, pext, res, 2 * I, J, K, T0, X0);
-        SplitRestrictPlane1(fv, pext, res, 2 * I + 1, J, K, T1, X1);
+        T T0, X0, T1, X1;
+        SplitRestrictPlane1<T>(fv, pext, res, 2 * I, J, K, T0, X0);
+        SplitRestrictPlane1<T>(fv, pext, res, 2 * I + 1, J, K, T1, X1);
         const long long c = (long long)I * cv.sI + (long long)J * cv.sJ + K;
         if (cv.code[c] & CODE_UNKNOWN)
-            rc[VecIdx(cv, I, J, K)] = ((0.25f * Tm2 + 0.75f * Tm1) + (0.75f * T0 + 0.25f * T1)) + (Xm1 + X0);
+            rc[VecIdx(cv, I, J, K)] = (((T)0.25 * Tm2 + (T)0.75 * Tm1) + ((T)0.75 * T0 + (T)0.25 * T1)) + (Xm1 + X0);
         Tm2 = T0;
         Tm1 = T1;
         Xm1 = X1;
     }
 }
 
+template <typename T>
 __global__ void __launch_bounds__(256) k_split_restrict1(LevelView fv, LevelView cv, const uint8_t *__restrict__ pext,
-                                                        const float *__restrict__ res, float *__restrict__ rc)
+                                                        const T *__restrict__ res, T *__restrict__ rc)
 {
     PdlWait();
     PdlTrigger();
-    SplitRestrict1(fv, cv, pext, res, rc, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, (int)gridDim.z);
+    SplitRestrict1<T>(fv, cv, pext, res, rc, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, (int)gridDim.z);
 }
 
 // Coarse levels with at least kRestrictQuadCells cells take the quad kernel (4x fewer loads per coarse cell), the
@@ -770,8 +846,9 @@ __global__ void __launch_bounds__(256) k_split_restrict1(LevelView fv, LevelView
 // Both sum the same products in the same order.
 constexpr long long kRestrictQuadCells = 1LL << 20;
 
-void LaunchSplitRestrict(const LevelView &fine, const LevelView &coarse, const uint8_t *pext, const float *resFine,
-                         float *rCoarse, int mode, cudaStream_t st)
+template <typename T>
+void LaunchSplitRestrict(const LevelView &fine, const LevelView &coarse, const uint8_t *pext, const T *resFine,
+                         T *rCoarse, int mode, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
     if (mode == 1 || (mode != 2 && coarse.cells < kRestrictQuadCells))
@@ -780,13 +857,13 @@ void LaunchSplitRestrict(const LevelView &fine, const LevelView &coarse, const u
         const int S = MarchPlanes(coarse.Ny - 2, perPlane);
         const dim3 grid((unsigned)((coarse.Nz - 2 + 31) / 32), (unsigned)((coarse.Nx - 2 + 7) / 8),
                         (unsigned)((coarse.Ny - 2 + S - 1) / S));
-        LaunchPdl(k_split_restrict1, grid, dim3(32, 8), 0, st, fine, coarse, pext, resFine, rCoarse);
+        LaunchPdl(k_split_restrict1<T>, grid, dim3(32, 8), 0, st, fine, coarse, pext, resFine, rCoarse);
         return;
     }
-    const long long nt = (long long)(coarse.Nx - 2) * ((coarse.Nz - 2 + 3) / 4);
+    const long long nt = (long long)(coarse.Nx - 2) * ((coarse.Nz - 2 + kQ<T> - 1) / kQ<T>);
     const long long perPlane = (nt + kPairThreads - 1) / kPairThreads, planes = coarse.Ny - 2 > 0 ? coarse.Ny - 2 : 1;
-    const long long bestS = BestMarch(perPlane, planes, (long long)SmCount() * Occ<k_split_restrict>());
-    LaunchPdl(k_split_restrict, dim3((unsigned)perPlane, (unsigned)((planes + bestS - 1) / bestS)), kPairThreads, 0,
+    const long long bestS = BestMarch(perPlane, planes, (long long)SmCount() * Occ<k_split_restrict<T>>());
+    LaunchPdl(k_split_restrict<T>, dim3((unsigned)perPlane, (unsigned)((planes + bestS - 1) / bestS)), kPairThreads, 0,
               st, fine, coarse, pext, resFine, rCoarse);
 }
 
@@ -799,90 +876,91 @@ __device__ __forceinline__ double SplitRzEff(const double *S, int base, double n
 }
 
 // p_new = U (z - mean + beta p_old), q = M p_new, sum p_new.q, both colours at a thread's quad position.
-template <bool kSingular>
+template <typename T, bool kSingular>
 __device__ __forceinline__ void SplitPApply(const LevelView &v, const uint8_t *__restrict__ du,
-                                            const float *__restrict__ z, float *p0, float *p1, float *__restrict__ q,
+                                            const T *__restrict__ z, T *p0, T *p1, T *__restrict__ q,
                                             const Reducer &R, const double *S, const int *it, int baseEven,
                                             int baseOdd, int slotN, int slotPQ, const Blk &blk)
 {
+    constexpr int N = kQ<T>;
     const int iter = *it, par = iter & 1;
-    const float *__restrict__ pIn = par ? p1 : p0;
-    float *__restrict__ pOut = par ? p0 : p1;
+    const T *__restrict__ pIn = par ? p1 : p0;
+    T *__restrict__ pOut = par ? p0 : p1;
     const int baseNew = par ? baseOdd : baseEven, baseOld = par ? baseEven : baseOdd;
     const double n = S[slotN];
     const double beta =
         iter == 0 ? 0.0 : SplitRzEff(S, baseNew, n, kSingular) / SplitRzEff(S, baseOld, n, kSingular);
-    const float bt = (float)beta;
-    const float mean = kSingular ? (float)(S[baseNew + 1] / n) : 0.f;
-    const QuadPos P = QuadStart(v, blk);
+    const T bt = (T)beta;
+    const T mean = kSingular ? (T)(S[baseNew + 1] / n) : (T)0;
+    const QuadPos P = QuadStart<N>(v, blk);
     if (TileIdle(v, blk.x, P.i0, P.i1))
     {
         double zero[1] = {0.0}; // p and q stay zero on these cells; the block adds its zero term to p.q
         GridReduceB<1>(R, zero, slotPQ, BlkId(blk), BlkCount(blk));
         return;
     }
-    const float g = (float)v.gamma, hg = 0.5f * (float)v.gamma;
+    const T g = (T)v.gamma, hg = (T)0.5 * (T)v.gamma;
     const long long hb = v.sHalf;
     auto pn = [&](long long base) {
-        const F4 zz = L4(z + base), pv = L4(pIn + base);
-        F4 out;
+        const Quad<T> zz = LQ(z + base), pv = LQ(pIn + base);
+        Quad<T> out;
 #pragma unroll
-        for (int x = 0; x < 4; x++) out.v[x] = (zz.v[x] - mean) + bt * pv.v[x];
+        for (int x = 0; x < N; x++) out.v[x] = (zz.v[x] - mean) + bt * pv.v[x];
         if (kSingular)
         {
-            const unsigned d = LdU4(du + base);
+            const unsigned d = LdB<N>(du + base);
 #pragma unroll
-            for (int x = 0; x < 4; x++) out.v[x] *= Unk(Byte(d, x));
+            for (int x = 0; x < N; x++) out.v[x] *= Unk<T>(Byte(d, x));
         }
         return out;
     };
     auto pn1 = [&](long long idx) {
-        float x = (z[idx] - mean) + bt * pIn[idx];
-        if (kSingular) x *= Unk(du[idx]);
+        T x = (z[idx] - mean) + bt * pIn[idx];
+        if (kSingular) x *= Unk<T>(du[idx]);
         return x;
     };
     const long long b0 = P.off, b1 = hb + P.off;
-    F4 M0 = pn(b0 - P.PS), M1 = pn(b1 - P.PS), C0 = pn(b0), C1 = pn(b1);
-    float facc = 0.f;
+    Quad<T> M0 = pn(b0 - P.PS), M1 = pn(b1 - P.PS), C0 = pn(b0), C1 = pn(b1);
+    T facc = (T)0;
     long long o = 0;
     for (int i = P.i0; i < P.i1; i++, o += P.PS)
     {
-        const F4 P0 = pn(b0 + o + P.PS), P1 = pn(b1 + o + P.PS);
-        const F4 Jp0 = pn(b0 + o + P.RS), Jp1 = pn(b1 + o + P.RS), Jm0 = pn(b0 + o - P.RS), Jm1 = pn(b1 + o - P.RS);
-        const unsigned d0 = LdU4(du + b0 + o), d1 = LdU4(du + b1 + o);
+        const Quad<T> P0 = pn(b0 + o + P.PS), P1 = pn(b1 + o + P.PS);
+        const Quad<T> Jp0 = pn(b0 + o + P.RS), Jp1 = pn(b1 + o + P.RS), Jm0 = pn(b0 + o - P.RS), Jm1 = pn(b1 + o - P.RS);
+        const unsigned d0 = LdB<N>(du + b0 + o), d1 = LdB<N>(du + b1 + o);
         const int q0 = (i + P.j) & 1, q1 = q0 ^ 1;
-        float pw0 = __shfl_up_sync(0xffffffffu, C0.v[3], 1), nx0 = __shfl_down_sync(0xffffffffu, C0.v[0], 1);
-        float pw1 = __shfl_up_sync(0xffffffffu, C1.v[3], 1), nx1 = __shfl_down_sync(0xffffffffu, C1.v[0], 1);
+        T pw0 = __shfl_up_sync(0xffffffffu, C0.v[N - 1], 1), nx0 = __shfl_down_sync(0xffffffffu, C0.v[0], 1);
+        T pw1 = __shfl_up_sync(0xffffffffu, C1.v[N - 1], 1), nx1 = __shfl_down_sync(0xffffffffu, C1.v[0], 1);
         if (P.lane == 0 && P.m0 > 0)
         {
             pw0 = pn1(b0 + o - 1);
             pw1 = pn1(b1 + o - 1);
         }
-        if (P.lane == 31 && P.m0 + 4 < P.RS)
+        if (P.lane == 31 && P.m0 + N < P.RS)
         {
-            nx0 = pn1(b0 + o + 4);
-            nx1 = pn1(b1 + o + 4);
+            nx0 = pn1(b0 + o + N);
+            nx1 = pn1(b1 + o + N);
         }
         // colour-0 cells see colour 1 shifted by q0, colour-1 cells see colour 0 shifted by q1
-        const F4 sh1 = KShift(C1, pw1, nx1, q0), sh0 = KShift(C0, pw0, nx0, q1);
-        F4 Q0, Q1;
+        const Quad<T> sh1 = KShift(C1, pw1, nx1, q0), sh0 = KShift(C0, pw0, nx0, q1);
+        Quad<T> Q0, Q1;
 #pragma unroll
-        for (int x = 0; x < 4; x++)
+        for (int x = 0; x < N; x++)
         {
             const unsigned a0 = Byte(d0, x), a1 = Byte(d1, x);
-            const float s0 = ((P1.v[x] + M1.v[x]) + (Jp1.v[x] + Jm1.v[x])) + (C1.v[x] + sh1.v[x]);
-            const float s1 = ((P0.v[x] + M0.v[x]) + (Jp0.v[x] + Jm0.v[x])) + (C0.v[x] + sh0.v[x]);
-            Q0.v[x] = Unk(a0) * (hg * (float)(a0 & 0x7Fu) * C0.v[x] - g * s0);
-            Q1.v[x] = Unk(a1) * (hg * (float)(a1 & 0x7Fu) * C1.v[x] - g * s1);
+            const T s0 = ((P1.v[x] + M1.v[x]) + (Jp1.v[x] + Jm1.v[x])) + (C1.v[x] + sh1.v[x]);
+            const T s1 = ((P0.v[x] + M0.v[x]) + (Jp0.v[x] + Jm0.v[x])) + (C0.v[x] + sh0.v[x]);
+            Q0.v[x] = Unk<T>(a0) * (hg * (T)(a0 & 0x7Fu) * C0.v[x] - g * s0);
+            Q1.v[x] = Unk<T>(a1) * (hg * (T)(a1 & 0x7Fu) * C1.v[x] - g * s1);
         }
         if (P.valid)
         {
-            S4(pOut + b0 + o, C0);
-            S4(pOut + b1 + o, C1);
-            S4(q + b0 + o, Q0);
-            S4(q + b1 + o, Q1);
+            SQ(pOut + b0 + o, C0);
+            SQ(pOut + b1 + o, C1);
+            SQ(q + b0 + o, Q0);
+            SQ(q + b1 + o, Q1);
 #pragma unroll
-            for (int x = 0; x < 4; x++) facc += C0.v[x] * Q0.v[x] + C1.v[x] * Q1.v[x];
+            for (int x = 0; x < N; x++) facc += C0.v[x] * Q0.v[x] + C1.v[x] * Q1.v[x];
         }
         M0 = C0;
         M1 = C1;
@@ -893,36 +971,39 @@ __device__ __forceinline__ void SplitPApply(const LevelView &v, const uint8_t *_
     GridReduceB<1>(R, acc, slotPQ, BlkId(blk), BlkCount(blk));
 }
 
-template <bool kSingular>
-__global__ void __launch_bounds__(kPairThreads, 4)
-    k_split_papply(LevelView v, const uint8_t *__restrict__ du, const float *__restrict__ z, float *p0, float *p1,
-                   float *__restrict__ q, Reducer R, const double *S, const int *it, int baseEven, int baseOdd,
+// FP64: 3 resident blocks (64 registers spill 132 bytes)
+template <typename T, bool kSingular>
+__global__ void __launch_bounds__(kPairThreads, sizeof(T) == 8 ? 3 : 4)
+    k_split_papply(LevelView v, const uint8_t *__restrict__ du, const T *__restrict__ z, T *p0, T *p1,
+                   T *__restrict__ q, Reducer R, const double *S, const int *it, int baseEven, int baseOdd,
                    int slotN, int slotPQ)
 {
     PdlWait();
     PdlTrigger();
-    SplitPApply<kSingular>(v, du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ, ThisBlk());
+    SplitPApply<T, kSingular>(v, du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ, ThisBlk());
 }
 
-void LaunchSplitPApply(const LevelView &v, const uint8_t *du, const float *z, float *p0, float *p1, float *q,
+template <typename T>
+void LaunchSplitPApply(const LevelView &v, const uint8_t *du, const T *z, T *p0, T *p1, T *q,
                        const Reducer &R, const double *S, const int *it, int baseEven, int baseOdd, int slotN,
                        int singular, int slotPQ, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
     if (singular)
-        LaunchPdl(k_split_papply<true>, QuadGrid(v, Occ<k_split_papply<true>>()), kPairThreads, 0, st, v, du, z, p0,
-                  p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ);
+        LaunchPdl(k_split_papply<T, true>, QuadGrid<kQ<T>>(v, Occ<k_split_papply<T, true>>()), kPairThreads, 0, st, v,
+                  du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ);
     else
-        LaunchPdl(k_split_papply<false>, QuadGrid(v, Occ<k_split_papply<false>>()), kPairThreads, 0, st, v, du, z, p0,
-                  p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ);
+        LaunchPdl(k_split_papply<T, false>, QuadGrid<kQ<T>>(v, Occ<k_split_papply<T, false>>()), kPairThreads, 0, st,
+                  v, du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// the FP64 side of level 0: FP64 arrays in the grid layout, the FP32 vectors colour-split
+// the outer FP64 side of level 0: FP64 arrays in the grid layout, the solver's vectors (T) colour-split
 // ---------------------------------------------------------------------------------------------------------------
 // r = sfac * b (split) and (sum b^2, sum b): the residual of a zero iterate. One thread per cell pair (k0 even).
 // bx of gx: this block among the launch's blocks (a grid-stride loop)
-__device__ __forceinline__ void SplitScaleSum(const LevelView &v, const double *__restrict__ b, float *__restrict__ r,
+template <typename T>
+__device__ __forceinline__ void SplitScaleSum(const LevelView &v, const double *__restrict__ b, T *__restrict__ r,
                                               double sfac, const Reducer &R, int slot, int bx, int gx)
 {
     double acc[2] = {0.0, 0.0};
@@ -937,8 +1018,8 @@ __device__ __forceinline__ void SplitScaleSum(const LevelView &v, const double *
         const int i = (int)(row / v.Nx), j = (int)(row - (long long)i * v.Nx);
         const int par = (i + j) & 1; // the colour of the pair's first cell
         const long long s = (long long)i * v.sPS + (long long)j * v.sRS + m;
-        r[par * v.sHalf + s] = (float)(x.x * sfac);
-        r[(par ^ 1) * v.sHalf + s] = (float)(x.y * sfac);
+        r[par * v.sHalf + s] = (T)(x.x * sfac);
+        r[(par ^ 1) * v.sHalf + s] = (T)(x.y * sfac);
         acc[0] += x.x * x.x + x.y * x.y;
         acc[1] += x.x + x.y;
     }
@@ -947,29 +1028,32 @@ __device__ __forceinline__ void SplitScaleSum(const LevelView &v, const double *
 
 constexpr int kScaleSumBlocks = 148 * 8;
 
+template <typename T>
 __global__ void __launch_bounds__(256) k_split_scale_sum(LevelView v, const double *__restrict__ b,
-                                                         float *__restrict__ r, double sfac, Reducer R, int slot)
+                                                         T *__restrict__ r, double sfac, Reducer R, int slot)
 {
-    SplitScaleSum(v, b, r, sfac, R, slot, (int)blockIdx.x, (int)gridDim.x);
+    SplitScaleSum<T>(v, b, r, sfac, R, slot, (int)blockIdx.x, (int)gridDim.x);
 }
 
-void LaunchSplitScaleSum(const LevelView &v, const double *b, float *r, double sfac, const Reducer &R, int slot,
+template <typename T>
+void LaunchSplitScaleSum(const LevelView &v, const double *b, T *r, double sfac, const Reducer &R, int slot,
                          cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    k_split_scale_sum<<<kScaleSumBlocks, 256, 0, st>>>(v, b, r, sfac, R, slot);
+    k_split_scale_sum<T><<<kScaleSumBlocks, 256, 0, st>>>(v, b, r, sfac, R, slot);
 }
 
 // The FP64 refinement step on a uniform split level 0 (k_pair_refine64's, with e read and r written split):
-// x_out = x_in + e; r = sfac (b - A x_out) in FP32; (sum (b - A x_out)^2, sum (b - A x_out)) in FP64. One thread per
+// x_out = x_in + e; r = sfac (b - A x_out) in T; (sum (b - A x_out)^2, sum (b - A x_out)) in FP64. One thread per
 // cell pair of the grid layout; the pair (k0, k0+1) of row (i, j) is element k0/2 of colours (i+j)&1 and its other.
 __device__ __forceinline__ double2 Ld2d(const double *p) { return *reinterpret_cast<const double2 *>(p); }
 
 // 3 resident blocks (80 registers, no spill) beat 4 with a 64-register cap that spills (measured 115 vs 122 us)
+template <typename T>
 __device__ __forceinline__ void SplitRefine64(const LevelView &v, const uint8_t *__restrict__ du,
                                               const double *__restrict__ b, const double *__restrict__ xin,
-                                              const float *__restrict__ e, double *__restrict__ xout,
-                                              float *__restrict__ r, double scale, double sfac, const Reducer &R,
+                                              const T *__restrict__ e, double *__restrict__ xout,
+                                              T *__restrict__ r, double scale, double sfac, const Reducer &R,
                                               int slot, const Blk &blk)
 {
     const PairPos P = PairStart(v, blk.x, blk.y, blk.gy);
@@ -978,7 +1062,7 @@ __device__ __forceinline__ void SplitRefine64(const LevelView &v, const uint8_t 
         // the block's pairs lie in rows j0 .. j1; with no unknown there, x_out = x_in + e and r stay zero
         const long long c0 = 2LL * kPairThreads * blk.x;
         const int j0 = (int)(c0 / v.Nz), j1 = min(v.Nx - 1, (int)((c0 + 2 * kPairThreads - 1) / v.Nz));
-        if (RowsIdle(v, j0, j1, P.i0, P.i1))
+        if (RowsIdle<kQ<T> * kPairThreads>(v, j0, j1, P.i0, P.i1))
         {
             double zero[2] = {0.0, 0.0};
             GridReduceB<2>(R, zero, slot, BlkId(blk), BlkCount(blk));
@@ -987,14 +1071,14 @@ __device__ __forceinline__ void SplitRefine64(const LevelView &v, const uint8_t 
     }
     const long long sb = (long long)P.i0 * v.sPS + (long long)P.j * v.sRS + (P.k0 >> 1);
     // the thread's element on plane i0 in colour 0 and colour 1
-    const float *e0 = e + sb, *e1 = e + v.sHalf + sb;
+    const T *e0 = e + sb, *e1 = e + v.sHalf + sb;
     const uint8_t *d0p = du + sb, *d1p = du + v.sHalf + sb;
-    float *r0p = r + sb, *r1p = r + v.sHalf + sb;
+    T *r0p = r + sb, *r1p = r + v.sHalf + sb;
     const double *xp = xin + P.base;
     // x_in + e at the pair `o` cells (grid layout) / `so` elements (split) away; par: the colour of its first cell
     auto X = [&](long long o, long long so, int par) {
         const double2 a = Ld2d(xp + o);
-        const float fa = e0[so], fb = e1[so];
+        const T fa = e0[so], fb = e1[so];
         return make_double2(a.x + (double)(par ? fb : fa), a.y + (double)(par ? fa : fb));
     };
     const int par0 = (P.i0 + P.j) & 1;
@@ -1022,7 +1106,7 @@ __device__ __forceinline__ void SplitRefine64(const LevelView &v, const uint8_t 
         if (P.valid)
         {
             *reinterpret_cast<double2 *>(xout + P.base + off) = XC;
-            const float f0 = (float)(r0 * sfac), f1 = (float)(r1 * sfac);
+            const T f0 = (T)(r0 * sfac), f1 = (T)(r1 * sfac);
             r0p[so] = par ? f1 : f0;
             r1p[so] = par ? f0 : f1;
             acc[0] += r0 * r0 + r1 * r1;
@@ -1035,22 +1119,24 @@ __device__ __forceinline__ void SplitRefine64(const LevelView &v, const uint8_t 
 }
 
 // swap (may be null): when *swap is odd, x_in and x_out trade places
+template <typename T>
 __global__ void __launch_bounds__(kPairThreads, 3)
     k_split_refine64(LevelView v, const uint8_t *__restrict__ du, const double *__restrict__ b,
-                     const double *xin, const float *__restrict__ e, double *xout,
-                     float *__restrict__ r, double scale, double sfac, Reducer R, int slot, const int *swap)
+                     const double *xin, const T *__restrict__ e, double *xout,
+                     T *__restrict__ r, double scale, double sfac, Reducer R, int slot, const int *swap)
 {
     const bool sw = swap && (*swap & 1);
-    SplitRefine64(v, du, b, sw ? xout : xin, e, sw ? const_cast<double *>(xin) : xout, r, scale, sfac, R, slot,
+    SplitRefine64<T>(v, du, b, sw ? xout : xin, e, sw ? const_cast<double *>(xin) : xout, r, scale, sfac, R, slot,
                   ThisBlk());
 }
 
-void LaunchSplitRefine64(const LevelView &v, const uint8_t *du, const double *b, const double *xin, const float *e,
-                         double *xout, float *r, double scale, double sfac, const Reducer &R, int slot,
+template <typename T>
+void LaunchSplitRefine64(const LevelView &v, const uint8_t *du, const double *b, const double *xin, const T *e,
+                         double *xout, T *r, double scale, double sfac, const Reducer &R, int slot,
                          cudaStream_t st, const int *swap)
 {
     NB_COUNT_LAUNCH();
-    k_split_refine64<<<PairGrid(v, kSplitReduceS), kPairThreads, 0, st>>>(v, du, b, xin, e, xout, r, scale, sfac, R,
+    k_split_refine64<T><<<PairGrid(v, kSplitReduceS), kPairThreads, 0, st>>>(v, du, b, xin, e, xout, r, scale, sfac, R,
                                                                            slot, swap);
 }
 
@@ -1069,7 +1155,7 @@ __global__ void __launch_bounds__(kPairThreads, 4) kb_split_first(const BatchLev
     const int q = BatchReqOf(a);
     if (q < 0) return;
     const BatchLevel &L = lv[q * ls + l];
-    SplitFirst(L.v, L.du, L.r, L.e, ThisBlk());
+    SplitFirst<float>(L.v, L.du, L.r, L.e, ThisBlk());
 }
 
 template <int kDot>
@@ -1084,10 +1170,10 @@ __global__ void __launch_bounds__(kPairThreads, kDot ? 3 : 4)
     const BatchLevel &L = lv[q * ls + l];
     const long long h = L.v.sHalf;
     if (kDot)
-        SplitHalf<kDot>(L.v, L.du + colour * h, L.r + colour * h, L.e + (colour ^ 1) * h, L.e + colour * h, colour,
+        SplitHalf<float, kDot>(L.v, L.du + colour * h, L.r + colour * h, L.e + (colour ^ 1) * h, L.e + colour * h, colour,
                         rq[q].red, rq[q].it, baseEven, baseOdd, partSlot, ThisBlk());
     else
-        SplitHalf<kDot>(L.v, L.du + colour * h, L.r + colour * h, L.e + (colour ^ 1) * h, L.e + colour * h, colour,
+        SplitHalf<float, kDot>(L.v, L.du + colour * h, L.r + colour * h, L.e + (colour ^ 1) * h, L.e + colour * h, colour,
                         Reducer{}, nullptr, baseEven, baseOdd, partSlot, ThisBlk());
 }
 
@@ -1099,7 +1185,7 @@ __global__ void __launch_bounds__(kPairThreads, 3) kb_split_residual(const Batch
     const int q = BatchReqOf(a);
     if (q < 0) return;
     const BatchLevel &L = lv[q * ls + l];
-    SplitResidual(L.v, L.du, L.r, L.e, L.res, ThisBlk());
+    SplitResidual<float>(L.v, L.du, L.r, L.e, L.res, ThisBlk());
 }
 
 __global__ void __launch_bounds__(kPairThreads) kb_split_prolong(const BatchLevel *__restrict__ lv, int ls, int l,
@@ -1110,7 +1196,7 @@ __global__ void __launch_bounds__(kPairThreads) kb_split_prolong(const BatchLeve
     const int q = BatchReqOf(a);
     if (q < 0) return;
     const BatchLevel &F = lv[q * ls + l], &C = lv[q * ls + l + 1];
-    SplitProlong(F.v, C.v, F.pext, C.e, F.e, ThisBlk());
+    SplitProlong<float>(F.v, C.v, F.pext, C.e, F.e, ThisBlk());
 }
 
 __global__ void __launch_bounds__(kPairThreads) kb_split_restrict(const BatchLevel *__restrict__ lv, int ls, int l,
@@ -1121,7 +1207,7 @@ __global__ void __launch_bounds__(kPairThreads) kb_split_restrict(const BatchLev
     const int q = BatchReqOf(a);
     if (q < 0) return;
     const BatchLevel &F = lv[q * ls + l], &C = lv[q * ls + l + 1];
-    SplitRestrictQ(F.v, C.v, F.pext, F.res, C.r, ThisBlk());
+    SplitRestrictQ<float>(F.v, C.v, F.pext, F.res, C.r, ThisBlk());
 }
 
 // grid (K tiles, J tiles x gz plane chunks, capacity)
@@ -1134,7 +1220,7 @@ __global__ void __launch_bounds__(256) kb_split_restrict1(const BatchLevel *__re
     if (q < 0) return;
     const BatchLevel &F = lv[q * ls + l], &C = lv[q * ls + l + 1];
     const int by = (int)blockIdx.y % gyJ, bz = (int)blockIdx.y / gyJ;
-    SplitRestrict1(F.v, C.v, F.pext, F.res, C.r, (int)blockIdx.x, by, bz, gz);
+    SplitRestrict1<float>(F.v, C.v, F.pext, F.res, C.r, (int)blockIdx.x, by, bz, gz);
 }
 
 // form -1: every request in its own form; 0 / 1: only the requests of that form (singular = 1)
@@ -1150,10 +1236,10 @@ __global__ void __launch_bounds__(kPairThreads, 4)
     const BatchReq &Q = rq[q];
     if (form >= 0 && (Q.singular != 0) != (form == 1)) return;
     if (Q.singular)
-        SplitPApply<true>(L.v, L.du, L.e, Q.p0, Q.p1, Q.q, Q.red, Q.red.out, Q.it, baseEven, baseOdd, slotN, slotPQ,
+        SplitPApply<float, true>(L.v, L.du, L.e, Q.p0, Q.p1, Q.q, Q.red, Q.red.out, Q.it, baseEven, baseOdd, slotN, slotPQ,
                           ThisBlk());
     else
-        SplitPApply<false>(L.v, L.du, L.e, Q.p0, Q.p1, Q.q, Q.red, Q.red.out, Q.it, baseEven, baseOdd, slotN, slotPQ,
+        SplitPApply<float, false>(L.v, L.du, L.e, Q.p0, Q.p1, Q.q, Q.red, Q.red.out, Q.it, baseEven, baseOdd, slotN, slotPQ,
                            ThisBlk());
 }
 
@@ -1164,7 +1250,7 @@ __global__ void __launch_bounds__(256) kb_split_scale_sum(const BatchLevel *__re
     if (q < 0) return;
     const BatchLevel &L = lv[q * ls];
     const BatchReq &Q = rq[q];
-    SplitScaleSum(L.v, Q.b, L.r, Q.sfac, Q.red, slot, (int)blockIdx.x, (int)gridDim.x);
+    SplitScaleSum<float>(L.v, Q.b, L.r, Q.sfac, Q.red, slot, (int)blockIdx.x, (int)gridDim.x);
 }
 
 // parity[q]: this pass reads x from xin (0) or xout (1) and writes the other
@@ -1177,7 +1263,7 @@ __global__ void __launch_bounds__(kPairThreads, 3)
     const BatchLevel &L = lv[q * ls];
     const BatchReq &Q = rq[q];
     const bool odd = parity[q] & 1;
-    SplitRefine64(L.v, L.du, Q.b, odd ? Q.xout : Q.xin, Q.x, odd ? Q.xin : Q.xout, L.r, Q.scale, Q.sfac, Q.red, slot,
+    SplitRefine64<float>(L.v, L.du, Q.b, odd ? Q.xout : Q.xin, Q.x, odd ? Q.xin : Q.xout, L.r, Q.scale, Q.sfac, Q.red, slot,
                   ThisBlk());
 }
 
@@ -1197,12 +1283,12 @@ int SplitDefaultS(const LevelView &v, int kind)
     int occ = 1;
     switch (kind)
     {
-    case NB_BK_FIRST: occ = Occ<k_split_first>(); break;
-    case NB_BK_HALF: occ = Occ<k_split_half<0>>(); break;
-    default: occ = Occ<k_split_residual>(); break;
+    case NB_BK_FIRST: occ = Occ<k_split_first<float>>(); break;
+    case NB_BK_HALF: occ = Occ<k_split_half<float, 0>>(); break;
+    default: occ = Occ<k_split_residual<float>>(); break;
     }
     const long long planes = v.Ny - 2 > 0 ? v.Ny - 2 : 1;
-    const dim3 g = QuadGrid(v, occ);
+    const dim3 g = QuadGrid<4>(v, occ);
     return (int)((planes + g.y - 1) / g.y);
 }
 
@@ -1215,17 +1301,17 @@ void LaunchBatchSplit(int kind, const LevelView &v, const LevelView *coarse, int
     switch (kind)
     {
     case NB_BK_FIRST:
-        LaunchPdl(kb_split_first, WithZ(QuadGridS(v, S), cap), kPairThreads, 0, st, lv, ls, l, a);
+        LaunchPdl(kb_split_first, WithZ(QuadGridS<4>(v, S), cap), kPairThreads, 0, st, lv, ls, l, a);
         break;
     case NB_BK_HALF:
-        LaunchPdl(kb_split_half<0>, WithZ(QuadGridS(v, S), cap), kPairThreads, 0, st, lv, ls, l, rq, a, colour, 0, 0,
+        LaunchPdl(kb_split_half<0>, WithZ(QuadGridS<4>(v, S), cap), kPairThreads, 0, st, lv, ls, l, rq, a, colour, 0, 0,
                   0);
         break;
     case NB_BK_RESIDUAL:
-        LaunchPdl(kb_split_residual, WithZ(QuadGridS(v, S), cap), kPairThreads, 0, st, lv, ls, l, a);
+        LaunchPdl(kb_split_residual, WithZ(QuadGridS<4>(v, S), cap), kPairThreads, 0, st, lv, ls, l, a);
         break;
     case NB_BK_PROLONG:
-        LaunchPdl(kb_split_prolong, WithZ(ProlongGridS(v, *coarse, S), cap), kPairThreads, 0, st, lv, ls, l, a);
+        LaunchPdl(kb_split_prolong, WithZ(ProlongGridS<4>(v, *coarse, S), cap), kPairThreads, 0, st, lv, ls, l, a);
         break;
     case NB_BK_RESTRICT:
     {
@@ -1257,10 +1343,10 @@ void LaunchBatchSplitHalfDot(const LevelView &v, const BatchLevel *lv, int ls, c
 {
     NB_COUNT_LAUNCH();
     if (last)
-        LaunchPdl(kb_split_half<2>, WithZ(QuadGrid(v, Occ<k_split_half<2>>()), cap), kPairThreads, 0, st, lv, ls, 0,
+        LaunchPdl(kb_split_half<2>, WithZ(QuadGrid<4>(v, Occ<k_split_half<float, 2>>()), cap), kPairThreads, 0, st, lv, ls, 0,
                   rq, a, colour, baseEven, baseOdd, partSlot);
     else
-        LaunchPdl(kb_split_half<1>, WithZ(QuadGrid(v, Occ<k_split_half<1>>()), cap), kPairThreads, 0, st, lv, ls, 0,
+        LaunchPdl(kb_split_half<1>, WithZ(QuadGrid<4>(v, Occ<k_split_half<float, 1>>()), cap), kPairThreads, 0, st, lv, ls, 0,
                   rq, a, colour, baseEven, baseOdd, partSlot);
 }
 
@@ -1269,7 +1355,7 @@ void LaunchBatchSplitPApply(const LevelView &v, const BatchLevel *lv, int ls, co
 {
     // a single solve launches its form (singular or not) on that form's grid; both have the same occupancy unless
     // the compiler gave them different register counts, and then each form gets a launch on its own grid
-    const dim3 gs = QuadGrid(v, Occ<k_split_papply<true>>()), gn = QuadGrid(v, Occ<k_split_papply<false>>());
+    const dim3 gs = QuadGrid<4>(v, Occ<k_split_papply<float, true>>()), gn = QuadGrid<4>(v, Occ<k_split_papply<float, false>>());
     if (gs.x == gn.x && gs.y == gn.y)
     {
         NB_COUNT_LAUNCH();
@@ -1301,45 +1387,78 @@ void LaunchBatchSplitRefine64(const LevelView &v, const BatchLevel *lv, int ls, 
 // ---------------------------------------------------------------------------------------------------------------
 // tile activity: one thread per (plane, tile), ORing the unknown bits of the tile's diagonal bytes in both colours
 // ---------------------------------------------------------------------------------------------------------------
-constexpr int kTileElems = 4 * kPairThreads;
+static int TileElems(int elemBytes) { return 16 / elemBytes * kPairThreads; }
 
-int SplitActivityTiles(const LevelView &v) { return (v.sPS + kTileElems - 1) / kTileElems; }
+int SplitActivityTiles(const LevelView &v, int elemBytes)
+{
+    return (v.sPS + TileElems(elemBytes) - 1) / TileElems(elemBytes);
+}
 
 __global__ void __launch_bounds__(256) k_split_activity(LevelView v, const uint8_t *__restrict__ du,
-                                                        uint8_t *__restrict__ act, int tiles)
+                                                        uint8_t *__restrict__ act, int tiles, int tileElems)
 {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= (long long)v.Ny * tiles) return;
     const int i = (int)(t / tiles), tile = (int)(t - (long long)i * tiles);
-    const int e0 = tile * kTileElems, e1 = min(e0 + kTileElems, v.sPS);
+    const int e0 = tile * tileElems, e1 = min(e0 + tileElems, v.sPS);
     unsigned any = 0;
     for (int c = 0; c < 2; c++)
     {
         const uint8_t *row = du + (long long)c * v.sHalf + (long long)i * v.sPS;
-        for (int e = e0; e < e1; e += 4) any |= LdU4(row + e); // sPS and e0 are multiples of 4
+        for (int e = e0; e < e1; e += 4) any |= LdB<4>(row + e); // sPS and e0 are multiples of 4
     }
     act[t] = (any & 0x80808080u) ? 1 : 0;
 }
 
-void LaunchSplitActivity(const LevelView &v, const uint8_t *du, uint8_t *act, int tiles, cudaStream_t st)
+void LaunchSplitActivity(const LevelView &v, const uint8_t *du, uint8_t *act, int tiles, int elemBytes,
+                         cudaStream_t st)
 {
     const long long n = (long long)v.Ny * tiles;
     NB_COUNT_LAUNCH();
-    k_split_activity<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(v, du, act, tiles);
+    k_split_activity<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(v, du, act, tiles, TileElems(elemBytes));
 }
 
 // The occupancy of every split kernel, read outside any stream capture (the launchers size their grids from it).
-void PrepareSplitKernels()
+template <typename T> static void PrepareSplit()
 {
-    (void)Occ<k_split_first>();
-    (void)Occ<k_split_half<0>>();
-    (void)Occ<k_split_half<1>>();
-    (void)Occ<k_split_half<2>>();
-    (void)Occ<k_split_residual>();
-    (void)Occ<k_split_prolong>();
-    (void)Occ<k_split_restrict>();
-    (void)Occ<k_split_papply<true>>();
-    (void)Occ<k_split_papply<false>>();
+    (void)Occ<k_split_first<T>>();
+    (void)Occ<k_split_half<T, 0>>();
+    (void)Occ<k_split_half<T, 1>>();
+    (void)Occ<k_split_half<T, 2>>();
+    (void)Occ<k_split_residual<T>>();
+    (void)Occ<k_split_prolong<T>>();
+    (void)Occ<k_split_restrict<T>>();
+    (void)Occ<k_split_papply<T, true>>();
+    (void)Occ<k_split_papply<T, false>>();
 }
+
+void PrepareSplitKernels(int elemBytes)
+{
+    if (elemBytes == 8) PrepareSplit<double>();
+    else PrepareSplit<float>();
+}
+
+#define NB_INST(T)                                                                                                 \
+    template void LaunchSplitFirst<T>(const LevelView &, const uint8_t *, const T *, T *, cudaStream_t);           \
+    template void LaunchSplitHalf<T>(const LevelView &, const uint8_t *, const T *, T *, int, cudaStream_t);       \
+    template void LaunchSplitHalfDot<T>(const LevelView &, const uint8_t *, const T *, T *, int, bool,             \
+                                        const Reducer &, const int *, int, int, int, cudaStream_t);                \
+    template void LaunchSplitResidual<T>(const LevelView &, const uint8_t *, const T *, const T *, T *,            \
+                                         cudaStream_t);                                                            \
+    template void LaunchSplitProlong<T>(const LevelView &, const LevelView &, const uint8_t *, const T *, T *,     \
+                                        cudaStream_t);                                                             \
+    template void LaunchSplitRestrict<T>(const LevelView &, const LevelView &, const uint8_t *, const T *, T *,    \
+                                         int, cudaStream_t);                                                       \
+    template void LaunchSplitPApply<T>(const LevelView &, const uint8_t *, const T *, T *, T *, T *,               \
+                                       const Reducer &, const double *, const int *, int, int, int, int, int,      \
+                                       cudaStream_t);                                                              \
+    template void LaunchSplitScaleSum<T>(const LevelView &, const double *, T *, double, const Reducer &, int,     \
+                                         cudaStream_t);                                                            \
+    template void LaunchSplitRefine64<T>(const LevelView &, const uint8_t *, const double *, const double *,       \
+                                         const T *, double *, T *, double, double, const Reducer &, int,           \
+                                         cudaStream_t, const int *);
+NB_INST(float)
+NB_INST(double)
+#undef NB_INST
 
 } // namespace nb

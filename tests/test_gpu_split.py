@@ -179,3 +179,39 @@ def test_device_refinement_loop_limits(nb):
     s.DestroyPressureSolver()
     assert r0.status == capi.NB_OK and r0.iters_outer == 0 and r0.iters_inner == 0 and r0.rel_res == 0.0
     assert not np.any(z.p[types == W.FLUID])
+
+
+# FP64: (interior x, y, z), outlet or closed; row lengths around the 16-byte quads and their padding, one tile and
+# several, the smallest grid with a split level above the coarse end and its neighbours
+FP64_SIZES = [(12, 12, 12), (14, 13, 16), (16, 16, 14), (30, 36, 26), (33, 40, 48), (64, 20, 34)]
+
+
+@pytest.mark.parametrize("closed", [False, True])
+@pytest.mark.parametrize("size", FP64_SIZES)
+def test_fp64_split_agrees_with_per_cell_kernels(nb, size, closed):
+    """The plain FP64 form on the colour-split layout against its per-cell kernels (pair_kernels = 0), both to 1e-12.
+    Each solution is within cond * 1e-12 of the exact one; cond <= 5 N^2 on N cells along the longest side (the lowest
+    mode a quarter wave), so the two agree within 1e-11 N^2."""
+    nx, ny, nz = size
+    h = 1.0 / min(nx, ny)
+    g = W.uniform_grid(3, (0.0, nx * h, 0.0, ny * h, 0.0, nz * h), min(nx, ny))
+    assert (g.Nx, g.Ny, g.Nz) == (nx + 2, ny + 2, nz + 2)
+    sph = W.Region(W.REGION_SOLID, W.PRIM_SPHERE, (0.5 * nx * h, 0.5 * ny * h, 0.5 * nz * h), radius=0.2 * min(size) * h)
+    case = W.Case("fp64", g, W.walls_scene(3, outlet_face=None if closed else 1, regions=[sph]), 31,
+                  needs_compat=closed)
+    types = capi.label_cells(g, case.scene)
+    u, v, w = W.face_velocities(g, types, case.seed)
+    out = []
+    for family in (2, 0):
+        m = MACGrid(g, types.copy(), u.copy(), v.copy(), w.copy(), np.zeros(g.cells), case.rho, case.dt)
+        s = PressureSolver("fp64", pair_kernels=family, tail_cells=512)
+        r = s.SolvePressure(m, tol=1e-12, needs_compat=closed)
+        assert r.status == capi.NB_OK and r.rel_res <= 1e-12
+        assert s.lib.nereus_b200_last_iterations(s.ctx) > 0
+        s.DestroyPressureSolver()
+        out.append(m)
+    a, b = out
+    bar = 1e-11 * max(size) ** 2
+    assert np.linalg.norm(a.p - b.p) <= bar * np.linalg.norm(b.p)
+    for x, y in ((a.u, b.u), (a.v, b.v), (a.w, b.w)):
+        assert np.linalg.norm(x - y) <= bar * np.linalg.norm(y)
