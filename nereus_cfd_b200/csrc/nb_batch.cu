@@ -340,7 +340,8 @@ struct Batch
         if (A.tailStart < 1 || A.tailStart >= (int)A.L.size())
             throw InputError("the batched form needs split levels above a shared-memory coarse end");
         for (int l = 0; l < A.tailStart; l++)
-            if (!A.Split(l)) throw InputError("the batched form needs colour-split levels above the coarse end");
+            if (!A.Split(l) || A.L[l].Nz % 2)
+                throw InputError("the batched form needs colour-split levels of even Nz above the coarse end");
         for (int i = 1; i < count; i++)
         {
             Context &B = *ctx[i];

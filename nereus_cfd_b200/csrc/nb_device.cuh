@@ -43,7 +43,7 @@ struct LevelView
     int fastLen, midLen, slowLen, slowChunk;
     // Colour-split layout of the level's solver vectors (sRS = 0: the grid layout). Cell (i, j, k) of colour
     // c = (i+j+k) & 1 sits at c*sHalf + i*sPS + j*sRS + (k >> 1): each colour is an Ny x Nx x sRS array whose rows
-    // hold the Nz/2 cells of that colour, padded with zeros to a multiple of 4.
+    // hold that colour's cells (at most (Nz+1)/2), padded with zeros to a multiple of 4.
     int sRS, sPS;
     long long sHalf;
     // Colour-split level: act[i * actTiles + t] != 0 when tile t of plane i (1024 FP32 or 512 FP64 elements of either
@@ -295,15 +295,16 @@ inline int MarchPlanes(long long planes, long long perPlane)
 
 // The launch grid of a pair kernel; minS: at least this many planes per thread (the launches that end in a
 // grid-wide sum keep their partial sums few).
-inline dim3 PairGrid(const LevelView &v, int minS = 1)
+inline dim3 PairGridOf(long long pairs, long long planes, int minS)
 {
-    const long long P = v.sI / 2, perPlane = (P + kPairThreads - 1) / kPairThreads, planes = v.Ny - 2;
+    const long long perPlane = (pairs + kPairThreads - 1) / kPairThreads;
     int S = MarchPlanes(planes, perPlane);
     const int cap = (int)(planes > 1 ? planes : 1);
     const int m = minS < cap ? minS : cap;
     if (m > S) S = m;
     return dim3((unsigned)perPlane, (unsigned)((planes + S - 1) / S));
 }
+inline dim3 PairGrid(const LevelView &v, int minS = 1) { return PairGridOf(v.sI / 2, v.Ny - 2, minS); }
 
 // Per-thread position of a pair kernel.
 struct PairPos

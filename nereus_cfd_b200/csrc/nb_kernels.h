@@ -110,8 +110,9 @@ void LaunchLinXR(long long cells, T *x, T *r, const T *p0, const T *p1, const T 
                  const double *S, int *it, int baseEven, int baseOdd, int slotN, int singular, int slotPQ, int slotRR,
                  cudaStream_t st);
 
-// ---- nb_split.cu: kernels for 3D levels with Nz even in the colour-split layout (LevelView::sRS), T = float (the
-//      mixed form's inner solve) or double (the plain FP64 form) ----
+// ---- nb_split.cu: kernels for 3D levels in the colour-split layout (LevelView::sRS), T = float (the mixed form's
+//      inner solve) or double (the plain FP64 form) ----
+bool SplitLevelShape(const LevelView &v);
 // uniform levels only; du: the level's diagonal units in that layout; pext: the red cells' bytes
 // reads the kernels' occupancy (their grids follow it); call before capturing launches into a graph
 void PrepareSplitKernels(int elemBytes);

@@ -3,8 +3,8 @@
 // plain FP64 form.
 //
 // Colour-split layout. Cell (i, j, k) has colour c = (i + j + k) & 1 and sits at c*H + i*PS + j*RS + (k >> 1) of a
-// level vector: each colour is an Ny x Nx x RS array whose rows hold the Nz/2 cells of that colour (RS = Nz/2
-// rounded up to 4, the padding kept at zero). In row (i, j) the cell of colour c at element m is k = 2m + q with
+// level vector: each colour is an Ny x Nx x RS array whose rows hold that colour's cells (RS = (Nz+1)/2 rounded up
+// to 4, the padding kept at zero; with Nz odd the rows of one colour hold a cell less, its element counts as padding). In row (i, j) the cell of colour c at element m is k = 2m + q with
 // q = (i + j + c) & 1, and its six neighbours all have the other colour:
 //   (i +- 1, j, m), (i, j +- 1, m), (i, j, m) and (i, j, m + (q ? 1 : -1)).
 // A half-sweep of colour c therefore reads the other colour, r and the diagonal bytes of colour c, and writes
@@ -32,6 +32,8 @@
 
 namespace nb
 {
+
+bool SplitLevelShape(const LevelView &v) { return v.dim == 3 && v.Nx >= 3 && v.Ny >= 3 && v.Nz >= 3; }
 
 namespace
 {
@@ -1000,21 +1002,37 @@ void LaunchSplitPApply(const LevelView &v, const uint8_t *du, const T *z, T *p0,
 // ---------------------------------------------------------------------------------------------------------------
 // the outer FP64 side of level 0: FP64 arrays in the grid layout, the solver's vectors (T) colour-split
 // ---------------------------------------------------------------------------------------------------------------
+// The two cells (i, j, k0), (i, j, k0 + 1), k0 even, of an FP64 grid-layout array: one aligned 16-byte access with Nz
+// even; with Nz odd two 8-byte ones, the second left out (and read as zero) past the row's last cell (two = false).
+template <bool kEven> __device__ __forceinline__ double2 LdPair(const double *p, bool two)
+{
+    if constexpr (kEven) return *reinterpret_cast<const double2 *>(p);
+    else return make_double2(p[0], two ? p[1] : 0.0);
+}
+template <bool kEven> __device__ __forceinline__ void StPair64(double *p, const double2 &x, bool two)
+{
+    if constexpr (kEven) *reinterpret_cast<double2 *>(p) = x;
+    else
+    {
+        p[0] = x.x;
+        if (two) p[1] = x.y;
+    }
+}
+
 // r = sfac * b (split) and (sum b^2, sum b): the residual of a zero iterate. One thread per cell pair (k0 even).
 // bx of gx: this block among the launch's blocks (a grid-stride loop)
-template <typename T>
+template <typename T, bool kEven>
 __device__ __forceinline__ void SplitScaleSum(const LevelView &v, const double *__restrict__ b, T *__restrict__ r,
                                               double sfac, const Reducer &R, int slot, int bx, int gx)
 {
     double acc[2] = {0.0, 0.0};
-    const long long pairs = v.cells >> 1, stride = (long long)gx * blockDim.x;
-    const int H = v.Nz >> 1;
-    const double2 *b2 = reinterpret_cast<const double2 *>(b);
+    const int H = (v.Nz + 1) >> 1;
+    const long long pairs = (long long)v.Ny * v.Nx * H, stride = (long long)gx * blockDim.x;
     for (long long t = bx * (long long)blockDim.x + threadIdx.x; t < pairs; t += stride)
     {
-        const double2 x = b2[t];
         const long long row = t / H; // i * Nx + j
         const int m = (int)(t - row * H);
+        const double2 x = LdPair<kEven>(b + row * v.Nz + 2 * m, 2 * m + 1 < v.Nz);
         const int i = (int)(row / v.Nx), j = (int)(row - (long long)i * v.Nx);
         const int par = (i + j) & 1; // the colour of the pair's first cell
         const long long s = (long long)i * v.sPS + (long long)j * v.sRS + m;
@@ -1028,11 +1046,11 @@ __device__ __forceinline__ void SplitScaleSum(const LevelView &v, const double *
 
 constexpr int kScaleSumBlocks = 148 * 8;
 
-template <typename T>
+template <typename T, bool kEven>
 __global__ void __launch_bounds__(256) k_split_scale_sum(LevelView v, const double *__restrict__ b,
                                                          T *__restrict__ r, double sfac, Reducer R, int slot)
 {
-    SplitScaleSum<T>(v, b, r, sfac, R, slot, (int)blockIdx.x, (int)gridDim.x);
+    SplitScaleSum<T, kEven>(v, b, r, sfac, R, slot, (int)blockIdx.x, (int)gridDim.x);
 }
 
 template <typename T>
@@ -1040,28 +1058,47 @@ void LaunchSplitScaleSum(const LevelView &v, const double *b, T *r, double sfac,
                          cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    k_split_scale_sum<T><<<kScaleSumBlocks, 256, 0, st>>>(v, b, r, sfac, R, slot);
+    if (v.Nz % 2 == 0) k_split_scale_sum<T, true><<<kScaleSumBlocks, 256, 0, st>>>(v, b, r, sfac, R, slot);
+    else k_split_scale_sum<T, false><<<kScaleSumBlocks, 256, 0, st>>>(v, b, r, sfac, R, slot);
 }
 
 // The FP64 refinement step on a uniform split level 0 (k_pair_refine64's, with e read and r written split):
 // x_out = x_in + e; r = sfac (b - A x_out) in T; (sum (b - A x_out)^2, sum (b - A x_out)) in FP64. One thread per
 // cell pair of the grid layout; the pair (k0, k0+1) of row (i, j) is element k0/2 of colours (i+j)&1 and its other.
-__device__ __forceinline__ double2 Ld2d(const double *p) { return *reinterpret_cast<const double2 *>(p); }
+// cell pairs of a row, and the position of a thread's pair with Nz odd (PairStart's with Nz even)
+__device__ __host__ __forceinline__ int RowPairs(const LevelView &v) { return (v.Nz + 1) >> 1; }
+
+template <bool kEven> __device__ __forceinline__ PairPos RowPairStart(const LevelView &v, const Blk &b)
+{
+    PairPos p = PairStart(v, b.x, b.y, b.gy);
+    if constexpr (!kEven)
+    {
+        const int H = RowPairs(v), P = v.Nx * H;
+        int q = b.x * kPairThreads + threadIdx.x;
+        p.valid = q < P;
+        if (!p.valid) q = P - 1;
+        p.j = q / H;
+        p.k0 = 2 * (q - p.j * H);
+        p.base = (long long)p.i0 * v.sI + (long long)p.j * v.sJ + p.k0;
+    }
+    return p;
+}
 
 // 3 resident blocks (80 registers, no spill) beat 4 with a 64-register cap that spills (measured 115 vs 122 us)
-template <typename T>
+template <typename T, bool kEven>
 __device__ __forceinline__ void SplitRefine64(const LevelView &v, const uint8_t *__restrict__ du,
                                               const double *__restrict__ b, const double *__restrict__ xin,
                                               const T *__restrict__ e, double *__restrict__ xout,
                                               T *__restrict__ r, double scale, double sfac, const Reducer &R,
                                               int slot, const Blk &blk)
 {
-    const PairPos P = PairStart(v, blk.x, blk.y, blk.gy);
+    const PairPos P = RowPairStart<kEven>(v, blk);
+    const bool in2 = kEven || P.k0 + 1 < v.Nz; // the pair has a second cell
     if (v.act)
     {
         // the block's pairs lie in rows j0 .. j1; with no unknown there, x_out = x_in + e and r stay zero
-        const long long c0 = 2LL * kPairThreads * blk.x;
-        const int j0 = (int)(c0 / v.Nz), j1 = min(v.Nx - 1, (int)((c0 + 2 * kPairThreads - 1) / v.Nz));
+        const int q0 = kPairThreads * blk.x, H = RowPairs(v);
+        const int j0 = q0 / H, j1 = min(v.Nx - 1, (q0 + kPairThreads - 1) / H);
         if (RowsIdle<kQ<T> * kPairThreads>(v, j0, j1, P.i0, P.i1))
         {
             double zero[2] = {0.0, 0.0};
@@ -1077,7 +1114,7 @@ __device__ __forceinline__ void SplitRefine64(const LevelView &v, const uint8_t 
     const double *xp = xin + P.base;
     // x_in + e at the pair `o` cells (grid layout) / `so` elements (split) away; par: the colour of its first cell
     auto X = [&](long long o, long long so, int par) {
-        const double2 a = Ld2d(xp + o);
+        const double2 a = LdPair<kEven>(xp + o, in2);
         const T fa = e0[so], fb = e1[so];
         return make_double2(a.x + (double)(par ? fb : fa), a.y + (double)(par ? fa : fb));
     };
@@ -1090,7 +1127,7 @@ __device__ __forceinline__ void SplitRefine64(const LevelView &v, const uint8_t 
         const int par = (i + P.j) & 1;
         const double2 XP = X(off + P.sI, so + v.sPS, par ^ 1);
         const double2 XJp = X(off + P.sJ, so + v.sRS, par ^ 1), XJm = X(off - P.sJ, so - v.sRS, par ^ 1);
-        const double2 bb = Ld2d(b + P.base + off);
+        const double2 bb = LdPair<kEven>(b + P.base + off, in2);
         const unsigned da = d0p[so], db = d1p[so];
         const unsigned d0 = par ? db : da, d1 = par ? da : db;
         double left = __shfl_up_sync(0xffffffffu, XC.y, 1);
@@ -1105,7 +1142,7 @@ __device__ __forceinline__ void SplitRefine64(const LevelView &v, const uint8_t 
         const double r1 = (d1 & 0x80u) ? bb.y - scale * (s1 - 0.5 * (double)(d1 & 0x7Fu) * XC.y) : 0.0;
         if (P.valid)
         {
-            *reinterpret_cast<double2 *>(xout + P.base + off) = XC;
+            StPair64<kEven>(xout + P.base + off, XC, in2);
             const T f0 = (T)(r0 * sfac), f1 = (T)(r1 * sfac);
             r0p[so] = par ? f1 : f0;
             r1p[so] = par ? f0 : f1;
@@ -1119,14 +1156,14 @@ __device__ __forceinline__ void SplitRefine64(const LevelView &v, const uint8_t 
 }
 
 // swap (may be null): when *swap is odd, x_in and x_out trade places
-template <typename T>
+template <typename T, bool kEven>
 __global__ void __launch_bounds__(kPairThreads, 3)
     k_split_refine64(LevelView v, const uint8_t *__restrict__ du, const double *__restrict__ b,
                      const double *xin, const T *__restrict__ e, double *xout,
                      T *__restrict__ r, double scale, double sfac, Reducer R, int slot, const int *swap)
 {
     const bool sw = swap && (*swap & 1);
-    SplitRefine64<T>(v, du, b, sw ? xout : xin, e, sw ? const_cast<double *>(xin) : xout, r, scale, sfac, R, slot,
+    SplitRefine64<T, kEven>(v, du, b, sw ? xout : xin, e, sw ? const_cast<double *>(xin) : xout, r, scale, sfac, R, slot,
                   ThisBlk());
 }
 
@@ -1136,8 +1173,12 @@ void LaunchSplitRefine64(const LevelView &v, const uint8_t *du, const double *b,
                          cudaStream_t st, const int *swap)
 {
     NB_COUNT_LAUNCH();
-    k_split_refine64<T><<<PairGrid(v, kSplitReduceS), kPairThreads, 0, st>>>(v, du, b, xin, e, xout, r, scale, sfac, R,
-                                                                           slot, swap);
+    const dim3 grid = PairGridOf((long long)v.Nx * RowPairs(v), v.Ny - 2, kSplitReduceS);
+    if (v.Nz % 2 == 0)
+        k_split_refine64<T, true><<<grid, kPairThreads, 0, st>>>(v, du, b, xin, e, xout, r, scale, sfac, R, slot, swap);
+    else
+        k_split_refine64<T, false><<<grid, kPairThreads, 0, st>>>(v, du, b, xin, e, xout, r, scale, sfac, R, slot,
+                                                                  swap);
 }
 
 
@@ -1250,7 +1291,7 @@ __global__ void __launch_bounds__(256) kb_split_scale_sum(const BatchLevel *__re
     if (q < 0) return;
     const BatchLevel &L = lv[q * ls];
     const BatchReq &Q = rq[q];
-    SplitScaleSum<float>(L.v, Q.b, L.r, Q.sfac, Q.red, slot, (int)blockIdx.x, (int)gridDim.x);
+    SplitScaleSum<float, true>(L.v, Q.b, L.r, Q.sfac, Q.red, slot, (int)blockIdx.x, (int)gridDim.x);
 }
 
 // parity[q]: this pass reads x from xin (0) or xout (1) and writes the other
@@ -1263,7 +1304,7 @@ __global__ void __launch_bounds__(kPairThreads, 3)
     const BatchLevel &L = lv[q * ls];
     const BatchReq &Q = rq[q];
     const bool odd = parity[q] & 1;
-    SplitRefine64<float>(L.v, L.du, Q.b, odd ? Q.xout : Q.xin, Q.x, odd ? Q.xin : Q.xout, L.r, Q.scale, Q.sfac, Q.red, slot,
+    SplitRefine64<float, true>(L.v, L.du, Q.b, odd ? Q.xout : Q.xin, Q.x, odd ? Q.xin : Q.xout, L.r, Q.scale, Q.sfac, Q.red, slot,
                   ThisBlk());
 }
 

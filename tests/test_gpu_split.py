@@ -181,6 +181,29 @@ def test_device_refinement_loop_limits(nb):
     assert not np.any(z.p[types == W.FLUID])
 
 
+def sphere_case(size, closed):
+    """A box of cubic cells of the given interior size around a solid sphere, closed or with an outlet."""
+    nx, ny, nz = size
+    h = 1.0 / min(nx, ny)
+    g = W.uniform_grid(3, (0.0, nx * h, 0.0, ny * h, 0.0, nz * h), min(nx, ny))
+    assert (g.Nx, g.Ny, g.Nz) == (nx + 2, ny + 2, nz + 2)
+    sph = W.Region(W.REGION_SOLID, W.PRIM_SPHERE, (0.5 * nx * h, 0.5 * ny * h, 0.5 * nz * h), radius=0.2 * min(size) * h)
+    case = W.Case("sphere", g, W.walls_scene(3, outlet_face=None if closed else 1, regions=[sph]), 31,
+                  needs_compat=closed)
+    return case, capi.label_cells(g, case.scene)
+
+
+def solve_family(case, types, family, precision, closed, tol=1e-12, **options):
+    g = case.grid
+    u, v, w = W.face_velocities(g, types, case.seed)
+    m = MACGrid(g, types.copy(), u, v, w, np.zeros(g.cells), case.rho, case.dt)
+    s = PressureSolver(precision, pair_kernels=family, **dict({"tail_cells": 512}, **options))
+    r = s.SolvePressure(m, tol=tol, needs_compat=closed)
+    assert r.status == capi.NB_OK and r.rel_res <= tol, r.as_dict()
+    s.DestroyPressureSolver()
+    return m
+
+
 # FP64: (interior x, y, z), outlet or closed; row lengths around the 16-byte quads and their padding, one tile and
 # several, the smallest grid with a split level above the coarse end and its neighbours
 FP64_SIZES = [(12, 12, 12), (14, 13, 16), (16, 16, 14), (30, 36, 26), (33, 40, 48), (64, 20, 34)]
@@ -192,26 +215,26 @@ def test_fp64_split_agrees_with_per_cell_kernels(nb, size, closed):
     """The plain FP64 form on the colour-split layout against its per-cell kernels (pair_kernels = 0), both to 1e-12.
     Each solution is within cond * 1e-12 of the exact one; cond <= 5 N^2 on N cells along the longest side (the lowest
     mode a quarter wave), so the two agree within 1e-11 N^2."""
-    nx, ny, nz = size
-    h = 1.0 / min(nx, ny)
-    g = W.uniform_grid(3, (0.0, nx * h, 0.0, ny * h, 0.0, nz * h), min(nx, ny))
-    assert (g.Nx, g.Ny, g.Nz) == (nx + 2, ny + 2, nz + 2)
-    sph = W.Region(W.REGION_SOLID, W.PRIM_SPHERE, (0.5 * nx * h, 0.5 * ny * h, 0.5 * nz * h), radius=0.2 * min(size) * h)
-    case = W.Case("fp64", g, W.walls_scene(3, outlet_face=None if closed else 1, regions=[sph]), 31,
-                  needs_compat=closed)
-    types = capi.label_cells(g, case.scene)
-    u, v, w = W.face_velocities(g, types, case.seed)
-    out = []
-    for family in (2, 0):
-        m = MACGrid(g, types.copy(), u.copy(), v.copy(), w.copy(), np.zeros(g.cells), case.rho, case.dt)
-        s = PressureSolver("fp64", pair_kernels=family, tail_cells=512)
-        r = s.SolvePressure(m, tol=1e-12, needs_compat=closed)
-        assert r.status == capi.NB_OK and r.rel_res <= 1e-12
-        assert s.lib.nereus_b200_last_iterations(s.ctx) > 0
-        s.DestroyPressureSolver()
-        out.append(m)
-    a, b = out
+    case, types = sphere_case(size, closed)
+    a, b = [solve_family(case, types, family, "fp64", closed) for family in (2, 0)]
     bar = 1e-11 * max(size) ** 2
-    assert np.linalg.norm(a.p - b.p) <= bar * np.linalg.norm(b.p)
-    for x, y in ((a.u, b.u), (a.v, b.v), (a.w, b.w)):
+    for x, y in ((a.p, b.p), (a.u, b.u), (a.v, b.v), (a.w, b.w)):
         assert np.linalg.norm(x - y) <= bar * np.linalg.norm(y)
+
+
+# Nz odd: the last cell of a row has no pair, and one colour's rows hold a cell less. (interior x, y, z), row lengths
+# around the quads and their padding; the last two have odd levels below an even one and above the coarse end
+ODD_SIZES = [(12, 12, 9), (16, 13, 15), (17, 15, 17), (24, 31, 33), (33, 40, 47), (20, 20, 38), (28, 36, 50)]
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("size", ODD_SIZES)
+def test_odd_rows_agree_with_per_cell_kernels(nb, size, precision):
+    """The colour-split layout on grids and levels of odd Nz against the per-cell kernels, closed and with an outlet,
+    all to 1e-12 (the bar of test_fp64_split_agrees_with_per_cell_kernels)."""
+    for closed in (False, True):
+        case, types = sphere_case(size, closed)
+        a, b = [solve_family(case, types, family, precision, closed) for family in (2, 0)]
+        bar = 1e-11 * max(size) ** 2
+        for x, y in ((a.p, b.p), (a.u, b.u), (a.v, b.v), (a.w, b.w)):
+            assert np.linalg.norm(x - y) <= bar * np.linalg.norm(y)
