@@ -74,9 +74,10 @@ typedef struct nb_options
                              batch: per 4 everywhere); 1: one thread per coarse cell everywhere; 2: one thread per 4
                              coarse cells everywhere. All three give the same result in a single solve */
     int pair_kernels;    /* kernels of 3D levels: 2 (default): the colour-split layout, red and black cells in separate
-                            arrays, so that one colour's sweep moves half the bytes (uniform levels, both
-                            precisions); 1: the mixed form's cell pairs in the grid layout (Nz even, uniform or
-                            stretched; also what 2 gives on its stretched levels); 0: the general per-cell kernels */
+                            arrays, so that one colour's sweep moves half the bytes (uniform levels in both
+                            precisions, stretched ones in FP64); 1: the mixed form's cell pairs in the grid layout
+                            (Nz even, uniform or stretched; also what 2 gives on its stretched levels); 0: the
+                            general per-cell kernels */
     int tail_cells;      /* the coarse end runs in one thread block from the first level with at most this many
                             cells (and shared memory for all of them); 0: no such block */
     int stretched_sweeps; /* red-black sweeps before and after the coarse correction on a stretched grid's levels

@@ -26,6 +26,7 @@ SOURCES = {
     "nb_tail.cu": [],
     "nb_pairs.cu": [],
     "nb_split.cu": [],
+    "nb_stretched.cu": [],
     "nb_solver.cu": [],
     "nb_capi.cu": [],
     "nb_noalloc.cu": [],
@@ -34,7 +35,7 @@ SOURCES = {
     "nb_server.cu": [],
     "nb_batch.cu": [],
 }
-HEADERS = ["nb_device.cuh", "nb_batch.cuh", "nb_kernels.h", "nb_solver.h", "nb_guard.h"]
+HEADERS = ["nb_device.cuh", "nb_quad.cuh", "nb_batch.cuh", "nb_kernels.h", "nb_solver.h", "nb_guard.h"]
 
 
 def _newest_input() -> float:

@@ -113,7 +113,8 @@ void LaunchLinXR(long long cells, T *x, T *r, const T *p0, const T *p1, const T 
 // ---- nb_split.cu: kernels for 3D levels in the colour-split layout (LevelView::sRS), T = float (the mixed form's
 //      inner solve) or double (the plain FP64 form) ----
 bool SplitLevelShape(const LevelView &v);
-// uniform levels only; du: the level's diagonal units in that layout; pext: the red cells' bytes
+// du: the level's diagonal units in that layout (a stretched level reads their unknown flag only, and runs the sweeps
+// of nb_stretched.cu, FP64 only); pext: the red cells' bytes
 // reads the kernels' occupancy (their grids follow it); call before capturing launches into a graph
 void PrepareSplitKernels(int elemBytes);
 // the first red-black sweep from a zero iterate
@@ -167,6 +168,19 @@ template <typename T>
 void LaunchSplitRefine64(const LevelView &v, const uint8_t *du, const double *b, const double *xin, const T *e,
                          double *xout, T *r, double scale, double sfac, const Reducer &R, int slot,
                          cudaStream_t st, const int *swap = nullptr);
+
+// ---- nb_stretched.cu: the FP64 sweeps of a stretched 3D level in the colour-split layout (LevelView::dg, idg) ----
+void PrepareStretchedKernels();
+void LaunchStretchedDiag(const LevelView &v, double *dg, double *idg, cudaStream_t st);
+void LaunchStretchedFirst(const LevelView &v, const double *r, double *e, cudaStream_t st);
+void LaunchStretchedHalf(const LevelView &v, const double *r, double *e, int colour, cudaStream_t st);
+void LaunchStretchedHalfDot(const LevelView &v, const double *r, double *e, int colour, bool last, const Reducer &R,
+                            const int *it, int baseEven, int baseOdd, int partSlot, cudaStream_t st);
+void LaunchStretchedResidual(const LevelView &v, const uint8_t *du, const double *r, const double *e, double *res,
+                             cudaStream_t st);
+void LaunchStretchedPApply(const LevelView &v, const uint8_t *du, const double *z, double *p0, double *p1, double *q,
+                           const Reducer &R, const double *S, const int *it, int baseEven, int baseOdd, int slotN,
+                           int singular, int slotPQ, cudaStream_t st);
 
 // ---- nb_kernels.cu: multigrid and PCG kernels, T = float (inner solve) or double (plain FP64) ----
 void LaunchBuildCodes(const LevelView &v, uint8_t *code, cudaStream_t st);

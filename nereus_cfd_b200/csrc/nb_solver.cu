@@ -63,12 +63,15 @@ LevelView LevelData::view() const
     v.gamma = gamma;
     v.xp = dxp;
     v.xr = dxr;
+    v.dg = diag.p;
+    v.idg = rdiag.p;
     for (int a = 0; a < 3; a++)
     {
         v.w[a] = dw[a];
         v.g[a] = dg[a];
         v.w32[a] = dw32[a];
         v.ig32[a] = dig32[a];
+        v.igd[a] = digd[a];
     }
     return v;
 }
@@ -91,7 +94,7 @@ void Context::UploadTables()
     for (const LevelData &Lv : L)
     {
         for (int a = 0; a < 3; a++)
-            bytes += 2 * pad(Lv.w[a].size() * 8) + 2 * pad(Lv.g[a].size() * 8);
+            bytes += 2 * pad(Lv.w[a].size() * 8) + 3 * pad(Lv.g[a].size() * 8);
         bytes += pad(Lv.xp.size() * 4) + pad(Lv.xr.size() * 4);
     }
     if (bytes > tablesHostCap)
@@ -112,7 +115,7 @@ void Context::UploadTables()
     };
     struct Off
     {
-        size_t w, g, w32, ig32;
+        size_t w, g, w32, ig32, igd;
     };
     std::vector<Off> offs(L.size() * 3);
     for (size_t l = 0; l < L.size(); l++)
@@ -130,6 +133,10 @@ void Context::UploadTables()
             for (size_t q = 0; q < Lv.g[a].size(); q++) ig32[q] = (float)(1.0 / Lv.g[a][q]);
             o.ig32 = off;
             off += pad(Lv.g[a].size() * 4);
+            double *igd = (double *)(tablesHost + off);
+            for (size_t q = 0; q < Lv.g[a].size(); q++) igd[q] = 1.0 / Lv.g[a][q];
+            o.igd = off;
+            off += pad(Lv.g[a].size() * 8);
         }
     std::vector<size_t> xOff(2 * L.size());
     for (size_t l = 0; l < L.size(); l++)
@@ -146,6 +153,7 @@ void Context::UploadTables()
             L[l].dg[a] = (const double *)(tables.p + o.g);
             L[l].dw32[a] = (const float *)(tables.p + o.w32);
             L[l].dig32[a] = (const float *)(tables.p + o.ig32);
+            L[l].digd[a] = (const double *)(tables.p + o.igd);
         }
     for (size_t l = 0; l < L.size(); l++)
     {
@@ -352,14 +360,14 @@ void Context::BuildHierarchy()
     NB_CK(cudaGetLastError());
 }
 
-// The colour-split levels (pair_kernels = 2): the uniform 3D levels above the coarse end, of either parity of Nz, as
-// long as every finer level is one too (a level's transfers read and write the next coarser level in either layout,
-// the grid-layout kernels only the grid layout). A grid of odd Nz ran the per-cell kernels before: on 125 x 101 x 117
-// cells the mixed step to 1e-12 took 8.7 ms there and takes 5.0 ms on this layout. A stretched grid keeps the cell-pair kernels: its
-// per-cell coefficients make the split kernels compute-bound (measured slower on the stretched cylinder).
+// The colour-split levels (pair_kernels = 2): the 3D levels above the coarse end, uniform ones in either precision and
+// stretched ones in FP64 (nb_stretched.cu), of either parity of Nz, as long as every finer level is one too (a level's
+// transfers read and write the next coarser level in either layout, the grid-layout kernels only the grid layout). A
+// grid of odd Nz ran the per-cell kernels before: on 125 x 101 x 117 cells the mixed step to 1e-12 took 8.7 ms there
+// and takes 5.0 ms on this layout. A stretched grid's FP32 levels keep the cell-pair kernels.
 void Context::AssignSplit()
 {
-    const bool on = opt.pair_kernels == 2 && !nonuniform;
+    const bool on = opt.pair_kernels == 2 && (!nonuniform || opt.precision == NB_PRECISION_FP64);
     bool finer = true;
     for (size_t l = 0; l < L.size(); l++)
     {
@@ -396,6 +404,19 @@ void Context::BuildPairData()
                 Lv.du.alloc((size_t)(2 * Lv.sHalf));
                 Lv.du.zero(st); // the padding
                 LaunchBuildDu(v, Lv.du.p, st);
+                if (Lv.stretched)
+                {
+                    Lv.diag.alloc((size_t)(2 * Lv.sHalf));
+                    Lv.rdiag.alloc((size_t)(2 * Lv.sHalf));
+                    Lv.diag.zero(st);
+                    Lv.rdiag.zero(st);
+                    LaunchStretchedDiag(Lv.view(), Lv.diag.p, Lv.rdiag.p, st);
+                }
+                else
+                {
+                    Lv.diag.release();
+                    Lv.rdiag.release();
+                }
                 if (opt.skip_idle_tiles)
                 {
                     Lv.actTiles = SplitActivityTiles(v, elem);
@@ -414,7 +435,12 @@ void Context::BuildPairData()
                 LaunchBuildDu(v, Lv.du.p, st);
             }
         }
-        else Lv.du.release();
+        else
+        {
+            Lv.du.release();
+            Lv.diag.release();
+            Lv.rdiag.release();
+        }
     }
     for (size_t l = 0; l < L.size(); l++)
     {
@@ -1574,7 +1600,8 @@ int Context::SolveFP64(double tol, double **xOut, nb_result *out, const double *
             ProfBegin(NB_K_REFINE, (8.0 + 8.0 + 1.0 + 8.0) * (double)Cells());
             if (split)
             {
-                LaunchSplitRefine64<double>(v0, L[0].du.p, b.p, x, x64.p, xo, r, scale, sfac, red, S_RES, st);
+                if (nonuniform) LaunchRefine64<double>(v0, b.p, x, x64.p, xo, r, scale, sfac, red, S_RES, st);
+                else LaunchSplitRefine64<double>(v0, L[0].du.p, b.p, x, x64.p, xo, r, scale, sfac, red, S_RES, st);
                 std::swap(x, xo);
             }
             else LaunchResidual64<double>(v0, b.p, x, r, scale, sfac, red, S_RES, st);

@@ -190,6 +190,7 @@ struct LevelData
     // the device copies of w, g (FP64) and of w, 1/g (FP32): pointers into the context's packed table array
     const double *dw[3] = {}, *dg[3] = {};
     const float *dw32[3] = {}, *dig32[3] = {};
+    const double *digd[3] = {};           // FP64 1/g
     // the x groups of the transfer to the next coarser level (LevelView::xp, xr) and their device copies in the
     // packed table array; empty: x cells paired by two like the other axes
     std::vector<int> xp, xr;
@@ -199,6 +200,7 @@ struct LevelData
                                           // Colour-split level: in that layout, and the codes on a stretched level
     DevArray<uint8_t> pext;               // unknown flag + moved prolongation weight toward the next coarser level
                                           // (colour-split level: the red cells only)
+    DevArray<double> diag, rdiag;         // stretched colour-split level (FP64): LevelView::dg, idg
     DevArray<uint8_t> act;                // colour-split level: which (plane, tile) holds an unknown (LevelView::act)
     int actTiles = 0;
     // the colour-split layout of the solver's vectors (nb_split.cu); sRS = 0: the grid layout

@@ -19,7 +19,7 @@
 // 0.24 of the measured copy bandwidth) to 9.8 ms (0.62).
 //
 // Every vector is zero off the unknowns (and on the padding), so the neighbour sum runs over all six neighbours. The
-// levels are uniform (a stretched grid keeps the cell-pair kernels of nb_pairs.cu): the coefficient is gamma
+// levels are uniform (a stretched level's sweeps are in nb_stretched.cu, the transfers here): the coefficient is gamma
 // everywhere and the diagonal is gamma/2 times the unit count in the level's byte array (0x80 | units, 0 off the
 // unknowns), divided through a 32-entry reciprocal table.
 //
@@ -28,221 +28,12 @@
 //   its restriction run over the red cells only;
 // - a black half-sweep does not read the black values it replaces, so the prolonged coarse correction is added to
 //   the red cells only before the post-smoothing, which starts black.
-#include "nb_kernels.h"
+#include "nb_quad.cuh"
 
 namespace nb
 {
 
 bool SplitLevelShape(const LevelView &v) { return v.dim == 3 && v.Nx >= 3 && v.Ny >= 3 && v.Nz >= 3; }
-
-namespace
-{
-
-// the 16 bytes a thread moves at a time
-template <typename T> struct Quad
-{
-    static constexpr int N = 16 / (int)sizeof(T);
-    T v[N];
-};
-template <typename T> constexpr int kQ = Quad<T>::N;
-
-__device__ __forceinline__ Quad<float> LQ(const float *p)
-{
-    const float4 a = *reinterpret_cast<const float4 *>(p);
-    return Quad<float>{{a.x, a.y, a.z, a.w}};
-}
-__device__ __forceinline__ Quad<double> LQ(const double *p)
-{
-    const double2 a = *reinterpret_cast<const double2 *>(p);
-    return Quad<double>{{a.x, a.y}};
-}
-__device__ __forceinline__ void SQ(float *p, const Quad<float> &a)
-{
-    *reinterpret_cast<float4 *>(p) = make_float4(a.v[0], a.v[1], a.v[2], a.v[3]);
-}
-__device__ __forceinline__ void SQ(double *p, const Quad<double> &a)
-{
-    *reinterpret_cast<double2 *>(p) = make_double2(a.v[0], a.v[1]);
-}
-// loads of values a kernel reads once (evict-first): measured to keep the half-sweep's j-row loads in L1 longer
-__device__ __forceinline__ Quad<float> LQOnce(const float *p)
-{
-    const float4 a = __ldcs(reinterpret_cast<const float4 *>(p));
-    return Quad<float>{{a.x, a.y, a.z, a.w}};
-}
-__device__ __forceinline__ Quad<double> LQOnce(const double *p)
-{
-    const double2 a = __ldcs(reinterpret_cast<const double2 *>(p));
-    return Quad<double>{{a.x, a.y}};
-}
-// a quad's N bytes of a byte array
-template <int N> __device__ __forceinline__ unsigned LdB(const uint8_t *p)
-{
-    static_assert(N == 4 || N == 2, "four or two bytes");
-    if constexpr (N == 4) return *reinterpret_cast<const unsigned *>(p);
-    else return *reinterpret_cast<const unsigned short *>(p);
-}
-template <int N> __device__ __forceinline__ unsigned LdBOnce(const uint8_t *p)
-{
-    if constexpr (N == 4) return __ldcs(reinterpret_cast<const unsigned *>(p));
-    else return __ldcs(reinterpret_cast<const unsigned short *>(p));
-}
-__device__ __forceinline__ unsigned Byte(unsigned d, int x) { return (d >> (8 * x)) & 0xFFu; }
-template <typename T> __device__ __forceinline__ T Unk(unsigned b) { return (b & 0x80u) ? (T)1 : (T)0; }
-
-// 1 / (gamma/2 * units), entry 0 = 0
-template <typename T> __device__ __forceinline__ void FillInv(T *inv, double gamma)
-{
-    if (threadIdx.x < 32) inv[threadIdx.x] = threadIdx.x ? (T)1 / ((T)0.5 * (T)gamma * (T)threadIdx.x) : (T)0;
-    __syncthreads();
-}
-
-// Per-thread position of a quad kernel.
-struct QuadPos
-{
-    int lane;
-    bool valid;  // false for the clamped threads past the plane's last quad (they still load and shuffle)
-    int i0, i1;  // planes [i0, i1)
-    int j, m0;   // row and first element of the quad
-    int RS, PS;
-    long long off; // element of the quad on plane i0, within one colour
-};
-
-template <int N> __device__ __forceinline__ QuadPos QuadStart(const LevelView &v, const Blk &b)
-{
-    QuadPos p;
-    const int Q = v.sRS / N, nq = v.Nx * Q;
-    p.lane = threadIdx.x & 31;
-    int t = b.x * kPairThreads + threadIdx.x;
-    p.valid = t < nq;
-    if (!p.valid) t = nq - 1;
-    // grid.y splits the Ny-2 interior planes into chunks of S (the host sized it); a block past the last plane starts
-    // at the ring plane and marches none
-    const int S = (v.Ny - 2 + b.gy - 1) / b.gy;
-    p.i0 = min(1 + b.y * S, v.Ny - 1);
-    p.i1 = min(p.i0 + S, v.Ny - 1);
-    p.RS = v.sRS;
-    p.PS = v.sPS;
-    p.j = t / Q;
-    p.m0 = N * (t - p.j * Q);
-    p.off = (long long)p.i0 * v.sPS + (long long)N * t;
-    return p;
-}
-
-// True when no tile this block owns on planes [i0, i1) holds an unknown (LevelView::act): the block's cells are
-// all zero in every vector and stay so, so it has nothing to compute, load or store.
-__device__ __forceinline__ bool TileIdle(const LevelView &v, int bx, int i0, int i1)
-{
-    if (!v.act) return false;
-    for (int i = i0; i < i1; i++)
-        if (v.act[(long long)i * v.actTiles + bx]) return false;
-    return true;
-}
-
-// The same for a block of a grid-layout pair kernel (PairStart): its rows j0 .. j1 of planes [i0, i1), checked
-// through the split tiles (of kTile elements) that hold those rows' cells in either colour.
-template <int kTile> __device__ __forceinline__ bool RowsIdle(const LevelView &v, int j0, int j1, int i0, int i1)
-{
-    if (!v.act) return false;
-    const int t0 = (int)(((long long)j0 * v.sRS) / kTile);
-    const int t1 = min(v.actTiles - 1, (int)(((long long)(j1 + 1) * v.sRS - 1) / kTile));
-    for (int i = i0; i < i1; i++)
-        for (int t = t0; t <= t1; t++)
-            if (v.act[(long long)i * v.actTiles + t]) return false;
-    return true;
-}
-
-// Resident blocks of a kernel per SM at kPairThreads threads (its registers and shared memory decide), and the SM
-// count of the current device.
-inline int ResidentBlocks(const void *fn)
-{
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, kPairThreads, 0) != cudaSuccess || n < 1) n = 1;
-    return n;
-}
-
-// read once per kernel (and before any stream capture: PrepareSplitKernels)
-template <auto kKernel> int Occ()
-{
-    static const int n = ResidentBlocks((const void *)kKernel);
-    return n;
-}
-
-inline int SmCount()
-{
-    int d = 0, c = 0;
-    if (cudaGetDevice(&d) != cudaSuccess) return 148;
-    if (cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, d) != cudaSuccess || c < 1) c = 148;
-    return c;
-}
-
-// The launch grid of a quad kernel with `resident` blocks per SM: the longest march (planes per thread, at most
-// kQuadMaxS) whose launch fills the last wave of resident blocks to at least 90%; the longer the march, the fewer
-// planes of a neighbour array are loaded twice (a chunk of S planes loads S + 2). Measured on a 258^3 level: one
-// 92%-full wave of 16-plane chunks beats two waves of 8 (and 1.03 waves of 15 runs at half speed). With no such S,
-// the best-filled one (a small level fills no wave: S = 1, all the parallelism there is).
-constexpr int kQuadMaxS = 16;
-
-// The march length S (planes per thread, 1 .. kQuadMaxS) for a grid of perPlane x ceil(planes / S) blocks on `slots`
-// resident blocks, by the rule above.
-inline long long BestMarch(long long perPlane, long long planes, long long slots)
-{
-    long long bestS = 1;
-    double bestU = -1.0;
-    for (long long S = kQuadMaxS; S >= 1; S--)
-    {
-        const long long blocks = perPlane * ((planes + S - 1) / S);
-        const long long waves = (blocks + slots - 1) / slots;
-        const double u = (double)blocks / (double)(waves * slots);
-        if (u >= 0.9) return S;
-        if (u > bestU + 1e-9)
-        {
-            bestU = u;
-            bestS = S;
-        }
-    }
-    return bestS;
-}
-
-// A quad kernel's grid with a march of S planes (S > 0), or sized as above (S = 0); N elements a thread.
-template <int N = 4> inline dim3 QuadGridS(const LevelView &v, int S)
-{
-    const long long nq = (long long)v.Nx * (v.sRS / N), perPlane = (nq + kPairThreads - 1) / kPairThreads;
-    const long long planes = v.Ny - 2 > 0 ? v.Ny - 2 : 1;
-    return dim3((unsigned)perPlane, (unsigned)((planes + S - 1) / S));
-}
-
-template <int N> inline dim3 QuadGrid(const LevelView &v, int resident)
-{
-    const long long nq = (long long)v.Nx * (v.sRS / N), perPlane = (nq + kPairThreads - 1) / kPairThreads;
-    const long long planes = v.Ny - 2 > 0 ? v.Ny - 2 : 1;
-    const long long bestS = BestMarch(perPlane, planes, (long long)SmCount() * (resident > 0 ? resident : 1));
-    return dim3((unsigned)perPlane, (unsigned)((planes + bestS - 1) / bestS));
-}
-
-// The other colour's k neighbours of a quad: the element at m (c) and the one at m + (q ? 1 : -1) (returned).
-__device__ __forceinline__ Quad<float> KShift(const Quad<float> &c, float prevW, float nextX, int q)
-{
-    return q ? Quad<float>{{c.v[1], c.v[2], c.v[3], nextX}} : Quad<float>{{prevW, c.v[0], c.v[1], c.v[2]}};
-}
-__device__ __forceinline__ Quad<double> KShift(const Quad<double> &c, double prevW, double nextX, int q)
-{
-    return q ? Quad<double>{{c.v[1], nextX}} : Quad<double>{{prevW, c.v[0]}};
-}
-
-// The elements just before and after this lane's quad in its row (0 past the row's ends; the values a lane takes
-// from a neighbouring row only reach ring or padding cells, whose results are masked).
-template <typename T>
-__device__ __forceinline__ void Edges(const QuadPos &P, const Quad<T> &c, const T *row, T &prevW, T &nextX)
-{
-    constexpr int N = kQ<T>;
-    prevW = __shfl_up_sync(0xffffffffu, c.v[N - 1], 1);
-    nextX = __shfl_down_sync(0xffffffffu, c.v[0], 1);
-    if (P.lane == 0) prevW = P.m0 > 0 ? row[-1] : (T)0;
-    if (P.lane == 31) nextX = P.m0 + N < P.RS ? row[N] : (T)0;
-}
-
-} // namespace
 
 // planes per thread at least in the pair-thread launches that end in a grid-wide sum
 constexpr int kSplitReduceS = 16;
@@ -421,6 +212,8 @@ __global__ void __launch_bounds__(kPairThreads, 4)
 template <typename T>
 void LaunchSplitFirst(const LevelView &v, const uint8_t *du, const T *r, T *e, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8)
+        if (v.stretched) return LaunchStretchedFirst(v, r, e, st);
     NB_COUNT_LAUNCH();
     LaunchPdl(k_split_first<T>, QuadGrid<kQ<T>>(v, Occ<k_split_first<T>>()), kPairThreads, 0, st, v, du, r, e);
 }
@@ -428,6 +221,8 @@ void LaunchSplitFirst(const LevelView &v, const uint8_t *du, const T *r, T *e, c
 template <typename T>
 void LaunchSplitHalf(const LevelView &v, const uint8_t *du, const T *r, T *e, int colour, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8)
+        if (v.stretched) return LaunchStretchedHalf(v, r, e, colour, st);
     NB_COUNT_LAUNCH();
     LaunchPdl(k_split_half<T, 0>, QuadGrid<kQ<T>>(v, Occ<k_split_half<T, 0>>()), kPairThreads, 0, st,
               NB_SPLIT_HALF_ARGS(colour), Reducer{}, (const int *)nullptr, 0, 0, 0);
@@ -437,6 +232,8 @@ template <typename T>
 void LaunchSplitHalfDot(const LevelView &v, const uint8_t *du, const T *r, T *e, int colour, bool last,
                         const Reducer &R, const int *it, int baseEven, int baseOdd, int partSlot, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8)
+        if (v.stretched) return LaunchStretchedHalfDot(v, r, e, colour, last, R, it, baseEven, baseOdd, partSlot, st);
     NB_COUNT_LAUNCH();
     if (last)
         LaunchPdl(k_split_half<T, 2>, QuadGrid<kQ<T>>(v, Occ<k_split_half<T, 2>>()), kPairThreads, 0, st,
@@ -510,6 +307,8 @@ __global__ void __launch_bounds__(kPairThreads, sizeof(T) == 8 ? 3 : 4) k_split_
 template <typename T>
 void LaunchSplitResidual(const LevelView &v, const uint8_t *du, const T *r, const T *e, T *res, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8)
+        if (v.stretched) return LaunchStretchedResidual(v, du, r, e, res, st);
     NB_COUNT_LAUNCH();
     LaunchPdl(k_split_residual<T>, QuadGrid<kQ<T>>(v, Occ<k_split_residual<T>>()), kPairThreads, 0, st, v, du, r, e,
               res);
@@ -566,10 +365,11 @@ __device__ __forceinline__ void CoarseRowK(const LevelView &cv, const T *__restr
     for (int t = 0; t <= N; t++) c[t] = ec[VecIdx(cv, A, B, min(m0 + t, Dmax))]; // past the row: masked cells only
 }
 
-// the coarse plane's rows interpolated across j for fine rows 2B-1 (y0) and 2B (y1), and row B itself (par)
+// the coarse plane's rows interpolated across j for fine rows 2B-1 (y0) and 2B (y1), and row B itself (par); one: row B
+// has a single fine row (x groups), which takes it whole
 template <typename T>
 __device__ __forceinline__ void CoarsePlaneRows(const LevelView &cv, const T *__restrict__ ec, int A, int B, int m0,
-                                                T y0[kQ<T> + 1], T y1[kQ<T> + 1], T par[kQ<T> + 1])
+                                                bool one, T y0[kQ<T> + 1], T y1[kQ<T> + 1], T par[kQ<T> + 1])
 {
     T cm[kQ<T> + 1], cp[kQ<T> + 1];
     CoarseRowK<T>(cv, ec, A, B, m0, par);
@@ -578,12 +378,13 @@ __device__ __forceinline__ void CoarsePlaneRows(const LevelView &cv, const T *__
 #pragma unroll
     for (int t = 0; t <= kQ<T>; t++)
     {
-        y0[t] = (T)0.75 * par[t] + (T)0.25 * cm[t];
+        y0[t] = one ? par[t] : (T)0.75 * par[t] + (T)0.25 * cm[t];
         y1[t] = (T)0.75 * par[t] + (T)0.25 * cp[t];
     }
 }
 
-template <typename T>
+// kX: the coarsening keeps some x cells whole (LevelView::xr: row B's first fine row, and whether it has a second)
+template <typename T, bool kX>
 __device__ __forceinline__ void SplitProlong(const LevelView &fv, const LevelView &cv,
                                              const uint8_t *__restrict__ pext, const T *__restrict__ ec,
                                              T *__restrict__ ef, const Blk &blk)
@@ -598,22 +399,24 @@ __device__ __forceinline__ void SplitProlong(const LevelView &fv, const LevelVie
     const int S = (cv.Ny - 2 + blk.gy - 1) / blk.gy;
     const int A0 = min(1 + blk.y * S, cv.Ny - 1), A1 = min(A0 + S, cv.Ny - 1);
     if (!valid || A0 >= A1) return;
+    const int xg = kX ? fv.xr[B] : 0;
+    const bool one = kX && !((xg >> 15) & 1);
+    const int fb0 = kX ? (xg & 0x7FFF) : 2 * B - 1, fb1 = one ? fb0 : fb0 + 1;
     T yM0[N + 1], yM1[N + 1], yC0[N + 1], yC1[N + 1], pC[N + 1], pD[N + 1];
-    CoarsePlaneRows<T>(cv, ec, A0 - 1, B, m0, yM0, yM1, pD);
-    CoarsePlaneRows<T>(cv, ec, A0, B, m0, yC0, yC1, pC);
-    const int fb0 = 2 * B - 1, fb1 = 2 * B;
+    CoarsePlaneRows<T>(cv, ec, A0 - 1, B, m0, one, yM0, yM1, pD);
+    CoarsePlaneRows<T>(cv, ec, A0, B, m0, one, yC0, yC1, pC);
     for (int A = A0; A < A1; A++)
     {
         T yP0[N + 1], yP1[N + 1], pP[N + 1];
-        CoarsePlaneRows<T>(cv, ec, A + 1, B, m0, yP0, yP1, pP);
+        CoarsePlaneRows<T>(cv, ec, A + 1, B, m0, one, yP0, yP1, pP);
         // fine planes 2A-1 (with coarse plane A-1) and 2A (with A+1), rows 2B-1 and 2B
 #pragma unroll
         for (int h = 0; h < 2; h++)
         {
             const int fa = 2 * A - 1 + h;
             const long long o0 = (long long)fa * fv.sPS + (long long)fb0 * fv.sRS + m0, o1 = o0 + fv.sRS;
-            const unsigned w0 = LdB<N>(pext + o0), w1 = LdB<N>(pext + o1);
-            Quad<T> e0 = LQ(ef + o0), e1 = LQ(ef + o1);
+            const unsigned w0 = LdB<N>(pext + o0), w1 = one ? 0u : LdB<N>(pext + o1);
+            Quad<T> e0 = LQ(ef + o0), e1 = one ? Quad<T>{} : LQ(ef + o1);
             const T *yo0 = h ? yP0 : yM0, *yo1 = h ? yP1 : yM1;
 #pragma unroll
             for (int rI = 0; rI < 2; rI++)
@@ -651,14 +454,14 @@ __device__ __forceinline__ void SplitProlong(const LevelView &fv, const LevelVie
 
 // 3 resident blocks (80 registers, 40 bytes spilled) where the kernel would take 88: measured 14% faster on the 258^3
 // level (its grid of one block per SM or so is latency-bound)
-template <typename T>
+template <typename T, bool kX>
 __global__ void __launch_bounds__(kPairThreads, 3) k_split_prolong(LevelView fv, LevelView cv,
                                                                 const uint8_t *__restrict__ pext,
                                                                 const T *__restrict__ ec, T *__restrict__ ef)
 {
     PdlWait();
     PdlTrigger();
-    SplitProlong<T>(fv, cv, pext, ec, ef, ThisBlk());
+    SplitProlong<T, kX>(fv, cv, pext, ec, ef, ThisBlk());
 }
 
 // The grid of k_split_prolong: threads over (coarse row, fine quad), grid.y chunks of coarse planes sized like
@@ -683,9 +486,17 @@ void LaunchSplitProlong(const LevelView &fine, const LevelView &coarse, const ui
                         T *eFine, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    const int occ = Occ<k_split_prolong<T>>();
-    LaunchPdl(k_split_prolong<T>, ProlongGrid<kQ<T>>(fine, coarse, occ), kPairThreads, 0, st, fine, coarse, pext, eCoarse,
-              eFine);
+    if constexpr (sizeof(T) == 8) // stretched grids run on this layout in FP64
+        if (fine.xr)
+        {
+            const int occ = Occ<k_split_prolong<T, true>>();
+            LaunchPdl(k_split_prolong<T, true>, ProlongGrid<kQ<T>>(fine, coarse, occ), kPairThreads, 0, st, fine,
+                      coarse, pext, eCoarse, eFine);
+            return;
+        }
+    const int occ = Occ<k_split_prolong<T, false>>();
+    LaunchPdl(k_split_prolong<T, false>, ProlongGrid<kQ<T>>(fine, coarse, occ), kPairThreads, 0, st, fine, coarse,
+              pext, eCoarse, eFine);
 }
 
 // r_c = R res_f = P^T res_f at the coarse unknowns, from the red fine residual. A thread owns N = 4 (FP64: 2) consecutive
@@ -694,21 +505,45 @@ void LaunchSplitProlong(const LevelView &fine, const LevelView &coarse, const ui
 // moved weights enter as X(a). In fine row (a, b) the red cells among k = 2K-2 .. 2K+1 are elements K-1 and K, at
 // k = 2K-2+q and 2K+q (q = (a + b) & 1), and the red child of coarse K is element K - q; the N + 1 elements
 // K0-1 .. K0+N-1 of a row are one aligned quad and one more.
-template <typename T>
+// The fine rows coarse row J gathers from and their weights: 2J-2 .. 2J+1, or with x groups (kX) those of
+// LevelView::xr; rows 1 and 2 are J's children (row 2 only with two).
+template <typename T, bool kX> struct RowTaps
+{
+    int b[4];
+    T w[4];
+    bool two;
+};
+template <typename T, bool kX> __device__ __forceinline__ RowTaps<T, kX> TapsOf(const LevelView &fv, int J)
+{
+    RowTaps<T, kX> t;
+    if constexpr (kX) XrTaps<T>(fv.xr[J], t.b, t.w, t.two);
+    else
+    {
+        t.two = true;
+#pragma unroll
+        for (int dj = 0; dj < 4; dj++)
+        {
+            t.b[dj] = 2 * J - 2 + dj;
+            t.w[dj] = dj == 0 || dj == 3 ? (T)0.25 : (T)0.75;
+        }
+    }
+    return t;
+}
+
+template <typename T, bool kX>
 __device__ __forceinline__ void SplitRestrictPlane(const LevelView &fv, const uint8_t *__restrict__ pext,
-                                                   const T *__restrict__ res, int a, int J, int K0, bool more,
-                                                   T (&Tw)[kQ<T>], T (&X)[kQ<T>])
+                                                   const T *__restrict__ res, int a, const RowTaps<T, kX> &J, int K0,
+                                                   bool more, T (&Tw)[kQ<T>], T (&X)[kQ<T>])
 {
     constexpr int N = kQ<T>;
 #pragma unroll
     for (int x = 0; x < N; x++) Tw[x] = X[x] = (T)0;
     if (a > fv.Ny - 1) return;
-    const T wt[4] = {(T)0.25, (T)0.75, (T)0.75, (T)0.25};
 #pragma unroll
     for (int dj = 0; dj < 4; dj++)
     {
-        const int b = 2 * J - 2 + dj;
-        if (b > fv.Nx - 1) continue;
+        const int b = J.b[dj];
+        if (kX ? J.w[dj] == (T)0 : b > fv.Nx - 1) continue;
         const int q = (a + b) & 1;
         const long long row = (long long)a * fv.sPS + (long long)b * fv.sRS + (K0 - 1);
         const Quad<T> r4 = LQ(res + row);
@@ -718,8 +553,8 @@ __device__ __forceinline__ void SplitRestrictPlane(const LevelView &fv, const ui
         R[N] = more ? res[row + N] : (T)0;
 #pragma unroll
         for (int x = 0; x < N; x++)
-            Tw[x] += wt[dj] * (q ? (T)0.75 * R[x] + (T)0.25 * R[x + 1] : (T)0.25 * R[x] + (T)0.75 * R[x + 1]);
-        if (dj == 1 || dj == 2)
+            Tw[x] += J.w[dj] * (q ? (T)0.75 * R[x] + (T)0.25 * R[x + 1] : (T)0.25 * R[x] + (T)0.75 * R[x + 1]);
+        if (dj == 1 || (dj == 2 && J.two))
         {
             const unsigned w = LdB<N>(pext + row);
             const unsigned wN = more ? pext[row + N] : 0u;
@@ -736,7 +571,7 @@ __device__ __forceinline__ void SplitRestrictPlane(const LevelView &fv, const ui
     for (int x = 0; x < N; x++) X[x] *= (T)(1.0 / 64.0);
 }
 
-template <typename T>
+template <typename T, bool kX>
 __device__ __forceinline__ void SplitRestrictQ(const LevelView &fv, const LevelView &cv,
                                                const uint8_t *__restrict__ pext, const T *__restrict__ res,
                                                T *__restrict__ rc, const Blk &blk)
@@ -750,14 +585,15 @@ __device__ __forceinline__ void SplitRestrictQ(const LevelView &fv, const LevelV
     const int I0 = 1 + blk.y * S, I1 = min(I0 + S, cv.Ny - 1);
     if (I0 >= I1) return;
     const bool more = K0 + N - 1 <= cv.Nz - 2; // element K0+N-1 is read only for coarse cell K0+N-1
+    const RowTaps<T, kX> taps = TapsOf<T, kX>(fv, J);
     T Tm2[N], Tm1[N], Xm1[N], Xd[N];
-    SplitRestrictPlane<T>(fv, pext, res, 2 * I0 - 2, J, K0, more, Tm2, Xd);
-    SplitRestrictPlane<T>(fv, pext, res, 2 * I0 - 1, J, K0, more, Tm1, Xm1);
+    SplitRestrictPlane<T, kX>(fv, pext, res, 2 * I0 - 2, taps, K0, more, Tm2, Xd);
+    SplitRestrictPlane<T, kX>(fv, pext, res, 2 * I0 - 1, taps, K0, more, Tm1, Xm1);
     for (int I = I0; I < I1; I++)
     {
         T T0[N], X0[N], T1[N], X1[N];
-        SplitRestrictPlane<T>(fv, pext, res, 2 * I, J, K0, more, T0, X0);
-        SplitRestrictPlane<T>(fv, pext, res, 2 * I + 1, J, K0, more, T1, X1);
+        SplitRestrictPlane<T, kX>(fv, pext, res, 2 * I, taps, K0, more, T0, X0);
+        SplitRestrictPlane<T, kX>(fv, pext, res, 2 * I + 1, taps, K0, more, T1, X1);
         const long long c = (long long)I * cv.sI + (long long)J * cv.sJ + K0;
 #pragma unroll
         for (int x = 0; x < N; x++)
@@ -772,42 +608,41 @@ __device__ __forceinline__ void SplitRestrictQ(const LevelView &fv, const LevelV
     }
 }
 
-template <typename T>
+template <typename T, bool kX>
 __global__ void __launch_bounds__(kPairThreads) k_split_restrict(LevelView fv, LevelView cv,
                                                                  const uint8_t *__restrict__ pext,
                                                                  const T *__restrict__ res, T *__restrict__ rc)
 {
     PdlWait();
     PdlTrigger();
-    SplitRestrictQ<T>(fv, cv, pext, res, rc, ThisBlk());
+    SplitRestrictQ<T, kX>(fv, cv, pext, res, rc, ThisBlk());
 }
 
 // The same restriction with one thread per coarse cell (K along the 32 lanes, J across the 8 warps), for the smaller
 // coarse levels: more threads, and their launches are latency-bound.
-template <typename T>
+template <typename T, bool kX>
 __device__ __forceinline__ void SplitRestrictPlane1(const LevelView &fv, const uint8_t *pext, const T *res, int a,
-                                                   int J, int K, T &Tw, T &X)
+                                                   const RowTaps<T, kX> &J, int K, T &Tw, T &X)
 {
     Tw = (T)0;
     X = (T)0;
     if (a > fv.Ny - 1) return;
-    const T wt[4] = {(T)0.25, (T)0.75, (T)0.75, (T)0.25};
 #pragma unroll
     for (int dj = 0; dj < 4; dj++)
     {
-        const int b = 2 * J - 2 + dj;
-        if (b > fv.Nx - 1) continue;
+        const int b = J.b[dj];
+        if (kX ? J.w[dj] == (T)0 : b > fv.Nx - 1) continue;
         const int q = (a + b) & 1;
         const long long row = (long long)a * fv.sPS + (long long)b * fv.sRS;
         const T lo = res[row + K - 1], hi = res[row + K];
-        Tw += wt[dj] * (q ? (T)0.75 * lo + (T)0.25 * hi : (T)0.25 * lo + (T)0.75 * hi);
-        if (dj == 1 || dj == 2) X += (T)(pext[row + K - q] & 0x3Fu) * (q ? lo : hi);
+        Tw += J.w[dj] * (q ? (T)0.75 * lo + (T)0.25 * hi : (T)0.25 * lo + (T)0.75 * hi);
+        if (dj == 1 || (dj == 2 && J.two)) X += (T)(pext[row + K - q] & 0x3Fu) * (q ? lo : hi);
     }
     X *= (T)(1.0 / 64.0);
 }
 
 // bx, by: the K and J tiles; bz of gz: the chunk of coarse planes
-template <typename T>
+template <typename T, bool kX>
 __device__ __forceinline__ void SplitRestrict1(const LevelView &fv, const LevelView &cv,
                                                const uint8_t *__restrict__ pext, const T *__restrict__ res,
                                                T *__restrict__ rc, int bx, int by, int bz, int gz)
@@ -817,14 +652,15 @@ __device__ __forceinline__ void SplitRestrict1(const LevelView &fv, const LevelV
     const int S = (cv.Ny - 2 + gz - 1) / gz;
     const int I0 = 1 + bz * S, I1 = min(I0 + S, cv.Ny - 1);
     if (I0 >= I1) return;
+    const RowTaps<T, kX> taps = TapsOf<T, kX>(fv, J);
     T Tm2, Tm1, Xm1, Xdummy;
-    SplitRestrictPlane1<T>(fv, pext, res, 2 * I0 - 2, J, K, Tm2, Xdummy);
-    SplitRestrictPlane1<T>(fv, pext, res, 2 * I0 - 1, J, K, Tm1, Xm1);
+    SplitRestrictPlane1<T, kX>(fv, pext, res, 2 * I0 - 2, taps, K, Tm2, Xdummy);
+    SplitRestrictPlane1<T, kX>(fv, pext, res, 2 * I0 - 1, taps, K, Tm1, Xm1);
     for (int I = I0; I < I1; I++)
     {
         T T0, X0, T1, X1;
-        SplitRestrictPlane1<T>(fv, pext, res, 2 * I, J, K, T0, X0);
-        SplitRestrictPlane1<T>(fv, pext, res, 2 * I + 1, J, K, T1, X1);
+        SplitRestrictPlane1<T, kX>(fv, pext, res, 2 * I, taps, K, T0, X0);
+        SplitRestrictPlane1<T, kX>(fv, pext, res, 2 * I + 1, taps, K, T1, X1);
         const long long c = (long long)I * cv.sI + (long long)J * cv.sJ + K;
         if (cv.code[c] & CODE_UNKNOWN)
             rc[VecIdx(cv, I, J, K)] = (((T)0.25 * Tm2 + (T)0.75 * Tm1) + ((T)0.75 * T0 + (T)0.25 * T1)) + (Xm1 + X0);
@@ -834,13 +670,13 @@ __device__ __forceinline__ void SplitRestrict1(const LevelView &fv, const LevelV
     }
 }
 
-template <typename T>
+template <typename T, bool kX>
 __global__ void __launch_bounds__(256) k_split_restrict1(LevelView fv, LevelView cv, const uint8_t *__restrict__ pext,
                                                         const T *__restrict__ res, T *__restrict__ rc)
 {
     PdlWait();
     PdlTrigger();
-    SplitRestrict1<T>(fv, cv, pext, res, rc, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, (int)gridDim.z);
+    SplitRestrict1<T, kX>(fv, cv, pext, res, rc, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, (int)gridDim.z);
 }
 
 // Coarse levels with at least kRestrictQuadCells cells take the quad kernel (4x fewer loads per coarse cell), the
@@ -848,25 +684,34 @@ __global__ void __launch_bounds__(256) k_split_restrict1(LevelView fv, LevelView
 // Both sum the same products in the same order.
 constexpr long long kRestrictQuadCells = 1LL << 20;
 
-template <typename T>
-void LaunchSplitRestrict(const LevelView &fine, const LevelView &coarse, const uint8_t *pext, const T *resFine,
-                         T *rCoarse, int mode, cudaStream_t st)
+template <typename T, bool kX>
+static void RestrictOn(const LevelView &fine, const LevelView &coarse, const uint8_t *pext, const T *resFine,
+                       T *rCoarse, int mode, cudaStream_t st)
 {
-    NB_COUNT_LAUNCH();
     if (mode == 1 || (mode != 2 && coarse.cells < kRestrictQuadCells))
     {
         const long long perPlane = (long long)((coarse.Nz - 2 + 31) / 32) * ((coarse.Nx - 2 + 7) / 8);
         const int S = MarchPlanes(coarse.Ny - 2, perPlane);
         const dim3 grid((unsigned)((coarse.Nz - 2 + 31) / 32), (unsigned)((coarse.Nx - 2 + 7) / 8),
                         (unsigned)((coarse.Ny - 2 + S - 1) / S));
-        LaunchPdl(k_split_restrict1<T>, grid, dim3(32, 8), 0, st, fine, coarse, pext, resFine, rCoarse);
+        LaunchPdl(k_split_restrict1<T, kX>, grid, dim3(32, 8), 0, st, fine, coarse, pext, resFine, rCoarse);
         return;
     }
     const long long nt = (long long)(coarse.Nx - 2) * ((coarse.Nz - 2 + kQ<T> - 1) / kQ<T>);
     const long long perPlane = (nt + kPairThreads - 1) / kPairThreads, planes = coarse.Ny - 2 > 0 ? coarse.Ny - 2 : 1;
-    const long long bestS = BestMarch(perPlane, planes, (long long)SmCount() * Occ<k_split_restrict<T>>());
-    LaunchPdl(k_split_restrict<T>, dim3((unsigned)perPlane, (unsigned)((planes + bestS - 1) / bestS)), kPairThreads, 0,
-              st, fine, coarse, pext, resFine, rCoarse);
+    const long long bestS = BestMarch(perPlane, planes, (long long)SmCount() * Occ<k_split_restrict<T, kX>>());
+    LaunchPdl(k_split_restrict<T, kX>, dim3((unsigned)perPlane, (unsigned)((planes + bestS - 1) / bestS)),
+              kPairThreads, 0, st, fine, coarse, pext, resFine, rCoarse);
+}
+
+template <typename T>
+void LaunchSplitRestrict(const LevelView &fine, const LevelView &coarse, const uint8_t *pext, const T *resFine,
+                         T *rCoarse, int mode, cudaStream_t st)
+{
+    NB_COUNT_LAUNCH();
+    if constexpr (sizeof(T) == 8) // stretched grids run on this layout in FP64
+        if (fine.xr) return RestrictOn<T, true>(fine, coarse, pext, resFine, rCoarse, mode, st);
+    RestrictOn<T, false>(fine, coarse, pext, resFine, rCoarse, mode, st);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -990,6 +835,8 @@ void LaunchSplitPApply(const LevelView &v, const uint8_t *du, const T *z, T *p0,
                        const Reducer &R, const double *S, const int *it, int baseEven, int baseOdd, int slotN,
                        int singular, int slotPQ, cudaStream_t st)
 {
+    if constexpr (sizeof(T) == 8)
+        if (v.stretched) return LaunchStretchedPApply(v, du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, st);
     NB_COUNT_LAUNCH();
     if (singular)
         LaunchPdl(k_split_papply<T, true>, QuadGrid<kQ<T>>(v, Occ<k_split_papply<T, true>>()), kPairThreads, 0, st, v,
@@ -1237,7 +1084,7 @@ __global__ void __launch_bounds__(kPairThreads) kb_split_prolong(const BatchLeve
     const int q = BatchReqOf(a);
     if (q < 0) return;
     const BatchLevel &F = lv[q * ls + l], &C = lv[q * ls + l + 1];
-    SplitProlong<float>(F.v, C.v, F.pext, C.e, F.e, ThisBlk());
+    SplitProlong<float, false>(F.v, C.v, F.pext, C.e, F.e, ThisBlk());
 }
 
 __global__ void __launch_bounds__(kPairThreads) kb_split_restrict(const BatchLevel *__restrict__ lv, int ls, int l,
@@ -1248,7 +1095,7 @@ __global__ void __launch_bounds__(kPairThreads) kb_split_restrict(const BatchLev
     const int q = BatchReqOf(a);
     if (q < 0) return;
     const BatchLevel &F = lv[q * ls + l], &C = lv[q * ls + l + 1];
-    SplitRestrictQ<float>(F.v, C.v, F.pext, F.res, C.r, ThisBlk());
+    SplitRestrictQ<float, false>(F.v, C.v, F.pext, F.res, C.r, ThisBlk());
 }
 
 // grid (K tiles, J tiles x gz plane chunks, capacity)
@@ -1261,7 +1108,7 @@ __global__ void __launch_bounds__(256) kb_split_restrict1(const BatchLevel *__re
     if (q < 0) return;
     const BatchLevel &F = lv[q * ls + l], &C = lv[q * ls + l + 1];
     const int by = (int)blockIdx.y % gyJ, bz = (int)blockIdx.y / gyJ;
-    SplitRestrict1<float>(F.v, C.v, F.pext, F.res, C.r, (int)blockIdx.x, by, bz, gz);
+    SplitRestrict1<float, false>(F.v, C.v, F.pext, F.res, C.r, (int)blockIdx.x, by, bz, gz);
 }
 
 // form -1: every request in its own form; 0 / 1: only the requests of that form (singular = 1)
@@ -1467,15 +1314,21 @@ template <typename T> static void PrepareSplit()
     (void)Occ<k_split_half<T, 1>>();
     (void)Occ<k_split_half<T, 2>>();
     (void)Occ<k_split_residual<T>>();
-    (void)Occ<k_split_prolong<T>>();
-    (void)Occ<k_split_restrict<T>>();
+    (void)Occ<k_split_prolong<T, false>>();
+    (void)Occ<k_split_restrict<T, false>>();
     (void)Occ<k_split_papply<T, true>>();
     (void)Occ<k_split_papply<T, false>>();
 }
 
 void PrepareSplitKernels(int elemBytes)
 {
-    if (elemBytes == 8) PrepareSplit<double>();
+    if (elemBytes == 8)
+    {
+        PrepareSplit<double>();
+        (void)Occ<k_split_prolong<double, true>>();
+        (void)Occ<k_split_restrict<double, true>>();
+        PrepareStretchedKernels();
+    }
     else PrepareSplit<float>();
 }
 

@@ -238,3 +238,28 @@ def test_odd_rows_agree_with_per_cell_kernels(nb, size, precision):
         bar = 1e-11 * max(size) ** 2
         for x, y in ((a.p, b.p), (a.u, b.u), (a.v, b.v), (a.w, b.w)):
             assert np.linalg.norm(x - y) <= bar * np.linalg.norm(y)
+
+
+# stretched FP64: (interior x, y, z) of the cylinder channel; Nz even and odd, one level above the coarse end and
+# several, x groups on and off
+@pytest.mark.parametrize("groups", [1, 0])
+@pytest.mark.parametrize("size", [(24, 16, 16), (32, 17, 15), (48, 32, 33), (64, 24, 40)])
+def test_stretched_fp64_agrees_with_per_cell_kernels(nb, size, groups):
+    """The stretched FP64 sweeps of the colour-split layout against the per-cell kernels. Both solve to 1e-12, so the
+    pressures agree within 2 cond(A) 1e-12, with cond(A) from the assembled matrix's extreme eigenvalues."""
+    import scipy.sparse as sp
+    import scipy.sparse.linalg as sl
+
+    case = W.stretched_cylinder_3d(*size)
+    types = capi.label_cells(case.grid, case.scene)
+    a, b = [solve_family(case, types, family, "fp64", False, x_groups=groups) for family in (2, 0)]
+    s = PressureSolver("fp64")
+    s.InitializePressureSolver(b)
+    rowptr, col, val, _ = s.ExportMatrix()
+    s.DestroyPressureSolver()
+    A = -sp.csr_matrix((val, col, rowptr))
+    top = sl.eigsh(A, k=1, which="LA", return_eigenvectors=False, tol=1e-3)[0]
+    low = sl.eigsh(A.tocsc(), k=1, sigma=0.0, return_eigenvectors=False)[0]
+    bar = 2.0 * top / low * 1e-12
+    idp = types.reshape(-1) == W.FLUID
+    assert np.linalg.norm((a.p - b.p)[idp]) <= bar * np.linalg.norm(b.p[idp])
