@@ -7,11 +7,19 @@
 //
 // What costs time here is latency, not bytes: each phase (one colour of a sweep, a residual, a transfer) is a short
 // loop over a level's unknowns followed by a barrier. So
-// - the per-colour lists of unknowns are built once per layout (k_tail_lists) and only copied in;
+// - what a layout fixes is built once per layout (k_tail_lists) in the order it has in shared memory and only copied
+//   in, 16 bytes at a time, before the dependent-launch wait: the per-colour lists of unknowns, the diagonal's
+//   half-units (uniform) or the codes and types (stretched), and the weights the transfers move off SOLID cells;
 // - a uniform level sums its six neighbours unmasked (every vector is zero off the unknowns) and divides through a
-//   per-level reciprocal table of the diagonal's half-units, computed once per launch;
+//   per-level reciprocal table of the diagonal's half-units;
+// - a thread keeps its red and its black cell's index, right-hand side and stencil in registers across a level's
+//   sweeps and residual, where a level has at most one unknown of each colour per thread (all but the first levels
+//   of unusually large coarse ends); a half-sweep then waits for its six neighbours only;
 // - the levels with at most 32 unknowns of each colour (the last two or three) run in warp 0 alone, with __syncwarp
 //   between their phases instead of a block-wide barrier.
+// Against a form that prepared the lists alone, decoded its cells and read its stencil again in every phase, this took
+// 10 us off each V-cycle of a 64^3 box (of 120), 8 off one of a 2D 128^2 box (of 86) and 21 off one of the stretched
+// FP64 cylinder (of 410; B200).
 #include "nb_kernels.h"
 
 #include <cstring>
@@ -21,13 +29,14 @@
 namespace nb
 {
 
-constexpr int kTailThreads = 256;
+// threads of the block: one per unknown of a colour on the usual coarse ends (a first level of at most 2048 cells)
+constexpr int kTailThreads = 256, kTailThreadsBig = 512;
 
 template <typename T> struct TailLevel
 {
     LevelView v;
     unsigned off;     // byte offset of the level's arrays in shared memory
-    unsigned listOff; // entry offset of the level's list in the global list array
+    unsigned listOff; // 4-byte offset of the level's prepared data in the global array
 };
 
 template <typename T> struct TailArgs
@@ -37,28 +46,39 @@ template <typename T> struct TailArgs
     const T *rIn; // residual of the first tail level (global)
     T *eOut;      // its correction (global)
     int pre, post, coarseSweeps;
-    const unsigned *lists; // per level: its cells' entries, red unknowns from the front, black ones from the back
+    const unsigned *lists; // per level: its prepared data (PrepBytes)
     const int *counts;     // [level][colour] unknowns
 };
 
-// The level's arrays in shared memory: r, e, res (T), then code, types and diagonal units (bytes), then the list of
-// its unknowns (4 bytes each: red ones from the front, black ones from the back), each padded to 16 bytes.
+__host__ __device__ inline unsigned Pad16(unsigned b) { return (b + 15u) / 16u * 16u; }
+
+// A level's prepared data, the same bytes in global and shared memory: the list of its unknowns (4 bytes each, packed
+// i << 20 | j << 10 | k: red ones from the front, black ones from the back), then three byte arrays: the diagonal's
+// half-units, the transfer weights and nothing (uniform), or the codes, the transfer weights and the types (stretched).
+__host__ __device__ inline unsigned PrepBytes(long long cells)
+{
+    return Pad16((unsigned)cells * 4u) + 3u * Pad16((unsigned)cells);
+}
+
+// The level's arrays in shared memory: r, e, res (T), then its prepared data, each padded to 16 bytes.
 template <typename T> __host__ __device__ inline unsigned LevelBytes(long long cells)
 {
-    const unsigned a = (unsigned)((cells * sizeof(T) + 15) / 16 * 16);
-    const unsigned b = (unsigned)((cells + 15) / 16 * 16);
-    const unsigned l = (unsigned)((cells * 4 + 15) / 16 * 16);
-    return 3 * a + 3 * b + l;
+    return 3u * Pad16((unsigned)(cells * sizeof(T))) + PrepBytes(cells);
 }
 
 template <typename T> struct SmemLevel
 {
-    LevelView v; // types/code point into shared memory
+    int sI, sJ, cells;
+    int Nx, Ny, Nz;
     T *r, *e, *res;
-    uint8_t *du;    // uniform level: 0x80 | diagonal half-units at an unknown, 0 elsewhere
-    unsigned *list; // packed (i << 20 | j << 10 | k) of the unknowns; red [0, nRed), black [cells - nBlack, cells)
+    unsigned *list;      // red [0, nRed), black [cells - nBlack, cells)
+    const uint8_t *unit; // uniform: 0x80 | diagonal half-units at an unknown, 0 elsewhere; stretched: the codes
+    const uint8_t *ext;  // 0x80 | 64ths of weight the transfers move onto the parent, at an unknown
+    const uint8_t *types; // stretched
     int nRed, nBlack;
-    const double *inv; // 1 / (gamma/2 * units), entry 0 = 0
+    T g, hg;             // gamma, gamma / 2 (uniform)
+    const double *inv;   // 1 / (gamma/2 * units), entry 0 = 0
+    const LevelView *v;  // the spacing tables (stretched)
 };
 
 __device__ __forceinline__ void Unpack(unsigned x, int &i, int &j, int &k)
@@ -71,18 +91,24 @@ __device__ __forceinline__ void Unpack(unsigned x, int &i, int &j, int &k)
 template <typename T> __device__ __forceinline__ SmemLevel<T> Bind(const TailLevel<T> &tl, unsigned char *smem)
 {
     SmemLevel<T> s;
-    s.v = tl.v;
-    const long long cells = tl.v.cells;
-    const unsigned a = (unsigned)((cells * sizeof(T) + 15) / 16 * 16);
-    const unsigned b = (unsigned)((cells + 15) / 16 * 16);
+    s.v = &tl.v;
+    s.sI = (int)tl.v.sI;
+    s.sJ = (int)tl.v.sJ;
+    s.cells = (int)tl.v.cells;
+    s.Nx = tl.v.Nx;
+    s.Ny = tl.v.Ny;
+    s.Nz = tl.v.Nz;
+    s.g = (T)tl.v.gamma;
+    s.hg = (T)0.5 * (T)tl.v.gamma;
+    const unsigned a = Pad16((unsigned)(s.cells * sizeof(T))), b = Pad16((unsigned)s.cells);
     unsigned char *base = smem + tl.off;
     s.r = (T *)base;
     s.e = (T *)(base + a);
     s.res = (T *)(base + 2 * a);
-    s.v.code = base + 3 * a;
-    s.v.types = base + 3 * a + b;
-    s.du = base + 3 * a + 2 * b;
-    s.list = (unsigned *)(base + 3 * a + 3 * b);
+    s.list = (unsigned *)(base + 3 * a);
+    s.unit = base + 3 * a + Pad16((unsigned)s.cells * 4u);
+    s.ext = s.unit + b;
+    s.types = s.ext + b;
     s.nRed = s.nBlack = 0;
     s.inv = nullptr;
     return s;
@@ -91,23 +117,14 @@ template <typename T> __device__ __forceinline__ SmemLevel<T> Bind(const TailLev
 // the t-th unknown of the given colour (0 red, 1 black, 2 both: red then black)
 template <typename T> __device__ __forceinline__ unsigned ListAt(const SmemLevel<T> &L, int colour, int t)
 {
-    const long long cells = L.v.cells;
     if (colour == 0) return L.list[t];
-    if (colour == 1) return L.list[cells - 1 - t];
-    return t < L.nRed ? L.list[t] : L.list[cells - 1 - (t - L.nRed)];
+    if (colour == 1) return L.list[L.cells - 1 - t];
+    return t < L.nRed ? L.list[t] : L.list[L.cells - 1 - (t - L.nRed)];
 }
 
 template <typename T> __device__ __forceinline__ int ListLen(const SmemLevel<T> &L, int colour)
 {
     return colour == 0 ? L.nRed : (colour == 1 ? L.nBlack : L.nRed + L.nBlack);
-}
-
-__device__ __forceinline__ void Decode(const LevelView &v, long long c, int &i, int &j, int &k)
-{
-    k = (int)(c % v.Nz);
-    const long long r = c / v.Nz;
-    j = (int)(r % v.Nx);
-    i = (int)(r / v.Nx);
 }
 
 // A phase runs over the whole block (kWarp false) or over warp 0 alone (kWarp true), and ends with the matching
@@ -120,317 +137,331 @@ template <bool kWarp> __device__ __forceinline__ void PhaseSync()
     else __syncthreads();
 }
 
-// the plain sum of a cell's neighbours on a uniform level (vectors are zero off the unknowns)
-template <typename T> __device__ __forceinline__ T NbrSum(const LevelView &v, const T *e, long long c)
+// One unknown of a level and its stencil
+template <typename T, bool k3D, bool kSt> struct Cell
 {
-    const T s = (e[c + v.sI] + e[c - v.sI]) + (e[c + v.sJ] + e[c - v.sJ]);
-    return v.dim == 3 ? s + (e[c + 1] + e[c - 1]) : s;
+    int c;
+    T r;
+    unsigned b;             // uniform: the half-units byte; stretched: the code
+    T inv;                  // uniform: 1 / diagonal
+    T cq[kSt ? 6 : 1], diag; // stretched
+};
+
+template <typename T, bool k3D, bool kSt>
+__device__ __forceinline__ Cell<T, k3D, kSt> LoadCell(const SmemLevel<T> &L, unsigned packed)
+{
+    Cell<T, k3D, kSt> o;
+    int i, j, k;
+    Unpack(packed, i, j, k);
+    o.c = i * L.sI + j * L.sJ + k;
+    o.r = L.r[o.c];
+    o.b = L.unit[o.c];
+    if constexpr (!kSt) o.inv = (T)L.inv[o.b & 0x7Fu];
+    else
+    {
+        LevelView v = *L.v;
+        v.types = L.types;
+        CodeStencil<T>(v, i, j, k, o.c, o.b, o.cq, o.diag);
+    }
+    return o;
 }
 
-template <typename T, bool kWarp> __device__ void TSmooth(const SmemLevel<T> &L, int colour, bool first)
+// the plain sum of a cell's neighbours on a uniform level (vectors are zero off the unknowns)
+template <typename T, bool k3D> __device__ __forceinline__ T NbrSum(const SmemLevel<T> &L, const T *e, int c)
 {
-    const LevelView &v = L.v;
-    const int n = ListLen(L, colour);
-    const T g = (T)v.gamma;
-    for (int t = PhaseStart<kWarp>(); t < n; t += PhaseStride<kWarp>())
+    const T s = (e[c + L.sI] + e[c - L.sI]) + (e[c + L.sJ] + e[c - L.sJ]);
+    return k3D ? s + (e[c + 1] + e[c - 1]) : s;
+}
+
+template <typename T, bool k3D, bool kSt>
+__device__ __forceinline__ void SmoothCell(const SmemLevel<T> &L, const Cell<T, k3D, kSt> &o, bool first)
+{
+    const int c = o.c;
+    T rhs = o.r;
+    if constexpr (!kSt)
     {
-        int i, j, k;
-        Unpack(ListAt(L, colour, t), i, j, k);
-        const long long c = (long long)i * v.sI + (long long)j * v.sJ + k;
-        if (!v.stretched)
-        {
-            T rhs = L.r[c];
-            if (!first) rhs += g * NbrSum(v, L.e, c);
-            L.e[c] = rhs * (T)L.inv[L.du[c] & 0x7Fu];
-            continue;
-        }
-        const unsigned code = v.code[c];
-        T cq[6], diag;
-        CodeStencil<T>(v, i, j, k, c, code, cq, diag);
-        T rhs = L.r[c];
+        if (!first) rhs += L.g * NbrSum<T, k3D>(L, L.e, c);
+        L.e[c] = rhs * o.inv;
+    }
+    else
+    {
         if (!first)
         {
-            if (code & 1u) rhs += cq[0] * L.e[c + v.sI];
-            if (code & 2u) rhs += cq[1] * L.e[c - v.sI];
-            if (code & 4u) rhs += cq[2] * L.e[c + v.sJ];
-            if (code & 8u) rhs += cq[3] * L.e[c - v.sJ];
-            if (code & 16u) rhs += cq[4] * L.e[c + 1];
-            if (code & 32u) rhs += cq[5] * L.e[c - 1];
+            if (o.b & 1u) rhs += o.cq[0] * L.e[c + L.sI];
+            if (o.b & 2u) rhs += o.cq[1] * L.e[c - L.sI];
+            if (o.b & 4u) rhs += o.cq[2] * L.e[c + L.sJ];
+            if (o.b & 8u) rhs += o.cq[3] * L.e[c - L.sJ];
+            if (o.b & 16u) rhs += o.cq[4] * L.e[c + 1];
+            if (o.b & 32u) rhs += o.cq[5] * L.e[c - 1];
         }
-        L.e[c] = diag != (T)0 ? rhs / diag : (T)0;
+        L.e[c] = o.diag != (T)0 ? rhs / o.diag : (T)0;
     }
-    PhaseSync<kWarp>();
 }
 
-template <typename T, bool kWarp> __device__ void TResidual(const SmemLevel<T> &L)
+template <typename T, bool k3D, bool kSt>
+__device__ __forceinline__ void ResidualCell(const SmemLevel<T> &L, const Cell<T, k3D, kSt> &o)
 {
-    const LevelView &v = L.v;
-    const int n = ListLen(L, 2);
-    const T g = (T)v.gamma, hg = (T)0.5 * (T)v.gamma;
-    for (int t = PhaseStart<kWarp>(); t < n; t += PhaseStride<kWarp>())
+    const int c = o.c;
+    if constexpr (!kSt)
+        L.res[c] = o.r - (L.hg * (T)(o.b & 0x7Fu) * L.e[c] - L.g * NbrSum<T, k3D>(L, L.e, c));
+    else
     {
-        int i, j, k;
-        Unpack(ListAt(L, 2, t), i, j, k);
-        const long long c = (long long)i * v.sI + (long long)j * v.sJ + k;
-        if (!v.stretched)
-        {
-            L.res[c] = L.r[c] - (hg * (T)(L.du[c] & 0x7Fu) * L.e[c] - g * NbrSum(v, L.e, c));
-            continue;
-        }
-        const unsigned code = v.code[c];
-        T cq[6], diag;
-        CodeStencil<T>(v, i, j, k, c, code, cq, diag);
-        T s = diag * L.e[c];
-        if (code & 1u) s -= cq[0] * L.e[c + v.sI];
-        if (code & 2u) s -= cq[1] * L.e[c - v.sI];
-        if (code & 4u) s -= cq[2] * L.e[c + v.sJ];
-        if (code & 8u) s -= cq[3] * L.e[c - v.sJ];
-        if (code & 16u) s -= cq[4] * L.e[c + 1];
-        if (code & 32u) s -= cq[5] * L.e[c - 1];
-        L.res[c] = L.r[c] - s;
+        T s = o.diag * L.e[c];
+        if (o.b & 1u) s -= o.cq[0] * L.e[c + L.sI];
+        if (o.b & 2u) s -= o.cq[1] * L.e[c - L.sI];
+        if (o.b & 4u) s -= o.cq[2] * L.e[c + L.sJ];
+        if (o.b & 8u) s -= o.cq[3] * L.e[c - L.sJ];
+        if (o.b & 16u) s -= o.cq[4] * L.e[c + 1];
+        if (o.b & 32u) s -= o.cq[5] * L.e[c - 1];
+        L.res[c] = o.r - s;
     }
-    PhaseSync<kWarp>();
 }
 
-template <typename T>
-__device__ __forceinline__ T TSolidWeight(const LevelView &cv, int I, int J, int K, int si, int sj, int sk)
+// Sweeps of a level by one thread's cells: `fwd` red-black pairs (the first from a zero iterate where zero is set),
+// then `bwd` black-red pairs, then the residual where res is set.
+template <typename T, bool k3D, bool kSt, bool kWarp>
+__device__ __forceinline__ void TSweeps(const SmemLevel<T> &L, int fwd, int bwd, bool zero, bool res)
 {
-    const T wv[2] = {(T)0.75, (T)0.25};
-    const long long parent = (long long)I * cv.sI + (long long)J * cv.sJ + K;
-    T extra = (T)0;
-    const int nk = cv.dim == 3 ? 2 : 1;
-    for (int di = 0; di < 2; di++)
-        for (int dj = 0; dj < 2; dj++)
-            for (int dk = 0; dk < nk; dk++)
-            {
-                if (!(di | dj | dk)) continue;
-                const long long cc = parent + (long long)(di * si) * cv.sI + (long long)(dj * sj) * cv.sJ + dk * sk;
-                if (cv.types[cc] == SOLID) extra += wv[di] * wv[dj] * (cv.dim == 3 ? wv[dk] : (T)1);
-            }
-    return extra;
+    const int t0 = PhaseStart<kWarp>(), stride = PhaseStride<kWarp>();
+    if (L.nRed <= stride && L.nBlack <= stride)
+    {
+        const bool hasR = t0 < L.nRed, hasB = t0 < L.nBlack;
+        Cell<T, k3D, kSt> red{}, black{};
+        if (hasR) red = LoadCell<T, k3D, kSt>(L, ListAt(L, 0, t0));
+        if (hasB) black = LoadCell<T, k3D, kSt>(L, ListAt(L, 1, t0));
+        for (int s = 0; s < fwd; s++)
+        {
+            if (hasR) SmoothCell(L, red, zero && s == 0);
+            PhaseSync<kWarp>();
+            if (hasB) SmoothCell(L, black, false);
+            PhaseSync<kWarp>();
+        }
+        for (int s = 0; s < bwd; s++)
+        {
+            if (hasB) SmoothCell(L, black, false);
+            PhaseSync<kWarp>();
+            if (hasR) SmoothCell(L, red, false);
+            PhaseSync<kWarp>();
+        }
+        if (res)
+        {
+            if (hasR) ResidualCell(L, red);
+            if (hasB) ResidualCell(L, black);
+            PhaseSync<kWarp>();
+        }
+        return;
+    }
+    auto half = [&](int colour, bool first) {
+        const int n = ListLen(L, colour);
+        for (int t = t0; t < n; t += stride) SmoothCell(L, LoadCell<T, k3D, kSt>(L, ListAt(L, colour, t)), first);
+        PhaseSync<kWarp>();
+    };
+    for (int s = 0; s < fwd; s++)
+    {
+        half(0, zero && s == 0);
+        half(1, false);
+    }
+    for (int s = 0; s < bwd; s++)
+    {
+        half(1, false);
+        half(0, false);
+    }
+    if (res)
+    {
+        const int n = ListLen(L, 2);
+        for (int t = t0; t < n; t += stride) ResidualCell(L, LoadCell<T, k3D, kSt>(L, ListAt(L, 2, t)));
+        PhaseSync<kWarp>();
+    }
 }
 
-template <typename T, bool kWarp> __device__ void TRestrict(const SmemLevel<T> &F, const SmemLevel<T> &C)
+// 64ths of moved weight at fine cell c, as a weight
+template <typename T> __device__ __forceinline__ T Moved(const SmemLevel<T> &F, int c)
 {
-    const LevelView &fv = F.v, &cv = C.v;
+    return (T)(F.ext[c] & 0x3Fu) * (T)(1.0 / 64.0);
+}
+
+template <typename T, bool k3D, bool kWarp> __device__ void TRestrict(const SmemLevel<T> &F, const SmemLevel<T> &C)
+{
     const int n = ListLen(C, 2);
+    const T wt[4] = {(T)0.25, (T)0.75, (T)0.75, (T)0.25};
     for (int t = PhaseStart<kWarp>(); t < n; t += PhaseStride<kWarp>())
     {
         int I, J, K;
         Unpack(ListAt(C, 2, t), I, J, K);
-        const long long c = (long long)I * cv.sI + (long long)J * cv.sJ + K;
         T acc = (T)0;
-        const T wt[4] = {(T)0.25, (T)0.75, (T)0.75, (T)0.25};
+#pragma unroll
         for (int di = 0; di < 4; di++)
         {
             const int a = 2 * I - 2 + di;
-            if (a > fv.Ny - 1) continue;
+            if (a > F.Ny - 1) continue;
+#pragma unroll
             for (int dj = 0; dj < 4; dj++)
             {
                 const int b = 2 * J - 2 + dj;
-                if (b > fv.Nx - 1) continue;
-                const long long rowBase = (long long)a * fv.sI + (long long)b * fv.sJ;
+                if (b > F.Nx - 1) continue;
+                const int rowBase = a * F.sI + b * F.sJ;
                 const T wij = wt[di] * wt[dj];
-                if (fv.dim == 3)
+                if (k3D)
                 {
-                    T t = (T)0;
+                    T s = (T)0;
+#pragma unroll
                     for (int dk = 0; dk < 4; dk++)
                     {
                         const int d = 2 * K - 2 + dk;
-                        if (d <= fv.Nz - 1) t += wt[dk] * F.res[rowBase + d];
+                        if (d <= F.Nz - 1) s += wt[dk] * F.res[rowBase + d];
                     }
-                    acc += wij * t;
+                    acc += wij * s;
                 }
                 else
                     acc += wij * F.res[rowBase];
             }
         }
-        const int nz = fv.dim == 3 ? 2 : 1;
+        // the children also carry the weight the prolongation moved off their SOLID coarse contributors
+#pragma unroll
         for (int ci = 0; ci < 2; ci++)
+#pragma unroll
             for (int cj = 0; cj < 2; cj++)
-                for (int ck = 0; ck < nz; ck++)
+#pragma unroll
+                for (int ck = 0; ck < (k3D ? 2 : 1); ck++)
                 {
-                    const int a = 2 * I - 1 + ci, b = 2 * J - 1 + cj, d = fv.dim == 3 ? 2 * K - 1 + ck : 0;
-                    if (a > fv.Ny - 2 || b > fv.Nx - 2 || (fv.dim == 3 && d > fv.Nz - 2)) continue;
-                    const T extra = TSolidWeight<T>(cv, I, J, K, ci ? 1 : -1, cj ? 1 : -1, ck ? 1 : -1);
-                    if (extra != (T)0) acc += extra * F.res[(long long)a * fv.sI + (long long)b * fv.sJ + d];
+                    const int a = 2 * I - 1 + ci, b = 2 * J - 1 + cj, d = k3D ? 2 * K - 1 + ck : 0;
+                    if (a > F.Ny - 2 || b > F.Nx - 2 || (k3D && d > F.Nz - 2)) continue;
+                    const int c = a * F.sI + b * F.sJ + d;
+                    const T extra = Moved(F, c);
+                    if (extra != (T)0) acc += extra * F.res[c];
                 }
-        C.r[c] = acc;
+        C.r[I * C.sI + J * C.sJ + K] = acc;
     }
     PhaseSync<kWarp>();
 }
 
-template <typename T, bool kWarp> __device__ void TProlong(const SmemLevel<T> &F, const SmemLevel<T> &C)
+template <typename T, bool k3D, bool kWarp> __device__ void TProlong(const SmemLevel<T> &F, const SmemLevel<T> &C)
 {
-    const LevelView &fv = F.v, &cv = C.v;
     const int n = ListLen(F, 2);
+    const T wv[2] = {(T)0.75, (T)0.25};
     for (int t = PhaseStart<kWarp>(); t < n; t += PhaseStride<kWarp>())
     {
         int a, b, d;
         Unpack(ListAt(F, 2, t), a, b, d);
-        const long long c = (long long)a * fv.sI + (long long)b * fv.sJ + d;
-        const int A = (a + 1) >> 1, B = (b + 1) >> 1;
-        const int D = fv.dim == 3 ? (d + 1) >> 1 : 0;
-        const int si = (a & 1) ? -1 : 1, sj = (b & 1) ? -1 : 1, sk = (d & 1) ? -1 : 1;
-        const T wv[2] = {(T)0.75, (T)0.25};
-        const long long parent = (long long)A * cv.sI + (long long)B * cv.sJ + D;
-        T acc = (T)0, extra = (T)0;
-        const int nk = fv.dim == 3 ? 2 : 1;
+        const int c = a * F.sI + b * F.sJ + d;
+        const int A = (a + 1) >> 1, B = (b + 1) >> 1, D = k3D ? (d + 1) >> 1 : 0;
+        const int si = (a & 1) ? -C.sI : C.sI, sj = (b & 1) ? -C.sJ : C.sJ, sk = (d & 1) ? -1 : 1;
+        const int parent = A * C.sI + B * C.sJ + D;
+        T acc = (T)0;
+#pragma unroll
         for (int di = 0; di < 2; di++)
+#pragma unroll
             for (int dj = 0; dj < 2; dj++)
-                for (int dk = 0; dk < nk; dk++)
+#pragma unroll
+                for (int dk = 0; dk < (k3D ? 2 : 1); dk++)
                 {
-                    const long long cc = parent + (long long)(di * si) * cv.sI + (long long)(dj * sj) * cv.sJ + dk * sk;
-                    const T w = wv[di] * wv[dj] * (fv.dim == 3 ? wv[dk] : (T)1);
-                    if ((di | dj | dk) && cv.types[cc] == SOLID) extra += w;
-                    else acc += w * C.e[cc];
+                    // e is zero at SOLID (and all other non-unknown) contributors
+                    const T w = wv[di] * wv[dj] * (k3D ? wv[dk] : (T)1);
+                    acc += w * C.e[parent + di * si + dj * sj + dk * sk];
                 }
-        F.e[c] += acc + extra * C.e[parent];
+        F.e[c] += acc + Moved(F, c) * C.e[parent];
     }
     PhaseSync<kWarp>();
 }
 
-// The descent through level l: the first sweep from zero, further sweeps, the residual and its restriction.
-template <typename T, bool kWarp>
+// The descent through level l: the sweeps from zero, the residual and its restriction.
+template <typename T, bool k3D, bool kSt, bool kWarp>
 __device__ void TDown(const SmemLevel<T> &F, const SmemLevel<T> &C, int pre)
 {
-    TSmooth<T, kWarp>(F, 0, true);
-    TSmooth<T, kWarp>(F, 1, false);
-    for (int s = 1; s < pre; s++)
-    {
-        TSmooth<T, kWarp>(F, 0, false);
-        TSmooth<T, kWarp>(F, 1, false);
-    }
-    TResidual<T, kWarp>(F);
-    TRestrict<T, kWarp>(F, C);
-}
-
-// The coarsest level: symmetric sweep pairs from zero.
-template <typename T, bool kWarp> __device__ void TCoarsest(const SmemLevel<T> &C, int sweeps)
-{
-    TSmooth<T, kWarp>(C, 0, true);
-    TSmooth<T, kWarp>(C, 1, false);
-    for (int s = 1; s < sweeps; s++)
-    {
-        TSmooth<T, kWarp>(C, 0, false);
-        TSmooth<T, kWarp>(C, 1, false);
-    }
-    for (int s = 0; s < sweeps; s++)
-    {
-        TSmooth<T, kWarp>(C, 1, false);
-        TSmooth<T, kWarp>(C, 0, false);
-    }
+    TSweeps<T, k3D, kSt, kWarp>(F, pre, 0, true, true);
+    TRestrict<T, k3D, kWarp>(F, C);
 }
 
 // The ascent into level l: the prolonged correction, then the post-sweeps black first.
-template <typename T, bool kWarp> __device__ void TUp(const SmemLevel<T> &F, const SmemLevel<T> &C, int post)
+template <typename T, bool k3D, bool kSt, bool kWarp>
+__device__ void TUp(const SmemLevel<T> &F, const SmemLevel<T> &C, int post)
 {
-    TProlong<T, kWarp>(F, C);
-    for (int s = 0; s < post; s++)
+    TProlong<T, k3D, kWarp>(F, C);
+    TSweeps<T, k3D, kSt, kWarp>(F, 0, post, false, false);
+}
+
+struct TailShared
+{
+    double inv[kMaxTailLevels][32]; // 1 / (gamma/2 * units), entry 0 = 0
+    int count[kMaxTailLevels][2];
+};
+
+// What a layout fixes, into shared memory, and zeroed vectors: nothing here depends on the launch before.
+template <typename T>
+__device__ __forceinline__ void TailStage(const TailArgs<T> &A, unsigned char *smem, TailShared &sh)
+{
+    for (int t = threadIdx.x; t < 32 * A.nlev; t += blockDim.x)
     {
-        TSmooth<T, kWarp>(F, 1, false);
-        TSmooth<T, kWarp>(F, 0, false);
+        const int l = t >> 5, u = t & 31;
+        sh.inv[l][u] = u ? 1.0 / (0.5 * A.lv[l].v.gamma * (double)u) : 0.0;
+        if (u < 2) sh.count[l][u] = A.counts[2 * l + u];
+    }
+    for (int l = 0; l < A.nlev; l++)
+    {
+        const SmemLevel<T> S = Bind<T>(A.lv[l], smem);
+        const unsigned a = Pad16((unsigned)(S.cells * sizeof(T)));
+        uint4 *z = reinterpret_cast<uint4 *>(S.r), *p = reinterpret_cast<uint4 *>(S.list);
+        const uint4 *g = reinterpret_cast<const uint4 *>(A.lists + A.lv[l].listOff);
+        for (unsigned t = threadIdx.x; t < 3 * a / 16; t += blockDim.x) z[t] = make_uint4(0, 0, 0, 0);
+        for (unsigned t = threadIdx.x; t < PrepBytes(S.cells) / 16; t += blockDim.x) p[t] = g[t];
     }
 }
 
-template <typename T> __device__ __forceinline__ void TailBody(const TailArgs<T> &A)
+template <typename T, bool k3D, bool kSt>
+__device__ __forceinline__ void TailBody(const TailArgs<T> &A, unsigned char *smem, const TailShared &sh)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ double sInv[kMaxTailLevels][32];
-    __shared__ int sCount[kMaxTailLevels][2];
-    // stage: cell types, codes and lists of every tail level, zero corrections and residuals, the first level's r
-    for (int l = 0; l < A.nlev; l++)
+    __syncthreads(); // the staged data; r of the first level overwrites its zeros
     {
-        const LevelView &g = A.lv[l].v;
-        const SmemLevel<T> S = Bind<T>(A.lv[l], smem);
-        const unsigned *gl = A.lists + A.lv[l].listOff;
-        for (long long c = threadIdx.x; c < g.cells; c += blockDim.x)
-        {
-            ((uint8_t *)S.v.code)[c] = g.code[c];
-            ((uint8_t *)S.v.types)[c] = g.types[c];
-            S.e[c] = (T)0;
-            S.res[c] = (T)0;
-            S.r[c] = l == 0 ? A.rIn[c] : (T)0;
-            S.list[c] = gl[c];
-        }
-        if (threadIdx.x < 32)
-            sInv[l][threadIdx.x] = threadIdx.x ? 1.0 / (0.5 * g.gamma * (double)threadIdx.x) : 0.0;
-        if (threadIdx.x < 2) sCount[l][threadIdx.x] = A.counts[2 * l + threadIdx.x];
-    }
-    __syncthreads();
-    // the diagonal half-units of the uniform levels' unknowns: 2 per FLUID neighbour, 2 per interior Dirichlet
-    // neighbour, 4 per Dirichlet ring neighbour (ring factor 2)
-    for (int l = 0; l < A.nlev; l++)
-    {
-        const SmemLevel<T> S = Bind<T>(A.lv[l], smem);
-        const LevelView &v = S.v;
-        if (v.stretched) continue;
-        const int nq = v.dim == 3 ? 6 : 4;
-        for (long long c = threadIdx.x; c < v.cells; c += blockDim.x)
-        {
-            const unsigned code = v.code[c];
-            unsigned units = 0;
-            if (code & CODE_UNKNOWN)
-            {
-                units = 2u * (unsigned)__popc(code & CODE_FLUID_MASK);
-                if (code & CODE_DIRICHLET)
-                {
-                    int i, j, k;
-                    Decode(v, c, i, j, k);
-                    for (int q = 0; q < nq; q++)
-                        if (IsDirichlet(v.types[c + NbrOffset(v, q)]))
-                        {
-                            const int ni = i + (q == 0) - (q == 1), nj = j + (q == 2) - (q == 3),
-                                      nk = k + (q == 4) - (q == 5);
-                            units += OnRing(v, ni, nj, nk) ? 4u : 2u;
-                        }
-                }
-                units |= 0x80u;
-            }
-            S.du[c] = (uint8_t)units;
-        }
+        const SmemLevel<T> F0 = Bind<T>(A.lv[0], smem);
+        for (int c = threadIdx.x; c < F0.cells; c += blockDim.x) F0.r[c] = A.rIn[c];
     }
     __syncthreads();
     auto lev = [&](int l) {
         SmemLevel<T> s = Bind<T>(A.lv[l], smem);
-        s.nRed = sCount[l][0];
-        s.nBlack = sCount[l][1];
-        s.inv = sInv[l];
+        s.nRed = sh.count[l][0];
+        s.nBlack = sh.count[l][1];
+        s.inv = sh.inv[l];
         return s;
     };
     const int last = A.nlev - 1;
     // wl: the first level from which every coarser one has at most 32 unknowns of each colour (warp 0 runs those)
     int wl = A.nlev;
-    for (int l = last; l >= 0 && sCount[l][0] <= 32 && sCount[l][1] <= 32; l--) wl = l;
+    for (int l = last; l >= 0 && sh.count[l][0] <= 32 && sh.count[l][1] <= 32; l--) wl = l;
     const int top = wl < last ? wl : last;
-    for (int l = 0; l < top; l++) TDown<T, false>(lev(l), lev(l + 1), A.pre);
-    if (wl > last) TCoarsest<T, false>(lev(last), A.coarseSweeps);
+    for (int l = 0; l < top; l++) TDown<T, k3D, kSt, false>(lev(l), lev(l + 1), A.pre);
+    // the coarsest level: symmetric sweep pairs from zero
+    if (wl > last) TSweeps<T, k3D, kSt, false>(lev(last), A.coarseSweeps, A.coarseSweeps, true, false);
     else
     {
         if (threadIdx.x < 32)
         {
-            for (int l = wl; l < last; l++) TDown<T, true>(lev(l), lev(l + 1), A.pre);
-            TCoarsest<T, true>(lev(last), A.coarseSweeps);
-            for (int l = last - 1; l >= wl; l--) TUp<T, true>(lev(l), lev(l + 1), A.post);
+            for (int l = wl; l < last; l++) TDown<T, k3D, kSt, true>(lev(l), lev(l + 1), A.pre);
+            TSweeps<T, k3D, kSt, true>(lev(last), A.coarseSweeps, A.coarseSweeps, true, false);
+            for (int l = last - 1; l >= wl; l--) TUp<T, k3D, kSt, true>(lev(l), lev(l + 1), A.post);
         }
         __syncthreads();
     }
-    for (int l = top - 1; l >= 0; l--) TUp<T, false>(lev(l), lev(l + 1), A.post);
+    for (int l = top - 1; l >= 0; l--) TUp<T, k3D, kSt, false>(lev(l), lev(l + 1), A.post);
     const SmemLevel<T> F0 = Bind<T>(A.lv[0], smem);
-    for (long long c = threadIdx.x; c < A.lv[0].v.cells; c += blockDim.x) A.eOut[c] = F0.e[c];
+    for (int c = threadIdx.x; c < F0.cells; c += blockDim.x) A.eOut[c] = F0.e[c];
 }
 
-template <typename T> __global__ void __launch_bounds__(kTailThreads) k_tail(TailArgs<T> A)
+template <typename T, bool k3D, bool kSt>
+__global__ void __launch_bounds__(kTailThreadsBig, 1) k_tail(const __grid_constant__ TailArgs<T> A)
 {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ TailShared sh;
+    TailStage<T>(A, smem, sh); // written when the layout was set: before any launch this one may overlap
     PdlWait();
     PdlTrigger();
-    TailBody<T>(A);
+    TailBody<T, k3D, kSt>(A, smem, sh);
 }
 
 // batched (nb_batch.cu): block z runs the coarse end of the request at list[z], its arguments copied from global
 // memory into shared memory first
-__global__ void __launch_bounds__(kTailThreads) kb_tail(const BatchReq *__restrict__ rq, BatchList a)
+__global__ void __launch_bounds__(kTailThreadsBig) kb_tail(const BatchReq *__restrict__ rq, BatchList a)
 {
+    extern __shared__ __align__(16) unsigned char smem[];
     PdlWait();
     PdlTrigger();
     const int q = BatchReqOf(a);
@@ -444,12 +475,13 @@ __global__ void __launch_bounds__(kTailThreads) kb_tail(const BatchReq *__restri
         for (int t = threadIdx.x; t < n; t += blockDim.x) dst[t] = src[t];
     }
     __syncthreads();
-    TailBody<float>(sA);
+    __shared__ TailShared sh;
+    TailStage<float>(sA, smem, sh);
+    TailBody<float, true, false>(sA, smem, sh); // batches are uniform 3D
 }
 
-// The per-colour lists of every tail level's unknowns, once per layout: entries packed (i << 20 | j << 10 | k), red
-// ones from the front of the level's segment, black ones from the back; their order within a colour does not matter
-// (the cells of one colour are updated independently).
+// Every tail level's prepared data, once per layout; the lists' order within a colour does not matter (the cells of one
+// colour are updated independently).
 __global__ void __launch_bounds__(1024) k_tail_lists(TailArgs<float> A)
 {
     __shared__ int cnt[kMaxTailLevels][2];
@@ -458,17 +490,55 @@ __global__ void __launch_bounds__(1024) k_tail_lists(TailArgs<float> A)
     for (int l = 0; l < A.nlev; l++)
     {
         const LevelView &g = A.lv[l].v;
+        const int cells = (int)g.cells, nq = g.dim == 3 ? 6 : 4;
         unsigned *list = const_cast<unsigned *>(A.lists) + A.lv[l].listOff;
-        for (long long c = threadIdx.x; c < g.cells; c += blockDim.x)
+        uint8_t *unit = (uint8_t *)list + Pad16((unsigned)cells * 4u), *ext = unit + Pad16((unsigned)cells);
+        uint8_t *types = ext + Pad16((unsigned)cells);
+        for (int c = threadIdx.x; c < cells; c += blockDim.x)
         {
-            if (!(g.code[c] & CODE_UNKNOWN)) continue;
-            int i, j, k;
-            Decode(g, c, i, j, k);
+            const unsigned code = g.code[c];
+            unit[c] = g.stretched ? (uint8_t)code : (uint8_t)0;
+            ext[c] = 0;
+            types[c] = g.stretched ? g.types[c] : (uint8_t)0;
+            if (!(code & CODE_UNKNOWN)) continue;
+            const int k = c % g.Nz, rr = c / g.Nz, j = rr % g.Nx, i = rr / g.Nx;
             const int col = (i + j + k) & 1;
             const int pos = atomicAdd(&cnt[l][col], 1);
             const unsigned packed = ((unsigned)i << 20) | ((unsigned)j << 10) | (unsigned)k;
             if (col == 0) list[pos] = packed;
-            else list[g.cells - 1 - pos] = packed;
+            else list[cells - 1 - pos] = packed;
+            if (!g.stretched)
+            {
+                // half-units of the diagonal: 2 per FLUID neighbour, 2 per interior Dirichlet neighbour, 4 per
+                // Dirichlet ring neighbour (ring factor 2)
+                unsigned units = 2u * (unsigned)__popc(code & CODE_FLUID_MASK);
+                if (code & CODE_DIRICHLET)
+                    for (int q = 0; q < nq; q++)
+                        if (IsDirichlet(g.types[c + NbrOffset(g, q)]))
+                        {
+                            const int ni = i + (q == 0) - (q == 1), nj = j + (q == 2) - (q == 3),
+                                      nk = k + (q == 4) - (q == 5);
+                            units += OnRing(g, ni, nj, nk) ? 4u : 2u;
+                        }
+                unit[c] = (uint8_t)(0x80u | units);
+            }
+            if (l + 1 < A.nlev)
+            {
+                // the trilinear (2D: bilinear) weights of the SOLID contributors, in 64ths
+                const LevelView &cv = A.lv[l + 1].v;
+                const bool d3 = g.dim == 3;
+                const int si = (i & 1) ? -1 : 1, sj = (j & 1) ? -1 : 1, sk = (k & 1) ? -1 : 1;
+                const long long parent = (long long)((i + 1) >> 1) * cv.sI + (long long)((j + 1) >> 1) * cv.sJ +
+                                         (d3 ? (k + 1) >> 1 : 0);
+                unsigned extra = 0;
+                for (int q = 1; q < (d3 ? 8 : 4); q++)
+                {
+                    const int di = q & 1, dj = (q >> 1) & 1, dk = q >> 2;
+                    if (cv.types[parent + (long long)(di * si) * cv.sI + (long long)(dj * sj) * cv.sJ + dk * sk] == SOLID)
+                        extra += (di ? 1u : 3u) * (dj ? 1u : 3u) * (d3 ? (dk ? 1u : 3u) : 4u);
+                }
+                ext[c] = (uint8_t)(0x80u | extra);
+            }
         }
     }
     __syncthreads();
@@ -478,21 +548,30 @@ __global__ void __launch_bounds__(1024) k_tail_lists(TailArgs<float> A)
 long long TailListEntries(const LevelView *levels, int nlev)
 {
     long long n = 0;
-    for (int l = 0; l < nlev; l++) n += levels[l].cells;
+    for (int l = 0; l < nlev; l++) n += PrepBytes(levels[l].cells) / 4;
     return n;
+}
+
+// the levels' places in shared memory and in the prepared data; returns the shared memory's bytes
+template <typename T> static unsigned PlaceLevels(TailArgs<T> &A, const LevelView *levels, int nlev)
+{
+    unsigned off = 0, listOff = 0;
+    for (int l = 0; l < nlev; l++)
+    {
+        A.lv[l].v = levels[l];
+        A.lv[l].off = off;
+        A.lv[l].listOff = listOff;
+        off += LevelBytes<T>(levels[l].cells);
+        listOff += PrepBytes(levels[l].cells) / 4;
+    }
+    A.nlev = nlev;
+    return off;
 }
 
 void LaunchTailLists(const LevelView *levels, int nlev, unsigned *lists, int *counts, cudaStream_t st)
 {
     TailArgs<float> A{};
-    unsigned off = 0;
-    for (int l = 0; l < nlev; l++)
-    {
-        A.lv[l].v = levels[l];
-        A.lv[l].listOff = off;
-        off += (unsigned)levels[l].cells;
-    }
-    A.nlev = nlev;
+    PlaceLevels(A, levels, nlev);
     A.lists = lists;
     A.counts = counts;
     NB_COUNT_LAUNCH();
@@ -508,11 +587,12 @@ template <typename T> size_t TailSmemBytes(const LevelView *levels, int nlev)
 
 template <typename T> static bool PrepareTailOnce()
 {
-    if (sizeof(T) == 4 &&
-        cudaFuncSetAttribute(kb_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailMaxSmem) != cudaSuccess)
-        return false;
-    return cudaFuncSetAttribute(k_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailMaxSmem) ==
-           cudaSuccess;
+    auto ok = [](const void *f) {
+        return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailMaxSmem) == cudaSuccess;
+    };
+    if (sizeof(T) == 4 && !ok((const void *)kb_tail)) return false;
+    return ok((const void *)k_tail<T, false, false>) && ok((const void *)k_tail<T, false, true>) &&
+           ok((const void *)k_tail<T, true, false>) && ok((const void *)k_tail<T, true, true>);
 }
 
 // Once per device and precision: changing a kernel's attribute on every layout change would take the driver's
@@ -537,16 +617,7 @@ void TailArgsFor(const LevelView *levels, int nlev, const float *rIn, float *eOu
                  int coarseSweeps, const unsigned *lists, const int *counts, void *out, size_t *bytes, size_t *smem)
 {
     TailArgs<float> A{};
-    unsigned off = 0, listOff = 0;
-    for (int l = 0; l < nlev; l++)
-    {
-        A.lv[l].v = levels[l];
-        A.lv[l].off = off;
-        A.lv[l].listOff = listOff;
-        off += LevelBytes<float>(levels[l].cells);
-        listOff += (unsigned)levels[l].cells;
-    }
-    A.nlev = nlev;
+    const unsigned off = PlaceLevels(A, levels, nlev);
     A.rIn = rIn;
     A.eOut = eOut;
     A.pre = pre < 1 ? 1 : pre;
@@ -570,16 +641,7 @@ void LaunchTail(const LevelView *levels, int nlev, const T *rIn, T *eOut, int pr
                 const unsigned *lists, const int *counts, cudaStream_t st)
 {
     TailArgs<T> A{};
-    unsigned off = 0, listOff = 0;
-    for (int l = 0; l < nlev; l++)
-    {
-        A.lv[l].v = levels[l];
-        A.lv[l].off = off;
-        A.lv[l].listOff = listOff;
-        off += LevelBytes<T>(levels[l].cells);
-        listOff += (unsigned)levels[l].cells;
-    }
-    A.nlev = nlev;
+    const unsigned off = PlaceLevels(A, levels, nlev);
     A.rIn = rIn;
     A.eOut = eOut;
     A.pre = pre < 1 ? 1 : pre;
@@ -587,8 +649,16 @@ void LaunchTail(const LevelView *levels, int nlev, const T *rIn, T *eOut, int pr
     A.coarseSweeps = coarseSweeps < 1 ? 1 : coarseSweeps;
     A.lists = lists;
     A.counts = counts;
+    const dim3 threads(levels[0].cells > 4 * kTailThreads ? kTailThreadsBig : kTailThreads);
     NB_COUNT_LAUNCH();
-    LaunchPdl(k_tail<T>, dim3(1), dim3(kTailThreads), (size_t)off, st, A);
+    if (levels[0].dim == 3 && !levels[0].stretched)
+        LaunchPdl(k_tail<T, true, false>, dim3(1), threads, (size_t)off, st, A);
+    else if (levels[0].dim == 3)
+        LaunchPdl(k_tail<T, true, true>, dim3(1), threads, (size_t)off, st, A);
+    else if (!levels[0].stretched)
+        LaunchPdl(k_tail<T, false, false>, dim3(1), threads, (size_t)off, st, A);
+    else
+        LaunchPdl(k_tail<T, false, true>, dim3(1), threads, (size_t)off, st, A);
 }
 
 template size_t TailSmemBytes<float>(const LevelView *, int);
