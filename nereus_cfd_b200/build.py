@@ -27,6 +27,7 @@ SOURCES = {
     "nb_pairs.cu": [],
     "nb_split.cu": [],
     "nb_stretched.cu": [],
+    "nb_legs.cu": [],
     "nb_solver.cu": [],
     "nb_capi.cu": [],
     "nb_noalloc.cu": [],

@@ -169,6 +169,19 @@ void LaunchSplitRefine64(const LevelView &v, const uint8_t *du, const double *b,
                          double *xout, T *r, double scale, double sfac, const Reducer &R, int slot,
                          cudaStream_t st, const int *swap = nullptr);
 
+// ---- nb_legs.cu: a small uniform colour-split level's descent and ascent in one launch each (one sweep before and after
+//      the coarse correction); tmp: a vector of the level other than e; Dot: the CG sums of level 0 ----
+template <typename T>
+void LaunchLegDown(const LevelView &v, const LevelView &cv, const uint8_t *du, const uint8_t *pext, const T *r, T *tmp,
+                   T *rc, cudaStream_t st);
+template <typename T>
+void LaunchLegUp(const LevelView &v, const LevelView &cv, const uint8_t *du, const uint8_t *pext, const T *r,
+                 const T *tmp, const T *ec, T *e, cudaStream_t st);
+template <typename T>
+void LaunchLegUpDot(const LevelView &v, const LevelView &cv, const uint8_t *du, const uint8_t *pext, const T *r,
+                    const T *tmp, const T *ec, T *e, const Reducer &R, const int *it, int baseEven, int baseOdd,
+                    cudaStream_t st);
+
 // ---- nb_stretched.cu: the FP64 sweeps of a stretched 3D level in the colour-split layout (LevelView::dg, idg) ----
 void PrepareStretchedKernels();
 void LaunchStretchedDiag(const LevelView &v, double *dg, double *idg, cudaStream_t st);

@@ -1033,6 +1033,24 @@ template <typename T> void Context::VCycleSplit(int l, T *r, T *e)
     // one colour: reads the other colour, and r and the bytes of its own; writes its own
     const double half = (3.0 * s + 1.0) / 2.0;
     const uint8_t *du = Lv.du.p;
+    if (Legs(l))
+    {
+        LevelData &Lc = L[l + 1];
+        const LevelView vc = Lc.view();
+        T *tmp = Lv.res<T>();
+        prof(NB_K_SMOOTH0, 2.0 * s + 1.0 + s / 8.0); // reads r and the bytes, writes the iterate and the coarse r
+        LaunchLegDown<T>(v, vc, du, Lv.pext.p, r, tmp, Lc.r<T>(), st);
+        ProfEnd();
+        if (l == 0) CoarseBracket<T>(l + 1, Lc.r<T>(), Lc.e<T>());
+        else VCycle<T>(l + 1, Lc.r<T>(), Lc.e<T>());
+        prof(NB_K_PROLONG0, 2.5 * s + 1.5 + s / 8.0); // reads the red iterate, r, the bytes and the coarse e, writes e
+        if (l == 0)
+            LaunchLegUpDot<T>(v, vc, du, Lv.pext.p, r, tmp, Lc.e<T>(), e, red, iter.p, S_RZ0, S_RZ1, st);
+        else
+            LaunchLegUp<T>(v, vc, du, Lv.pext.p, r, tmp, Lc.e<T>(), e, st);
+        ProfEnd();
+        return;
+    }
     prof(NB_K_SMOOTH0, 2.0 * s + 1.0); // reads r and the bytes, writes e
     LaunchSplitFirst(v, du, r, e, st);
     ProfEnd();

@@ -411,6 +411,13 @@ struct Context
     bool PairLevel(int l) const { return opt.pair_kernels && L[l].du.p != nullptr; }
     // the solver's vectors of this level are colour-split and its V-cycle runs the split kernels
     bool Split(int l) const { return L[l].sRS != 0; }
+    // Levels of at most this many cells run their legs in one launch each: measured faster on 66^3 and below, slower on
+    // 130^3 (nb_legs.cu)
+    static constexpr long long kLegCells = 300000;
+    bool Legs(int l) const
+    {
+        return Split(l) && !L[l].stretched && L[l].cells <= kLegCells && PreSweeps(l) == 1 && PostSweeps(l) == 1;
+    }
     // elements of a level-0 solver vector (the split layout pads its rows)
     size_t VecLen0() const { return L[0].VecLen(); }
     void VCyclePairs(int l, float *r, float *e);

@@ -209,14 +209,17 @@ def solve_family(case, types, family, precision, closed, tol=1e-12, **options):
 FP64_SIZES = [(12, 12, 12), (14, 13, 16), (16, 16, 14), (30, 36, 26), (33, 40, 48), (64, 20, 34)]
 
 
+# sweeps: small levels run one launch per leg with one sweep, and a launch per operation with two
+@pytest.mark.parametrize("sweeps", [1, 2])
 @pytest.mark.parametrize("closed", [False, True])
 @pytest.mark.parametrize("size", FP64_SIZES)
-def test_fp64_split_agrees_with_per_cell_kernels(nb, size, closed):
+def test_fp64_split_agrees_with_per_cell_kernels(nb, size, closed, sweeps):
     """The plain FP64 form on the colour-split layout against its per-cell kernels (pair_kernels = 0), both to 1e-12.
     Each solution is within cond * 1e-12 of the exact one; cond <= 5 N^2 on N cells along the longest side (the lowest
     mode a quarter wave), so the two agree within 1e-11 N^2."""
     case, types = sphere_case(size, closed)
-    a, b = [solve_family(case, types, family, "fp64", closed) for family in (2, 0)]
+    a, b = [solve_family(case, types, family, "fp64", closed, pre_sweeps=sweeps, post_sweeps=sweeps)
+            for family in (2, 0)]
     bar = 1e-11 * max(size) ** 2
     for x, y in ((a.p, b.p), (a.u, b.u), (a.v, b.v), (a.w, b.w)):
         assert np.linalg.norm(x - y) <= bar * np.linalg.norm(y)
@@ -227,14 +230,16 @@ def test_fp64_split_agrees_with_per_cell_kernels(nb, size, closed):
 ODD_SIZES = [(12, 12, 9), (16, 13, 15), (17, 15, 17), (24, 31, 33), (33, 40, 47), (20, 20, 38), (28, 36, 50)]
 
 
+@pytest.mark.parametrize("sweeps", [1, 2])
 @pytest.mark.parametrize("precision", ["mixed", "fp64"])
 @pytest.mark.parametrize("size", ODD_SIZES)
-def test_odd_rows_agree_with_per_cell_kernels(nb, size, precision):
+def test_odd_rows_agree_with_per_cell_kernels(nb, size, precision, sweeps):
     """The colour-split layout on grids and levels of odd Nz against the per-cell kernels, closed and with an outlet,
     all to 1e-12 (the bar of test_fp64_split_agrees_with_per_cell_kernels)."""
     for closed in (False, True):
         case, types = sphere_case(size, closed)
-        a, b = [solve_family(case, types, family, precision, closed) for family in (2, 0)]
+        a, b = [solve_family(case, types, family, precision, closed, pre_sweeps=sweeps, post_sweeps=sweeps)
+                for family in (2, 0)]
         bar = 1e-11 * max(size) ** 2
         for x, y in ((a.p, b.p), (a.u, b.u), (a.v, b.v), (a.w, b.w)):
             assert np.linalg.norm(x - y) <= bar * np.linalg.norm(y)
