@@ -77,7 +77,8 @@ typedef struct nb_options
                             arrays, so that one colour's sweep moves half the bytes (uniform levels in both
                             precisions, stretched ones in FP64); 1: the mixed form's cell pairs in the grid layout
                             (Nz even, uniform or stretched; also what 2 gives on its stretched levels); 0: the
-                            general per-cell kernels */
+                            general per-cell kernels. 2D levels: 2 (with one or two sweeps): a launch per leg of the
+                            V-cycle; else the per-cell kernels */
     int tail_cells;      /* the coarse end runs in one thread block from the first level with at most this many
                             cells (and shared memory for all of them); 0: no such block */
     int stretched_sweeps; /* red-black sweeps before and after the coarse correction on a stretched grid's levels

@@ -28,6 +28,7 @@ SOURCES = {
     "nb_split.cu": [],
     "nb_stretched.cu": [],
     "nb_legs.cu": [],
+    "nb_legs2d.cu": [],
     "nb_solver.cu": [],
     "nb_capi.cu": [],
     "nb_noalloc.cu": [],

@@ -7,6 +7,8 @@
 
 #include <cub/device/device_scan.cuh>
 
+#include <algorithm>
+
 namespace nb
 {
 
@@ -766,6 +768,63 @@ __device__ __forceinline__ void RingEntry(const LevelView &v, double *p, long lo
     else if (t != PRESSURE) p[d] = p[s];
 }
 
+// What the passes below leave on ring cell (i, j, k), in one launch: the last pass whose face holds the cell decides
+// (0 at EMPTY, kept at PRESSURE), else it copies inward along that axis a cell that the earlier passes decide in turn.
+// Only ring cells that are not PRESSURE are written and only PRESSURE and interior cells are read, so no order between
+// threads matters. A step replays the ring twice or three times; each replay took two or three launches.
+__device__ __forceinline__ double RingValue(const LevelView &v, const double *p, int i, int j, int k)
+{
+    while (true)
+    {
+        const long long c = (long long)i * v.sI + (long long)j * v.sJ + k;
+        const bool onZ = v.dim == 3 && (k == 0 || k == v.Nz - 1), onX = j == 0 || j == v.Nx - 1;
+        if (!onZ && !onX && i > 0 && i < v.Ny - 1) return p[c];
+        const int t = v.types[c];
+        if (t == EMPTY) return 0.0;
+        if (t == PRESSURE) return p[c];
+        if (onZ) k = k == 0 ? 1 : v.Nz - 2;
+        else if (onX) j = j == 0 ? 1 : v.Nx - 2;
+        else i = i == 0 ? 1 : v.Ny - 2;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_ring_once(LevelView v, double *p)
+{
+    const int Nx = v.Nx, Ny = v.Ny, Nz = v.Nz;
+    // the y faces whole, the x faces without them, the z faces without either
+    const long long nY = 2LL * Nx * Nz, nX = 2LL * (Ny - 2) * Nz, nZ = v.dim == 3 ? 2LL * (Ny - 2) * (Nx - 2) : 0;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nY + nX + nZ;
+         t += (long long)gridDim.x * blockDim.x)
+    {
+        int i, j, k;
+        if (t < nY)
+        {
+            const int s = t >= nY / 2, q = (int)(t - (s ? nY / 2 : 0));
+            i = s ? Ny - 1 : 0;
+            j = q / Nz;
+            k = q - j * Nz;
+        }
+        else if (t < nY + nX)
+        {
+            const long long u = t - nY;
+            const int s = u >= nX / 2, q = (int)(u - (s ? nX / 2 : 0));
+            i = 1 + q / Nz;
+            j = s ? Nx - 1 : 0;
+            k = q - (i - 1) * Nz;
+        }
+        else
+        {
+            const long long u = t - nY - nX;
+            const int s = u >= nZ / 2, q = (int)(u - (s ? nZ / 2 : 0));
+            i = 1 + q / (Nx - 2);
+            j = 1 + q - (i - 1) * (Nx - 2);
+            k = s ? Nz - 1 : 0;
+        }
+        const long long c = (long long)i * v.sI + (long long)j * v.sJ + k;
+        if (v.types[c] != PRESSURE) p[c] = RingValue(v, p, i, j, k);
+    }
+}
+
 // pass 0: y faces (i = 0, Ny-1) over (j, k); pass 1: x faces (j = 0, Nx-1) over (i, k); pass 2: z faces over (i, j)
 __global__ void k_ring(LevelView v, double *p, int pass)
 {
@@ -800,6 +859,14 @@ __global__ void k_ring(LevelView v, double *p, int pass)
 void LaunchRing(const LevelView &v, double *p, cudaStream_t st)
 {
     const int passes = v.dim == 3 ? 3 : 2;
+    if (v.Nx >= 3 && v.Ny >= 3 && (v.dim == 2 || v.Nz >= 3))
+    {
+        const long long n = 2LL * v.Nx * v.Nz + 2LL * v.Ny * v.Nz + (v.dim == 3 ? 2LL * v.Ny * v.Nx : 0);
+        NB_COUNT_LAUNCH();
+        k_ring_once<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, st>>>(v, p);
+        return;
+    }
+    // a side without interior cells: a face's inward cell is the other face's, and the passes' order counts
     for (int pass = 0; pass < passes; pass++)
     {
         const long long A = pass == 0 ? v.Nx : v.Ny;

@@ -630,6 +630,8 @@ __global__ void __launch_bounds__(256) k_update_p_apply(LevelView v, const T *__
                                                         T *__restrict__ q, Reducer R, const double *S, const int *it,
                                                         int baseEven, int baseOdd, int slotN, int singular, int slotPQ)
 {
+    PdlWait();
+    PdlTrigger();
     const int iter = *it, par = iter & 1;
     const T *__restrict__ pIn = par ? p1 : p0;
     T *__restrict__ pOut = par ? p0 : p1;
@@ -684,11 +686,11 @@ void LaunchUpdatePApply(const LevelView &v, const T *z, T *p0, T *p1, T *q, cons
 {
     NB_COUNT_LAUNCH();
     if (exact)
-        k_update_p_apply<T, true><<<TileGrid(v), kTile, 0, st>>>(v, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN,
-                                                                 singular, slotPQ);
+        LaunchPdl(k_update_p_apply<T, true>, TileGrid(v), kTile, 0, st, v, z, p0, p1, q, R, S, it, baseEven, baseOdd,
+                  slotN, singular, slotPQ);
     else
-        k_update_p_apply<T, false><<<TileGrid(v), kTile, 0, st>>>(v, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN,
-                                                                  singular, slotPQ);
+        LaunchPdl(k_update_p_apply<T, false>, TileGrid(v), kTile, 0, st, v, z, p0, p1, q, R, S, it, baseEven, baseOdd,
+                  slotN, singular, slotPQ);
 }
 
 // alpha = rz/pq; x += alpha p_new; r -= alpha q; sum r.r. The last block advances the iteration counter.

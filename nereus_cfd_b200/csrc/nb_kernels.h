@@ -182,6 +182,17 @@ void LaunchLegUpDot(const LevelView &v, const LevelView &cv, const uint8_t *du, 
                     const T *tmp, const T *ec, T *e, const Reducer &R, const int *it, int baseEven, int baseOdd,
                     cudaStream_t st);
 
+// ---- nb_legs2d.cu: a 2D level's descent and ascent in one launch each (1 or 2 sweeps before and after the coarse
+//      correction); ext: the moved transfer weights, with the diagonal and its reciprocal built once per layout ----
+void LaunchBuild2D(const LevelView &v, const LevelView &cv, double *dg, double *idg, uint8_t *ext, cudaStream_t st);
+template <typename T>
+void LaunchLeg2Down(const LevelView &v, const LevelView &cv, const uint8_t *ext, const T *r, T *tmp, T *rc, int sweeps,
+                    cudaStream_t st);
+template <typename T>
+void LaunchLeg2Up(const LevelView &v, const LevelView &cv, const uint8_t *ext, const T *r, const T *tmp, const T *ec,
+                  T *e, int sweeps, bool dot, const Reducer &R, const int *it, int baseEven, int baseOdd,
+                  cudaStream_t st);
+
 // ---- nb_stretched.cu: the FP64 sweeps of a stretched 3D level in the colour-split layout (LevelView::dg, idg) ----
 void PrepareStretchedKernels();
 void LaunchStretchedDiag(const LevelView &v, double *dg, double *idg, cudaStream_t st);

@@ -1108,8 +1108,9 @@ void LaunchLinXR(long long cells, T *x, T *r, const T *p0, const T *p1, const T 
                  const double *S, int *it, int baseEven, int baseOdd, int slotN, int singular, int slotPQ, int slotRR,
                  cudaStream_t st)
 {
+    const long long quads = cells * (long long)sizeof(T) / 16, want = (quads + 255) / 256;
     NB_COUNT_LAUNCH();
-    LaunchPdl(k_lin_xr<T>, dim3(kLinBlocks), dim3(256), 0, st, cells, x, r, p0, p1, q, R, S, it, baseEven, baseOdd,
+    LaunchPdl(k_lin_xr<T>, dim3((unsigned)(want < 1 ? 1 : std::min<long long>(want, kLinBlocks))), dim3(256), 0, st, cells, x, r, p0, p1, q, R, S, it, baseEven, baseOdd,
               slotN, singular, slotPQ, slotRR);
 }
 
@@ -1123,11 +1124,14 @@ void LaunchSplitLinXR(const LevelView &v, long long vecLen, T *x, T *r, const T 
         LaunchLinXR<T>(vecLen, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, st);
         return;
     }
+    // no more blocks than tiles: on a 66^3 level the last block had 1184 partial sums to add for 396 tiles
     NB_COUNT_LAUNCH();
-    LaunchPdl(k_lin_xr_tiles<T>, dim3(kLinBlocks), dim3(256), 0, st, v, x, r, p0, p1, q, R, S, it, baseEven, baseOdd,
+    LaunchPdl(k_lin_xr_tiles<T>, dim3((unsigned)std::min(2 * v.Ny * v.actTiles, kLinBlocks)), dim3(256), 0, st, v, x, r, p0, p1, q, R, S, it, baseEven, baseOdd,
               slotN, singular, slotPQ, slotRR);
 }
 
+template void LaunchLinXR<double>(long long, double *, double *, const double *, const double *, const double *,
+                                  const Reducer &, const double *, int *, int, int, int, int, int, int, cudaStream_t);
 template void LaunchLinXR<float>(long long, float *, float *, const float *, const float *, const float *,
                                  const Reducer &, const double *, int *, int, int, int, int, int, int, cudaStream_t);
 template void LaunchSplitLinXR<float>(const LevelView &, long long, float *, float *, const float *, const float *,

@@ -444,7 +444,15 @@ void Context::BuildPairData()
     }
     for (size_t l = 0; l < L.size(); l++)
     {
-        if (L[l].du.p && l + 1 < L.size())
+        if (Legs2D((int)l))
+        {
+            const size_t c = (size_t)L[l].cells;
+            L[l].diag.alloc(c);
+            L[l].rdiag.alloc(c);
+            L[l].pext.alloc(c);
+            LaunchBuild2D(L[l].view(), L[l + 1].view(), L[l].diag.p, L[l].rdiag.p, L[l].pext.p, st);
+        }
+        else if (L[l].du.p && l + 1 < L.size())
         {
             if (L[l].sRS)
             {
@@ -896,6 +904,21 @@ template <typename T> void Context::VCycle(int l, T *r, T *e)
         VCycleSplit<T>(l, r, e);
         return;
     }
+    if (Legs2D(l))
+    {
+        LevelData &Lc = L[l + 1];
+        const LevelView vc = Lc.view();
+        prof(NB_K_SMOOTH0, 2.0 * s + 8.0 + s / 4.0); // reads r and the reciprocals, writes the iterate and the coarse r
+        LaunchLeg2Down<T>(v, vc, Lv.pext.p, r, Lv.res<T>(), Lc.r<T>(), PreSweeps(l), st);
+        ProfEnd();
+        if (l == 0) CoarseBracket<T>(l + 1, Lc.r<T>(), Lc.e<T>());
+        else VCycle<T>(l + 1, Lc.r<T>(), Lc.e<T>());
+        prof(NB_K_PROLONG0, 3.0 * s + 9.0 + s / 4.0); // reads the iterate, r, the reciprocals and bytes, writes e
+        LaunchLeg2Up<T>(v, vc, Lv.pext.p, r, Lv.res<T>(), Lc.e<T>(), e, PostSweeps(l), l == 0, red, iter.p, S_RZ0, S_RZ1,
+                        st);
+        ProfEnd();
+        return;
+    }
     if constexpr (std::is_same<T, float>::value)
     {
         if (PairLevel(l))
@@ -1132,14 +1155,19 @@ template <typename T> void Context::IterBody(T *x, T *r, T *z, T *p0, T *p1, T *
             return;
         }
     }
-    ProfBegin(NB_K_DOT, 2.0 * s * cells);
-    LaunchDot<T>(v0, r, z, red, iter.p, S_RZ0, S_RZ1, st);
-    ProfEnd();
+    if (!Legs2D(0)) // there r.z came with the V-cycle's last sweep
+    {
+        ProfBegin(NB_K_DOT, 2.0 * s * cells);
+        LaunchDot<T>(v0, r, z, red, iter.p, S_RZ0, S_RZ1, st);
+        ProfEnd();
+    }
     ProfBegin(NB_K_PAPPLY, (4.0 * s + 1.0) * cells);
     LaunchUpdatePApply<T>(v0, z, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, exact ? 1 : 0, st);
     ProfEnd();
     ProfBegin(NB_K_XR, 6.0 * s * cells);
-    LaunchUpdateXR<T>(v0, x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, S_RR, st);
+    if (Legs2D(0))
+        LaunchLinXR<T>(L[0].cells, x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, S_RR, st);
+    else LaunchUpdateXR<T>(v0, x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, S_RR, st);
     ProfEnd();
     if (copyRR) NB_CK(cudaMemcpyAsync(hostSlots + S_RR, slots.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, st));
 }

@@ -200,7 +200,7 @@ struct LevelData
                                           // Colour-split level: in that layout, and the codes on a stretched level
     DevArray<uint8_t> pext;               // unknown flag + moved prolongation weight toward the next coarser level
                                           // (colour-split level: the red cells only)
-    DevArray<double> diag, rdiag;         // stretched colour-split level (FP64): LevelView::dg, idg
+    DevArray<double> diag, rdiag;         // stretched colour-split level (FP64), 2D level: LevelView::dg, idg
     DevArray<uint8_t> act;                // colour-split level: which (plane, tile) holds an unknown (LevelView::act)
     int actTiles = 0;
     // the colour-split layout of the solver's vectors (nb_split.cu); sRS = 0: the grid layout
@@ -417,6 +417,12 @@ struct Context
     bool Legs(int l) const
     {
         return Split(l) && !L[l].stretched && L[l].cells <= kLegCells && PreSweeps(l) == 1 && PostSweeps(l) == 1;
+    }
+    // a 2D level above the coarse end whose legs run in one launch each (nb_legs2d.cu)
+    bool Legs2D(int l) const
+    {
+        return opt.pair_kernels == 2 && L[l].dim == 2 && l < tailStart && l + 1 < (int)L.size() &&
+               PreSweeps(l) <= 2 && PostSweeps(l) == PreSweeps(l);
     }
     // elements of a level-0 solver vector (the split layout pads its rows)
     size_t VecLen0() const { return L[0].VecLen(); }

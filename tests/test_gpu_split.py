@@ -268,3 +268,79 @@ def test_stretched_fp64_agrees_with_per_cell_kernels(nb, size, groups):
     bar = 2.0 * top / low * 1e-12
     idp = types.reshape(-1) == W.FLUID
     assert np.linalg.norm((a.p - b.p)[idp]) <= bar * np.linalg.norm(b.p[idp])
+
+
+# 2D: (interior x, y) around the 32 x 16 cells a block of the legs owns; one level above the coarse end and several
+@pytest.mark.parametrize("sweeps", [1, 2, 3])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("size", [(20, 20), (31, 33), (32, 48), (33, 65), (64, 50), (97, 80)])
+def test_2d_legs_agree_with_per_cell_kernels(nb, size, precision, sweeps):
+    """2D levels with a launch per leg (pair_kernels = 2 and up to two sweeps) against a launch per operation, closed and
+    with an outlet, all to 1e-12 (the bar of test_fp64_split_agrees_with_per_cell_kernels)."""
+    nx, ny = size
+    h = 1.0 / min(size)
+    g = W.uniform_grid(2, (0.0, nx * h, 0.0, ny * h, 0.0, 1.0), min(size))
+    assert (g.Nx, g.Ny) == (nx + 2, ny + 2)
+    disc = W.Region(W.REGION_SOLID, W.PRIM_CYLINDER, (0.4 * nx * h, 0.5 * ny * h, 0.0), radius=0.2)
+    for closed in (False, True):
+        case = W.Case("disc", g, W.walls_scene(2, outlet_face=None if closed else 1, regions=[disc]), 37,
+                      needs_compat=closed)
+        types = capi.label_cells(g, case.scene)
+        a, b = [solve_family(case, types, family, precision, closed, pre_sweeps=sweeps, post_sweeps=sweeps,
+                             tail_cells=128) for family in (2, 0)]
+        bar = 1e-11 * max(size) ** 2
+        for x, y in ((a.p, b.p), (a.u, b.u), (a.v, b.v)):
+            assert np.linalg.norm(x - y) <= bar * np.linalg.norm(y)
+
+
+@pytest.mark.parametrize("sweeps", [1, 2, 3])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("size", [(40, 24), (65, 33)])
+def test_2d_stretched_legs_agree_with_per_cell_kernels(nb, size, precision, sweeps):
+    """The same on the stretched channel; each solution within cond(A) 1e-11 of the exact one."""
+    import scipy.sparse as sp
+    import scipy.sparse.linalg as sl
+
+    case = W.channel_2d_stretched(*size)
+    types = capi.label_cells(case.grid, case.scene)
+    a, b = [solve_family(case, types, family, precision, False, tol=1e-11, stretched_sweeps=sweeps, tail_cells=128)
+            for family in (2, 0)]
+    s = PressureSolver("fp64")
+    s.InitializePressureSolver(b)
+    rowptr, col, val, _ = s.ExportMatrix()
+    s.DestroyPressureSolver()
+    A = -sp.csr_matrix((val, col, rowptr))
+    top = sl.eigsh(A, k=1, which="LA", return_eigenvectors=False, tol=1e-3)[0]
+    low = sl.eigsh(A.tocsc(), k=1, sigma=0.0, return_eigenvectors=False)[0]
+    assert np.linalg.norm(a.p - b.p) <= 2.0 * top / low * 1e-11 * np.linalg.norm(b.p)
+
+
+@pytest.mark.parametrize("shape", [(3, 3, 3), (5, 4, 7), (9, 12, 6), (2, 5, 4), (5, 2, 4), (6, 5, 2), (7, 6, 1), (3, 2, 1)])
+def test_pressure_ring_replay(nb, shape):
+    """EnforcePressureBC's passes (y, x, then z faces; EMPTY 0, PRESSURE kept, any other ring cell copies inward) on
+    random ring labels: on a grid without unknowns the step only replays the ring. Exact; the last shapes have sides
+    without interior cells."""
+    Ny, Nx, Nz = shape
+    dim = 2 if Nz == 1 else 3
+    rng = np.random.default_rng(Ny * 100 + Nx * 10 + Nz)
+    axis = lambda n: W.Axis(np.full(n, 0.1), 0.1 * np.arange(n + 1), 0.1 * np.arange(n) + 0.05)
+    g = W.Grid(dim, [axis(Nx), axis(Ny), axis(Nz)], 0.1, False, (0.0, 1.0) * 3)
+    types = rng.choice([W.SOLID, W.EMPTY, W.INFLOW, W.PRESSURE, W.OUTFLOW], size=shape).astype(np.uint8)
+    p = rng.standard_normal(shape)
+    expect = p.copy()
+    for _ in range(2):  # at the start of the step and after the (empty) solve
+        for ax in range(dim if dim == 2 else 3):
+            n = shape[ax]
+            for at, src in ((0, 1), (n - 1, n - 2)):
+                t, d, s = types.take(at, ax), expect.take(at, ax), expect.take(src, ax)
+                face = np.where(t == W.EMPTY, 0.0, np.where(t == W.PRESSURE, d, s))
+                expect[tuple(at if a == ax else slice(None) for a in range(3))] = face
+    zeros = lambda s: np.zeros(int(np.prod(s)))
+    m = MACGrid(g, types.reshape(-1).copy(), zeros(g.u_shape()), zeros(g.v_shape()), zeros(g.w_shape()),
+                p.reshape(-1).copy(), 1.0, 1e-3)
+    s = PressureSolver("mixed")
+    s.InitializePressureSolver(m)
+    assert s.SystemSize() == 0
+    s.SolvePressure(m, tol=1e-8)
+    s.DestroyPressureSolver()
+    assert np.array_equal(m.p.reshape(shape), expect)
