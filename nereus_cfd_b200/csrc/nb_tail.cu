@@ -203,7 +203,12 @@ __device__ __forceinline__ void ResidualCell(const SmemLevel<T> &L, const Cell<T
 {
     const int c = o.c;
     if constexpr (!kSt)
-        L.res[c] = o.r - (L.hg * (T)(o.b & 0x7Fu) * L.e[c] - L.g * NbrSum<T, k3D>(L, L.e, c));
+    {
+        // the products' rounding written out: contracted another way, the FP32 V-cycle's corrections (and with them a
+        // mixed solve's last digits, 1e-8 to 3e-7 of the pressure) would differ from those of the per-cell kernels
+        const T M = fma(-L.g, NbrSum<T, k3D>(L, L.e, c), L.hg * (T)(o.b & 0x7Fu) * L.e[c]);
+        L.res[c] = o.r - M;
+    }
     else
     {
         T s = o.diag * L.e[c];
