@@ -399,6 +399,13 @@ __device__ __forceinline__ void SplitProlong(const LevelView &fv, const LevelVie
     const int S = (cv.Ny - 2 + blk.gy - 1) / blk.gy;
     const int A0 = min(1 + blk.y * S, cv.Ny - 1), A1 = min(A0 + S, cv.Ny - 1);
     if (!valid || A0 >= A1) return;
+    // a block whose fine rows hold no unknown on its planes adds nothing (the air of a tank)
+    {
+        const int t0 = blk.x * kPairThreads, B0 = 1 + t0 / Q, B1 = 1 + min(t0 + kPairThreads, nq) / Q;
+        const int f0 = kX ? (fv.xr[B0] & 0x7FFF) : 2 * B0 - 1;
+        const int f1 = kX ? (fv.xr[min(B1, nrow)] & 0x7FFF) + 1 : 2 * min(B1, nrow);
+        if (RowsIdle<N * kPairThreads>(fv, f0, min(f1, fv.Nx - 1), 2 * A0 - 1, 2 * A1 - 1)) return;
+    }
     const int xg = kX ? fv.xr[B] : 0;
     const bool one = kX && !((xg >> 15) & 1);
     const int fb0 = kX ? (xg & 0x7FFF) : 2 * B - 1, fb1 = one ? fb0 : fb0 + 1;
@@ -584,6 +591,12 @@ __device__ __forceinline__ void SplitRestrictQ(const LevelView &fv, const LevelV
     const int S = (cv.Ny - 2 + blk.gy - 1) / blk.gy;
     const int I0 = 1 + blk.y * S, I1 = min(I0 + S, cv.Ny - 1);
     if (I0 >= I1) return;
+    // a block none of whose coarse cells' children is an unknown has no coarse unknown either
+    {
+        const int t0 = blk.x * kPairThreads, Ja = 1 + t0 / nq, Jb = 1 + (min(t0 + kPairThreads, nt) - 1) / nq;
+        const int f0 = kX ? (fv.xr[Ja] & 0x7FFF) : 2 * Ja - 1, f1 = kX ? (fv.xr[Jb] & 0x7FFF) + 1 : 2 * Jb;
+        if (RowsIdle<N * kPairThreads>(fv, f0, min(f1, fv.Nx - 1), 2 * I0 - 1, min(2 * I1 - 1, fv.Ny))) return;
+    }
     const bool more = K0 + N - 1 <= cv.Nz - 2; // element K0+N-1 is read only for coarse cell K0+N-1
     const RowTaps<T, kX> taps = TapsOf<T, kX>(fv, J);
     T Tm2[N], Tm1[N], Xm1[N], Xd[N];
@@ -652,6 +665,11 @@ __device__ __forceinline__ void SplitRestrict1(const LevelView &fv, const LevelV
     const int S = (cv.Ny - 2 + gz - 1) / gz;
     const int I0 = 1 + bz * S, I1 = min(I0 + S, cv.Ny - 1);
     if (I0 >= I1) return;
+    {
+        const int Ja = 1 + by * 8, Jb = min(Ja + 7, cv.Nx - 2); // idle as SplitRestrictQ's
+        const int f0 = kX ? (fv.xr[Ja] & 0x7FFF) : 2 * Ja - 1, f1 = kX ? (fv.xr[Jb] & 0x7FFF) + 1 : 2 * Jb;
+        if (RowsIdle<kQ<T> * kPairThreads>(fv, f0, min(f1, fv.Nx - 1), 2 * I0 - 1, min(2 * I1 - 1, fv.Ny))) return;
+    }
     const RowTaps<T, kX> taps = TapsOf<T, kX>(fv, J);
     T Tm2, Tm1, Xm1, Xdummy;
     SplitRestrictPlane1<T, kX>(fv, pext, res, 2 * I0 - 2, taps, K, Tm2, Xdummy);
