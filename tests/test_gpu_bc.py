@@ -92,3 +92,59 @@ def test_replay_in_a_cuda_graph(nb):
             assert np.array_equal(got, want)
     del graph
     bc.close()
+
+
+def random_lists(seed, n=7, dense=False):
+    """Lists on an n^3 grid that no scene would make: repeated destinations, chains of copies, sources written before and
+    after they are read (dense: most programs then do not resolve into independent writes), rows and single entries."""
+    rng = np.random.default_rng(seed)
+    sizes = [n * n * (n + 1)] * 3
+    pick = lambda size, count: rng.integers(0, size, count)
+    z = {}
+    for c in range(3):
+        z["solid%d" % c] = np.concatenate([np.arange(5, 5 + rng.integers(1, 300)), pick(sizes[c], 20)]) % sizes[c]
+    m = 400 if dense else 60
+    comp = np.sort(rng.integers(0, 3, m))
+    z["presc_comp"], z["presc_index"] = comp, pick(sizes[0], m)
+    z["presc_value"] = rng.normal(size=m)
+    comp = np.repeat(np.arange(3), m)
+    z["copy_comp"] = comp
+    if dense:
+        z["copy_dst"], z["copy_src"] = pick(sizes[0], 3 * m), pick(sizes[0], 3 * m)
+    else:  # from a block no copy writes, or along a chain of entries copied just before
+        z["copy_dst"] = np.tile(np.arange(100, 100 + m), 3)
+        z["copy_src"] = np.where(rng.random(3 * m) < 0.5, 300 + pick(40, 3 * m), np.maximum(z["copy_dst"] - 1, 100))
+        z["copy_src"][::m] = 350
+    r = 500 if dense else 120
+    z["ring_dst"] = pick(n ** 3, r) if dense else np.arange(0, 2 * r, 2)
+    z["ring_kind"], z["ring_value"] = rng.integers(0, 3, r), rng.normal(size=r)
+    z["ring_src"] = pick(n ** 3, r) if dense else 2 * pick(60, r) + 1
+    for k in ("inlet_comp", "inlet_index", "inlet_area", "inlet_sign", "outflow_comp", "outflow_index", "outflow_outer",
+              "outflow_area", "outflow_sign"):
+        z[k] = np.zeros(0)
+    return z
+
+
+@pytest.mark.parametrize("values", [True, False])
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("seed", range(6))
+def test_random_programs_match_the_serial_replay(nb, seed, dense, values):
+    import torch
+
+    n = 7
+    z = random_lists(seed, n, dense)
+    rng = np.random.default_rng(100 + seed)
+    ins = [rng.normal(size=n * n * (n + 1)) for _ in range(3)] + [rng.normal(size=n ** 3)]
+    bc = BoundaryReplay(z, 3, n, n, n)
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a, dtype=np.float64)).to("cuda")
+    fields = [d(a) for a in ins]
+    bc.EnforceVelocityBC(*fields[:3], d(z["presc_value"]) if values else None)
+    bc.EnforcePressureBC(fields[3], d(z["ring_value"]) if values else None)
+    torch.cuda.synchronize()
+    lists = dict(z)
+    if not values:
+        lists["ring_value"] = np.zeros_like(z["ring_value"])
+    ref = cpu.bc_replay(lists, *ins, with_velocity_function=values)
+    for got, want in zip(_host(fields), ref):
+        assert np.array_equal(got, want)
+    bc.close()
