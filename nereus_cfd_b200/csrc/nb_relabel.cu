@@ -7,18 +7,19 @@
 // caller may capture them in a graph):
 //   1. reset: every cell that is not SOLID, INFLOW, OUTFLOW or PRESSURE becomes EMPTY. k_relabel_reset, 16 bytes per
 //      thread; it also zeroes the pending-list counter and the skipped-particle count.
-//   2. mark: each particle's cell, if EMPTY, becomes FLUID. k_relabel_mark, one wave of threads striding over the
-//      particles four at a time, reading
-//      x, y, z through a stride so that the reference's own Particle array (x, y, z at doubles 1..3 of 7) and plain
-//      position arrays both serve. The index is the reference's (truncation of (x - origin) / dh toward zero, clamped
+//   2. mark: each particle's cell, if EMPTY, becomes FLUID. Positions that lie in rows of at most kMaxRow doubles (plain
+//      x, y, z rows, or the reference's own Particle array with x, y, z at doubles 1..3 of 7) stream through shared
+//      memory (k_relabel_mark_rows); separate or widely strided arrays are read directly, four particles in flight a
+//      thread (k_relabel_mark). The index is the reference's (truncation of (x - origin) / dh toward zero, clamped
 //      above); a particle more than one cell below the grid or with a non-finite coordinate, which the reference
 //      would index outside its labels with, is skipped and counted.
 //   3. hole filling: one pass over the interior in (i, j, k) order, IN PLACE: an EMPTY cell with >= 5 (3D) / >= 3
 //      (2D) FLUID neighbours becomes FLUID, and a cell filled earlier in the pass counts for the later ones. So a cell
 //      sees its upper neighbours (i+1, j+1, k+1) as they were before the pass and its lower ones (i-1, j-1, k-1) as
 //      the pass left them. The result is the unique solution of that recurrence, which is what is computed here:
-//        k_relabel_fill: one thread per interior cell, consecutive threads along the fast axis, whole columns per
-//          block step. Filled cells get the
+//        k_relabel_fill: four cells a thread, read as words; a cell none of whose upper neighbours is FLUID can get at
+//          most as many FLUID neighbours as it has lower ones, too few, so most of the air is passed over by
+//          comparing words. Filled cells get the
 //          marker kFilled, which counts as FLUID for the cells above and not at all for the cells below (they read
 //          the label from before the pass). A filled cell has at most one uncounted neighbour, so at most one of its
 //          upper neighbours can continue a chain of fills: the thread walks up that chain at once. A cell still EMPTY
@@ -32,7 +33,10 @@
 //        k_relabel_finish: kFilled -> FLUID.
 #include "nb_solver.h"
 
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
+#include <cstring>
 
 namespace nb
 {
@@ -54,6 +58,7 @@ struct RelabelGrid
     int nCols;                 // interior columns
     int march;                 // interior cells along the march axis (3D: Nz - 2; 2D: Nx - 2)
     int thr;                   // FLUID neighbours that fill a hole: 5 (3D), 3 (2D)
+    int nearHi;                // ParticleIndex's bound of nearness to an integer: the high word of that double
 };
 
 __device__ __forceinline__ uint8_t ResetByte(uint8_t b)
@@ -130,21 +135,30 @@ __global__ void __launch_bounds__(kThreads) k_relabel_finish(uint8_t *__restrict
 // UpdateFluidCells' index of one coordinate (FLIP3D.cpp:796-802): trunc((x - origin) / dh), at most N - 1; -1 for a
 // quotient at or below -1 or not finite (outside the labels in the reference). A quotient at or above N takes N - 1
 // without a conversion.
-// The quotient is first taken as (x - origin) * inv with inv = 1 / dh rounded, which is within 2^-51 |q| of the
-// correctly rounded quotient q (two roundings of 2^-53 each, plus the one of q). Every decision below compares q with
-// an integer (the truncation, -1, N), so where the product lies farther than that bound (2^-48 |q| here, with margin)
-// from both integers around it, q lies strictly between the same two integers and every decision agrees; otherwise
-// (and for a non-finite product) the exact IEEE division decides.
-__device__ __forceinline__ int ParticleIndex(double x, double origin, double dh, double inv, int N)
+// The quotient is first taken as q = (x - origin) * inv with inv = 1 / dh rounded, which is within 2^-51 |q| of the
+// correctly rounded one (two roundings of 2^-53 each, plus the one of the quotient). Every decision compares it with an
+// integer (the truncation, -1, N), so where q lies farther than g.nearHi's bound, 2^-48 (max N + 2), from the integer
+// nearest to it, the two lie strictly between the same integers and every decision agrees (a |q| beyond N + 2 is beyond
+// N and -1 by more than its error); next to an integer, and for a q that is not finite or above 2^30, the exact IEEE
+// division decides. The nearest integer comes from adding 1.5 * 2^52, the comparisons are on the high words: no
+// conversion (those run at a sixteenth of the rate of the additions) and few FP64 instructions.
+__device__ __noinline__ int ParticleIndexExact(double d, double dh, int N)
 {
-    const double d = x - origin;
-    double q = d * inv;
-    const double fl = floor(q);
-    const double tol = fabs(q) * 0x1p-48 + 0x1p-60;
-    if (!(q - fl > tol && fl + 1.0 - q > tol)) q = d / dh;
+    const double q = d / dh;
     if (!(q > -1.0)) return -1;
     if (q >= (double)N) return N - 1;
     return (int)q;
+}
+
+__device__ __forceinline__ int ParticleIndex(double x, double origin, double dh, double inv, int N, int nearHi)
+{
+    const double shift = 0x1.8p52;
+    const double d = x - origin, q = __dmul_rn(d, inv), r = __dadd_rn(q, shift);
+    const double f = __dsub_rn(q, __dsub_rn(r, shift)); // q less the integer nearest to it, exact
+    const int qh = __double2hiint(q) & 0x7FFFFFFF, fh = __double2hiint(f);
+    if (qh >= 0x41D00000 || (fh & 0x7FFFFFFF) <= nearHi) return ParticleIndexExact(d, dh, N); // 0x41D00000: 2^30
+    const int fl = __double2loint(r) + (fh >> 31); // floor(q)
+    return fl < -1 ? -1 : min(max(fl, 0), N - 1);
 }
 
 constexpr int kMarkBatch = 4; // particles in flight per thread
@@ -174,17 +188,17 @@ __global__ void __launch_bounds__(kThreads, 4)
     if (p0 < count) load(p0);
     while (p0 < count)
     {
-        long long c[kMarkBatch];
+        int c[kMarkBatch];
 #pragma unroll
         for (int b = 0; b < kMarkBatch; b++)
         {
-            const int i = ParticleIndex(y[b], oy, dh, inv, g.Ny);
-            const int j = ParticleIndex(x[b], ox, dh, inv, g.Nx);
-            const int k = g.dim == 3 ? ParticleIndex(z[b], oz, dh, inv, g.Nz) : 0;
+            const int i = ParticleIndex(y[b], oy, dh, inv, g.Ny, g.nearHi);
+            const int j = ParticleIndex(x[b], ox, dh, inv, g.Nx, g.nearHi);
+            const int k = g.dim == 3 ? ParticleIndex(z[b], oz, dh, inv, g.Nz, g.nearHi) : 0;
             const bool live = p0 + b * nt < count;
             const bool out = (i | j | k) < 0;
             mine += live && out;
-            c[b] = live && !out ? ((long long)i * g.Nx + j) * g.Nz + k : -1;
+            c[b] = live && !out ? (i * g.Nx + j) * g.Nz + k : -1;
         }
         // the next batch's positions are in flight while this batch's labels are read and written
         const long long p1 = p0 + step;
@@ -196,6 +210,82 @@ __global__ void __launch_bounds__(kThreads, 4)
     }
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, s);
+    if (skipped && (threadIdx.x & 31) == 0 && mine) atomicAdd(skipped, mine);
+}
+
+// The same for positions in rows: coordinates of particle p at base[p * stride + ox0, oy0, oz0] (doubles), stride at
+// most kMaxRow. Reading them with one 8-byte load per coordinate left the pass at 3.6 TB/s (the rows of 24 bytes take
+// every sector three times through L1, and the loads are tied to the index arithmetic); here a block copies chunks of
+// kRowChunk rows to shared memory 16 bytes at a time, kRowStages chunks ahead (cp.async), and works from there. A lane
+// whose particle lies in the previous lane's cell leaves the label to it: particles come cell by cell. 67 M particles
+// in (x, y, z) rows, 256^3 labels, the whole call (B200): 0.648 ms before, 0.498 ms now.
+constexpr int kMaxRow = 8, kRowChunk = 512, kRowStages = 3;
+
+__device__ __forceinline__ void CopyAsync16(void *smem, const void *gmem)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+
+// bytes of a stage: a chunk's rows, and a granule for a start that is not on a 16-byte boundary
+__host__ __device__ inline int RowStageBytes(int stride) { return kRowChunk * stride * 8 + 16; }
+
+__global__ void __launch_bounds__(kThreads)
+    k_relabel_mark_rows(const double *__restrict__ base, int stride, int offX, int offY, int offZ, int span,
+                        long long count, RelabelGrid g, double ox, double oy, double oz, double dh, double inv,
+                        uint8_t *__restrict__ t, unsigned long long *skipped)
+{
+    extern __shared__ __align__(16) unsigned char rows[];
+    const long long chunks = (count + kRowChunk - 1) / kRowChunk;
+    const int stageBytes = RowStageBytes(stride);
+    const unsigned char *src = reinterpret_cast<const unsigned char *>(base);
+    const int mis = (int)((uintptr_t)src & 15); // every chunk starts as far from a 16-byte boundary (512 rows of 8 n)
+    // chunk c into stage s: the granules that hold its rows' coordinates (the last row ends after `span` doubles);
+    // a granule that holds one valid byte lies inside the array's allocation
+    auto fetch = [&](long long c, int s) {
+        if (c < chunks)
+        {
+            const long long n = min((long long)kRowChunk, count - c * kRowChunk);
+            const int bytes = mis + (int)(((n - 1) * stride + span) * 8);
+            const unsigned char *from = src - mis + c * (long long)kRowChunk * stride * 8;
+            for (int o = 16 * (int)threadIdx.x; o < bytes; o += 16 * kThreads)
+                CopyAsync16(rows + s * stageBytes + o, from + o);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    unsigned long long mine = 0;
+    for (int s = 0; s < kRowStages - 1; s++) fetch(blockIdx.x + (long long)s * gridDim.x, s);
+    int s = 0;
+    for (long long c = blockIdx.x; c < chunks; c += gridDim.x, s = s + 1 == kRowStages ? 0 : s + 1)
+    {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kRowStages - 2) : "memory");
+        __syncthreads(); // this chunk is in; the stage fetched next was read in the round before
+        fetch(c + (long long)(kRowStages - 1) * gridDim.x, s + kRowStages - 1 >= kRowStages ? s - 1 : s + kRowStages - 1);
+        const double *rd = reinterpret_cast<const double *>(rows + s * stageBytes + mis);
+        const int here = (int)min((long long)kRowChunk, count - c * kRowChunk); // rows of this chunk
+        int cell[kRowChunk / kThreads];
+#pragma unroll
+        for (int b = 0; b < kRowChunk / kThreads; b++)
+        {
+            const int p = threadIdx.x + b * kThreads;
+            const bool live = p < here;
+            const double *q = rd + (live ? p * stride : 0);
+            const int i = ParticleIndex(q[offY], oy, dh, inv, g.Ny, g.nearHi);
+            const int j = ParticleIndex(q[offX], ox, dh, inv, g.Nx, g.nearHi);
+            const int k = g.dim == 3 ? ParticleIndex(q[offZ], oz, dh, inv, g.Nz, g.nearHi) : 0;
+            const bool out = (i | j | k) < 0;
+            mine += live && out;
+            const int at = live && !out ? (i * g.Nx + j) * g.Nz + k : -1;
+            const int before = __shfl_up_sync(0xffffffffu, at, 1);
+            cell[b] = (threadIdx.x & 31) != 0 && before == at ? -1 : at;
+        }
+#pragma unroll
+        for (int b = 0; b < kRowChunk / kThreads; b++)
+            if (cell[b] >= 0 && t[cell[b]] == EMPTY) t[cell[b]] = (uint8_t)FLUID;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, d);
     if (skipped && (threadIdx.x & 31) == 0 && mine) atomicAdd(skipped, mine);
 }
 
@@ -288,27 +378,62 @@ __device__ __forceinline__ long long InteriorCell(const RelabelGrid &g, long lon
     return (g.dim == 3 ? ((long long)i * g.Nx + j) * g.Nz : (long long)i * g.Nx) + m;
 }
 
-// Each block step takes whole columns: `span` threads per column along the march axis (consecutive threads on
-// consecutive cells), kThreads / span columns per step. A cell that reaches the threshold with the labels as this
-// thread reads them is filled (and the chain above it followed); one that could still reach it once its EMPTY lower
-// neighbours are filled goes on the pending list.
+// bytes of w equal to b (b repeated in every byte of bbbb): 0x80 in each
+__device__ __forceinline__ unsigned BytesEqual(unsigned w, unsigned bbbb)
+{
+    const unsigned x = w ^ bbbb;
+    return ~(((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u;
+}
+// the four bytes at p (any alignment; the word after the last one's may be read)
+__device__ __forceinline__ unsigned Bytes4(const uint8_t *p)
+{
+    const unsigned m = (unsigned)((uintptr_t)p & 3);
+    const unsigned *w = reinterpret_cast<const unsigned *>(p - m);
+    return m ? __funnelshift_r(w[0], w[1], 8 * m) : w[0];
+}
+
+// Four cells a thread, on 4-byte boundaries of the label array, over the planes i = 1 .. Ny-2. A cell that reaches the
+// threshold with the labels as this thread reads them is filled (and the chain above it followed); one that could
+// still reach it once its EMPTY lower neighbours are filled goes on the pending list. A cell with no FLUID upper
+// neighbour needs neither (the threshold is one less than twice the dimension, the lower neighbours are as many as
+// the dimension), and what FLUID upper neighbours there are does not change during the pass.
 __global__ void __launch_bounds__(kThreads)
     k_relabel_fill(RelabelGrid g, uint8_t *t, int *hdr, int *list, int cap)
 {
-    const int span = g.march < kThreads ? g.march : kThreads;
-    const int cpb = kThreads / span;
-    const int lc = threadIdx.x / span, lm = threadIdx.x - lc * span;
-    if (lc >= cpb) return;
-    for (int col0 = blockIdx.x * cpb; col0 < g.nCols; col0 += gridDim.x * cpb)
+    const long long mis = (long long)((4 - ((uintptr_t)t & 3)) & 3);
+    // words [w0, w1): those that touch the inner planes; the few cells before the first and after the last 4-byte
+    // boundary are ring cells
+    const long long w0 = g.sI > mis ? (g.sI - mis) >> 2 : 0, w1 = (g.cells - g.sI - mis + 3) >> 2;
+    for (long long w = w0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; w < w1;
+         w += (long long)gridDim.x * blockDim.x)
     {
-        const int col = col0 + lc;
-        if (col >= g.nCols) return;
-        const int i = 1 + col / g.colsX;
-        const int j = g.dim == 3 ? 1 + (col - (i - 1) * g.colsX) : 0;
-        const long long base = g.dim == 3 ? ((long long)i * g.Nx + j) * g.Nz : (long long)i * g.Nx;
-        for (int m = 1 + lm; m <= g.march; m += span)
+        const long long c0 = mis + 4 * w;
+        const uint8_t *p = t + c0;
+        unsigned cand;
+        if (c0 + g.sI + 8 <= g.cells) // the words read below stay inside the array
         {
-            const long long c = base + m;
+            const unsigned own = *reinterpret_cast<const unsigned *>(p);
+            cand = BytesEqual(own, 0x01010101u * EMPTY);
+            if (!cand) continue;
+            unsigned up = BytesEqual(__funnelshift_r(own, *reinterpret_cast<const unsigned *>(p + 4), 8), 0u) |
+                          BytesEqual(Bytes4(p + g.sI), 0u);
+            if (g.dim == 3) up |= BytesEqual(Bytes4(p + g.sJ), 0u);
+            cand &= up;
+        }
+        else
+        {
+            cand = 0;
+            for (int b = 0; b < 4; b++)
+                if (c0 + b < g.cells && p[b] == EMPTY) cand |= 0x80u << (8 * b);
+        }
+        while (cand)
+        {
+            const int b = (__ffs((int)cand) - 1) >> 3;
+            cand &= cand - 1;
+            const long long c = c0 + b;
+            int i, j, m;
+            CellCoords(g, c, i, j, m);
+            if (i < 1 || i > g.Ny - 2 || m < 1 || m > g.march || (g.dim == 3 && (j < 1 || j > g.Nx - 2))) continue;
             if (t[c] != EMPTY) continue;
             int maybe = 0;
             const int f = FluidCountOnce(g, t, c, i, j, m, maybe);
@@ -400,6 +525,10 @@ void UpdateFluidCellsDevice(int dim, int Nx, int Ny, int Nz, double ox, double o
     g.nCols = (Ny > 2 ? Ny - 2 : 0) * g.colsX;
     g.march = dim == 3 ? (nz > 2 ? nz - 2 : 0) : (Nx > 2 ? Nx - 2 : 0);
     g.thr = 2 * dim - 1;
+    const double bound = std::ldexp((double)std::max(Nx, std::max(Ny, nz)) + 2.0, -48);
+    uint64_t bits;
+    std::memcpy(&bits, &bound, sizeof bits);
+    g.nearHi = (int)(bits >> 32);
     int *hdr = (int *)scratch;
     int *list = hdr + kHeaderInts;
     const long long capLL = (long long)(scratchBytes / sizeof(int)) - kHeaderInts;
@@ -413,14 +542,30 @@ void UpdateFluidCellsDevice(int dim, int Nx, int Ny, int Nz, double ox, double o
     if (count > 0)
     {
         NB_COUNT_LAUNCH();
+        // rows: the coordinates of a particle within one row of `stride` doubles (compared as addresses, since separate
+        // arrays are separate objects)
+        const uintptr_t ax = (uintptr_t)px, ay = (uintptr_t)py, az = dim == 3 ? (uintptr_t)pz : ax;
+        const uintptr_t lo = std::min(ax, std::min(ay, az)), hi = std::max(ax, std::max(ay, az));
+        if (stride <= kMaxRow && (lo & 7) == 0 && ((ax - lo) | (ay - lo) | (az - lo)) % 8 == 0 &&
+            hi - lo < (uintptr_t)stride * 8)
+        {
+            const int s = (int)stride, smem = kRowStages * RowStageBytes(s);
+            if (smem > (48 << 10)) // more than a kernel gets unasked
+                NB_CK(cudaFuncSetAttribute(k_relabel_mark_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           kRowStages * RowStageBytes(kMaxRow)));
+            const int perSm = std::max(1, std::min(6, (200 << 10) / smem));
+            k_relabel_mark_rows<<<Blocks(count, kRowChunk, sms * perSm), kThreads, smem, st>>>(
+                (const double *)lo, s, (int)((ax - lo) / 8), (int)((ay - lo) / 8), (int)((az - lo) / 8),
+                (int)((hi - lo) / 8) + 1, count, g, ox, oy, oz, dh, 1.0 / dh, cellTypes, skipped);
+        }
+        else
         k_relabel_mark<<<Blocks((count + kMarkBatch - 1) / kMarkBatch, kThreads, sms * 4), kThreads, 0, st>>>(
             px, py, pz, count, stride, g, ox, oy, oz, dh, 1.0 / dh, cellTypes, skipped);
     }
     if (g.nCols > 0 && g.march > 0)
     {
         NB_COUNT_LAUNCHES(3);
-        const int span = g.march < kThreads ? g.march : kThreads;
-        k_relabel_fill<<<Blocks(g.nCols, kThreads / span, sms * 8), kThreads, 0, st>>>(g, cellTypes, hdr, list, cap);
+        k_relabel_fill<<<Blocks(cells / 4 + 1, kThreads, sms * 8), kThreads, 0, st>>>(g, cellTypes, hdr, list, cap);
         k_relabel_settle<<<1, kSettleThreads, 0, st>>>(g, cellTypes, hdr, list, cap);
         k_relabel_finish<<<Blocks(cells / 16 + 1, kThreads, sms * 8), kThreads, 0, st>>>(cellTypes, cells);
     }

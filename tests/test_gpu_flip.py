@@ -190,3 +190,47 @@ def test_relabel_then_projection_matches_reference(nb, name, precision):
     assert np.abs(m.v - z["v_out"]).max() <= 1e-6 * scale
     if g.dim == 3:
         assert np.abs(m.w - z["w_out"]).max() <= 1e-6 * scale
+
+
+def oracle_labels(grid, types, xyz, origin):
+    return cpu.update_fluid_cells(grid, types, np.ascontiguousarray(xyz), origin)
+
+
+# counts around a chunk of 512 rows and a block's 256 threads; row widths up to the widest that streams (8) and past it;
+# starts on and off a 16-byte boundary; labels on any byte boundary
+@pytest.mark.parametrize("count", [1, 255, 257, 511, 512, 513, 1024, 5000])
+@pytest.mark.parametrize("stride,first", [(3, 0), (3, 1), (4, 1), (7, 1), (8, 5), (9, 2)])
+def test_particle_rows_stream_like_the_oracle(nb, count, stride, first):
+    import torch
+
+    case = W.flip_tank_3d(13, a=0.6, b=0.6)
+    g = case.grid
+    types = capi.label_cells(g, case.scene)
+    rng = np.random.default_rng(stride * 10000 + first * 1000 + count)
+    xyz = rng.uniform(-0.02, 1.02, size=(count, 3)) * np.array([0.6, 1.0, 0.6])
+    xyz[rng.random(count) < 0.05] -= 0.5  # skipped: more than a cell below the grid
+    expect, skip = oracle_labels(g, types, xyz, _origin(g))[:2]
+    # one buffer: `first` doubles before the first row's x, rows of `stride` doubles, nothing after the last z
+    buf = np.full(first + (count - 1) * stride + 3, np.nan)
+    for q in range(3):
+        buf[first + q::stride][:count] = xyz[:, q]
+    d = torch.from_numpy(buf).to("cuda")
+    base = d.data_ptr() + 8 * first
+    lab = torch.zeros(types.size + 8, dtype=torch.uint8, device="cuda")
+    sb = nb.nereus_b200_update_fluid_cells_scratch_bytes(3, g.Nx, g.Ny, g.Nz)
+    scratch = torch.zeros(sb // 4 + 1, dtype=torch.int32, device="cuda")
+    skipped = torch.zeros(1, dtype=torch.int64, device="cuda")
+    for shift in range(4):
+        view = lab[shift:shift + types.size]
+        view.copy_(torch.from_numpy(types.reshape(-1)))
+        lab[:shift] = 77
+        lab[shift + types.size:] = 77
+        capi.check(nb.nereus_b200_update_fluid_cells_device(
+            torch.cuda.current_device(), 3, g.Nx, g.Ny, g.Nz, *_origin(g), g.dh, ctypes.c_void_p(base),
+            ctypes.c_void_p(base + 8), ctypes.c_void_p(base + 16), count, stride, ctypes.c_void_p(view.data_ptr()),
+            ctypes.c_void_p(scratch.data_ptr()), sb, ctypes.c_void_p(skipped.data_ptr()),
+            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        torch.cuda.synchronize()
+        assert np.array_equal(view.cpu().numpy(), np.asarray(expect).reshape(-1))
+        assert int(skipped.item()) == skip
+        assert bool((lab[:shift] == 77).all()) and bool((lab[shift + types.size:] == 77).all())
