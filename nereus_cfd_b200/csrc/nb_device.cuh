@@ -34,9 +34,9 @@ struct LevelView
     const double *g[3]; // padded FaceGap tables, entry n at [n+1] (n = -1..N-1)
     const float *w32[3];
     const float *ig32[3]; // 1 / FaceGap, FP32
-    const double *igd[3]; // 1 / FaceGap, FP64 (the kernels of stretched colour-split and 2D levels)
-    // a stretched colour-split level (in that layout) or a 2D one (nb_legs2d.cu): each cell's diagonal and its
-    // reciprocal, zero off the unknowns
+    const double *igd[3]; // 1 / FaceGap, FP64 (a stretched colour-split level's kernels)
+    // a stretched colour-split level: each cell's diagonal and its reciprocal, in that layout, zero off the unknowns;
+    // a 2D level (nb_legs2d.cu): the diagonal
     const double *dg, *idg;
     // Per-cell code of the level: bits 0-5 neighbour q is FLUID, bit 6 a neighbour is Dirichlet, bit 7 the cell is
     // an unknown (interior FLUID). Built once per layout (k_build_codes).

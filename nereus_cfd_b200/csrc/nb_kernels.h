@@ -183,8 +183,8 @@ void LaunchLegUpDot(const LevelView &v, const LevelView &cv, const uint8_t *du, 
                     cudaStream_t st);
 
 // ---- nb_legs2d.cu: a 2D level's descent and ascent in one launch each (1 or 2 sweeps before and after the coarse
-//      correction); ext: the moved transfer weights, with the diagonal and its reciprocal built once per layout ----
-void LaunchBuild2D(const LevelView &v, const LevelView &cv, double *dg, double *idg, uint8_t *ext, cudaStream_t st);
+//      correction); ext: the moved transfer weights, built with the diagonal once per layout ----
+void LaunchBuild2D(const LevelView &v, const LevelView &cv, int elemBytes, double *dg, uint8_t *ext, cudaStream_t st);
 template <typename T>
 void LaunchLeg2Down(const LevelView &v, const LevelView &cv, const uint8_t *ext, const T *r, T *tmp, T *rc, int sweeps,
                     cudaStream_t st);

@@ -8,10 +8,12 @@
 // 20 x 36 for the ascent. The descent writes the smoothed iterate to the level's residual vector, the ascent reads it
 // there and writes the level's e, so no block reads what another one writes.
 //
-// The stencil at cell (i, j) is w_x (e_i+ / g + e_i- / g) + w_y (e_j+ / g + e_j- / g), with all entries 1 on a uniform
-// level (whose unit-form coefficient is 1); the diagonal and its reciprocal are kept per cell (FP64, once per layout).
+// The values are those of the per-cell kernels (nb_kernels.cu): the same coefficients (the level's FP32 tables; 1 on a
+// uniform level), diagonal (kept per cell, once per layout), sums in the same order and division, so that a solve ends
+// where it ended with a launch per operation. Reciprocals and sums by pairs instead were no faster and moved the
+// pressure by 3e-8 of itself (FP32 rounding, carried through a solve to 1e-8).
 //
-// Measured (B200): the 128^2 closed box's step in mixed precision to 1e-10 (13 iterations, two such levels) 1.03 -> 0.74 ms
+// Measured (B200): the 128^2 closed box's step in mixed precision to 1e-10 (13 iterations, two such levels) 1.03 -> 0.79 ms
 // with the ring replay in one launch.
 #include "nb_kernels.h"
 
@@ -36,7 +38,7 @@ template <int kHalo> struct Region2
     }
 };
 
-// the region's 1D tables: Width and 1/FaceGap along both axes (1 on a uniform level)
+// the region's 1D tables: Width and 1/FaceGap (FP32, as LevelCoefs reads them) along both axes, 1 on a uniform level
 template <typename T, int kR, int kC> struct Tables2
 {
     T wy[kR], gy[kR + 1], wx[kC], gx[kC + 1]; // g[n]: the face below cell n of the region
@@ -45,25 +47,35 @@ template <typename T, int kR, int kC> struct Tables2
 template <typename T, int kR, int kC>
 __device__ __forceinline__ void LoadTables(const LevelView &v, int i0, int j0, Tables2<T, kR, kC> &s)
 {
-    auto entry = [](const double *tab, int n, int last) { return (T)tab[n < 0 ? 0 : (n > last ? last : n)]; };
+    auto entry = [](const float *tab, int n, int last) { return (T)tab[n < 0 ? 0 : (n > last ? last : n)]; };
     for (int n = threadIdx.x; n <= kR; n += kThreads2)
     {
-        if (n < kR) s.wy[n] = v.stretched ? entry(v.w[1], i0 + n + 1, v.Ny + 1) : (T)1;
-        s.gy[n] = v.stretched ? entry(v.igd[1], i0 + n, v.Ny) : (T)1;
+        if (n < kR) s.wy[n] = v.stretched ? entry(v.w32[1], i0 + n + 1, v.Ny + 1) : (T)1;
+        s.gy[n] = v.stretched ? entry(v.ig32[1], i0 + n, v.Ny) : (T)1;
     }
     for (int n = threadIdx.x; n <= kC; n += kThreads2)
     {
-        if (n < kC) s.wx[n] = v.stretched ? entry(v.w[0], j0 + n + 1, v.Nx + 1) : (T)1;
-        s.gx[n] = v.stretched ? entry(v.igd[0], j0 + n, v.Nx) : (T)1;
+        if (n < kC) s.wx[n] = v.stretched ? entry(v.w32[0], j0 + n + 1, v.Nx + 1) : (T)1;
+        s.gx[n] = v.stretched ? entry(v.ig32[0], j0 + n, v.Nx) : (T)1;
     }
 }
 
+// the coefficient-weighted sum of a cell's neighbours, in MaskedSum's order (a neighbour that is no unknown holds zero)
 template <typename T, int kR, int kC>
 __device__ __forceinline__ T Sum2(const Tables2<T, kR, kC> &s, const T *e, int li, int lj)
 {
     const T *p = e + li * kC + lj;
-    return s.wx[lj] * (s.gy[li + 1] * p[kC] + s.gy[li] * p[-kC]) + s.wy[li] * (s.gx[lj + 1] * p[1] + s.gx[lj] * p[-1]);
+    const T wx = s.wx[lj], wy = s.wy[li];
+    const T c0 = wx * s.gy[li + 1], c1 = wx * s.gy[li], c2 = wy * s.gx[lj + 1], c3 = wy * s.gx[lj];
+    T x = c0 * p[kC];
+    x += c1 * p[-kC];
+    x += c2 * p[1];
+    x += c3 * p[-1];
+    return x;
 }
+
+// a sweep's new value: rhs / diagonal (zero off the unknowns and at an unknown without neighbours)
+template <typename T> __device__ __forceinline__ T OverDiag(T rhs, T d) { return d != (T)0 ? rhs / d : (T)0; }
 
 // Runs f(li, lj) over the cells of the colour in the region shrunk by `m` on every side, then the barrier.
 template <int kR, int kC, typename F>
@@ -86,38 +98,22 @@ __device__ __forceinline__ bool InGrid(const LevelView &v, int i, int j)
 
 } // namespace
 
-// per layout: the diagonal and its reciprocal of every unknown (zero elsewhere), and the weights the transfers move off
-// SOLID coarse contributors (0x80 | 64ths at an unknown)
+// per layout: the diagonal of every unknown as the per-cell kernels of the solver's precision form it (zero elsewhere),
+// and the weights the transfers move off SOLID coarse contributors (0x80 | 64ths at an unknown)
+template <typename T>
 __global__ void __launch_bounds__(256) k_build_2d(LevelView v, LevelView cv, double *__restrict__ dg,
-                                                  double *__restrict__ idg, uint8_t *__restrict__ ext)
+                                                  uint8_t *__restrict__ ext)
 {
     const int c = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (c >= (int)v.cells) return;
     const unsigned code = v.code[c];
-    double d = 0.0;
+    T d = (T)0;
     unsigned moved = 0;
     if (code & CODE_UNKNOWN)
     {
         const int i = c / v.Nx, j = c - i * v.Nx;
-        double cq[4] = {1.0, 1.0, 1.0, 1.0};
-        if (v.stretched)
-        {
-            cq[0] = Wd(v, 0, j) / Gp(v, 1, i);
-            cq[1] = Wd(v, 0, j) / Gp(v, 1, i - 1);
-            cq[2] = Wd(v, 1, i) / Gp(v, 0, j);
-            cq[3] = Wd(v, 1, i) / Gp(v, 0, j - 1);
-        }
-        for (int q = 0; q < 4; q++)
-        {
-            if (code >> q & 1u) d += cq[q];
-            else if ((code & CODE_DIRICHLET) && IsDirichlet(v.types[c + NbrOffset(v, q)]))
-            {
-                const int a = q < 2 ? 1 : 0, n = q < 2 ? i : j;
-                const bool ring = OnRing(v, i + (q == 0) - (q == 1), j + (q == 2) - (q == 3), 0);
-                const double f = !v.stretched ? 2.0 : Gp(v, a, (q & 1) ? n - 1 : n) / (0.5 * Wd(v, a, n));
-                d += ring ? cq[q] * f : cq[q];
-            }
-        }
+        T cq[6];
+        CodeStencil<T>(v, i, j, 0, c, code, cq, d);
         const int I = (i + 1) >> 1, J = (j + 1) >> 1, si = (i & 1) ? -1 : 1, sj = (j & 1) ? -1 : 1;
         moved = 0x80u;
         for (int q = 1; q < 4; q++)
@@ -126,18 +122,19 @@ __global__ void __launch_bounds__(256) k_build_2d(LevelView v, LevelView cv, dou
             if (cv.types[(long long)(I + di * si) * cv.sI + J + dj * sj] == SOLID) moved += 4u * (di ? 1u : 3u) * (dj ? 1u : 3u);
         }
     }
-    dg[c] = d;
-    idg[c] = d != 0.0 ? 1.0 / d : 0.0;
+    dg[c] = (double)d;
     ext[c] = (uint8_t)moved;
 }
 
-void LaunchBuild2D(const LevelView &v, const LevelView &cv, double *dg, double *idg, uint8_t *ext, cudaStream_t st)
+void LaunchBuild2D(const LevelView &v, const LevelView &cv, int elemBytes, double *dg, uint8_t *ext, cudaStream_t st)
 {
+    const unsigned blocks = (unsigned)((v.cells + 255) / 256);
     NB_COUNT_LAUNCH();
-    k_build_2d<<<(unsigned)((v.cells + 255) / 256), 256, 0, st>>>(v, cv, dg, idg, ext);
+    if (elemBytes == 8) k_build_2d<double><<<blocks, 256, 0, st>>>(v, cv, dg, ext);
+    else k_build_2d<float><<<blocks, 256, 0, st>>>(v, cv, dg, ext);
 }
 
-// tmp = kS red-black sweeps from zero; rc = R (r - M tmp). The sweeps end black: the black residual is zero.
+// tmp = kS red-black sweeps from zero; rc = R (r - M tmp)
 template <typename T, int kS>
 __global__ void __launch_bounds__(kThreads2) k_leg2_down(LevelView v, LevelView cv, const uint8_t *__restrict__ ext,
                                                          const T *__restrict__ r, T *__restrict__ tmp,
@@ -152,7 +149,7 @@ __global__ void __launch_bounds__(kThreads2) k_leg2_down(LevelView v, LevelView 
     for (int t = threadIdx.x; t < G::kN; t += kThreads2)
     {
         const int i = P.i0 + t / G::kC, j = P.j0 + t % G::kC;
-        sd[t] = InGrid(v, i, j) ? (T)v.idg[i * v.Nx + j] : (T)0;
+        sd[t] = InGrid(v, i, j) ? (T)v.dg[i * v.Nx + j] : (T)0;
     }
     PdlWait();
     PdlTrigger();
@@ -161,46 +158,51 @@ __global__ void __launch_bounds__(kThreads2) k_leg2_down(LevelView v, LevelView 
         const int i = P.i0 + t / G::kC, j = P.j0 + t % G::kC;
         const T x = InGrid(v, i, j) ? r[i * v.Nx + j] : (T)0;
         sr[t] = x;
-        se[t] = x * sd[t]; // the red half from zero (the black values are replaced unread)
+        se[t] = OverDiag(x, sd[t]); // the red half from zero (the black values are replaced unread)
     }
     __syncthreads();
 #pragma unroll
     for (int h = 1; h < 2 * kS; h++)
         ForColour<G::kR, G::kC>(P.i0, P.j0, h, h & 1, [&](int li, int lj) {
             const int t = li * G::kC + lj;
-            se[t] = (sr[t] + Sum2<T, G::kR, G::kC>(tab, se, li, lj)) * sd[t];
+            se[t] = OverDiag(sr[t] + Sum2<T, G::kR, G::kC>(tab, se, li, lj), sd[t]);
         });
     for (int t = threadIdx.x; t < kOwnI * kOwnJ; t += kThreads2)
     {
         const int li = kHalo + t / kOwnJ, lj = kHalo + t % kOwnJ, i = P.i0 + li, j = P.j0 + lj;
         if (i <= v.Ny - 2 && j <= v.Nx - 2) tmp[i * v.Nx + j] = se[li * G::kC + lj];
     }
-    // the red residual, over r; the black one is zero
-    ForColour<G::kR, G::kC>(P.i0, P.j0, 2 * kS, 0, [&](int li, int lj) {
-        const int t = li * G::kC + lj, i = P.i0 + li, j = P.j0 + lj;
-        T x = (T)0;
-        if (InGrid(v, i, j) && (v.code[i * v.Nx + j] & CODE_UNKNOWN))
-            x = sr[t] - ((T)v.dg[i * v.Nx + j] * se[t] - Sum2<T, G::kR, G::kC>(tab, se, li, lj));
-        sr[t] = x;
-    });
+    // the residual, over r (of both colours: the black one is what the division's rounding leaves, as in the per-cell
+    // kernels)
+#pragma unroll
+    for (int colour = 0; colour < 2; colour++)
+        ForColour<G::kR, G::kC>(P.i0, P.j0, 2 * kS, colour, [&](int li, int lj) {
+            const int t = li * G::kC + lj, i = P.i0 + li, j = P.j0 + lj;
+            T x = (T)0;
+            if (InGrid(v, i, j) && (v.code[i * v.Nx + j] & CODE_UNKNOWN))
+                x = sr[t] - (sd[t] * se[t] - Sum2<T, G::kR, G::kC>(tab, se, li, lj));
+            sr[t] = x;
+        });
     if (threadIdx.x >= (kOwnI / 2) * (kOwnJ / 2)) return;
     const int ii = threadIdx.x / (kOwnJ / 2), jj = threadIdx.x % (kOwnJ / 2);
     const int I = (P.i0 + kHalo + 1) / 2 + ii, J = (P.j0 + kHalo + 1) / 2 + jj;
     if (I > cv.Ny - 2 || J > cv.Nx - 2 || !(cv.code[I * cv.Nx + J] & CODE_UNKNOWN)) return;
     const T wt[4] = {(T)0.25, (T)0.75, (T)0.75, (T)0.25};
     T acc = (T)0;
+    // fine cell (2I - 2 + di, 2J - 2 + dj): I, J are the own region's (ii, jj)-th, whose first child is its first cell
+    const T *x = sr + (kHalo - 1 + 2 * ii) * G::kC + kHalo - 1 + 2 * jj;
 #pragma unroll
     for (int di = 0; di < 4; di++)
 #pragma unroll
-        for (int dj = 0; dj < 4; dj++)
+        for (int dj = 0; dj < 4; dj++) acc += wt[di] * wt[dj] * x[di * G::kC + dj];
+#pragma unroll
+    for (int di = 1; di < 3; di++)
+#pragma unroll
+        for (int dj = 1; dj < 3; dj++)
         {
-            // fine cell (2I - 2 + di, 2J - 2 + dj): I, J are the own region's (ii, jj)-th, whose first child is own
-            const int li = kHalo - 1 + 2 * ii + di, lj = kHalo - 1 + 2 * jj + dj, i = P.i0 + li, j = P.j0 + lj;
-            if ((i + j) & 1) continue;
-            const T x = sr[li * G::kC + lj];
-            acc += wt[di] * wt[dj] * x;
-            if ((di == 1 || di == 2) && (dj == 1 || dj == 2) && InGrid(v, i, j))
-                acc += (T)(ext[i * v.Nx + j] & 0x3Fu) * (T)(1.0 / 64.0) * x;
+            const int i = 2 * I - 2 + di, j = 2 * J - 2 + dj;
+            const unsigned m = InGrid(v, i, j) ? ext[i * v.Nx + j] & 0x3Fu : 0u;
+            if (m) acc += (T)m * (T)(1.0 / 64.0) * x[di * G::kC + dj];
         }
     rc[I * cv.Nx + J] = acc;
 }
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__(kThreads2) k_leg2_up(LevelView v, LevelView cv
     for (int t = threadIdx.x; t < G::kN; t += kThreads2)
     {
         const int i = P.i0 + t / G::kC, j = P.j0 + t % G::kC;
-        sd[t] = InGrid(v, i, j) ? (T)v.idg[i * v.Nx + j] : (T)0;
+        sd[t] = InGrid(v, i, j) ? (T)v.dg[i * v.Nx + j] : (T)0;
     }
     const int A0 = (P.i0 + kHalo + 1) / 2 - kS - 1, B0 = (P.j0 + kHalo + 1) / 2 - kS - 1;
     PdlWait();
@@ -248,14 +250,18 @@ __global__ void __launch_bounds__(kThreads2) k_leg2_up(LevelView v, LevelView cv
         if (!(x & 0x80u)) return;
         const int si = (i & 1) ? -kCC : kCC, sj = (j & 1) ? -1 : 1;
         const T *p = sc + (((i + 1) >> 1) - A0) * kCC + ((j + 1) >> 1) - B0;
-        se[li * G::kC + lj] += ((T)0.5625 * p[0] + (T)0.1875 * (p[si] + p[sj]) + (T)0.0625 * p[si + sj]) +
-                               (T)(x & 0x3Fu) * (T)(1.0 / 64.0) * p[0];
+        T acc = (T)0;
+        acc += (T)0.5625 * p[0];
+        acc += (T)0.1875 * p[sj];
+        acc += (T)0.1875 * p[si];
+        acc += (T)0.0625 * p[si + sj];
+        se[li * G::kC + lj] += acc + (T)(x & 0x3Fu) * (T)(1.0 / 64.0) * p[0];
     });
 #pragma unroll
     for (int h = 1; h <= 2 * kS; h++)
         ForColour<G::kR, G::kC>(P.i0, P.j0, h, h & 1, [&](int li, int lj) {
             const int t = li * G::kC + lj;
-            se[t] = (sr[t] + Sum2<T, G::kR, G::kC>(tab, se, li, lj)) * sd[t];
+            se[t] = OverDiag(sr[t] + Sum2<T, G::kR, G::kC>(tab, se, li, lj), sd[t]);
         });
     double acc[3] = {0.0, 0.0, 0.0};
     for (int t = threadIdx.x; t < kOwnI * kOwnJ; t += kThreads2)

@@ -448,9 +448,8 @@ void Context::BuildPairData()
         {
             const size_t c = (size_t)L[l].cells;
             L[l].diag.alloc(c);
-            L[l].rdiag.alloc(c);
             L[l].pext.alloc(c);
-            LaunchBuild2D(L[l].view(), L[l + 1].view(), L[l].diag.p, L[l].rdiag.p, L[l].pext.p, st);
+            LaunchBuild2D(L[l].view(), L[l + 1].view(), elem, L[l].diag.p, L[l].pext.p, st);
         }
         else if (L[l].du.p && l + 1 < L.size())
         {
@@ -908,12 +907,12 @@ template <typename T> void Context::VCycle(int l, T *r, T *e)
     {
         LevelData &Lc = L[l + 1];
         const LevelView vc = Lc.view();
-        prof(NB_K_SMOOTH0, 2.0 * s + 8.0 + s / 4.0); // reads r and the reciprocals, writes the iterate and the coarse r
+        prof(NB_K_SMOOTH0, 2.0 * s + 8.0 + s / 4.0); // reads r and the diagonals, writes the iterate and the coarse r
         LaunchLeg2Down<T>(v, vc, Lv.pext.p, r, Lv.res<T>(), Lc.r<T>(), PreSweeps(l), st);
         ProfEnd();
         if (l == 0) CoarseBracket<T>(l + 1, Lc.r<T>(), Lc.e<T>());
         else VCycle<T>(l + 1, Lc.r<T>(), Lc.e<T>());
-        prof(NB_K_PROLONG0, 3.0 * s + 9.0 + s / 4.0); // reads the iterate, r, the reciprocals and bytes, writes e
+        prof(NB_K_PROLONG0, 3.0 * s + 9.0 + s / 4.0); // reads the iterate, r, the diagonals and bytes, writes e
         LaunchLeg2Up<T>(v, vc, Lv.pext.p, r, Lv.res<T>(), Lc.e<T>(), e, PostSweeps(l), l == 0, red, iter.p, S_RZ0, S_RZ1,
                         st);
         ProfEnd();
