@@ -176,7 +176,7 @@ __global__ void kb_pass_begin(const BatchReq *__restrict__ rq, BatchList pass, i
 }
 
 // After a batched CG iteration: each listed request goes on while its iterations are below its cap and its r.r is
-// above its target and finite (the single solve's k_loop_cond); the list keeps those in order, and the WHILE node
+// above its target and finite (the single solve's LoopNext); the list keeps those in order, and the WHILE node
 // goes on while any is left. The loop also ends after maxLoop iterations whatever the requests' state (every
 // request's cap is below it), so it ends by construction. One block of up to 1024 threads (capacity <= 1024).
 __global__ void __launch_bounds__(1024) kb_inner_cond(cudaGraphConditionalHandle h, const BatchReq *__restrict__ rq,

@@ -383,9 +383,9 @@ constexpr int kWarps = kBlock / 32;
 // every block of the launch has read before any block can be the last).
 // addSlot0 >= 0 (sums only): each total also adds out[addSlot0 + s], the totals an earlier launch left there.
 // GridReduceB: the same over the blocks bid = 0 .. nblk-1 of one reduction (a batched launch runs one reduction per
-// request, each over its own blocks and Reducer).
+// request, each over its own blocks and Reducer). True on the one thread that stored the totals.
 template <int NV>
-__device__ __forceinline__ void GridReduceB(const Reducer &R, double (&val)[NV], int slot0, unsigned bid,
+__device__ __forceinline__ bool GridReduceB(const Reducer &R, double (&val)[NV], int slot0, unsigned bid,
                                             unsigned nblk, int op = 0, int *bump = nullptr, int addSlot0 = -1)
 {
     __shared__ double sh[NV][32];
@@ -414,7 +414,7 @@ __device__ __forceinline__ void GridReduceB(const Reducer &R, double (&val)[NV],
         amLast = (done == nblk - 1);
     }
     __syncthreads();
-    if (!amLast) return;
+    if (!amLast) return false;
     __threadfence();
 #pragma unroll
     for (int s = 0; s < NV; s++)
@@ -446,14 +446,29 @@ __device__ __forceinline__ void GridReduceB(const Reducer &R, double (&val)[NV],
         if (bump) *bump += 1;
         *R.counter = 0u;
     }
+    return tid == 0;
 }
 
 template <int NV>
-__device__ __forceinline__ void GridReduce(const Reducer &R, double (&val)[NV], int slot0, int op = 0,
+__device__ __forceinline__ bool GridReduce(const Reducer &R, double (&val)[NV], int slot0, int op = 0,
                                            int *bump = nullptr, int addSlot0 = -1)
 {
-    GridReduceB<NV>(R, val, slot0, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z),
+    return GridReduceB<NV>(R, val, slot0, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z),
                     gridDim.x * gridDim.y * gridDim.z, op, bump, addSlot0);
+}
+
+// The condition of the device-side CG loop (a WHILE node's handle), set by the x/r update that ends an iteration: go on
+// while the iterations done are below the cap, r.r is above its target and finite (the host loop's test). A launch of
+// its own for this took 2 us an iteration. on = 0: not inside the loop.
+struct LoopCond
+{
+    cudaGraphConditionalHandle h;
+    int on, slotTgt, slotMax, slotIts;
+};
+__device__ __forceinline__ void LoopNext(const LoopCond &c, double *S, int done, double rr)
+{
+    S[c.slotIts] = (double)done;
+    cudaGraphSetConditional(c.h, done < (int)S[c.slotMax] && rr > S[c.slotTgt] && isfinite(rr) ? 1u : 0u);
 }
 
 // The block coordinates of a launch's blocks within one request's grid: a single launch passes blockIdx and gridDim,

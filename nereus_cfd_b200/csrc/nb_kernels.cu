@@ -698,7 +698,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_update_xr(LevelView v, T *__restrict__ x, T *__restrict__ r, const T *p0,
                                                    const T *p1, const T *__restrict__ q, Reducer R, const double *S,
                                                    int *it, int baseEven, int baseOdd, int slotN, int singular,
-                                                   int slotPQ, int slotRR)
+                                                   int slotPQ, int slotRR, LoopCond lc)
 {
     const int par = *it & 1;
     const T *__restrict__ p = par ? p0 : p1;
@@ -717,17 +717,17 @@ __global__ void __launch_bounds__(256) k_update_xr(LevelView v, T *__restrict__ 
         r[c] = rn;
         acc[0] += (double)rn * (double)rn;
     }
-    GridReduce<1>(R, acc, slotRR, 0, it);
+    if (GridReduce<1>(R, acc, slotRR, 0, it) && lc.on) LoopNext(lc, R.out, *it, R.out[slotRR]);
 }
 
 template <typename T>
 void LaunchUpdateXR(const LevelView &v, T *x, T *r, const T *p0, const T *p1, const T *q, const Reducer &R,
                     const double *S, int *it, int baseEven, int baseOdd, int slotN, int singular, int slotPQ, int slotRR,
-                    cudaStream_t st)
+                    cudaStream_t st, const LoopCond &lc)
 {
     NB_COUNT_LAUNCH();
     k_update_xr<T><<<TileGrid(v), kTile, 0, st>>>(v, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular,
-                                                  slotPQ, slotRR);
+                                                  slotPQ, slotRR, lc);
 }
 
 template <typename Tin, typename Tout>
@@ -829,7 +829,8 @@ template void LaunchScaleSum<double>(long long, const double *, double *, double
     template void LaunchUpdatePApply<T>(const LevelView &, const T *, T *, T *, T *, const Reducer &,              \
                                         const double *, const int *, int, int, int, int, int, int, cudaStream_t);  \
     template void LaunchUpdateXR<T>(const LevelView &, T *, T *, const T *, const T *, const T *, const Reducer &, \
-                                    const double *, int *, int, int, int, int, int, int, cudaStream_t);
+                                    const double *, int *, int, int, int, int, int, int, cudaStream_t,         \
+                                    const LoopCond &);
 NB_INST(float)
 NB_INST(double)
 template void LaunchScaleCopy<double, float>(const LevelView &, const double *, float *, double, cudaStream_t);

@@ -102,13 +102,13 @@ void LaunchLinDot(long long cells, const float *r, const float *z, const Reducer
 template <typename T>
 void LaunchSplitLinXR(const LevelView &v, long long vecLen, T *x, T *r, const T *p0, const T *p1, const T *q,
                       const Reducer &R, const double *S, int *it, int baseEven, int baseOdd, int slotN,
-                      int singular, int slotPQ, int slotRR, cudaStream_t st);
+                      int singular, int slotPQ, int slotRR, cudaStream_t st, const LoopCond &lc = LoopCond{});
 void LaunchBatchLinXR(const BatchLevel *lv, int ls, const BatchReq *rq, BatchList a, int cap, int baseEven,
                       int baseOdd, int slotN, int slotPQ, int slotRR, cudaStream_t st);
 template <typename T>
 void LaunchLinXR(long long cells, T *x, T *r, const T *p0, const T *p1, const T *q, const Reducer &R,
                  const double *S, int *it, int baseEven, int baseOdd, int slotN, int singular, int slotPQ, int slotRR,
-                 cudaStream_t st);
+                 cudaStream_t st, const LoopCond &lc = LoopCond{});
 
 // ---- nb_split.cu: kernels for 3D levels in the colour-split layout (LevelView::sRS), T = float (the mixed form's
 //      inner solve) or double (the plain FP64 form) ----
@@ -242,7 +242,7 @@ void LaunchUpdatePApply(const LevelView &v, const T *z, T *p0, T *p1, T *q, cons
 template <typename T>
 void LaunchUpdateXR(const LevelView &v, T *x, T *r, const T *p0, const T *p1, const T *q, const Reducer &R,
                     const double *S, int *it, int baseEven, int baseOdd, int slotN, int singular, int slotPQ, int slotRR,
-                    cudaStream_t st);
+                    cudaStream_t st, const LoopCond &lc = LoopCond{});
 // r = sfac * b over all `cells` and out[slot..slot+1] = (sum b^2, sum b): the residual of a zero iterate
 template <typename T>
 void LaunchScaleSum(long long cells, const double *b, T *r, double sfac, const Reducer &R, int slot, cudaStream_t st);

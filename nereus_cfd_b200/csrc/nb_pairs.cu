@@ -977,7 +977,7 @@ template <typename T>
 __device__ __forceinline__ void LinXR(long long cells, T *__restrict__ x, T *__restrict__ r, const T *p0,
                                       const T *p1, const T *__restrict__ q, const Reducer &R, const double *S,
                                       int *it, int baseEven, int baseOdd, int slotN, int singular, int slotPQ,
-                                      int slotRR, int bx, int gx)
+                                      int slotRR, int bx, int gx, const LoopCond &lc = LoopCond{})
 {
     using V = typename Vec16<T>::V;
     constexpr int N = 16 / (int)sizeof(T);
@@ -1005,7 +1005,8 @@ __device__ __forceinline__ void LinXR(long long cells, T *__restrict__ x, T *__r
         r[t] = rn;
         acc[0] += (double)rn * rn;
     }
-    GridReduceB<1>(R, acc, slotRR, (unsigned)bx, (unsigned)gx, 0, it);
+    if (GridReduceB<1>(R, acc, slotRR, (unsigned)bx, (unsigned)gx, 0, it) && lc.on)
+        LoopNext(lc, R.out, *it, R.out[slotRR]);
 }
 
 // The same update on a colour-split level 0 with its tile activity (LevelView::act): the vector walked tile by tile
@@ -1015,7 +1016,8 @@ template <typename T>
 __device__ __forceinline__ void LinXRTiles(const LevelView &v, T *__restrict__ x, T *__restrict__ r,
                                            const T *p0, const T *p1, const T *__restrict__ q,
                                            const Reducer &R, const double *S, int *it, int baseEven, int baseOdd,
-                                           int slotN, int singular, int slotPQ, int slotRR, int bx, int gx)
+                                           int slotN, int singular, int slotPQ, int slotRR, int bx, int gx,
+                                           const LoopCond &lc = LoopCond{})
 {
     using V = typename Vec16<T>::V;
     constexpr int N = 16 / (int)sizeof(T);
@@ -1042,31 +1044,32 @@ __device__ __forceinline__ void LinXRTiles(const LevelView &v, T *__restrict__ x
             acc[0] += rr;
         }
     }
-    GridReduceB<1>(R, acc, slotRR, (unsigned)bx, (unsigned)gx, 0, it);
+    if (GridReduceB<1>(R, acc, slotRR, (unsigned)bx, (unsigned)gx, 0, it) && lc.on)
+        LoopNext(lc, R.out, *it, R.out[slotRR]);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_lin_xr_tiles(LevelView v, T *__restrict__ x, T *__restrict__ r,
                                                       const T *p0, const T *p1, const T *__restrict__ q,
                                                       Reducer R, const double *S, int *it, int baseEven, int baseOdd,
-                                                      int slotN, int singular, int slotPQ, int slotRR)
+                                                      int slotN, int singular, int slotPQ, int slotRR, LoopCond lc)
 {
     PdlWait();
     PdlTrigger();
     LinXRTiles<T>(v, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, (int)blockIdx.x,
-                  (int)gridDim.x);
+                  (int)gridDim.x, lc);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256) k_lin_xr(long long cells, T *__restrict__ x, T *__restrict__ r,
                                                 const T *p0, const T *p1, const T *__restrict__ q,
                                                 Reducer R, const double *S, int *it, int baseEven, int baseOdd, int slotN,
-                                                int singular, int slotPQ, int slotRR)
+                                                int singular, int slotPQ, int slotRR, LoopCond lc)
 {
     PdlWait();
     PdlTrigger();
     LinXR<T>(cells, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, (int)blockIdx.x,
-             (int)gridDim.x);
+             (int)gridDim.x, lc);
 }
 
 // batched (nb_batch.cu): block z runs the request at list[z]; r is its level 0's r
@@ -1106,39 +1109,43 @@ void LaunchBatchLinXR(const BatchLevel *lv, int ls, const BatchReq *rq, BatchLis
 template <typename T>
 void LaunchLinXR(long long cells, T *x, T *r, const T *p0, const T *p1, const T *q, const Reducer &R,
                  const double *S, int *it, int baseEven, int baseOdd, int slotN, int singular, int slotPQ, int slotRR,
-                 cudaStream_t st)
+                 cudaStream_t st, const LoopCond &lc)
 {
     const long long quads = cells * (long long)sizeof(T) / 16, want = (quads + 255) / 256;
     NB_COUNT_LAUNCH();
     LaunchPdl(k_lin_xr<T>, dim3((unsigned)(want < 1 ? 1 : std::min<long long>(want, kLinBlocks))), dim3(256), 0, st, cells, x, r, p0, p1, q, R, S, it, baseEven, baseOdd,
-              slotN, singular, slotPQ, slotRR);
+              slotN, singular, slotPQ, slotRR, lc);
 }
 
 template <typename T>
 void LaunchSplitLinXR(const LevelView &v, long long vecLen, T *x, T *r, const T *p0, const T *p1, const T *q,
                       const Reducer &R, const double *S, int *it, int baseEven, int baseOdd, int slotN, int singular,
-                      int slotPQ, int slotRR, cudaStream_t st)
+                      int slotPQ, int slotRR, cudaStream_t st, const LoopCond &lc)
 {
     if (!v.act)
     {
-        LaunchLinXR<T>(vecLen, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, st);
+        LaunchLinXR<T>(vecLen, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, st, lc);
         return;
     }
     // no more blocks than tiles: on a 66^3 level the last block had 1184 partial sums to add for 396 tiles
     NB_COUNT_LAUNCH();
     LaunchPdl(k_lin_xr_tiles<T>, dim3((unsigned)std::min(2 * v.Ny * v.actTiles, kLinBlocks)), dim3(256), 0, st, v, x, r, p0, p1, q, R, S, it, baseEven, baseOdd,
-              slotN, singular, slotPQ, slotRR);
+              slotN, singular, slotPQ, slotRR, lc);
 }
 
 template void LaunchLinXR<double>(long long, double *, double *, const double *, const double *, const double *,
-                                  const Reducer &, const double *, int *, int, int, int, int, int, int, cudaStream_t);
+                                  const Reducer &, const double *, int *, int, int, int, int, int, int, cudaStream_t,
+    const LoopCond &);
 template void LaunchLinXR<float>(long long, float *, float *, const float *, const float *, const float *,
-                                 const Reducer &, const double *, int *, int, int, int, int, int, int, cudaStream_t);
+                                 const Reducer &, const double *, int *, int, int, int, int, int, int, cudaStream_t,
+    const LoopCond &);
 template void LaunchSplitLinXR<float>(const LevelView &, long long, float *, float *, const float *, const float *,
                                       const float *, const Reducer &, const double *, int *, int, int, int, int, int,
-                                      int, cudaStream_t);
+                                      int, cudaStream_t,
+    const LoopCond &);
 template void LaunchSplitLinXR<double>(const LevelView &, long long, double *, double *, const double *,
                                        const double *, const double *, const Reducer &, const double *, int *, int,
-                                       int, int, int, int, int, cudaStream_t);
+                                       int, int, int, int, int, cudaStream_t,
+    const LoopCond &);
 
 } // namespace nb

@@ -1114,7 +1114,8 @@ template <typename T> void Context::VCycleSplit(int l, T *r, T *e)
 
 // One CG iteration on level 0: z = V-cycle(r), r.z, p = z + beta p (and q = M p, p.q), x += alpha p, r -= alpha q,
 // r.r copied to the host. The iteration number and the parity of the p buffers live on the device.
-template <typename T> void Context::IterBody(T *x, T *r, T *z, T *p0, T *p1, T *q, bool exact, bool copyRR)
+template <typename T>
+void Context::IterBody(T *x, T *r, T *z, T *p0, T *p1, T *q, bool exact, bool copyRR, const LoopCond &lc)
 {
     const LevelView v0 = L[0].view();
     const double s = sizeof(T), cells = (double)Cells();
@@ -1127,7 +1128,7 @@ template <typename T> void Context::IterBody(T *x, T *r, T *z, T *p0, T *p1, T *
         ProfEnd();
         ProfBegin(NB_K_XR, 6.0 * s * cells);
         LaunchSplitLinXR<T>(v0, (long long)VecLen0(), x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing,
-                            S_PQ, S_RR, st);
+                            S_PQ, S_RR, st, lc);
         ProfEnd();
         if (copyRR) NB_CK(cudaMemcpyAsync(hostSlots + S_RR, slots.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, st));
         return;
@@ -1147,7 +1148,8 @@ template <typename T> void Context::IterBody(T *x, T *r, T *z, T *p0, T *p1, T *
             LaunchPairPApply(v0, L[0].du.p, z, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, st);
             ProfEnd();
             ProfBegin(NB_K_XR, 6.0 * s * cells);
-            LaunchLinXR<float>(L[0].cells, x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, S_RR, st);
+            LaunchLinXR<float>(L[0].cells, x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, S_RR, st,
+                               lc);
             ProfEnd();
             if (copyRR)
                 NB_CK(cudaMemcpyAsync(hostSlots + S_RR, slots.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -1165,22 +1167,10 @@ template <typename T> void Context::IterBody(T *x, T *r, T *z, T *p0, T *p1, T *
     ProfEnd();
     ProfBegin(NB_K_XR, 6.0 * s * cells);
     if (Legs2D(0))
-        LaunchLinXR<T>(L[0].cells, x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, S_RR, st);
-    else LaunchUpdateXR<T>(v0, x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, S_RR, st);
+        LaunchLinXR<T>(L[0].cells, x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, S_RR, st, lc);
+    else LaunchUpdateXR<T>(v0, x, r, p0, p1, q, red, slots.p, iter.p, S_RZ0, S_RZ1, S_NUNK, sing, S_PQ, S_RR, st, lc);
     ProfEnd();
     if (copyRR) NB_CK(cudaMemcpyAsync(hostSlots + S_RR, slots.p + S_RR, sizeof(double), cudaMemcpyDeviceToHost, st));
-}
-
-// The loop condition of the device-side CG loop, after an iteration's x/r update: go on while the iterations done are
-// below the cap, r.r is above its target and finite (the host loop's test).
-__global__ void k_loop_cond(cudaGraphConditionalHandle h, double *S, const int *it, int slotRR, int slotTgt,
-                            int slotMax, int slotIts)
-{
-    const double rr = S[slotRR];
-    const int n = *it;
-    S[slotIts] = (double)n;
-    const bool go = n < (int)S[slotMax] && rr > S[slotTgt] && isfinite(rr);
-    cudaGraphSetConditional(h, go ? 1u : 0u);
 }
 
 template <typename T> void Context::BuildLoop(IterGraph *G, T *x, T *r, T *z, T *p0, T *p1, T *q, bool exact)
@@ -1211,9 +1201,7 @@ template <typename T> void Context::BuildLoop(IterGraph *G, T *x, T *r, T *z, T 
     bool ok = true;
     try
     {
-        IterBody<T>(x, r, z, p0, p1, q, exact, false);
-        NB_COUNT_LAUNCH();
-        k_loop_cond<<<1, 1, 0, st>>>(h, slots.p, iter.p, S_RR, S_TGT, S_MAXIT, S_ITS);
+        IterBody<T>(x, r, z, p0, p1, q, exact, false, LoopCond{h, 1, S_TGT, S_MAXIT, S_ITS});
     }
     catch (...)
     {
@@ -1475,9 +1463,8 @@ void Context::BuildSolveGraph()
         return unavailable();
     try
     {
-        IterBody<float>(x32.p, r32, z32, p32[0].p, p32[1].p, q32.p, false, false);
-        NB_COUNT_LAUNCH();
-        k_loop_cond<<<1, 1, 0, st>>>(hInner, slots.p, iter.p, S_RR, S_TGT, S_MAXIT, S_ITS);
+        IterBody<float>(x32.p, r32, z32, p32[0].p, p32[1].p, q32.p, false, false,
+                        LoopCond{hInner, 1, S_TGT, S_MAXIT, S_ITS});
     }
     catch (...)
     {

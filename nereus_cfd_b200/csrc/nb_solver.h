@@ -432,7 +432,9 @@ struct Context
     void AssignSplit();
     void BuildTailLists();
     // copyRR: end with the copy of r.r to the host (not inside the device-side loop)
-    template <typename T> void IterBody(T *x, T *r, T *z, T *p0, T *p1, T *q, bool exact, bool copyRR = true);
+    // lc: the loop condition the iteration sets when it is captured inside one
+    template <typename T>
+    void IterBody(T *x, T *r, T *z, T *p0, T *p1, T *q, bool exact, bool copyRR = true, const LoopCond &lc = LoopCond{});
     template <typename T> void BuildLoop(IterGraph *G, T *x, T *r, T *z, T *p0, T *p1, T *q, bool exact);
     template <typename T>
     int RunPCG(T *x, T *r, T *z, T *p0, T *p1, T *q, double rrStart, double rrTarget, int maxIt, bool exact,
