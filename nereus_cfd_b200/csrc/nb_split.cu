@@ -415,6 +415,21 @@ __device__ __forceinline__ void SplitProlong(const LevelView &fv, const LevelVie
     for (int A = A0; A < A1; A++)
     {
         T yP0[N + 1], yP1[N + 1], pP[N + 1];
+        // the four fine quads and their bytes, loaded with the coarse plane's rows: behind the stores of the first two,
+        // the last two waited for memory once more (258^3 level, FP32, B200: 31.8 -> 25.0 us)
+        Quad<T> ev[2][2];
+        unsigned wv[2][2];
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+        {
+            const long long o0 = (long long)min(2 * A - 1 + h, fv.Ny - 1) * fv.sPS + (long long)fb0 * fv.sRS + m0;
+            const long long o1 = one ? o0 : (long long)min(fb1, fv.Nx - 1) * fv.sRS - (long long)fb0 * fv.sRS + o0;
+            wv[h][0] = LdB<N>(pext + o0);
+            wv[h][1] = LdB<N>(pext + o1);
+            ev[h][0] = LQ(ef + o0);
+            ev[h][1] = LQ(ef + o1);
+            if (one) wv[h][1] = 0u;
+        }
         CoarsePlaneRows<T>(cv, ec, A + 1, B, m0, one, yP0, yP1, pP);
         // fine planes 2A-1 (with coarse plane A-1) and 2A (with A+1), rows 2B-1 and 2B
 #pragma unroll
@@ -422,8 +437,8 @@ __device__ __forceinline__ void SplitProlong(const LevelView &fv, const LevelVie
         {
             const int fa = 2 * A - 1 + h;
             const long long o0 = (long long)fa * fv.sPS + (long long)fb0 * fv.sRS + m0, o1 = o0 + fv.sRS;
-            const unsigned w0 = LdB<N>(pext + o0), w1 = one ? 0u : LdB<N>(pext + o1);
-            Quad<T> e0 = LQ(ef + o0), e1 = one ? Quad<T>{} : LQ(ef + o1);
+            const unsigned w0 = wv[h][0], w1 = wv[h][1];
+            Quad<T> &e0 = ev[h][0], &e1 = ev[h][1];
             const T *yo0 = h ? yP0 : yM0, *yo1 = h ? yP1 : yM1;
 #pragma unroll
             for (int rI = 0; rI < 2; rI++)
@@ -435,16 +450,16 @@ __device__ __forceinline__ void SplitProlong(const LevelView &fv, const LevelVie
 #pragma unroll
                 for (int k = 0; k <= N; k++)
                     z[k] = rI ? (T)0.75 * yC1[k] + (T)0.25 * yo1[k] : (T)0.75 * yC0[k] + (T)0.25 * yo0[k];
-                Quad<T> &ev = rI ? e1 : e0;
+                Quad<T> &er = rI ? e1 : e0;
 #pragma unroll
                 for (int x = 0; x < N; x++)
                 {
                     const unsigned px = Byte(w, x);
                     if (!(px & 0x80u)) continue;
                     const T lohi = q ? (T)0.25 * z[x] + (T)0.75 * z[x + 1] : (T)0.75 * z[x] + (T)0.25 * z[x + 1];
-                    ev.v[x] += lohi + (T)(px & 0x3Fu) * (T)(1.0 / 64.0) * (q ? pC[x + 1] : pC[x]);
+                    er.v[x] += lohi + (T)(px & 0x3Fu) * (T)(1.0 / 64.0) * (q ? pC[x + 1] : pC[x]);
                 }
-                SQ(ef + (rI ? o1 : o0), ev);
+                SQ(ef + (rI ? o1 : o0), er);
             }
         }
 #pragma unroll
@@ -459,10 +474,9 @@ __device__ __forceinline__ void SplitProlong(const LevelView &fv, const LevelVie
     }
 }
 
-// 3 resident blocks (80 registers, 40 bytes spilled) where the kernel would take 88: measured 14% faster on the 258^3
-// level (its grid of one block per SM or so is latency-bound)
+// 2 resident blocks: at 3 (80 registers) 136 bytes are spilled and the 258^3 level takes 28.1 us, here 25.0
 template <typename T, bool kX>
-__global__ void __launch_bounds__(kPairThreads, 3) k_split_prolong(LevelView fv, LevelView cv,
+__global__ void __launch_bounds__(kPairThreads, 2) k_split_prolong(LevelView fv, LevelView cv,
                                                                 const uint8_t *__restrict__ pext,
                                                                 const T *__restrict__ ec, T *__restrict__ ef)
 {
@@ -537,39 +551,64 @@ template <typename T, bool kX> __device__ __forceinline__ RowTaps<T, kX> TapsOf(
     return t;
 }
 
+// What one fine plane gives: four rows of N + 1 elements and the children's transfer bytes, all loaded before any is
+// used. With a branch around each row past the level's edge the rows were loaded one after the other, each waiting for
+// the last (258^3 level, FP32, B200: 31.7 -> 21.9 us); now such rows and planes read the ring, which is zero.
+template <typename T> struct RestrictLoads
+{
+    Quad<T> r[4];
+    T rN[4];
+    unsigned w[2], wN[2];
+};
 template <typename T, bool kX>
-__device__ __forceinline__ void SplitRestrictPlane(const LevelView &fv, const uint8_t *__restrict__ pext,
-                                                   const T *__restrict__ res, int a, const RowTaps<T, kX> &J, int K0,
-                                                   bool more, T (&Tw)[kQ<T>], T (&X)[kQ<T>])
+__device__ __forceinline__ RestrictLoads<T> LoadRestrict(const LevelView &fv, const uint8_t *__restrict__ pext,
+                                                         const T *__restrict__ res, int a, const RowTaps<T, kX> &J,
+                                                         int K0, bool more)
+{
+    constexpr int N = kQ<T>;
+    RestrictLoads<T> l;
+    const long long base = (long long)min(a, fv.Ny - 1) * fv.sPS + (K0 - 1);
+#pragma unroll
+    for (int dj = 0; dj < 4; dj++)
+    {
+        const long long row = base + (long long)min(J.b[dj], fv.Nx - 1) * fv.sRS;
+        l.r[dj] = LQ(res + row);
+        l.rN[dj] = more ? res[row + N] : (T)0;
+        if (dj == 1 || dj == 2)
+        {
+            l.w[dj - 1] = LdB<N>(pext + row);
+            l.wN[dj - 1] = more ? pext[row + N] : 0u;
+        }
+    }
+    return l;
+}
+
+template <typename T, bool kX>
+__device__ __forceinline__ void SplitRestrictPlane(const RestrictLoads<T> &l, int a, const RowTaps<T, kX> &J,
+                                                   T (&Tw)[kQ<T>], T (&X)[kQ<T>])
 {
     constexpr int N = kQ<T>;
 #pragma unroll
     for (int x = 0; x < N; x++) Tw[x] = X[x] = (T)0;
-    if (a > fv.Ny - 1) return;
 #pragma unroll
     for (int dj = 0; dj < 4; dj++)
     {
-        const int b = J.b[dj];
-        if (kX ? J.w[dj] == (T)0 : b > fv.Nx - 1) continue;
-        const int q = (a + b) & 1;
-        const long long row = (long long)a * fv.sPS + (long long)b * fv.sRS + (K0 - 1);
-        const Quad<T> r4 = LQ(res + row);
+        const int q = (a + J.b[dj]) & 1;
+        const bool none = kX && J.w[dj] == (T)0; // a tap that is not there
         T R[N + 1];
 #pragma unroll
-        for (int x = 0; x < N; x++) R[x] = r4.v[x];
-        R[N] = more ? res[row + N] : (T)0;
+        for (int x = 0; x < N; x++) R[x] = none ? (T)0 : l.r[dj].v[x];
+        R[N] = none ? (T)0 : l.rN[dj];
 #pragma unroll
         for (int x = 0; x < N; x++)
             Tw[x] += J.w[dj] * (q ? (T)0.75 * R[x] + (T)0.25 * R[x + 1] : (T)0.25 * R[x] + (T)0.75 * R[x + 1]);
         if (dj == 1 || (dj == 2 && J.two))
         {
-            const unsigned w = LdB<N>(pext + row);
-            const unsigned wN = more ? pext[row + N] : 0u;
 #pragma unroll
             for (int x = 0; x < N; x++)
             {
                 // the red child of coarse K0 + x is element K0 + x - q: index x + 1 - q of the N + 1
-                const unsigned pw = q ? Byte(w, x) : (x < N - 1 ? Byte(w, x + 1) : wN);
+                const unsigned pw = q ? Byte(l.w[dj - 1], x) : (x < N - 1 ? Byte(l.w[dj - 1], x + 1) : l.wN[dj - 1]);
                 X[x] += (T)(pw & 0x3Fu) * R[x + 1 - q];
             }
         }
@@ -600,13 +639,19 @@ __device__ __forceinline__ void SplitRestrictQ(const LevelView &fv, const LevelV
     const bool more = K0 + N - 1 <= cv.Nz - 2; // element K0+N-1 is read only for coarse cell K0+N-1
     const RowTaps<T, kX> taps = TapsOf<T, kX>(fv, J);
     T Tm2[N], Tm1[N], Xm1[N], Xd[N];
-    SplitRestrictPlane<T, kX>(fv, pext, res, 2 * I0 - 2, taps, K0, more, Tm2, Xd);
-    SplitRestrictPlane<T, kX>(fv, pext, res, 2 * I0 - 1, taps, K0, more, Tm1, Xm1);
+    {
+        const RestrictLoads<T> l0 = LoadRestrict<T, kX>(fv, pext, res, 2 * I0 - 2, taps, K0, more);
+        const RestrictLoads<T> l1 = LoadRestrict<T, kX>(fv, pext, res, 2 * I0 - 1, taps, K0, more);
+        SplitRestrictPlane<T, kX>(l0, 2 * I0 - 2, taps, Tm2, Xd);
+        SplitRestrictPlane<T, kX>(l1, 2 * I0 - 1, taps, Tm1, Xm1);
+    }
     for (int I = I0; I < I1; I++)
     {
         T T0[N], X0[N], T1[N], X1[N];
-        SplitRestrictPlane<T, kX>(fv, pext, res, 2 * I, taps, K0, more, T0, X0);
-        SplitRestrictPlane<T, kX>(fv, pext, res, 2 * I + 1, taps, K0, more, T1, X1);
+        const RestrictLoads<T> l0 = LoadRestrict<T, kX>(fv, pext, res, 2 * I, taps, K0, more);
+        const RestrictLoads<T> l1 = LoadRestrict<T, kX>(fv, pext, res, 2 * I + 1, taps, K0, more);
+        SplitRestrictPlane<T, kX>(l0, 2 * I, taps, T0, X0);
+        SplitRestrictPlane<T, kX>(l1, 2 * I + 1, taps, T1, X1);
         const long long c = (long long)I * cv.sI + (long long)J * cv.sJ + K0;
 #pragma unroll
         for (int x = 0; x < N; x++)
@@ -633,23 +678,42 @@ __global__ void __launch_bounds__(kPairThreads) k_split_restrict(LevelView fv, L
 
 // The same restriction with one thread per coarse cell (K along the 32 lanes, J across the 8 warps), for the smaller
 // coarse levels: more threads, and their launches are latency-bound.
-template <typename T, bool kX>
-__device__ __forceinline__ void SplitRestrictPlane1(const LevelView &fv, const uint8_t *pext, const T *res, int a,
-                                                   const RowTaps<T, kX> &J, int K, T &Tw, T &X)
+template <typename T> struct RestrictLoads1
 {
-    Tw = (T)0;
-    X = (T)0;
-    if (a > fv.Ny - 1) return;
+    T lo[4], hi[4];
+    unsigned w[2];
+};
+template <typename T, bool kX>
+__device__ __forceinline__ RestrictLoads1<T> LoadRestrict1(const LevelView &fv, const uint8_t *__restrict__ pext,
+                                                           const T *__restrict__ res, int a, const RowTaps<T, kX> &J,
+                                                           int K)
+{
+    RestrictLoads1<T> l;
 #pragma unroll
     for (int dj = 0; dj < 4; dj++)
     {
-        const int b = J.b[dj];
-        if (kX ? J.w[dj] == (T)0 : b > fv.Nx - 1) continue;
-        const int q = (a + b) & 1;
-        const long long row = (long long)a * fv.sPS + (long long)b * fv.sRS;
-        const T lo = res[row + K - 1], hi = res[row + K];
+        const long long row = (long long)min(a, fv.Ny - 1) * fv.sPS + (long long)min(J.b[dj], fv.Nx - 1) * fv.sRS + K;
+        l.lo[dj] = res[row - 1];
+        l.hi[dj] = res[row];
+        if (dj == 1 || dj == 2) l.w[dj - 1] = pext[row - ((a + J.b[dj]) & 1)];
+    }
+    return l;
+}
+
+template <typename T, bool kX>
+__device__ __forceinline__ void SplitRestrictPlane1(const RestrictLoads1<T> &l, int a, const RowTaps<T, kX> &J, T &Tw,
+                                                   T &X)
+{
+    Tw = (T)0;
+    X = (T)0;
+#pragma unroll
+    for (int dj = 0; dj < 4; dj++)
+    {
+        const int q = (a + J.b[dj]) & 1;
+        const bool none = kX && J.w[dj] == (T)0;
+        const T lo = none ? (T)0 : l.lo[dj], hi = none ? (T)0 : l.hi[dj];
         Tw += J.w[dj] * (q ? (T)0.75 * lo + (T)0.25 * hi : (T)0.25 * lo + (T)0.75 * hi);
-        if (dj == 1 || (dj == 2 && J.two)) X += (T)(pext[row + K - q] & 0x3Fu) * (q ? lo : hi);
+        if (dj == 1 || (dj == 2 && J.two)) X += (T)(l.w[dj - 1] & 0x3Fu) * (q ? lo : hi);
     }
     X *= (T)(1.0 / 64.0);
 }
@@ -672,13 +736,19 @@ __device__ __forceinline__ void SplitRestrict1(const LevelView &fv, const LevelV
     }
     const RowTaps<T, kX> taps = TapsOf<T, kX>(fv, J);
     T Tm2, Tm1, Xm1, Xdummy;
-    SplitRestrictPlane1<T, kX>(fv, pext, res, 2 * I0 - 2, taps, K, Tm2, Xdummy);
-    SplitRestrictPlane1<T, kX>(fv, pext, res, 2 * I0 - 1, taps, K, Tm1, Xm1);
+    {
+        const RestrictLoads1<T> l0 = LoadRestrict1<T, kX>(fv, pext, res, 2 * I0 - 2, taps, K);
+        const RestrictLoads1<T> l1 = LoadRestrict1<T, kX>(fv, pext, res, 2 * I0 - 1, taps, K);
+        SplitRestrictPlane1<T, kX>(l0, 2 * I0 - 2, taps, Tm2, Xdummy);
+        SplitRestrictPlane1<T, kX>(l1, 2 * I0 - 1, taps, Tm1, Xm1);
+    }
     for (int I = I0; I < I1; I++)
     {
         T T0, X0, T1, X1;
-        SplitRestrictPlane1<T, kX>(fv, pext, res, 2 * I, taps, K, T0, X0);
-        SplitRestrictPlane1<T, kX>(fv, pext, res, 2 * I + 1, taps, K, T1, X1);
+        const RestrictLoads1<T> l0 = LoadRestrict1<T, kX>(fv, pext, res, 2 * I, taps, K);
+        const RestrictLoads1<T> l1 = LoadRestrict1<T, kX>(fv, pext, res, 2 * I + 1, taps, K);
+        SplitRestrictPlane1<T, kX>(l0, 2 * I, taps, T0, X0);
+        SplitRestrictPlane1<T, kX>(l1, 2 * I + 1, taps, T1, X1);
         const long long c = (long long)I * cv.sI + (long long)J * cv.sJ + K;
         if (cv.code[c] & CODE_UNKNOWN)
             rc[VecIdx(cv, I, J, K)] = (((T)0.25 * Tm2 + (T)0.75 * Tm1) + ((T)0.75 * T0 + (T)0.25 * T1)) + (Xm1 + X0);
