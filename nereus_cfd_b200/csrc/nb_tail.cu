@@ -37,6 +37,7 @@ template <typename T> struct TailLevel
     LevelView v;
     unsigned off;     // byte offset of the level's arrays in shared memory
     unsigned listOff; // 4-byte offset of the level's prepared data in the global array
+    unsigned vecs; // vectors in shared memory: r, e and, but for the coarsest level, res
 };
 
 template <typename T> struct TailArgs
@@ -60,10 +61,11 @@ __host__ __device__ inline unsigned PrepBytes(long long cells)
     return Pad16((unsigned)cells * 4u) + 3u * Pad16((unsigned)cells);
 }
 
-// The level's arrays in shared memory: r, e, res (T), then its prepared data, each padded to 16 bytes.
-template <typename T> __host__ __device__ inline unsigned LevelBytes(long long cells)
+// The level's arrays in shared memory: r, e and, but for the coarsest level, res (T), then its prepared data, each padded
+// to 16 bytes.
+template <typename T> __host__ __device__ inline unsigned LevelBytes(long long cells, bool last)
 {
-    return 3u * Pad16((unsigned)(cells * sizeof(T))) + PrepBytes(cells);
+    return (last ? 2u : 3u) * Pad16((unsigned)(cells * sizeof(T))) + PrepBytes(cells);
 }
 
 template <typename T> struct SmemLevel
@@ -105,8 +107,8 @@ template <typename T> __device__ __forceinline__ SmemLevel<T> Bind(const TailLev
     s.r = (T *)base;
     s.e = (T *)(base + a);
     s.res = (T *)(base + 2 * a);
-    s.list = (unsigned *)(base + 3 * a);
-    s.unit = base + 3 * a + Pad16((unsigned)s.cells * 4u);
+    s.list = (unsigned *)(base + tl.vecs * a);
+    s.unit = base + tl.vecs * a + Pad16((unsigned)s.cells * 4u);
     s.ext = s.unit + b;
     s.types = s.ext + b;
     s.nRed = s.nBlack = 0;
@@ -407,7 +409,7 @@ __device__ __forceinline__ void TailStage(const TailArgs<T> &A, unsigned char *s
         const unsigned a = Pad16((unsigned)(S.cells * sizeof(T)));
         uint4 *z = reinterpret_cast<uint4 *>(S.r), *p = reinterpret_cast<uint4 *>(S.list);
         const uint4 *g = reinterpret_cast<const uint4 *>(A.lists + A.lv[l].listOff);
-        for (unsigned t = threadIdx.x; t < 3 * a / 16; t += blockDim.x) z[t] = make_uint4(0, 0, 0, 0);
+        for (unsigned t = threadIdx.x; t < A.lv[l].vecs * a / 16; t += blockDim.x) z[t] = make_uint4(0, 0, 0, 0);
         for (unsigned t = threadIdx.x; t < PrepBytes(S.cells) / 16; t += blockDim.x) p[t] = g[t];
     }
 }
@@ -566,7 +568,8 @@ template <typename T> static unsigned PlaceLevels(TailArgs<T> &A, const LevelVie
         A.lv[l].v = levels[l];
         A.lv[l].off = off;
         A.lv[l].listOff = listOff;
-        off += LevelBytes<T>(levels[l].cells);
+        A.lv[l].vecs = l + 1 < nlev ? 3 : 2;
+        off += LevelBytes<T>(levels[l].cells, l + 1 == nlev);
         listOff += PrepBytes(levels[l].cells) / 4;
     }
     A.nlev = nlev;
@@ -586,7 +589,7 @@ void LaunchTailLists(const LevelView *levels, int nlev, unsigned *lists, int *co
 template <typename T> size_t TailSmemBytes(const LevelView *levels, int nlev)
 {
     size_t bytes = 0;
-    for (int l = 0; l < nlev; l++) bytes += LevelBytes<T>(levels[l].cells);
+    for (int l = 0; l < nlev; l++) bytes += LevelBytes<T>(levels[l].cells, l + 1 == nlev);
     return bytes;
 }
 

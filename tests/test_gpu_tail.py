@@ -26,8 +26,9 @@ CASES = {"box_2d": lambda: W.closed_box_2d(67), "outlet_2d": lambda: W.cavity_ou
          "cylinder_3d": lambda: W.stretched_cylinder_3d(48, 20, 20)}
 
 
-# 256: warp-sized levels; 2048 (the default) and 5000: up to, and more than, an unknown of each colour per thread
-@pytest.mark.parametrize("tail_cells", [256, 2048, 5000])
+# 64: the coarsest level alone, although it has more cells; 256: warp-sized levels; 2048 (the default) and 5000: up to,
+# and more than, an unknown of each colour per thread
+@pytest.mark.parametrize("tail_cells", [64, 256, 2048, 5000])
 @pytest.mark.parametrize("precision", ["mixed", "fp64"])
 @pytest.mark.parametrize("name", sorted(CASES))
 def test_tail_agrees_with_its_levels_own_launches(nb, name, precision, tail_cells):
