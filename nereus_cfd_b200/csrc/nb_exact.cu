@@ -419,26 +419,47 @@ __global__ void k_rhs(LevelView v, Faces F, const double *p, double rhoDt, doubl
 // The same right-hand side on a uniform 3D grid with Nz even, two cells along k per thread (nb_device.cuh, PairPos):
 // the u faces of a pair are one aligned 16-byte load per row (u rows have Nz entries), the v faces one per plane (the
 // v plane of i+1 is kept for the next step of the march), the w faces three scalars (w rows have Nz+1 entries). Each
-// cell's expression is k_rhs's, operation for operation.
-__global__ void __launch_bounds__(kPairThreads, 4) k_pair_rhs(LevelView v, Faces F, const double *p, double rhoDt,
-                                                           double scale, double dh, double *b)
+// cell's expression is k_rhs's, operation for operation. A
+// plane's loads are issued a plane ahead, before the stores and divisions of the plane in hand: loading each plane where
+// it is used left the march waiting for memory (258^3 level, B200: 171 -> 157 us, at two blocks of 128 registers an SM).
+struct DivLoads
 {
-    const PairPos P = PairStart(v);
-    const long long uPlane = F.uI, wPlane = F.wI;
-    const int Nz = v.Nz;
+    double2 u0, u1, vP;  // the pair's u faces at j and j+1, its v faces at i+1
+    double w0, w1, w2;
+    unsigned code2;
+};
+__device__ __forceinline__ DivLoads LoadDiv(const LevelView &v, const Faces &F, const PairPos &P, int i)
+{
+    const long long c = P.base + (long long)(i - P.i0) * P.sI;
+    const long long cu = (long long)i * F.uI + (long long)P.j * v.Nz + P.k0;
+    const long long cw = (long long)i * F.wI + (long long)P.j * (v.Nz + 1) + P.k0;
+    DivLoads d;
+    d.u0 = *reinterpret_cast<const double2 *>(F.u + cu);
+    d.u1 = *reinterpret_cast<const double2 *>(F.u + cu + v.Nz);
+    d.vP = *reinterpret_cast<const double2 *>(F.v + c + P.sI);
+    d.w0 = F.w[cw];
+    d.w1 = F.w[cw + 1];
+    d.w2 = F.w[cw + 2];
+    d.code2 = *reinterpret_cast<const unsigned short *>(v.code + c);
+    return d;
+}
+
+__device__ __forceinline__ void PairRhs(const LevelView &v, const Faces &F, const double *p, double rhoDt,
+                                        double scale, double dh, double *b, const PairPos &P)
+{
+    if (P.i0 >= P.i1) return;
     // plane i's v faces (i, j, k) are the pair at the cell index; (i+1, j, k) one plane on
     double2 vC = *reinterpret_cast<const double2 *>(F.v + P.base);
+    DivLoads next = LoadDiv(v, F, P, P.i0);
     int off = 0;
     for (int i = P.i0; i < P.i1; i++, off += P.sI)
     {
         const long long c = P.base + off;
-        const long long cu = (long long)i * uPlane + (long long)P.j * Nz + P.k0;
-        const long long cw = (long long)i * wPlane + (long long)P.j * (Nz + 1) + P.k0;
-        const double2 u0 = *reinterpret_cast<const double2 *>(F.u + cu);
-        const double2 u1 = *reinterpret_cast<const double2 *>(F.u + cu + Nz);
-        const double2 vP = *reinterpret_cast<const double2 *>(F.v + c + P.sI);
-        const double w0 = F.w[cw], w1 = F.w[cw + 1], w2 = F.w[cw + 2];
-        const unsigned code2 = *reinterpret_cast<const unsigned short *>(v.code + c);
+        const DivLoads d = next;
+        if (i + 1 < P.i1) next = LoadDiv(v, F, P, i + 1);
+        const double2 u0 = d.u0, u1 = d.u1, vP = d.vP;
+        const double w0 = d.w0, w1 = d.w1, w2 = d.w2;
+        const unsigned code2 = d.code2;
         if (P.valid && (code2 & ((unsigned)CODE_UNKNOWN | ((unsigned)CODE_UNKNOWN << 8))))
         {
             double out[2];
@@ -473,7 +494,13 @@ __global__ void __launch_bounds__(kPairThreads, 4) k_pair_rhs(LevelView v, Faces
     }
 }
 
-Faces MakeFaces(const LevelView &v, const double *u, const double *vv, const double *w)
+__global__ void __launch_bounds__(kPairThreads, 2) k_pair_rhs(LevelView v, Faces F, const double *p, double rhoDt,
+                                                           double scale, double dh, double *b)
+{
+    PairRhs(v, F, p, rhoDt, scale, dh, b, PairStart(v));
+}
+
+__host__ __device__ Faces MakeFaces(const LevelView &v, const double *u, const double *vv, const double *w)
 {
     Faces F;
     F.u = u; F.v = vv; F.w = w;
@@ -514,23 +541,19 @@ __global__ void k_max_div(LevelView v, Faces F, double dh, Reducer R, int slot)
 }
 
 // The same check on a uniform 3D grid with Nz even, two cells per thread (the face loads of k_pair_rhs).
-__global__ void __launch_bounds__(kPairThreads) k_pair_max_div(LevelView v, Faces F, double dh, Reducer R, int slot)
+__device__ __forceinline__ void PairMaxDiv(const LevelView &v, const Faces &F, double dh, const Reducer &R, int slot,
+                                           const Blk &blk)
 {
-    const PairPos P = PairStart(v);
-    const int Nz = v.Nz;
+    const PairPos P = PairStart(v, blk.x, blk.y, blk.gy);
     double m[1] = {0.0};
-    double2 vC = *reinterpret_cast<const double2 *>(F.v + P.base);
-    int off = 0;
-    for (int i = P.i0; i < P.i1; i++, off += P.sI)
+    double2 vC = make_double2(0.0, 0.0);
+    if (P.i0 < P.i1) vC = *reinterpret_cast<const double2 *>(F.v + P.base);
+    for (int i = P.i0; i < P.i1; i++)
     {
-        const long long c = P.base + off;
-        const long long cu = (long long)i * F.uI + (long long)P.j * Nz + P.k0;
-        const long long cw = (long long)i * F.wI + (long long)P.j * (Nz + 1) + P.k0;
-        const double2 u0 = *reinterpret_cast<const double2 *>(F.u + cu);
-        const double2 u1 = *reinterpret_cast<const double2 *>(F.u + cu + Nz);
-        const double2 vP = *reinterpret_cast<const double2 *>(F.v + c + P.sI);
-        const double w0 = F.w[cw], w1 = F.w[cw + 1], w2 = F.w[cw + 2];
-        const unsigned code2 = *reinterpret_cast<const unsigned short *>(v.code + c);
+        const DivLoads L = LoadDiv(v, F, P, i);
+        const double2 u0 = L.u0, u1 = L.u1, vP = L.vP;
+        const double w0 = L.w0, w1 = L.w1, w2 = L.w2;
+        const unsigned code2 = L.code2;
         if (P.valid)
         {
             if (code2 & CODE_UNKNOWN)
@@ -546,7 +569,12 @@ __global__ void __launch_bounds__(kPairThreads) k_pair_max_div(LevelView v, Face
         }
         vC = vP;
     }
-    GridReduce<1>(R, m, slot, 1);
+    GridReduceB<1>(R, m, slot, BlkId(blk), BlkCount(blk), 1);
+}
+
+__global__ void __launch_bounds__(kPairThreads) k_pair_max_div(LevelView v, Faces F, double dh, Reducer R, int slot)
+{
+    PairMaxDiv(v, F, dh, R, slot, ThisBlk());
 }
 
 void LaunchMaxDiv(const LevelView &v, const double *u, const double *vv, const double *w, double dh,
@@ -736,9 +764,8 @@ void LaunchSumUnknowns(const LevelView &v, const double *x, const Reducer &R, in
 }
 
 // The same over the whole array in order, the unknowns told by their code byte (interior FLUID cells).
-__global__ void __launch_bounds__(256) k_lin_sub_mean_scatter(long long cells, const uint8_t *__restrict__ code,
-                                                              double *x, const double *sums, int n, int sub,
-                                                              double *p)
+__device__ __forceinline__ void LinSubMeanScatter(long long cells, const uint8_t *__restrict__ code, double *x,
+                                                  const double *sums, int n, int sub, double *p)
 {
     const double mean = sub ? (sums[0] + sums[1]) / (double)n : 0.0;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < cells;
@@ -749,6 +776,13 @@ __global__ void __launch_bounds__(256) k_lin_sub_mean_scatter(long long cells, c
         if (sub) x[t] = y;
         if (p) p[t] = y;
     }
+}
+
+__global__ void __launch_bounds__(256) k_lin_sub_mean_scatter(long long cells, const uint8_t *__restrict__ code,
+                                                              double *x, const double *sums, int n, int sub,
+                                                              double *p)
+{
+    LinSubMeanScatter(cells, code, x, sums, n, sub, p);
 }
 
 void LaunchSubMeanScatter(const LevelView &v, double *x, const double *sums, int n, int sub, double *p, cudaStream_t st)
@@ -788,7 +822,7 @@ __device__ __forceinline__ double RingValue(const LevelView &v, const double *p,
     }
 }
 
-__global__ void __launch_bounds__(256) k_ring_once(LevelView v, double *p)
+__device__ __forceinline__ void RingOnce(const LevelView &v, double *p)
 {
     const int Nx = v.Nx, Ny = v.Ny, Nz = v.Nz;
     // the y faces whole, the x faces without them, the z faces without either
@@ -824,6 +858,8 @@ __global__ void __launch_bounds__(256) k_ring_once(LevelView v, double *p)
         if (v.types[c] != PRESSURE) p[c] = RingValue(v, p, i, j, k);
     }
 }
+
+__global__ void __launch_bounds__(256) k_ring_once(LevelView v, double *p) { RingOnce(v, p); }
 
 // pass 0: y faces (i = 0, Ny-1) over (j, k); pass 1: x faces (j = 0, Nx-1) over (i, k); pass 2: z faces over (i, j)
 __global__ void k_ring(LevelView v, double *p, int pass)
@@ -971,86 +1007,119 @@ __device__ __forceinline__ double ProjGradV(const LevelView &g, int a, int i, in
 // behind a wall is stored back unchanged), its two w faces scalars; the pressures of the low neighbours come from
 // the pair loads of the previous plane and row and, along k, from the neighbouring lane. The block whose planes end
 // at Ny-2 also does the v faces of plane Ny-1 (v's loop runs to Ny-1).
-__global__ void __launch_bounds__(kPairThreads) k_pair_project(LevelView g, double *u, double *v, double *w,
-                                                               const double *p, double f)
+__device__ __forceinline__ void PairProject(const LevelView &g, double *u, double *v, double *w, const double *p,
+                                            double f, const PairPos &P)
 {
-    const PairPos P = PairStart(g);
     const int Nx = g.Nx, Ny = g.Ny, Nz = g.Nz, j = P.j;
     const int iEnd = (P.i0 < P.i1 && P.i1 == Ny - 1) ? Ny : P.i1;
+    // a plane's loads, all issued before anything of it is computed: with each load where it is used, behind the stores
+    // of the component before, a plane waited for memory four times (258^3, B200: 261 -> 243 us; loading a plane ahead
+    // as well takes 114 registers, and with two blocks an SM 337 us)
+    struct Loads
+    {
+        double2 pC, pJ, uu, vv;
+        double w0, w1, pEdge;
+        unsigned tC, tJ, tEdge;
+    };
+    const bool doU = P.valid && j >= 1, doV = doU && j <= Nx - 2;
+    auto load = [&](int i) {
+        const long long c = P.base + (long long)(i - P.i0) * P.sI;
+        Loads l = {};
+        l.pC = *reinterpret_cast<const double2 *>(p + c);
+        l.tC = *reinterpret_cast<const unsigned short *>(g.types + c);
+        if (P.lane == 0)
+        {
+            l.pEdge = p[c - 1];
+            l.tEdge = g.types[c - 1];
+        }
+        if (i <= Ny - 2 && doU)
+        {
+            l.uu = *reinterpret_cast<const double2 *>(u + ((long long)i * (Nx + 1) + j) * Nz + P.k0);
+            l.pJ = *reinterpret_cast<const double2 *>(p + c - P.sJ);
+            l.tJ = *reinterpret_cast<const unsigned short *>(g.types + c - P.sJ);
+            if (doV)
+            {
+                const long long fw = ((long long)i * Nx + j) * (Nz + 1) + P.k0;
+                l.w0 = w[fw];
+                l.w1 = w[fw + 1];
+            }
+        }
+        if (doV) l.vv = *reinterpret_cast<const double2 *>(v + c);
+        return l;
+    };
+    if (P.i0 >= iEnd) return;
     double2 pM = *reinterpret_cast<const double2 *>(p + P.base - P.sI);
     unsigned tM = *reinterpret_cast<const unsigned short *>(g.types + P.base - P.sI);
     int off = 0;
     for (int i = P.i0; i < iEnd; i++, off += P.sI)
     {
         const long long c = P.base + off;
-        const double2 pC = *reinterpret_cast<const double2 *>(p + c);
-        const unsigned tC = *reinterpret_cast<const unsigned short *>(g.types + c);
+        const Loads l = load(i);
+        const double2 pC = l.pC;
+        const unsigned tC = l.tC;
         double pKm = __shfl_up_sync(0xffffffffu, pC.y, 1);
         unsigned tKm = __shfl_up_sync(0xffffffffu, tC >> 8, 1);
         if (P.lane == 0)
         {
-            pKm = p[c - 1];
-            tKm = g.types[c - 1];
+            pKm = l.pEdge;
+            tKm = l.tEdge;
         }
-        if (P.valid)
+        const bool inner = i <= Ny - 2;
+        const double pc[2] = {pC.x, pC.y}, pm[2] = {pM.x, pM.y};
+        const int tc[2] = {(int)(tC & 0xFFu), (int)(tC >> 8)}, tm[2] = {(int)(tM & 0xFFu), (int)(tM >> 8)};
+        // u faces (i, j, k): i in [1, Ny-2], j in [1, Nx-1], k in [1, Nz-2]
+        if (inner && doU)
         {
-            const bool inner = i <= Ny - 2;
-            const double pc[2] = {pC.x, pC.y}, pm[2] = {pM.x, pM.y};
-            const int tc[2] = {(int)(tC & 0xFFu), (int)(tC >> 8)}, tm[2] = {(int)(tM & 0xFFu), (int)(tM >> 8)};
-            // u faces (i, j, k): i in [1, Ny-2], j in [1, Nx-1], k in [1, Nz-2]
-            if (inner && j >= 1)
-            {
-                const long long fu = ((long long)i * (Nx + 1) + j) * Nz + P.k0;
-                double2 uu = *reinterpret_cast<double2 *>(u + fu);
-                const double2 pJ = *reinterpret_cast<const double2 *>(p + c - P.sJ);
-                const unsigned tJ = *reinterpret_cast<const unsigned short *>(g.types + c - P.sJ);
-                double ux[2] = {uu.x, uu.y};
-                const double pj[2] = {pJ.x, pJ.y};
+            double ux[2] = {l.uu.x, l.uu.y};
+            const double pj[2] = {l.pJ.x, l.pJ.y};
 #pragma unroll
-                for (int h = 0; h < 2; h++)
-                {
-                    const int k = P.k0 + h;
-                    if (k < 1 || k > Nz - 2) continue;
-                    if (tc[h] == SOLID || (int)((tJ >> (8 * h)) & 0xFFu) == SOLID) continue;
-                    ux[h] = ux[h] - f * ProjGradV(g, 0, i, j, k, pc[h], pj[h]);
-                }
-                *reinterpret_cast<double2 *>(u + fu) = make_double2(ux[0], ux[1]);
+            for (int h = 0; h < 2; h++)
+            {
+                const int k = P.k0 + h;
+                if (k < 1 || k > Nz - 2) continue;
+                if (tc[h] == SOLID || (int)((l.tJ >> (8 * h)) & 0xFFu) == SOLID) continue;
+                ux[h] = ux[h] - f * ProjGradV(g, 0, i, j, k, pc[h], pj[h]);
             }
-            // v faces: i in [1, Ny-1], j in [1, Nx-2], k in [1, Nz-2]
-            if (j >= 1 && j <= Nx - 2)
-            {
-                const long long fv = c; // ((i * Nx + j) * Nz + k): the cell index
-                double2 vv = *reinterpret_cast<double2 *>(v + fv);
-                double vx[2] = {vv.x, vv.y};
+            *reinterpret_cast<double2 *>(u + ((long long)i * (Nx + 1) + j) * Nz + P.k0) = make_double2(ux[0], ux[1]);
+        }
+        // v faces: i in [1, Ny-1], j in [1, Nx-2], k in [1, Nz-2]
+        if (doV)
+        {
+            double vx[2] = {l.vv.x, l.vv.y};
 #pragma unroll
-                for (int h = 0; h < 2; h++)
-                {
-                    const int k = P.k0 + h;
-                    if (k < 1 || k > Nz - 2) continue;
-                    if (tc[h] == SOLID || tm[h] == SOLID) continue;
-                    vx[h] = vx[h] - f * ProjGradV(g, 1, i, j, k, pc[h], pm[h]);
-                }
-                *reinterpret_cast<double2 *>(v + fv) = make_double2(vx[0], vx[1]);
+            for (int h = 0; h < 2; h++)
+            {
+                const int k = P.k0 + h;
+                if (k < 1 || k > Nz - 2) continue;
+                if (tc[h] == SOLID || tm[h] == SOLID) continue;
+                vx[h] = vx[h] - f * ProjGradV(g, 1, i, j, k, pc[h], pm[h]);
             }
-            // w faces: i in [1, Ny-2], j in [1, Nx-2], k in [1, Nz-1]
-            if (inner && j >= 1 && j <= Nx - 2)
-            {
-                const long long fw = ((long long)i * Nx + j) * (Nz + 1) + P.k0;
-                const double plow[2] = {pKm, pC.x};
-                const int tlow[2] = {(int)tKm, tc[0]};
+            *reinterpret_cast<double2 *>(v + c) = make_double2(vx[0], vx[1]); // ((i * Nx + j) * Nz + k): the cell index
+        }
+        // w faces: i in [1, Ny-2], j in [1, Nx-2], k in [1, Nz-1]
+        if (inner && doV)
+        {
+            const long long fw = ((long long)i * Nx + j) * (Nz + 1) + P.k0;
+            const double plow[2] = {pKm, pC.x}, wx[2] = {l.w0, l.w1};
+            const int tlow[2] = {(int)tKm, tc[0]};
 #pragma unroll
-                for (int h = 0; h < 2; h++)
-                {
-                    const int k = P.k0 + h;
-                    if (k < 1 || k > Nz - 1) continue;
-                    if (tc[h] == SOLID || tlow[h] == SOLID) continue;
-                    w[fw + h] = w[fw + h] - f * ProjGradV(g, 2, i, j, k, pc[h], plow[h]);
-                }
+            for (int h = 0; h < 2; h++)
+            {
+                const int k = P.k0 + h;
+                if (k < 1 || k > Nz - 1) continue;
+                if (tc[h] == SOLID || tlow[h] == SOLID) continue;
+                w[fw + h] = wx[h] - f * ProjGradV(g, 2, i, j, k, pc[h], plow[h]);
             }
         }
         pM = pC;
         tM = tC;
     }
+}
+
+__global__ void __launch_bounds__(kPairThreads) k_pair_project(LevelView g, double *u, double *v, double *w,
+                                                               const double *p, double f)
+{
+    PairProject(g, u, v, w, p, f, PairStart(g));
 }
 
 void LaunchProject(const LevelView &g, double *u, double *v, double *w, const double *p, double dtOverRho,
