@@ -337,7 +337,7 @@ struct Batch
         Context &A = *ctx[0];
         if (A.opt.precision != NB_PRECISION_MIXED) throw InputError("the batched form runs the mixed precision");
         if (A.dim != 3 || A.nonuniform) throw InputError("the batched form takes uniform 3D grids");
-        if (A.tailStart < 1 || A.tailStart >= (int)A.L.size())
+        if (A.tailStart < 1 || A.tailStart >= (int)A.L.size() || A.L[A.tailStart].cells > (long long)A.opt.tail_cells)
             throw InputError("the batched form needs split levels above a shared-memory coarse end");
         for (int l = 0; l < A.tailStart; l++)
             if (!A.Split(l) || A.L[l].Nz % 2)
