@@ -11,8 +11,8 @@
 //     checks every listed request's r.r against its own target and iteration cap, compacts the work list (the
 //     converged requests leave it) and ends the loop when the list is empty;
 //   * the FP64 refinement around the inner solves is batched the same way, one host synchronisation per pass;
-//   * the FP64 steps before and after the solve (ring, right-hand side, compatibility, levelling, scatter,
-//     projection) run per request on the batch's stream.
+//   * the FP64 steps before and after the solve (ring, right-hand side, scatter, projection) run in one launch each for
+//     all requests; per request where one has a compatibility step.
 // Each request's sums run over its own blocks in a fixed order, so its result does not depend on the other requests
 // of the batch (alone or in any mix, in any slot, the same bits); the autotuner only picks shapes that cannot change
 // a result: the march length of the smoothing, residual and transfer kernels, timed on the batch itself and cached
@@ -250,6 +250,8 @@ struct Batch
                             // [2 cap + 1]: inner count, [2 cap + 2]: the inner loop's iterations
     DevArray<int> dParity;  // per request: this pass's iterate parity
     DevArray<double> dParams, dOut;
+    DevArray<BatchStep> dStep;   // the step around the solve, per request
+    BatchStep *hStep = nullptr;  // pinned
     double *hOut = nullptr; // pinned: params (2 cap), gathered slots (4 cap)
     int *hInt = nullptr;    // pinned: the pass list [0, cap), its count [2 cap], the parities [2 cap + 2, 3 cap + 2)
     bool dirty = true;      // a layout changed since the tables were written
@@ -289,6 +291,8 @@ struct Batch
         dOut.alloc(4 * (size_t)cap);
         NB_CK(cudaMallocHost((void **)&hOut, sizeof(double) * 6 * cap));
         NB_CK(cudaMallocHost((void **)&hInt, sizeof(int) * (3 * cap + 2)));
+        dStep.alloc(cap);
+        NB_CK(cudaMallocHost((void **)&hStep, sizeof(BatchStep) * cap));
     }
 
     ~Batch()
@@ -297,6 +301,7 @@ struct Batch
         ReleaseGraph();
         if (hOut) cudaFreeHost(hOut);
         if (hInt) cudaFreeHost(hInt);
+        if (hStep) cudaFreeHost(hStep);
         ctx.clear();
         if (ownStream && st) cudaStreamDestroy(st);
     }
@@ -634,11 +639,35 @@ struct Batch
         NB_CK(cudaEventCreate(&ev0));
         NB_CK(cudaEventCreate(&ev1));
         NB_CK(cudaEventRecord(ev0, st));
-        // ring, right-hand side, compatibility per request
+        // ring and right-hand side of all; with a compatibility step in one of them (its sums are launches of its own),
+        // request by request
+        bool compat = false;
         for (int i = 0; i < count; i++)
         {
             const nb_batch_item &it = items[i];
-            ctx[i]->BatchBegin(it.u, it.v, it.w, it.p, it.rho, it.dt, it.needs_compat);
+            ctx[i]->BatchCheck(it.u, it.v, it.w, it.p, it.rho, it.dt);
+            compat |= it.needs_compat && ctx[i]->singular && ctx[i]->n > 0;
+        }
+        auto steps = [&](auto &&x) {
+            for (int i = 0; i < count; i++)
+            {
+                const nb_batch_item &it = items[i];
+                const Context &C = *ctx[i];
+                hStep[i] = BatchStep{it.u,        it.v,          it.w,    it.p, C.b.p, x(i), it.rho / it.dt,
+                                     it.dt / it.rho, C.scale, C.dh, C.red};
+            }
+            NB_CK(cudaMemcpyAsync(dStep.p, hStep, sizeof(BatchStep) * count, cudaMemcpyHostToDevice, st));
+        };
+        if (!compat)
+        {
+            steps([&](int i) { return ctx[i]->xa.p; });
+            LaunchBatchRing(views[0], dLev.p, ls, dStep.p, count, st);
+            LaunchBatchRhs(views[0], dLev.p, ls, dStep.p, count, st);
+        }
+        for (int i = 0; i < count; i++)
+        {
+            const nb_batch_item &it = items[i];
+            if (compat) ctx[i]->BatchBegin(it.u, it.v, it.w, it.p, it.rho, it.dt, it.needs_compat);
             ctx[i]->xa.zero(st);
         }
         // the residual of x = 0 and ||b||^2 for all
@@ -715,12 +744,21 @@ struct Batch
             passes++;
         }
         // levelling, scatter, ring, velocity correction per request; max |div u| for all
-        for (int i = 0; i < count; i++)
+        auto solution = [&](int i) { return S[i].parity ? ctx[i]->xb.p : ctx[i]->xa.p; };
+        if (compat)
+            for (int i = 0; i < count; i++)
+            {
+                const nb_batch_item &it = items[i];
+                ctx[i]->BatchEnd(solution(i), it.u, it.v, it.w, it.p, it.rho, it.dt, it.needs_compat);
+            }
+        else
         {
-            Context &C = *ctx[i];
-            double *x = S[i].parity ? C.xb.p : C.xa.p;
-            const nb_batch_item &it = items[i];
-            C.BatchEnd(x, it.u, it.v, it.w, it.p, it.rho, it.dt, it.needs_compat);
+            // hStep's first copy is done: every path here has synchronised on the passes since
+            steps(solution);
+            LaunchBatchScatter(dLev.p, ls, dStep.p, count, st);
+            LaunchBatchRing(views[0], dLev.p, ls, dStep.p, count, st);
+            LaunchBatchProject(views[0], dLev.p, ls, dStep.p, count, st);
+            LaunchBatchMaxDiv(views[0], dLev.p, ls, dStep.p, count, S_DIV, st);
         }
         ListAll(count);
         NB_COUNT_LAUNCH();

@@ -31,6 +31,14 @@ struct BatchReq
     const void *tail; // its coarse end's TailArgs<float> (device memory)
 };
 
+// one request's step around the solve (fields in the grid layout; x: its solution)
+struct BatchStep
+{
+    double *u, *v, *w, *p, *b, *x;
+    double rhoDt, dtOverRho, scale, dh;
+    Reducer red;
+};
+
 // the requests a launch runs
 struct BatchList
 {

@@ -1192,4 +1192,84 @@ void LaunchScatterVolume(const LevelView &v, const int32_t *idp, const double *c
     k_scatter_volume<<<LineGrid(v.nLines, 148 * 8), kBlock, 0, st>>>(v, idp, compact, grid, volume);
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// the steps around a batch's solve (nb_batch.cu), one launch each for all its requests: block z runs request z. One
+// request of 128^3 fills the device for a fraction of its launch (16 x 6 launches took 1.8 ms of a 15.8 ms step).
+// ---------------------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) kb_ring(const BatchLevel *__restrict__ lv, int ls, const BatchStep *__restrict__ rq)
+{
+    RingOnce(lv[blockIdx.z * ls].v, rq[blockIdx.z].p);
+}
+
+__global__ void __launch_bounds__(kPairThreads, 2)
+    kb_pair_rhs(const BatchLevel *__restrict__ lv, int ls, const BatchStep *__restrict__ rq)
+{
+    const LevelView &v = lv[blockIdx.z * ls].v;
+    const BatchStep &q = rq[blockIdx.z];
+    PairRhs(v, MakeFaces(v, q.u, q.v, q.w), q.p, q.rhoDt, q.scale, q.dh, q.b, PairStart(v));
+}
+
+__global__ void __launch_bounds__(256)
+    kb_scatter(const BatchLevel *__restrict__ lv, int ls, const BatchStep *__restrict__ rq)
+{
+    const LevelView &v = lv[blockIdx.z * ls].v;
+    const BatchStep &q = rq[blockIdx.z];
+    LinSubMeanScatter(v.cells, v.code, q.x, nullptr, 1, 0, q.p);
+}
+
+__global__ void __launch_bounds__(kPairThreads)
+    kb_pair_project(const BatchLevel *__restrict__ lv, int ls, const BatchStep *__restrict__ rq)
+{
+    const LevelView &v = lv[blockIdx.z * ls].v;
+    const BatchStep &q = rq[blockIdx.z];
+    PairProject(v, q.u, q.v, q.w, q.p, q.dtOverRho, PairStart(v));
+}
+
+__global__ void __launch_bounds__(kPairThreads)
+    kb_pair_max_div(const BatchLevel *__restrict__ lv, int ls, const BatchStep *__restrict__ rq, int slot)
+{
+    const LevelView &v = lv[blockIdx.z * ls].v;
+    const BatchStep &q = rq[blockIdx.z];
+    PairMaxDiv(v, MakeFaces(v, q.u, q.v, q.w), q.dh, q.red, slot, ThisBlk());
+}
+
+static dim3 ForAll(dim3 g, int count)
+{
+    g.z = (unsigned)count;
+    return g;
+}
+
+void LaunchBatchRing(const LevelView &v, const BatchLevel *lv, int ls, const BatchStep *rq, int count, cudaStream_t st)
+{
+    const long long n = 2LL * v.Nx * v.Nz + 2LL * v.Ny * v.Nz + 2LL * v.Ny * v.Nx;
+    NB_COUNT_LAUNCH();
+    kb_ring<<<dim3((unsigned)std::min<long long>((n + 255) / 256, 148 * 8), 1, (unsigned)count), 256, 0, st>>>(lv, ls, rq);
+}
+
+void LaunchBatchRhs(const LevelView &v, const BatchLevel *lv, int ls, const BatchStep *rq, int count, cudaStream_t st)
+{
+    NB_COUNT_LAUNCH();
+    kb_pair_rhs<<<ForAll(PairGrid(v), count), kPairThreads, 0, st>>>(lv, ls, rq);
+}
+
+void LaunchBatchScatter(const BatchLevel *lv, int ls, const BatchStep *rq, int count, cudaStream_t st)
+{
+    NB_COUNT_LAUNCH();
+    kb_scatter<<<dim3(148 * 2, 1, (unsigned)count), 256, 0, st>>>(lv, ls, rq);
+}
+
+void LaunchBatchProject(const LevelView &v, const BatchLevel *lv, int ls, const BatchStep *rq, int count,
+                        cudaStream_t st)
+{
+    NB_COUNT_LAUNCH();
+    kb_pair_project<<<ForAll(PairGrid(v), count), kPairThreads, 0, st>>>(lv, ls, rq);
+}
+
+void LaunchBatchMaxDiv(const LevelView &v, const BatchLevel *lv, int ls, const BatchStep *rq, int count, int slot,
+                       cudaStream_t st)
+{
+    NB_COUNT_LAUNCH();
+    kb_pair_max_div<<<ForAll(PairGrid(v, 16), count), kPairThreads, 0, st>>>(lv, ls, rq, slot);
+}
+
 } // namespace nb

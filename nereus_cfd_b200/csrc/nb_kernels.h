@@ -51,6 +51,15 @@ void LaunchGather(const LevelView &v, const int32_t *idp, const double *grid, do
 void LaunchScatterVolume(const LevelView &v, const int32_t *idp, const double *compact, double *grid, int volume,
                          cudaStream_t st);
 
+// the steps around a batch's solve, for all its requests at once (requests without compatibility)
+void LaunchBatchRing(const LevelView &v, const BatchLevel *lv, int ls, const BatchStep *rq, int count, cudaStream_t st);
+void LaunchBatchRhs(const LevelView &v, const BatchLevel *lv, int ls, const BatchStep *rq, int count, cudaStream_t st);
+void LaunchBatchScatter(const BatchLevel *lv, int ls, const BatchStep *rq, int count, cudaStream_t st);
+void LaunchBatchProject(const LevelView &v, const BatchLevel *lv, int ls, const BatchStep *rq, int count,
+                        cudaStream_t st);
+void LaunchBatchMaxDiv(const LevelView &v, const BatchLevel *lv, int ls, const BatchStep *rq, int count, int slot,
+                       cudaStream_t st);
+
 // ---- nb_tail.cu: the coarse end of the V-cycle in one thread block, in shared memory ----
 constexpr int kMaxTailLevels = 8;
 constexpr size_t kTailMaxSmem = 200 * 1024;

@@ -1810,11 +1810,17 @@ int Context::ProjectDevice(double *u, double *v, double *w, double *p, double rh
     return status;
 }
 
-void Context::BatchBegin(double *u, double *v, double *w, double *p, double rho, double dt, int compat)
+void Context::BatchCheck(const double *u, const double *v, const double *w, const double *p, double rho,
+                         double dt) const
 {
     if (!built) throw InputError("set_layout has not been called");
     if (!u || !v || !p || (dim == 3 && !w)) throw InputError("null field pointer");
     if (!(rho > 0.0) || !(dt > 0.0)) throw InputError("rho and dt must be positive");
+}
+
+void Context::BatchBegin(double *u, double *v, double *w, double *p, double rho, double dt, int compat)
+{
+    BatchCheck(u, v, w, p, rho, dt);
     const LevelView v0 = L[0].view();
     LaunchRing(v0, p, st);
     LaunchRhs(v0, u, v, w, p, rho / dt, scale, dh, b.p, st);

@@ -348,6 +348,7 @@ struct Context
     // A batch's halves of the Chorin step around its solve (nb_batch.cu), on this context's stream: Begin checks the
     // call and runs the ring, the right-hand side and the compatibility step; End levels x, scatters it into p, runs
     // the ring and the velocity correction and leaves max |div u| in slot S_DIV.
+    void BatchCheck(const double *u, const double *v, const double *w, const double *p, double rho, double dt) const;
     void BatchBegin(double *u, double *v, double *w, double *p, double rho, double dt, int compat);
     void BatchEnd(double *x, double *u, double *v, double *w, double *p, double rho, double dt, int compat);
     void Rhs(const double *u, const double *v, const double *w, const double *p, double rho, double dt, double *bOut);
