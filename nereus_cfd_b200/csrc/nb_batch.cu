@@ -269,6 +269,7 @@ struct Batch
     std::vector<LevelTune> tuning;
     cudaGraph_t loop = nullptr;
     cudaGraphExec_t loopExec = nullptr;
+    int forms = 0; // the forms the loop launches: bit 0 requests that are not singular, bit 1 singular ones
     long long loopLaunches = 0;
     double tuneMs = 0.0;
 
@@ -474,7 +475,7 @@ struct Batch
     void IterBody(BatchList a)
     {
         VCycle(a);
-        LaunchBatchSplitPApply(views[0], dLev.p, ls, dReq.p, a, cap, S_RZ0, S_RZ1, S_NUNK, S_PQ, st);
+        LaunchBatchSplitPApply(views[0], dLev.p, ls, dReq.p, a, cap, S_RZ0, S_RZ1, S_NUNK, S_PQ, forms, st);
         LaunchBatchLinXR(dLev.p, ls, dReq.p, a, cap, S_RZ0, S_RZ1, S_NUNK, S_PQ, S_RR, st);
     }
 
@@ -631,6 +632,13 @@ struct Batch
         if (tuning.size() != (size_t)nLev)
         {
             Tune(count);
+            ReleaseGraph();
+        }
+        int need = 0;
+        for (int i = 0; i < count; i++) need |= ctx[i]->singular ? 2 : 1;
+        if (need & ~forms)
+        {
+            forms |= need;
             ReleaseGraph();
         }
         if (!loopExec) BuildLoop();

@@ -168,7 +168,7 @@ void LaunchBatchSplit(int kind, const LevelView &v, const LevelView *coarse, int
 void LaunchBatchSplitHalfDot(const LevelView &v, const BatchLevel *lv, int ls, const BatchReq *rq, BatchList a,
                              int cap, int colour, bool last, int baseEven, int baseOdd, int partSlot, cudaStream_t st);
 void LaunchBatchSplitPApply(const LevelView &v, const BatchLevel *lv, int ls, const BatchReq *rq, BatchList a,
-                            int cap, int baseEven, int baseOdd, int slotN, int slotPQ, cudaStream_t st);
+                            int cap, int baseEven, int baseOdd, int slotN, int slotPQ, int forms, cudaStream_t st);
 void LaunchBatchSplitScaleSum(const BatchLevel *lv, int ls, const BatchReq *rq, BatchList a, int cap, int slot,
                               cudaStream_t st);
 void LaunchBatchSplitRefine64(const LevelView &v, const BatchLevel *lv, int ls, const BatchReq *rq, BatchList a,

@@ -1199,10 +1199,13 @@ __global__ void __launch_bounds__(256) kb_split_restrict1(const BatchLevel *__re
     SplitRestrict1<float, false>(F.v, C.v, F.pext, F.res, C.r, (int)blockIdx.x, by, bz, gz);
 }
 
-// form -1: every request in its own form; 0 / 1: only the requests of that form (singular = 1)
-__global__ void __launch_bounds__(kPairThreads, 4)
+// The requests of one form (singular or not), each form in a kernel and a launch of its own: both inlined into one
+// kernel took 64 registers with 552 bytes spilled, apart they spill 128 and 180 at 80 registers. 16 tanks of 128^3, the
+// step: 16.1 ms in one kernel, 15.8 apart at 3 blocks an SM, 16.2 at 2.
+template <bool kSingular>
+__global__ void __launch_bounds__(kPairThreads, 3)
     kb_split_papply(const BatchLevel *__restrict__ lv, int ls, const BatchReq *__restrict__ rq, BatchList a,
-                    int baseEven, int baseOdd, int slotN, int slotPQ, int form)
+                    int baseEven, int baseOdd, int slotN, int slotPQ)
 {
     PdlWait();
     PdlTrigger();
@@ -1210,13 +1213,9 @@ __global__ void __launch_bounds__(kPairThreads, 4)
     if (q < 0) return;
     const BatchLevel &L = lv[q * ls];
     const BatchReq &Q = rq[q];
-    if (form >= 0 && (Q.singular != 0) != (form == 1)) return;
-    if (Q.singular)
-        SplitPApply<float, true>(L.v, L.du, L.e, Q.p0, Q.p1, Q.q, Q.red, Q.red.out, Q.it, baseEven, baseOdd, slotN, slotPQ,
-                          ThisBlk());
-    else
-        SplitPApply<float, false>(L.v, L.du, L.e, Q.p0, Q.p1, Q.q, Q.red, Q.red.out, Q.it, baseEven, baseOdd, slotN, slotPQ,
-                           ThisBlk());
+    if ((Q.singular != 0) != kSingular) return;
+    SplitPApply<float, kSingular>(L.v, L.du, L.e, Q.p0, Q.p1, Q.q, Q.red, Q.red.out, Q.it, baseEven, baseOdd, slotN,
+                                  slotPQ, ThisBlk());
 }
 
 __global__ void __launch_bounds__(256) kb_split_scale_sum(const BatchLevel *__restrict__ lv, int ls,
@@ -1326,24 +1325,22 @@ void LaunchBatchSplitHalfDot(const LevelView &v, const BatchLevel *lv, int ls, c
                   rq, a, colour, baseEven, baseOdd, partSlot);
 }
 
+// forms: bit 0, some request is not singular; bit 1, some request is. Each on the grid a single solve of its form uses.
 void LaunchBatchSplitPApply(const LevelView &v, const BatchLevel *lv, int ls, const BatchReq *rq, BatchList a,
-                            int cap, int baseEven, int baseOdd, int slotN, int slotPQ, cudaStream_t st)
+                            int cap, int baseEven, int baseOdd, int slotN, int slotPQ, int forms, cudaStream_t st)
 {
-    // a single solve launches its form (singular or not) on that form's grid; both have the same occupancy unless
-    // the compiler gave them different register counts, and then each form gets a launch on its own grid
-    const dim3 gs = QuadGrid<4>(v, Occ<k_split_papply<float, true>>()), gn = QuadGrid<4>(v, Occ<k_split_papply<float, false>>());
-    if (gs.x == gn.x && gs.y == gn.y)
+    if (forms & 1)
     {
         NB_COUNT_LAUNCH();
-        LaunchPdl(kb_split_papply, WithZ(gn, cap), kPairThreads, 0, st, lv, ls, rq, a, baseEven, baseOdd, slotN,
-                  slotPQ, -1);
-        return;
+        LaunchPdl(kb_split_papply<false>, WithZ(QuadGrid<4>(v, Occ<k_split_papply<float, false>>()), cap), kPairThreads, 0,
+                  st, lv, ls, rq, a, baseEven, baseOdd, slotN, slotPQ);
     }
-    NB_COUNT_LAUNCHES(2);
-    LaunchPdl(kb_split_papply, WithZ(gn, cap), kPairThreads, 0, st, lv, ls, rq, a, baseEven, baseOdd, slotN, slotPQ,
-              0);
-    LaunchPdl(kb_split_papply, WithZ(gs, cap), kPairThreads, 0, st, lv, ls, rq, a, baseEven, baseOdd, slotN, slotPQ,
-              1);
+    if (forms & 2)
+    {
+        NB_COUNT_LAUNCH();
+        LaunchPdl(kb_split_papply<true>, WithZ(QuadGrid<4>(v, Occ<k_split_papply<float, true>>()), cap), kPairThreads, 0,
+                  st, lv, ls, rq, a, baseEven, baseOdd, slotN, slotPQ);
+    }
 }
 
 void LaunchBatchSplitScaleSum(const BatchLevel *lv, int ls, const BatchReq *rq, BatchList a, int cap, int slot,
