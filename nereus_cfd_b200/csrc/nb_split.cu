@@ -63,7 +63,7 @@ __device__ __forceinline__ void SplitFirst(const LevelView &v, const uint8_t *__
         Quad<T> a = LQ(R0 + o);
         const unsigned d = LdB<N>(D0 + o);
 #pragma unroll
-        for (int x = 0; x < 4; x++) a.v[x] *= inv[Byte(d, x) & 0x7Fu];
+        for (int x = 0; x < N; x++) a.v[x] *= inv[Byte(d, x) & 0x7Fu];
         return a;
     };
     auto red1 = [&](long long o) { return R0[o] * inv[D0[o] & 0x7Fu]; };
