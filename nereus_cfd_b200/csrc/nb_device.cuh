@@ -385,9 +385,10 @@ constexpr int kWarps = kBlock / 32;
 // GridReduceB: the same over the blocks bid = 0 .. nblk-1 of one reduction (a batched launch runs one reduction per
 // request, each over its own blocks and Reducer). True on the one thread that stored the totals.
 //
-// Its latency ends every launch of a CG iteration that sums (about 5 us of a 12 us half-sweep on a 130^3 level), so: a lane
-// per value adds the warps' sums, one acquire-release addition to the counter orders the partials (two full fences and
-// one thread adding all the sums before; with this, box 128^2 0.81 -> 0.76 ms, 128^3 FLIP step 12.9 -> 12.6), and the totals to add are read before the partials.
+// Its latency ends every launch of a CG iteration that sums (about 5 us of a 12 us half-sweep on a 130^3 level), so a lane
+// per value adds the warps' sums, one acquire-release addition to the counter orders the partials, and the totals to add
+// are read before the partials. With one thread adding all the sums and two full fences: 128^2 box 0.81 ms (0.76 now), a
+// FLIP pass at 128^3 12.9 ms (12.6).
 __device__ __forceinline__ unsigned CountUp(unsigned *counter)
 {
     unsigned old;

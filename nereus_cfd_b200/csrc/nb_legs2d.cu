@@ -10,8 +10,8 @@
 //
 // The values are those of the per-cell kernels (nb_kernels.cu): the same coefficients (the level's FP32 tables; 1 on a
 // uniform level), diagonal (kept per cell, once per layout), sums in the same order and division, so that a solve ends
-// where it ended with a launch per operation. Reciprocals and sums by pairs instead were no faster and moved the
-// pressure by 3e-8 of itself (FP32 rounding, carried through a solve to 1e-8).
+// where it ended with a launch per operation. Reciprocals and sums by pairs instead took 6% off the step and
+// moved the pressure by up to 3e-7 of itself (FP32 rounding, carried through a solve to 1e-8).
 //
 // Measured (B200): the 128^2 closed box's step in mixed precision to 1e-10 (13 iterations, two such levels) 1.03 -> 0.79 ms
 // with the ring replay in one launch.
