@@ -70,7 +70,7 @@ typedef struct nb_options
                             captured from a layout's second solve on: the first solve after a change of shape
                             launches plainly (capturing costs more than it saves once). All give the same result */
     int transfer_kernels; /* the restriction of colour-split levels: 0 (default): one thread per 4 coarse cells
-                             where the coarse level has at least 2^20 cells, else one thread per coarse cell (a
+                             where the coarse level has at least 2^17 cells, else one thread per coarse cell (a
                              batch: per 4 everywhere); 1: one thread per coarse cell everywhere; 2: one thread per 4
                              coarse cells everywhere. All three give the same result in a single solve */
     int pair_kernels;    /* kernels of 3D levels: 2 (default): the colour-split layout, red and black cells in separate

@@ -529,7 +529,7 @@ struct Batch
                                                                      : SplitDefaultS(views[l], k);
             // one thread per four coarse cells at every level unless forced: a batched launch has the capacity times
             // a single solve's threads, so the per-cell kernel's extra threads buy nothing (measured on 64 tanks of
-            // 128^3: 3.7% faster whole steps than per cell below 2^20 coarse cells, the single solve's rule)
+            // 128^3: 3.7% faster whole steps than per cell below 2^20 coarse cells, the single solve's rule then)
             T.mode = (opt.transfer_kernels == 1 || opt.transfer_kernels == 2) ? opt.transfer_kernels : 2;
         }
         if (!opt.autotune) return;

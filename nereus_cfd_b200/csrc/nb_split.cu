@@ -769,8 +769,10 @@ __global__ void __launch_bounds__(256) k_split_restrict1(LevelView fv, LevelView
 
 // Coarse levels with at least kRestrictQuadCells cells take the quad kernel (4x fewer loads per coarse cell), the
 // smaller ones the per-cell kernel (mode 0); mode 1 takes the per-cell kernel and mode 2 the quad kernel everywhere.
-// Both sum the same products in the same order.
-constexpr long long kRestrictQuadCells = 1LL << 20;
+// Both sum the same products in the same order. Restriction from 194^3, 162^3, 130^3 and 98^3, per cell against quads
+// (B200, us): FP32 17.9 / 15.6, 15.8 / 13.4, 11.6 / 9.8, 9.6 / 9.4; FP64 25.1 / 17.8, 16.5 / 15.3, 15.5 / 12.2,
+// 9.5 / 9.6. The line lies between the last two (coarse levels of 66^3 and 50^3).
+constexpr long long kRestrictQuadCells = 1LL << 17;
 
 template <typename T, bool kX>
 static void RestrictOn(const LevelView &fine, const LevelView &coarse, const uint8_t *pext, const T *resFine,
