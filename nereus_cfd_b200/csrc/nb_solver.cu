@@ -396,8 +396,9 @@ void Context::BuildPairData()
     // are FP32 (the mixed form's inner solve)
     const bool mixed = opt.precision == NB_PRECISION_MIXED;
     const int elem = mixed ? (int)sizeof(float) : (int)sizeof(double);
-    for (auto &Lv : L)
+    for (size_t l = 0; l < L.size(); l++)
     {
+        LevelData &Lv = L[l];
         const LevelView v = Lv.view();
         if (Lv.sRS || (mixed && opt.pair_kernels && PairLevelShape(v)))
         {
@@ -441,7 +442,7 @@ void Context::BuildPairData()
         else
         {
             Lv.du.release();
-            Lv.diag.release();
+            if (!Legs2D((int)l)) Lv.diag.release(); // built below, in place: captured iterations hold its pointer
             Lv.rdiag.release();
         }
     }
@@ -468,10 +469,20 @@ void Context::BuildPairData()
     }
 }
 
+// The device arrays a captured iteration reads besides the solver's vectors.
+std::vector<const void *> Context::LayoutPointers() const
+{
+    std::vector<const void *> out{tables.p, tailLists.p, tailCounts.p};
+    for (const LevelData &Lv : L)
+        out.insert(out.end(), {Lv.types.p, Lv.code.p, Lv.du.p, Lv.pext.p, Lv.diag.p, Lv.rdiag.p, Lv.act.p});
+    return out;
+}
+
 // A new layout with the hierarchy's shape (sizes and spacing tables) unchanged: the cell types, codes and pair bytes of
 // every level are rebuilt in the arrays they have; pointers, tail and captured iterations stay as they are.
 void Context::RefillHierarchy()
 {
+    const std::vector<const void *> before = LayoutPointers();
     L[0].types.upload(layout.data(), layout.size(), st);
     LaunchBuildCodes(L[0].view(), L[0].code.p, st);
     for (size_t l = 1; l < L.size(); l++)
@@ -482,6 +493,7 @@ void Context::RefillHierarchy()
     BuildPairData();
     BuildTailLists();
     NB_CK(cudaGetLastError());
+    if (LayoutPointers() != before) throw std::logic_error("a refilled hierarchy's arrays moved");
 }
 
 // The tail levels' lists of unknowns by colour (they follow the cell types).

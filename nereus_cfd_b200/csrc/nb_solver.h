@@ -365,6 +365,7 @@ struct Context
     friend struct Batch;
     void BuildHierarchy();
     void RefillHierarchy();
+    std::vector<const void *> LayoutPointers() const;
     void BuildPairData();
     void EnsureIdp();
     void AllocVectors();
