@@ -795,6 +795,7 @@ struct Batch
             r.max_div = hOut[i];
             r.seconds = ms * 1e-3;
             r.status = S[i].status;
+            if (!std::isfinite(r.rel_res)) C.ClearVectors();
             C.lastIterations = r.iters_inner;
             if (r.status != NB_OK) worst = r.status;
         }

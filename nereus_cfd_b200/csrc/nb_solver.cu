@@ -561,6 +561,22 @@ void Context::AllocVectors()
     }
 }
 
+// The solver's vectors as a layout starts with them. The kernels keep what is no unknown (solids, ring, the colour-split
+// rows' padding) at zero by multiplying with zero, which an infinity or a NaN survives: after a solve that overflowed they
+// are zeroed again, or the next one would start from what it left there.
+void Context::ClearVectors()
+{
+    for (auto &Lv : L)
+    {
+        Lv.r32.zero(st); Lv.e32.zero(st); Lv.res32.zero(st);
+        Lv.r64.zero(st); Lv.e64.zero(st); Lv.res64.zero(st);
+    }
+    for (auto &a : p32) a.zero(st);
+    for (auto &a : p64) a.zero(st);
+    q32.zero(st); x32.zero(st);
+    q64.zero(st); x64.zero(st);
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // context
 // ---------------------------------------------------------------------------------------------------------------
@@ -1678,6 +1694,7 @@ int Context::Solve(double tol, double **xOut, nb_result *out, const double *gues
     }
     const int status = opt.precision == NB_PRECISION_MIXED ? SolveMixed(tol, xOut, out, guess, refNorm)
                                                            : SolveFP64(tol, xOut, out, guess, refNorm);
+    if (!std::isfinite(out->rel_res)) ClearVectors();
     solvesOnShape++;
     return status;
 }

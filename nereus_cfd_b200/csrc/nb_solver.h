@@ -369,6 +369,7 @@ struct Context
     void BuildPairData();
     void EnsureIdp();
     void AllocVectors();
+    void ClearVectors();
     double ReadSlot(int s);
     void ReadSlots(int s, int count);
     // Solve A x = b (b in this->b, grid layout); the solution ends in *xOut (xa or xb). Fills out->iters/rel_res.

@@ -344,3 +344,46 @@ def test_pressure_ring_replay(nb, shape):
     s.SolvePressure(m, tol=1e-8)
     s.DestroyPressureSolver()
     assert np.array_equal(m.p.reshape(shape), expect)
+
+
+# (interior x, y, z): Nz odd and even, both with rows that the colour-split layout pads
+@pytest.mark.parametrize("sweeps", [1, 2])
+@pytest.mark.parametrize("form", ["mixed_odd", "mixed_even", "fp64_odd", "fp64_even", "fp64_stretched"])
+def test_an_overflowed_solve_leaves_nothing_behind(nb, form, sweeps):
+    """A step whose solve overflows (NOT_CONVERGED, no finite pressure), then an ordinary one on the same solver: what a
+    fresh solver gives, bit for bit. The mixed form overflows in FP32 from velocities of 1e60. The FP64 form's products
+    have to pass 1.8e308 where |b|^2 stays below: on cells of 1e6 the solver's units scale b by 1e12; on the stretched
+    grid of thin cells r.z is above r.r (an eigenvalue of the operator is at most twice its diagonal, here below 0.4)."""
+    precision, shape = form.split("_")
+    dh = 1.0 if precision == "mixed" else 1e6
+    if shape == "stretched":
+        case = W.stretched_cylinder_3d(24, 16, 17)
+    else:
+        n = (20, 18, 17 if shape == "odd" else 18)
+        g = W.uniform_grid(3, (0.0, n[0] * dh, 0.0, n[1] * dh, 0.0, n[2] * dh), 18)
+        assert (g.Nx, g.Ny, g.Nz) == (n[0] + 2, n[1] + 2, n[2] + 2)
+        case = W.Case("box", g, W.walls_scene(3, outlet_face=1), 41)
+    g, types = case.grid, capi.label_cells(case.grid, case.scene)
+    assert 2 * ((((g.Nz + 1) // 2) + 3) // 4 * 4) >= g.Nz + 2
+    u, v, w = W.face_velocities(g, types, case.seed)
+
+    def step(s, scale):
+        m = MACGrid(g, types.copy(), scale * u, scale * v, scale * w, np.zeros(g.cells), case.rho, case.dt)
+        return s.SolvePressure(m, tol=1e-9), m
+
+    options = dict(pre_sweeps=sweeps, post_sweeps=sweeps, stretched_sweeps=sweeps)
+    fresh = PressureSolver(precision, **options)
+    r0, m0 = step(fresh, 1.0)
+    assert r0.status == capi.NB_OK and r0.levels >= 2
+    fresh.DestroyPressureSolver()
+    s = PressureSolver(precision, **options)
+    big = 1e60 if precision == "mixed" else (1.2e154 if shape == "stretched" else 1e147) / r0.b_norm
+    for _ in range(2):
+        r, m = step(s, big)
+        assert r.status == capi.NB_NOT_CONVERGED and np.isfinite(r.b_norm) and not np.all(np.isfinite(m.p))
+        for _ in range(2):
+            r, m = step(s, 1.0)
+            assert (r.status, r.iters_inner, r.rel_res) == (r0.status, r0.iters_inner, r0.rel_res)
+            for a, b in ((m.p, m0.p), (m.u, m0.u), (m.v, m0.v), (m.w, m0.w)):
+                assert np.array_equal(a, b)
+    s.DestroyPressureSolver()
