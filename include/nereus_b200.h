@@ -437,6 +437,9 @@ int nereus_b200_x_groups(const double *widths, int n, double yz_min, int32_t *co
  * Returns the coarse extent Nc (rings included; xr needs room for n + 2), 0 when the groups are the regular pairing
  * of every axis (nothing written), or NB_BAD_INPUT. */
 int nereus_b200_x_maps(const double *widths, int n, double yz_min, int32_t *xp, int32_t *xr);
+/* The partial sums (thread blocks of the largest launch that ends in a grid-wide sum) a solver keeps per value for a
+ * grid of these sizes, ring included, at least 65536 (host only). NB_BAD_INPUT for sizes no layout may have. */
+int nereus_b200_sum_blocks(int dim, int Nx, int Ny, int Nz);
 int nereus_b200_tune_key(int Nx, int Ny, int Nz, int level, int kind, int capacity, char *buf, int size);
 int nereus_b200_tune_cache_dump(char *buf, int size);
 int nereus_b200_tune_cache_load(const char *text);

@@ -585,6 +585,12 @@ int nereus_b200_x_groups(const double *widths, int n, double yz_min, int32_t *co
     return (int)c.size();
 }
 
+int nereus_b200_sum_blocks(int dim, int Nx, int Ny, int Nz)
+{
+    if ((dim != 2 && dim != 3) || Nx < 2 || Ny < 2 || (dim == 3 && Nz < 2)) return Fail(NB_BAD_INPUT, "bad grid sizes");
+    return nb::SumBlocks(dim, Nx, Ny, dim == 3 ? Nz : 1);
+}
+
 int nereus_b200_x_maps(const double *widths, int n, double yz_min, int32_t *xp, int32_t *xr)
 {
     if (!widths || !xp || !xr || n < 1 || !(yz_min > 0.0)) return Fail(NB_BAD_INPUT, "bad x widths");

@@ -9,6 +9,7 @@
 
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <stdexcept>
 
 namespace nb
 {
@@ -297,8 +298,11 @@ inline int MarchPlanes(long long planes, long long perPlane)
     return (int)(s < 1 ? 1 : (s > kPairS ? kPairS : s));
 }
 
-// The launch grid of a pair kernel; minS: at least this many planes per thread (the launches that end in a
-// grid-wide sum keep their partial sums few).
+// planes per thread at least in the pair-thread launches that end in a grid-wide sum: fewer blocks, fewer partial sums for
+// the last block to add (measured: 16 beats the 8 of the plain sweeps there)
+constexpr int kSumPlanes = 16;
+
+// The launch grid of a pair kernel; minS: at least this many planes per thread.
 inline dim3 PairGridOf(long long pairs, long long planes, int minS)
 {
     const long long perPlane = (pairs + kPairThreads - 1) / kPairThreads;
@@ -373,6 +377,14 @@ struct Reducer
     double *out;        // scalar slots
     int maxBlocks;
 };
+
+// The grid of a launch that ends in a grid-wide sum over R. With more blocks than R holds partial sums for, those of one
+// value would run into the next one's (Context::SetLayout sizes R for the layout's largest such grid).
+inline dim3 SumGrid(const Reducer &R, dim3 g)
+{
+    if ((long long)g.x * g.y * g.z > R.maxBlocks) throw std::length_error("more blocks than a reduction has partial sums");
+    return g;
+}
 
 constexpr int kBlock = 256;            // threads per block of the line kernels
 constexpr int kWarps = kBlock / 32;

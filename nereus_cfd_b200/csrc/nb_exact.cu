@@ -582,9 +582,9 @@ void LaunchMaxDiv(const LevelView &v, const double *u, const double *vv, const d
 {
     NB_COUNT_LAUNCH();
     if (v.dim == 3 && !v.stretched && v.Nz % 2 == 0 && v.code && v.Ny >= 3)
-        k_pair_max_div<<<PairGrid(v, 16), kPairThreads, 0, st>>>(v, MakeFaces(v, u, vv, w), dh, R, slot);
+        k_pair_max_div<<<SumGrid(R, PairGrid(v, kSumPlanes)), kPairThreads, 0, st>>>(v, MakeFaces(v, u, vv, w), dh, R, slot);
     else
-        k_max_div<<<TileGrid(v), dim3(kTileF, kTileM), 0, st>>>(v, MakeFaces(v, u, vv, w), dh, R, slot);
+        k_max_div<<<SumGrid(R, TileGrid(v)), dim3(kTileF, kTileM), 0, st>>>(v, MakeFaces(v, u, vv, w), dh, R, slot);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -688,10 +688,9 @@ template <typename T>
 void LaunchResidual64(const LevelView &v, const double *b, const double *x, T *rOut, double scale, double sfac,
                       const Reducer &R, int slot, cudaStream_t st)
 {
-    const int blocks = LineGrid(v.nLines > 0 ? v.nLines : 1, R.maxBlocks);
     NB_COUNT_LAUNCH();
-    k_residual64<T, false><<<TileGrid(v), dim3(kTileF, kTileM), 0, st>>>(v, b, x, (const T *)nullptr, nullptr, rOut,
-                                                                          scale, sfac, R, slot, nullptr);
+    k_residual64<T, false><<<SumGrid(R, TileGrid(v)), dim3(kTileF, kTileM), 0, st>>>(
+        v, b, x, (const T *)nullptr, nullptr, rOut, scale, sfac, R, slot, nullptr);
 }
 
 template <typename T>
@@ -699,8 +698,8 @@ void LaunchRefine64(const LevelView &v, const double *b, const double *xin, cons
                     double scale, double sfac, const Reducer &R, int slot, cudaStream_t st, const int *swap)
 {
     NB_COUNT_LAUNCH();
-    k_residual64<T, true><<<TileGrid(v), dim3(kTileF, kTileM), 0, st>>>(v, b, xin, e, xout, rOut, scale, sfac, R, slot,
-                                                                         swap);
+    k_residual64<T, true><<<SumGrid(R, TileGrid(v)), dim3(kTileF, kTileM), 0, st>>>(v, b, xin, e, xout, rOut, scale, sfac,
+                                                                                    R, slot, swap);
 }
 
 template void LaunchResidual64<float>(const LevelView &, const double *, const double *, float *, double, double,
@@ -758,9 +757,8 @@ __global__ void k_sub_mean_scatter(LevelView v, double *x, const double *sums, i
 
 void LaunchSumUnknowns(const LevelView &v, const double *x, const Reducer &R, int slot, cudaStream_t st)
 {
-    const int blocks = LineGrid(v.nLines > 0 ? v.nLines : 1, R.maxBlocks);
     NB_COUNT_LAUNCH();
-    k_sum_unknowns<<<TileGrid(v), dim3(kTileF, kTileM), 0, st>>>(v, x, R, slot);
+    k_sum_unknowns<<<SumGrid(R, TileGrid(v)), dim3(kTileF, kTileM), 0, st>>>(v, x, R, slot);
 }
 
 // The same over the whole array in order, the unknowns told by their code byte (interior FLUID cells).
@@ -1269,7 +1267,7 @@ void LaunchBatchMaxDiv(const LevelView &v, const BatchLevel *lv, int ls, const B
                        cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    kb_pair_max_div<<<ForAll(PairGrid(v, 16), count), kPairThreads, 0, st>>>(lv, ls, rq, slot);
+    kb_pair_max_div<<<ForAll(PairGrid(v, kSumPlanes), count), kPairThreads, 0, st>>>(lv, ls, rq, slot);
 }
 
 } // namespace nb

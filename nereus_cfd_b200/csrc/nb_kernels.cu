@@ -613,7 +613,7 @@ void LaunchDot(const LevelView &v, const T *r, const T *z, const Reducer &R, con
                cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    k_dot<T><<<TileGrid(v), kTile, 0, st>>>(v, r, z, R, it, baseEven, baseOdd);
+    k_dot<T><<<SumGrid(R, TileGrid(v)), kTile, 0, st>>>(v, r, z, R, it, baseEven, baseOdd);
 }
 
 // n (the unknowns) is read from S[slotN] on the device, so a captured iteration outlives a change of the layout
@@ -686,11 +686,11 @@ void LaunchUpdatePApply(const LevelView &v, const T *z, T *p0, T *p1, T *q, cons
 {
     NB_COUNT_LAUNCH();
     if (exact)
-        LaunchPdl(k_update_p_apply<T, true>, TileGrid(v), kTile, 0, st, v, z, p0, p1, q, R, S, it, baseEven, baseOdd,
-                  slotN, singular, slotPQ);
+        LaunchPdl(k_update_p_apply<T, true>, SumGrid(R, TileGrid(v)), kTile, 0, st, v, z, p0, p1, q, R, S, it, baseEven,
+                  baseOdd, slotN, singular, slotPQ);
     else
-        LaunchPdl(k_update_p_apply<T, false>, TileGrid(v), kTile, 0, st, v, z, p0, p1, q, R, S, it, baseEven, baseOdd,
-                  slotN, singular, slotPQ);
+        LaunchPdl(k_update_p_apply<T, false>, SumGrid(R, TileGrid(v)), kTile, 0, st, v, z, p0, p1, q, R, S, it, baseEven,
+                  baseOdd, slotN, singular, slotPQ);
 }
 
 // alpha = rz/pq; x += alpha p_new; r -= alpha q; sum r.r. The last block advances the iteration counter.
@@ -726,8 +726,8 @@ void LaunchUpdateXR(const LevelView &v, T *x, T *r, const T *p0, const T *p1, co
                     cudaStream_t st, const LoopCond &lc)
 {
     NB_COUNT_LAUNCH();
-    k_update_xr<T><<<TileGrid(v), kTile, 0, st>>>(v, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular,
-                                                  slotPQ, slotRR, lc);
+    k_update_xr<T><<<SumGrid(R, TileGrid(v)), kTile, 0, st>>>(v, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN,
+                                                              singular, slotPQ, slotRR, lc);
 }
 
 template <typename Tin, typename Tout>
@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(256) k_count_unknowns(LevelView v, Reducer R, 
 void LaunchCountUnknowns(const LevelView &v, const Reducer &R, int slot, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    k_count_unknowns<<<TileGrid(v), kTile, 0, st>>>(v, R, slot);
+    k_count_unknowns<<<SumGrid(R, TileGrid(v)), kTile, 0, st>>>(v, R, slot);
 }
 
 // r = sfac * b over the whole level and (sum b^2, sum b): the FP64 residual b - A x of a zero iterate. b is zero off

@@ -122,6 +122,8 @@ void LaunchLinXR(long long cells, T *x, T *r, const T *p0, const T *p1, const T 
 // ---- nb_split.cu: kernels for 3D levels in the colour-split layout (LevelView::sRS), T = float (the mixed form's
 //      inner solve) or double (the plain FP64 form) ----
 bool SplitLevelShape(const LevelView &v);
+// the most blocks a launch takes that ends in a grid-wide sum over a level of this shape (either precision)
+long long SplitSumBlocks(const LevelView &v);
 // du: the level's diagonal units in that layout (a stretched level reads their unknown flag only, and runs the sweeps
 // of nb_stretched.cu, FP64 only); pext: the red cells' bytes
 // reads the kernels' occupancy (their grids follow it); call before capturing launches into a graph
@@ -193,6 +195,7 @@ void LaunchLegUpDot(const LevelView &v, const LevelView &cv, const uint8_t *du, 
 
 // ---- nb_legs2d.cu: a 2D level's descent and ascent in one launch each (1 or 2 sweeps before and after the coarse
 //      correction); ext: the moved transfer weights, built with the diagonal once per layout ----
+long long Leg2SumBlocks(const LevelView &v); // the blocks of the ascent's sums
 void LaunchBuild2D(const LevelView &v, const LevelView &cv, int elemBytes, double *dg, uint8_t *ext, cudaStream_t st);
 template <typename T>
 void LaunchLeg2Down(const LevelView &v, const LevelView &cv, const uint8_t *ext, const T *r, T *tmp, T *rc, int sweeps,

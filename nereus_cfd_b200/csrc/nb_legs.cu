@@ -340,8 +340,8 @@ void LaunchLegUpDot(const LevelView &v, const LevelView &cv, const uint8_t *du, 
                     cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    LaunchPdl(k_leg_up<T, true>, LegGrid(cv), dim3(kLegThreads), 0, st, v, cv, du, pext, r, tmp, ec, e, R, it, baseEven,
-              baseOdd);
+    LaunchPdl(k_leg_up<T, true>, SumGrid(R, LegGrid(cv)), dim3(kLegThreads), 0, st, v, cv, du, pext, r, tmp, ec, e, R, it,
+              baseEven, baseOdd);
 }
 
 #define NB_INST(T)                                                                                                 \

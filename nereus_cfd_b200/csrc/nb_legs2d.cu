@@ -286,6 +286,12 @@ static dim3 Leg2Grid(const LevelView &v)
     return dim3((unsigned)((v.Nx - 2 + kOwnJ - 1) / kOwnJ), (unsigned)((v.Ny - 2 + kOwnI - 1) / kOwnI));
 }
 
+long long Leg2SumBlocks(const LevelView &v)
+{
+    const dim3 g = Leg2Grid(v);
+    return (long long)g.x * g.y;
+}
+
 template <typename T>
 void LaunchLeg2Down(const LevelView &v, const LevelView &cv, const uint8_t *ext, const T *r, T *tmp, T *rc, int sweeps,
                     cudaStream_t st)
@@ -302,7 +308,8 @@ void LaunchLeg2Up(const LevelView &v, const LevelView &cv, const uint8_t *ext, c
 {
     NB_COUNT_LAUNCH();
     auto go = [&](auto kernel) {
-        LaunchPdl(kernel, Leg2Grid(v), dim3(kThreads2), 0, st, v, cv, ext, r, tmp, ec, e, R, it, baseEven, baseOdd);
+        LaunchPdl(kernel, dot ? SumGrid(R, Leg2Grid(v)) : Leg2Grid(v), dim3(kThreads2), 0, st, v, cv, ext, r, tmp, ec, e, R,
+                  it, baseEven, baseOdd);
     };
     if (sweeps == 1) dot ? go(k_leg2_up<T, 1, true>) : go(k_leg2_up<T, 1, false>);
     else dot ? go(k_leg2_up<T, 2, true>) : go(k_leg2_up<T, 2, false>);

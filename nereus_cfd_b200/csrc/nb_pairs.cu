@@ -80,10 +80,6 @@ void LaunchBuildDu(const LevelView &v, uint8_t *du, cudaStream_t st)
     k_build_du<<<blocks, 256, 0, st>>>(v, du);
 }
 
-// planes per thread at least in the launches that end in a grid-wide sum: fewer blocks, fewer partial sums for the
-// last block to add (measured: 16 beats the 8 of the plain sweeps there)
-constexpr int kReduceS = 16;
-
 // ---------------------------------------------------------------------------------------------------------------
 // smoothing
 // ---------------------------------------------------------------------------------------------------------------
@@ -476,8 +472,8 @@ void LaunchPairHalfStDot(const LevelView &v, const float *r, float *e, int colou
                          int baseEven, int baseOdd, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    k_pair_half_st<true, false><<<PairGrid(v, kReduceS), kPairThreads, 0, st>>>(v, r, e, colour, R, it, baseEven,
-                                                                               baseOdd);
+    k_pair_half_st<true, false><<<SumGrid(R, PairGrid(v, kSumPlanes)), kPairThreads, 0, st>>>(v, r, e, colour, R, it,
+                                                                                             baseEven, baseOdd);
 }
 
 void LaunchPairResidualSt(const LevelView &v, const float *r, const float *e, float *res, cudaStream_t st)
@@ -502,7 +498,8 @@ void LaunchPairHalfDot(const LevelView &v, const uint8_t *du, const float *r, fl
                        const int *it, int baseEven, int baseOdd, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    k_pair_half<true><<<PairGrid(v, kReduceS), kPairThreads, 0, st>>>(v, du, r, e, colour, R, it, baseEven, baseOdd);
+    k_pair_half<true><<<SumGrid(R, PairGrid(v, kSumPlanes)), kPairThreads, 0, st>>>(v, du, r, e, colour, R, it, baseEven,
+                                                                                   baseOdd);
 }
 
 void LaunchPairResidual(const LevelView &v, const uint8_t *du, const float *r, const float *e, float *res,
@@ -838,7 +835,7 @@ void LaunchPairPApply(const LevelView &v, const uint8_t *du, const float *z, flo
                       int singular, int slotPQ, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    const dim3 grid = PairGrid(v, kReduceS);
+    const dim3 grid = SumGrid(R, PairGrid(v, kSumPlanes));
     const uint8_t *bytes = v.stretched ? v.code : du;
 #define NB_PAPPLY(SING, ST)                                                                                        \
     k_pair_papply<SING, ST><<<grid, kPairThreads, 0, st>>>(v, bytes, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, \
@@ -915,8 +912,8 @@ void LaunchPairRefine64(const LevelView &v, const uint8_t *du, const double *b, 
                         cudaStream_t st, const int *swap)
 {
     NB_COUNT_LAUNCH();
-    k_pair_refine64<<<PairGrid(v, kReduceS), kPairThreads, 0, st>>>(v, du, b, xin, e, xout, r, scale, sfac, R,
-                                                                      slot, swap);
+    k_pair_refine64<<<SumGrid(R, PairGrid(v, kSumPlanes)), kPairThreads, 0, st>>>(v, du, b, xin, e, xout, r, scale, sfac,
+                                                                                 R, slot, swap);
 }
 
 // Whole-array kernels (every entry off the unknowns is zero): 16-byte loads over the level's cells.

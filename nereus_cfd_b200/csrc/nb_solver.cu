@@ -378,12 +378,7 @@ void Context::AssignSplit()
         Lv.sRS = Lv.sPS = 0;
         Lv.sHalf = 0;
         const bool s = on && finer && (int)l < tailStart && l + 1 < L.size() && SplitLevelShape(Lv.view());
-        if (s)
-        {
-            Lv.sRS = ((Lv.Nz + 1) / 2 + 3) & ~3;
-            Lv.sPS = Lv.Nx * Lv.sRS;
-            Lv.sHalf = ((long long)Lv.Ny * Lv.sPS + 63) & ~63LL; // each colour starts 256-byte aligned
-        }
+        if (s) Lv.PlaceSplit();
         finer = s;
     }
 }
@@ -512,6 +507,24 @@ void Context::BuildTailLists()
     LaunchTailLists(views.data(), (int)views.size(), tailLists.p, tailCounts.p, st);
 }
 
+// The partial sums (per value) the reductions of a grid's level 0 need, whatever its form: level 0 alone runs launches
+// that end in a grid-wide sum.
+int SumBlocks(int dim, int Nx, int Ny, int Nz)
+{
+    LevelData Lv;
+    Lv.dim = dim;
+    Lv.Nx = Nx;
+    Lv.Ny = Ny;
+    Lv.Nz = Nz;
+    Lv.PlaceSplit();
+    const LevelView v = Lv.view();
+    auto count = [](const dim3 &g) { return (long long)g.x * g.y * g.z; };
+    long long n = std::max((long long)kSumBlocksMin, count(TileGrid(v)));
+    if (dim == 2) n = std::max(n, Leg2SumBlocks(v));
+    else n = std::max(n, std::max(count(PairGrid(v, kSumPlanes)), SplitSumBlocks(v)));
+    return (int)n;
+}
+
 void Context::AllocVectors()
 {
     const bool mixed = opt.precision == NB_PRECISION_MIXED;
@@ -592,7 +605,7 @@ Context::Context(const nb_options &o) : opt(o)
         ownStream = true;
     }
     arrays.Init(device, st);
-    red.maxBlocks = 1 << 16; // partial sums per reduction launch (the tile grids stay well below)
+    red.maxBlocks = kSumBlocksMin;
     partials.alloc((size_t)red.maxBlocks * 4);
     slots.alloc(S_COUNT);
     slots.zero(st);
@@ -847,6 +860,9 @@ void Context::SetLayout(int dim_, int Nx_, int Ny_, int Nz_, const uint8_t *type
         Nx = Nx_;
         Ny = Ny_;
         Nz = Nz_;
+        red.maxBlocks = SumBlocks(dim, Nx, Ny, Nz);
+        partials.alloc((size_t)red.maxBlocks * 4);
+        red.partials = partials.p;
         nonuniform = nonUniform != 0;
         dh = dh_;
         scale = nonuniform ? 1.0 : 1.0 / (dh * dh); // MatrixScale3D (PressureSolver3D.cpp:34-37)

@@ -206,6 +206,13 @@ struct LevelData
     // the colour-split layout of the solver's vectors (nb_split.cu); sRS = 0: the grid layout
     int sRS = 0, sPS = 0;
     long long sHalf = 0;
+    // the layout of a colour-split level of these sizes
+    void PlaceSplit()
+    {
+        sRS = ((Nz + 1) / 2 + 3) & ~3;
+        sPS = Nx * sRS;
+        sHalf = ((long long)Ny * sPS + 63) & ~63LL; // each colour starts 256-byte aligned
+    }
     size_t VecLen() const { return sRS ? (size_t)(2 * sHalf) : (size_t)cells; }
     DevArray<float> r32, e32, res32;
     DevArray<double> r64, e64, res64;
@@ -470,6 +477,10 @@ void PlanXGroups(const double *w, int n, double yzMin, std::vector<int> &count);
 // are the regular pairing of every axis.
 bool XMaps(const double *w, int nf, double yzMin, int &Nc, std::vector<double> &size, std::vector<int> &xp,
            std::vector<int> &xr);
+
+// The partial sums a reduction has room for at least, and those a grid's largest one needs
+constexpr int kSumBlocksMin = 1 << 16;
+int SumBlocks(int dim, int Nx, int Ny, int Nz);
 
 void CheckBcLists(const nb_bc_lists &lists);
 // The level of each operation of the two replays, in list order (solid faces of u, v, w, prescribed entries, copies;

@@ -35,9 +35,6 @@ namespace nb
 
 bool SplitLevelShape(const LevelView &v) { return v.dim == 3 && v.Nx >= 3 && v.Ny >= 3 && v.Nz >= 3; }
 
-// planes per thread at least in the pair-thread launches that end in a grid-wide sum
-constexpr int kSplitReduceS = 16;
-
 // ---------------------------------------------------------------------------------------------------------------
 // smoothing
 // ---------------------------------------------------------------------------------------------------------------
@@ -236,10 +233,10 @@ void LaunchSplitHalfDot(const LevelView &v, const uint8_t *du, const T *r, T *e,
         if (v.stretched) return LaunchStretchedHalfDot(v, r, e, colour, last, R, it, baseEven, baseOdd, partSlot, st);
     NB_COUNT_LAUNCH();
     if (last)
-        LaunchPdl(k_split_half<T, 2>, QuadGrid<kQ<T>>(v, Occ<k_split_half<T, 2>>()), kPairThreads, 0, st,
+        LaunchPdl(k_split_half<T, 2>, SumGrid(R, QuadGrid<kQ<T>>(v, Occ<k_split_half<T, 2>>())), kPairThreads, 0, st,
                   NB_SPLIT_HALF_ARGS(colour), R, it, baseEven, baseOdd, partSlot);
     else
-        LaunchPdl(k_split_half<T, 1>, QuadGrid<kQ<T>>(v, Occ<k_split_half<T, 1>>()), kPairThreads, 0, st,
+        LaunchPdl(k_split_half<T, 1>, SumGrid(R, QuadGrid<kQ<T>>(v, Occ<k_split_half<T, 1>>())), kPairThreads, 0, st,
                   NB_SPLIT_HALF_ARGS(colour), R, it, baseEven, baseOdd, partSlot);
 }
 #undef NB_SPLIT_HALF_ARGS
@@ -929,11 +926,11 @@ void LaunchSplitPApply(const LevelView &v, const uint8_t *du, const T *z, T *p0,
         if (v.stretched) return LaunchStretchedPApply(v, du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, st);
     NB_COUNT_LAUNCH();
     if (singular)
-        LaunchPdl(k_split_papply<T, true>, QuadGrid<kQ<T>>(v, Occ<k_split_papply<T, true>>()), kPairThreads, 0, st, v,
-                  du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ);
+        LaunchPdl(k_split_papply<T, true>, SumGrid(R, QuadGrid<kQ<T>>(v, Occ<k_split_papply<T, true>>())), kPairThreads, 0,
+                  st, v, du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ);
     else
-        LaunchPdl(k_split_papply<T, false>, QuadGrid<kQ<T>>(v, Occ<k_split_papply<T, false>>()), kPairThreads, 0, st,
-                  v, du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ);
+        LaunchPdl(k_split_papply<T, false>, SumGrid(R, QuadGrid<kQ<T>>(v, Occ<k_split_papply<T, false>>())), kPairThreads,
+                  0, st, v, du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -1110,7 +1107,7 @@ void LaunchSplitRefine64(const LevelView &v, const uint8_t *du, const double *b,
                          cudaStream_t st, const int *swap)
 {
     NB_COUNT_LAUNCH();
-    const dim3 grid = PairGridOf((long long)v.Nx * RowPairs(v), v.Ny - 2, kSplitReduceS);
+    const dim3 grid = SumGrid(R, PairGridOf((long long)v.Nx * RowPairs(v), v.Ny - 2, kSumPlanes));
     if (v.Nz % 2 == 0)
         k_split_refine64<T, true><<<grid, kPairThreads, 0, st>>>(v, du, b, xin, e, xout, r, scale, sfac, R, slot, swap);
     else
@@ -1118,6 +1115,15 @@ void LaunchSplitRefine64(const LevelView &v, const uint8_t *du, const double *b,
                                                                   swap);
 }
 
+// The most blocks such a launch takes: a quad kernel with two doubles a thread, on kQuadMaxS planes where that fills ten
+// waves (BestMarch stops there; with fewer waves, the longest shorter march has at most twice the blocks of one that fills
+// less than ten), or a pair-thread one.
+long long SplitSumBlocks(const LevelView &v)
+{
+    const long long few = 2LL * 10 * 148 * 8;
+    const dim3 q = QuadGridS<2>(v, kQuadMaxS), p = PairGridOf((long long)v.Nx * RowPairs(v), v.Ny - 2, kSumPlanes);
+    return std::max(few, std::max((long long)q.x * q.y, (long long)p.x * p.y));
+}
 
 // ---------------------------------------------------------------------------------------------------------------
 // batched launches (nb_batch.cu): grid z = the batch's capacity, block z runs the request at list[z] on the x, y tiles
@@ -1356,7 +1362,7 @@ void LaunchBatchSplitRefine64(const LevelView &v, const BatchLevel *lv, int ls, 
                               int cap, const int *parity, int slot, cudaStream_t st)
 {
     NB_COUNT_LAUNCH();
-    kb_split_refine64<<<WithZ(PairGrid(v, kSplitReduceS), cap), kPairThreads, 0, st>>>(lv, ls, rq, a, parity, slot);
+    kb_split_refine64<<<WithZ(PairGrid(v, kSumPlanes), cap), kPairThreads, 0, st>>>(lv, ls, rq, a, parity, slot);
 }
 
 // ---------------------------------------------------------------------------------------------------------------

@@ -377,9 +377,9 @@ static void HalfOn(const LevelView &v, const double *r, double *e, int c, const 
 {
     const long long h = v.sHalf;
     NB_COUNT_LAUNCH();
-    LaunchPdl(k_stretched_half<kDot>, QuadGrid<kN>(v, Occ<k_stretched_half<kDot>>()), kPairThreads, 0, st, v,
-              v.idg + c * h, r + c * h, (const double *)(e + (c ^ 1) * h), e + c * h, c, R, it, baseEven, baseOdd,
-              partSlot);
+    const dim3 grid = QuadGrid<kN>(v, Occ<k_stretched_half<kDot>>());
+    LaunchPdl(k_stretched_half<kDot>, kDot ? SumGrid(R, grid) : grid, kPairThreads, 0, st, v, v.idg + c * h, r + c * h,
+              (const double *)(e + (c ^ 1) * h), e + c * h, c, R, it, baseEven, baseOdd, partSlot);
 }
 
 void LaunchStretchedHalf(const LevelView &v, const double *r, double *e, int colour, cudaStream_t st)
@@ -408,11 +408,11 @@ void LaunchStretchedPApply(const LevelView &v, const uint8_t *du, const double *
 {
     NB_COUNT_LAUNCH();
     if (singular)
-        LaunchPdl(k_stretched_papply<true>, QuadGrid<kN>(v, Occ<k_stretched_papply<true>>()), kPairThreads, 0, st, v, du,
-                  z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ);
+        LaunchPdl(k_stretched_papply<true>, SumGrid(R, QuadGrid<kN>(v, Occ<k_stretched_papply<true>>())), kPairThreads, 0,
+                  st, v, du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ);
     else
-        LaunchPdl(k_stretched_papply<false>, QuadGrid<kN>(v, Occ<k_stretched_papply<false>>()), kPairThreads, 0, st, v,
-                  du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ);
+        LaunchPdl(k_stretched_papply<false>, SumGrid(R, QuadGrid<kN>(v, Occ<k_stretched_papply<false>>())), kPairThreads, 0,
+                  st, v, du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, slotPQ);
 }
 
 // the kernels' occupancy, read outside any stream capture

@@ -103,3 +103,36 @@ def test_headline_size_against_reference(nb, big, reference, precision):
     scale = np.abs(r12.p).max()
     assert np.abs(m.p[~mask] - r12.p[~mask]).max() <= 1e-6 * scale
     assert r.max_div <= 10.0 * r8.max_div, (r.max_div, r8.max_div)
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_sums_over_more_blocks_than_the_least_room(nb, precision):
+    """A 2D box of 4608^2 cells, whose grid-wide sums run over 82,944 blocks where a solver keeps room for 65,536 at least:
+    the count of unknowns, the reported residual and divergence against numpy's. The residual's own rounding is of the
+    order of 8 (products and sums per cell) times 2^-53 of |A| |p| / |b|; after a few iterations on this box |A| |p| is
+    below 1e3 |b|, so the two agree to 1e-12 of |b|, and rel_res is far above that."""
+    n, rho, dt = 4608, 1.0, 1e-3
+    assert capi.load().nereus_b200_sum_blocks(2, n + 2, n + 2, 1) == 144 * 576
+    g = W.uniform_grid(2, (0.0, 1.0, 0.0, 1.0, 0.0, 1.0), n)
+    types = capi.label_cells(g, W.walls_scene(2))
+    rng = np.random.default_rng(12)
+    u, v = np.zeros((n + 2, n + 3)), np.zeros((n + 3, n + 2))
+    u[1:-1, 2:-2] = rng.normal(size=(n, n - 1))
+    v[2:-2, 1:-1] = rng.normal(size=(n - 1, n))
+    m = MACGrid(g, types, u.reshape(-1).copy(), v.reshape(-1).copy(), np.zeros(1), np.zeros(g.cells), rho, dt)
+    s = PressureSolver(precision, max_iters=3, max_outer=1)
+    r = s.SolvePressure(m, tol=1e-10)
+    s.DestroyPressureSolver()
+    assert r.status == capi.NB_NOT_CONVERGED and r.n == n * n
+
+    def divergence(u, v):
+        return (u[1:-1, 2:-1] - u[1:-1, 1:-2]) / g.dh + (v[2:-1, 1:-1] - v[1:-2, 1:-1]) / g.dh
+
+    b = rho / dt * divergence(u, v)
+    p = np.pad(m.p.reshape(n + 2, n + 2)[1:-1, 1:-1], 1, mode="edge")
+    inner = p[1:-1, 1:-1]
+    lap = ((p[2:, 1:-1] - inner) + (p[:-2, 1:-1] - inner) + (p[1:-1, 2:] - inner) + (p[1:-1, :-2] - inner)) / g.dh ** 2
+    rel = np.linalg.norm(b - lap) / np.linalg.norm(b)
+    assert rel > 1e-6 and abs(r.rel_res - rel) <= 1e-12
+    after = np.abs(divergence(m.u.reshape(u.shape), m.v.reshape(v.shape))).max()
+    assert abs(r.max_div - after) <= 1e-12 * after
