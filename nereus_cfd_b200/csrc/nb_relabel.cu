@@ -7,12 +7,11 @@
 // caller may capture them in a graph):
 //   1. reset: every cell that is not SOLID, INFLOW, OUTFLOW or PRESSURE becomes EMPTY. k_relabel_reset, 16 bytes per
 //      thread; it also zeroes the pending-list counter and the skipped-particle count.
-//   2. mark: each particle's cell, if EMPTY, becomes FLUID. Positions that lie in rows of at most kMaxRow doubles (plain
-//      x, y, z rows, or the reference's own Particle array with x, y, z at doubles 1..3 of 7) stream through shared
-//      memory (k_relabel_mark_rows); separate or widely strided arrays are read directly, four particles in flight a
-//      thread (k_relabel_mark). The index is the reference's (truncation of (x - origin) / dh toward zero, clamped
-//      above); a particle more than one cell below the grid or with a non-finite coordinate, which the reference
-//      would index outside its labels with, is skipped and counted.
+//   2. mark: each particle's cell, if EMPTY, becomes FLUID. k_relabel_mark, one wave of threads striding over the
+//      particles four at a time, reading x, y, z through a stride so that the reference's own Particle array (x, y, z at
+//      doubles 1..3 of 7), plain rows and separate arrays all serve. The index is the reference's (truncation of
+//      (x - origin) / dh toward zero, clamped above); a particle more than one cell below the grid or with a non-finite
+//      coordinate, which the reference would index outside its labels with, is skipped and counted.
 //   3. hole filling: one pass over the interior in (i, j, k) order, IN PLACE: an EMPTY cell with >= 5 (3D) / >= 3
 //      (2D) FLUID neighbours becomes FLUID, and a cell filled earlier in the pass counts for the later ones. So a cell
 //      sees its upper neighbours (i+1, j+1, k+1) as they were before the pass and its lower ones (i-1, j-1, k-1) as
@@ -163,6 +162,11 @@ __device__ __forceinline__ int ParticleIndex(double x, double origin, double dh,
 
 constexpr int kMarkBatch = 4; // particles in flight per thread
 
+// The whole call on 65 M particles and 256^3 labels by row width (doubles a particle; B200, us), with a floor and a
+// conversion per coordinate and with ParticleIndex above: 3: 661 / 489, 4: 670 / 513, 5: 703 / 563, 6: 757 / 646,
+// 7: 838 / 732, 8: 888 / 791, separate arrays: 666 / 497. What bounds it is the rows' bytes from DRAM. Streaming the rows
+// through shared memory (cp.async, 512 rows a stage, three stages) was slower at every width with the same index: 511,
+// 614, 734, 955, 987, 1073.
 __global__ void __launch_bounds__(kThreads, 4)
     k_relabel_mark(const double *__restrict__ px, const double *__restrict__ py, const double *__restrict__ pz,
                    long long count, long long stride, RelabelGrid g, double ox, double oy, double oz, double dh,
@@ -210,82 +214,6 @@ __global__ void __launch_bounds__(kThreads, 4)
     }
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, s);
-    if (skipped && (threadIdx.x & 31) == 0 && mine) atomicAdd(skipped, mine);
-}
-
-// The same for positions in rows: coordinates of particle p at base[p * stride + ox0, oy0, oz0] (doubles), stride at
-// most kMaxRow. Reading them with one 8-byte load per coordinate left the pass at 3.6 TB/s (the rows of 24 bytes take
-// every sector three times through L1, and the loads are tied to the index arithmetic); here a block copies chunks of
-// kRowChunk rows to shared memory 16 bytes at a time, kRowStages chunks ahead (cp.async), and works from there. A lane
-// whose particle lies in the previous lane's cell leaves the label to it: particles come cell by cell. 67 M particles
-// in (x, y, z) rows, 256^3 labels, the whole call (B200): 0.648 ms before, 0.498 ms now.
-constexpr int kMaxRow = 8, kRowChunk = 512, kRowStages = 3;
-
-__device__ __forceinline__ void CopyAsync16(void *smem, const void *gmem)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
-                 : "memory");
-}
-
-// bytes of a stage: a chunk's rows, and a granule for a start that is not on a 16-byte boundary
-__host__ __device__ inline int RowStageBytes(int stride) { return kRowChunk * stride * 8 + 16; }
-
-__global__ void __launch_bounds__(kThreads)
-    k_relabel_mark_rows(const double *__restrict__ base, int stride, int offX, int offY, int offZ, int span,
-                        long long count, RelabelGrid g, double ox, double oy, double oz, double dh, double inv,
-                        uint8_t *__restrict__ t, unsigned long long *skipped)
-{
-    extern __shared__ __align__(16) unsigned char rows[];
-    const long long chunks = (count + kRowChunk - 1) / kRowChunk;
-    const int stageBytes = RowStageBytes(stride);
-    const unsigned char *src = reinterpret_cast<const unsigned char *>(base);
-    const int mis = (int)((uintptr_t)src & 15); // every chunk starts as far from a 16-byte boundary (512 rows of 8 n)
-    // chunk c into stage s: the granules that hold its rows' coordinates (the last row ends after `span` doubles);
-    // a granule that holds one valid byte lies inside the array's allocation
-    auto fetch = [&](long long c, int s) {
-        if (c < chunks)
-        {
-            const long long n = min((long long)kRowChunk, count - c * kRowChunk);
-            const int bytes = mis + (int)(((n - 1) * stride + span) * 8);
-            const unsigned char *from = src - mis + c * (long long)kRowChunk * stride * 8;
-            for (int o = 16 * (int)threadIdx.x; o < bytes; o += 16 * kThreads)
-                CopyAsync16(rows + s * stageBytes + o, from + o);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    unsigned long long mine = 0;
-    for (int s = 0; s < kRowStages - 1; s++) fetch(blockIdx.x + (long long)s * gridDim.x, s);
-    int s = 0;
-    for (long long c = blockIdx.x; c < chunks; c += gridDim.x, s = s + 1 == kRowStages ? 0 : s + 1)
-    {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kRowStages - 2) : "memory");
-        __syncthreads(); // this chunk is in; the stage fetched next was read in the round before
-        fetch(c + (long long)(kRowStages - 1) * gridDim.x, s + kRowStages - 1 >= kRowStages ? s - 1 : s + kRowStages - 1);
-        const double *rd = reinterpret_cast<const double *>(rows + s * stageBytes + mis);
-        const int here = (int)min((long long)kRowChunk, count - c * kRowChunk); // rows of this chunk
-        int cell[kRowChunk / kThreads];
-#pragma unroll
-        for (int b = 0; b < kRowChunk / kThreads; b++)
-        {
-            const int p = threadIdx.x + b * kThreads;
-            const bool live = p < here;
-            const double *q = rd + (live ? p * stride : 0);
-            const int i = ParticleIndex(q[offY], oy, dh, inv, g.Ny, g.nearHi);
-            const int j = ParticleIndex(q[offX], ox, dh, inv, g.Nx, g.nearHi);
-            const int k = g.dim == 3 ? ParticleIndex(q[offZ], oz, dh, inv, g.Nz, g.nearHi) : 0;
-            const bool out = (i | j | k) < 0;
-            mine += live && out;
-            const int at = live && !out ? (i * g.Nx + j) * g.Nz + k : -1;
-            const int before = __shfl_up_sync(0xffffffffu, at, 1);
-            cell[b] = (threadIdx.x & 31) != 0 && before == at ? -1 : at;
-        }
-#pragma unroll
-        for (int b = 0; b < kRowChunk / kThreads; b++)
-            if (cell[b] >= 0 && t[cell[b]] == EMPTY) t[cell[b]] = (uint8_t)FLUID;
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, d);
     if (skipped && (threadIdx.x & 31) == 0 && mine) atomicAdd(skipped, mine);
 }
 
@@ -542,23 +470,6 @@ void UpdateFluidCellsDevice(int dim, int Nx, int Ny, int Nz, double ox, double o
     if (count > 0)
     {
         NB_COUNT_LAUNCH();
-        // rows: the coordinates of a particle within one row of `stride` doubles (compared as addresses, since separate
-        // arrays are separate objects)
-        const uintptr_t ax = (uintptr_t)px, ay = (uintptr_t)py, az = dim == 3 ? (uintptr_t)pz : ax;
-        const uintptr_t lo = std::min(ax, std::min(ay, az)), hi = std::max(ax, std::max(ay, az));
-        if (stride <= kMaxRow && (lo & 7) == 0 && ((ax - lo) | (ay - lo) | (az - lo)) % 8 == 0 &&
-            hi - lo < (uintptr_t)stride * 8)
-        {
-            const int s = (int)stride, smem = kRowStages * RowStageBytes(s);
-            if (smem > (48 << 10)) // more than a kernel gets unasked
-                NB_CK(cudaFuncSetAttribute(k_relabel_mark_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           kRowStages * RowStageBytes(kMaxRow)));
-            const int perSm = std::max(1, std::min(6, (200 << 10) / smem));
-            k_relabel_mark_rows<<<Blocks(count, kRowChunk, sms * perSm), kThreads, smem, st>>>(
-                (const double *)lo, s, (int)((ax - lo) / 8), (int)((ay - lo) / 8), (int)((az - lo) / 8),
-                (int)((hi - lo) / 8) + 1, count, g, ox, oy, oz, dh, 1.0 / dh, cellTypes, skipped);
-        }
-        else
         k_relabel_mark<<<Blocks((count + kMarkBatch - 1) / kMarkBatch, kThreads, sms * 4), kThreads, 0, st>>>(
             px, py, pz, count, stride, g, ox, oy, oz, dh, 1.0 / dh, cellTypes, skipped);
     }

@@ -196,8 +196,8 @@ def oracle_labels(grid, types, xyz, origin):
     return cpu.update_fluid_cells(grid, types, np.ascontiguousarray(xyz), origin)
 
 
-# counts around a chunk of 512 rows and a block's 256 threads; row widths up to the widest that streams (8) and past it;
-# starts on and off a 16-byte boundary; labels on any byte boundary
+# counts around one and two blocks of 256 threads; row widths around the reference's 7 doubles; starts on and off a 16-byte
+# boundary; labels on any byte boundary
 @pytest.mark.parametrize("count", [1, 255, 257, 511, 512, 513, 1024, 5000])
 @pytest.mark.parametrize("stride,first", [(3, 0), (3, 1), (4, 1), (7, 1), (8, 5), (9, 2)])
 def test_particle_rows_stream_like_the_oracle(nb, count, stride, first):
