@@ -373,8 +373,10 @@ int nereus_b200_wait(nb_server *srv, uint64_t ticket, double timeout_s, nb_resul
 int nereus_b200_server_stats(nb_server *srv, nb_server_stats *stats);
 /* Starts the statistics afresh (counts, latencies, the clock) from now; queued and running requests are kept. */
 int nereus_b200_server_reset_stats(nb_server *srv);
-/* Estimated device bytes of one solve (the admission cost): fields, right-hand side and solution, level vectors. */
+/* Estimated device bytes of one solve (the admission cost): fields, right-hand side and solution, level vectors. _ex:
+ * of a uniform or a stretched grid (a stretched FP64 solve keeps its levels' diagonals); without it, a uniform one. */
 double nereus_b200_request_bytes(int dim, int Nx, int Ny, int Nz, int precision);
+double nereus_b200_request_bytes_ex(int dim, int Nx, int Ny, int Nz, int precision, int nonuniform);
 /* Host only: a deterministic least-loaded assignment of n requests with the given costs to k devices (or processes):
  * in submission order, each goes to the device with the smallest assigned total (lowest index on ties). */
 int nereus_b200_plan(const double *costs, int n, int k, int *device_of);

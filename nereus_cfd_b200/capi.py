@@ -180,6 +180,7 @@ SIGNATURES = {
     "nereus_b200_server_reset_stats": (ctypes.c_int, [ctypes.c_void_p]),
     "nereus_b200_request_bytes": (ctypes.c_double, [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                                     ctypes.c_int]),
+    "nereus_b200_request_bytes_ex": (ctypes.c_double, [ctypes.c_int] * 6),
     "nereus_b200_plan": (ctypes.c_int, [_dp, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]),
     "nereus_b200_number_unknowns_noalloc": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                                            ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p,

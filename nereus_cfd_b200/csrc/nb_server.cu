@@ -44,13 +44,32 @@ struct Record
 
 } // namespace
 
-double RequestBytes(int dim, int Nx, int Ny, int Nz, int precision)
+// The device bytes a request's solve holds: a flat count per cell (what the forms held before stretched FP64 levels kept
+// their diagonals and colour-split rows were padded), or the arrays level by level where those come to more.
+double RequestBytes(int dim, int Nx, int Ny, int Nz, int precision, bool stretched)
 {
-    const double cells = (double)Nx * Ny * (dim == 3 ? Nz : 1);
+    const bool fp64 = precision != NB_PRECISION_MIXED;
+    const double s = fp64 ? 8.0 : 4.0;
+    const double cells0 = (double)Nx * Ny * Nz;
     // fields u, v, w, p, p_prev (5 x 8), b and two solutions (3 x 8), types/codes/du/pext (4), level-0 solver
     // vectors (r, e, res, p0, p1, q, x: 7 x 4 or 8) and the coarser levels (x 8/7 in 3D)
-    const double s = precision == NB_PRECISION_MIXED ? 4.0 : 8.0;
-    return cells * (5 * 8 + 3 * 8 + 4 + 7 * s * (dim == 3 ? 8.0 / 7.0 : 4.0 / 3.0)) + (64 << 20);
+    const double flat = cells0 * (5 * 8 + 3 * 8 + 4 + 7 * s * (dim == 3 ? 8.0 / 7.0 : 4.0 / 3.0));
+    double levels = cells0 * ((dim == 3 ? 5 : 4) * 8 + 3 * 8);
+    for (int l = 0;; l++)
+    {
+        const double cells = (double)Nx * Ny * Nz, pad = dim == 3 ? 2.0 * Nx * Ny * (((Nz + 1) / 2 + 3) & ~3) : cells;
+        levels += 2 * cells + 1.5 * pad;              // types and codes; du and pext
+        levels += (l == 0 ? 7 : 3) * s * pad;         // r, e, res; on level 0 also p0, p1, q, x
+        if (dim == 2) levels += 8 * cells;            // the diagonal
+        else if (stretched && fp64) levels += 16 * pad; // the diagonal and its reciprocal
+        const int nx = Nx - 2, ny = Ny - 2, nz = dim == 3 ? Nz - 2 : 1;
+        if (std::min(nx, std::min(ny, dim == 3 ? nz : ny)) < 8 || (double)nx * ny * nz <= 64) break;
+        // x groups may keep every x cell of a stretched level (the mixed form's levels stay below the flat count)
+        if (dim == 2 || !stretched || !fp64) Nx = (nx + 1) / 2 + 2;
+        Ny = (ny + 1) / 2 + 2;
+        if (dim == 3) Nz = (nz + 1) / 2 + 2;
+    }
+    return std::max(flat, levels) + (64 << 20);
 }
 
 void Plan(const double *costs, int n, int k, int *deviceOf)
@@ -290,7 +309,7 @@ int nereus_b200_submit(nb_server *srv, const nb_request *req, uint64_t *ticket)
             q->tables[a].assign(r.width[a], r.width[a] + N[a] + 2);
             q->tables[3 + a].assign(r.gap[a], r.gap[a] + N[a] + 1);
         }
-        q->bytes = nb::RequestBytes(r.dim, r.Nx, r.Ny, Nz, srv->opt.solver.precision);
+        q->bytes = nb::RequestBytes(r.dim, r.Nx, r.Ny, Nz, srv->opt.solver.precision, r.non_uniform != 0);
         if (q->bytes > srv->budget) throw nb::InputError("request larger than the device memory budget");
         {
             std::lock_guard<std::mutex> lock(srv->mu);
@@ -392,7 +411,12 @@ int nereus_b200_server_reset_stats(nb_server *srv)
 
 double nereus_b200_request_bytes(int dim, int Nx, int Ny, int Nz, int precision)
 {
-    return nb::RequestBytes(dim, Nx, Ny, dim == 3 ? Nz : 1, precision);
+    return nb::RequestBytes(dim, Nx, Ny, dim == 3 ? Nz : 1, precision, false);
+}
+
+double nereus_b200_request_bytes_ex(int dim, int Nx, int Ny, int Nz, int precision, int nonuniform)
+{
+    return nb::RequestBytes(dim, Nx, Ny, dim == 3 ? Nz : 1, precision, nonuniform != 0);
 }
 
 int nereus_b200_plan(const double *costs, int n, int k, int *device_of)

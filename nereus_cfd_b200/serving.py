@@ -84,7 +84,7 @@ def tank_batch(count: int = 64, n: int = 128, seed: int = 4) -> list:
 
 def request_bytes(job: Job, precision: int = capi.PRECISION_MIXED) -> float:
     g = job.grid.grid
-    return capi.load().nereus_b200_request_bytes(g.dim, g.Nx, g.Ny, g.Nz, precision)
+    return capi.load().nereus_b200_request_bytes_ex(g.dim, g.Nx, g.Ny, g.Nz, precision, int(g.nonuniform))
 
 
 def plan(costs: Sequence[float], k: int) -> List[int]:

@@ -70,6 +70,48 @@ def test_device_fields_equal_host_fields(nb):
             assert np.array_equal(getattr(a.grid, f), getattr(b.grid, f)), f
 
 
+def slab(dim, n, stretched=False):
+    """A grid of n interior cells a side, its cell widths along x growing from the middle when stretched."""
+    if stretched:
+        w = [W.band_stretched_widths(n[0], 2.2, max(2, n[0] // 8 // 2 * 2), 0.5, 1.04)]
+        w += [np.full(m, 0.41 / m) for m in n[1:]]
+        g = W.stretched_grid(dim, (0.0, 2.2, 0.0, 0.41, 0.0, 0.41), w)
+    else:
+        h = 1.0 / min(n[:2])
+        g = W.uniform_grid(dim, (0.0, n[0] * h, 0.0, n[1] * h, 0.0, n[-1] * h), min(n[:2]))
+    return W.Case("slab", g, W.walls_scene(dim, outlet_face=1), 3)
+
+
+# stretched 3D grids in FP64 (whose levels keep their diagonals) of both parities of Nz, a thin one whose padded rows are
+# 1.6 times its cells, a 2D one
+@pytest.mark.parametrize("dim,n,stretched,precision", [
+    (3, (384, 192, 192), True, "fp64"), (3, (400, 200, 151), True, "fp64"), (3, (200, 200, 251), False, "fp64"),
+    (3, (1000, 1100, 8), False, "fp64"), (3, (1000, 1100, 8), False, "mixed"), (3, (240, 240, 240), False, "mixed"),
+    (3, (384, 192, 192), True, "mixed"), (2, (3000, 3000), False, "fp64"), (2, (3000, 3000), False, "mixed")])
+def test_request_bytes_cover_what_a_solve_takes(nb, dim, n, stretched, precision):
+    """The admission estimate against the device memory a context holds after a step on host fields."""
+    import torch
+
+    g = slab(dim, n, stretched).grid
+    types = capi.label_cells(g, W.walls_scene(dim, outlet_face=1))
+    fields = [np.zeros(k) for k in (g.Ny * (g.Nx + 1) * g.Nz, (g.Ny + 1) * g.Nx * g.Nz,
+                                    g.Ny * g.Nx * (g.Nz + 1) if dim == 3 else 1, g.cells)]
+    fields[0][:] = np.random.default_rng(1).normal(size=fields[0].size)
+    for warm in (True, False):  # the kernels' code is loaded by a first, small solve
+        h = slab(dim, (24, 24, 16)[:dim], stretched).grid if warm else g
+        t = capi.label_cells(h, W.walls_scene(dim, outlet_face=1)) if warm else types
+        f = [np.zeros(k) for k in (h.Ny * (h.Nx + 1) * h.Nz, (h.Ny + 1) * h.Nx * h.Nz,
+                                   h.Ny * h.Nx * (h.Nz + 1) if dim == 3 else 1, h.cells)] if warm else fields
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        s = PressureSolver(precision, max_iters=3, max_outer=1)
+        s.SolvePressure(MACGrid(h, t, *f), tol=1e-8)
+        used = free - torch.cuda.mem_get_info()[0]
+        s.DestroyPressureSolver()
+    prec = capi.PRECISION_FP64 if precision == "fp64" else capi.PRECISION_MIXED
+    assert used <= serving.request_bytes(serving.Job(MACGrid(g, types, *fields)), prec)
+
+
 def test_admission_budget(nb):
     job = mix()[0]
     with serving.Server(hbm_budget_gb=0.01) as srv:
