@@ -2,11 +2,11 @@
 
 * The 2D 128^2 closed box (all-Neumann, compatibility on) at its own tolerance 1e-10, against the reference's Eigen-CG
   solution at 1e-12 (tests/golden/closed_box_2d_128.npz): mean-free pressure within 1e-6 relative L2.
-* The 3D sphere-outlet workload at 208^3, the first size at which a coarse level (106^3 = 1,191,016 cells) reaches the
-  2^20 cells from which the colour-split restriction runs one thread per four coarse cells, as it does on the 256^3
-  headline grid:
+* The 3D sphere-outlet workload at 208^3, whose first coarse levels (106^3 = 1,191,016 and 55^3 = 166,375 cells) lie above
+  the 2^17 cells from which the colour-split restriction runs one thread per four coarse cells, as they do on the 256^3
+  headline grid, and whose next one lies below:
   - the two restriction kernels (one thread per coarse cell, one per four) give the same bits through a whole mixed
-    solve, and the default choice is the quad kernel there;
+    solve, and so does the default choice between them;
   - the mixed and the plain FP64 solves to 1e-8 against the reference's own solve of the same system
     (oracle/_ref/ref_harness, AMGCL SA+SPAI0 CG, run on this host): relative residual <= 1e-8, pressure within 1e-6
     relative L2 of the reference's solve at 1e-12, and max |div u| within 10x of the reference's at 1e-8, driven the
@@ -74,7 +74,7 @@ def test_quad_and_per_cell_restriction_agree(nb, big):
     assert (r1.iters_inner, r1.iters_outer) == (r2.iters_inner, r2.iters_outer)
     assert np.array_equal(m1.p, m2.p), np.abs(m1.p - m2.p).max()
     assert np.array_equal(m1.u, m2.u) and np.array_equal(m1.v, m2.v) and np.array_equal(m1.w, m2.w)
-    # the default picks the quad kernel for the 106^3 level
+    # the default runs one kernel on the larger levels and the other on the smaller
     assert np.array_equal(m0.p, m2.p)
 
 

@@ -245,6 +245,37 @@ def test_odd_rows_agree_with_per_cell_kernels(nb, size, precision, sweeps):
             assert np.linalg.norm(x - y) <= bar * np.linalg.norm(y)
 
 
+# (interior x, y, z): fine rows around the restriction's quads of coarse cells (2 doubles, 4 floats) and a last quad that is
+# partly past the row, Nz even and odd, one coarse split level and several
+RESTRICT_SIZES = FP64_SIZES + ODD_SIZES + [(40, 24, 18), (26, 22, 70)]
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("size", RESTRICT_SIZES)
+def test_restriction_by_quads_equals_per_cell(nb, size, precision):
+    """The restriction of colour-split levels with one thread per coarse cell (transfer_kernels = 1) and with one per quad
+    of them (2): the same sums in the same order, so whole solves agree bit for bit. Two sweeps, because with one a launch
+    per leg takes levels of these sizes."""
+    for closed in (False, True):
+        case, types = sphere_case(size, closed)
+        a, b = [solve_family(case, types, 2, precision, closed, tol=1e-10, pre_sweeps=2, post_sweeps=2,
+                             transfer_kernels=mode) for mode in (1, 2)]
+        for f in ("p", "u", "v", "w"):
+            assert np.array_equal(getattr(a, f), getattr(b, f)), f
+
+
+@pytest.mark.parametrize("groups", [1, 0])
+@pytest.mark.parametrize("size", [(24, 16, 16), (32, 17, 15), (48, 32, 33), (64, 24, 40), (97, 30, 21)])
+def test_stretched_restriction_by_quads_equals_per_cell(nb, size, groups):
+    """The same on stretched FP64 grids, x groups on and off."""
+    case = W.stretched_cylinder_3d(*size)
+    types = capi.label_cells(case.grid, case.scene)
+    a, b = [solve_family(case, types, 2, "fp64", False, tol=1e-10, x_groups=groups, transfer_kernels=mode)
+            for mode in (1, 2)]
+    for f in ("p", "u", "v", "w"):
+        assert np.array_equal(getattr(a, f), getattr(b, f)), f
+
+
 # stretched FP64: (interior x, y, z) of the cylinder channel; Nz even and odd, one level above the coarse end and
 # several, x groups on and off
 @pytest.mark.parametrize("groups", [1, 0])
