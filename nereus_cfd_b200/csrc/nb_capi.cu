@@ -122,10 +122,7 @@ int nereus_b200_project(nb_ctx *ctx, double *u, double *v, double *w, double *p,
         if (!u || !v || !p || (C.dim == 3 && !w)) throw nb::InputError("null field pointer");
         nb_result local{};
         nb_result *r = out ? out : &local;
-        C.du.upload(u, C.FieldSizeU(), C.st);
-        C.dv.upload(v, C.FieldSizeV(), C.st);
-        if (C.dim == 3) C.dw.upload(w, C.FieldSizeW(), C.st);
-        C.dp.upload(p, C.Cells(), C.st);
+        C.UploadFields(u, v, w, p);
         // p and then u, v, w go back to the host on the context's copy stream as soon as each is final, beside the
         // velocity correction and the divergence check
         struct HostFields
@@ -172,11 +169,7 @@ int nereus_b200_project_ex(nb_ctx *ctx, double *u, double *v, double *w, double 
         if (!u || !v || !p || (C.dim == 3 && !w)) throw nb::InputError("null field pointer");
         nb_result local{};
         nb_result *r = out ? out : &local;
-        C.du.upload(u, C.FieldSizeU(), C.st);
-        C.dv.upload(v, C.FieldSizeV(), C.st);
-        if (C.dim == 3) C.dw.upload(w, C.FieldSizeW(), C.st);
-        C.dp.upload(p, C.Cells(), C.st);
-        if (pPrev) C.dpPrev.upload(pPrev, C.Cells(), C.st);
+        C.UploadFields(u, v, w, p, pPrev);
         const int status = C.ProjectDevice(C.du.p, C.dv.p, C.dim == 3 ? C.dw.p : C.du.p, C.dp.p, rho, dt,
                                            needsCompat, tol, r, true, true, pPrev ? C.dpPrev.p : nullptr, scheme,
                                            warmStart != 0);
@@ -214,10 +207,7 @@ int nereus_b200_solve_pressure(nb_ctx *ctx, const double *u, const double *v, co
         if (!C.built) throw nb::InputError("set_layout has not been called");
         if (!u || !v || !p || (C.dim == 3 && !w)) throw nb::InputError("null field pointer");
         nb_result local{};
-        C.du.upload(u, C.FieldSizeU(), C.st);
-        C.dv.upload(v, C.FieldSizeV(), C.st);
-        if (C.dim == 3) C.dw.upload(w, C.FieldSizeW(), C.st);
-        C.dp.upload(p, C.Cells(), C.st);
+        C.UploadFields(u, v, w, p);
         const int status = C.ProjectDevice(C.du.p, C.dv.p, C.dim == 3 ? C.dw.p : C.du.p, C.dp.p, rho, dt,
                                            needsCompat, tol, out ? out : &local, true, false);
         NB_CK(cudaMemcpyAsync(p, C.dp.p, C.dp.bytes(), cudaMemcpyDeviceToHost, C.st));
@@ -236,10 +226,7 @@ int nereus_b200_project_velocity(nb_ctx *ctx, double *u, double *v, double *w, c
         if (!C.built) throw nb::InputError("set_layout has not been called");
         if (!u || !v || !p || (C.dim == 3 && !w)) throw nb::InputError("null field pointer");
         nb_result local{};
-        C.du.upload(u, C.FieldSizeU(), C.st);
-        C.dv.upload(v, C.FieldSizeV(), C.st);
-        if (C.dim == 3) C.dw.upload(w, C.FieldSizeW(), C.st);
-        C.dp.upload(p, C.Cells(), C.st);
+        C.UploadFields(u, v, w, p);
         C.ProjectDevice(C.du.p, C.dv.p, C.dim == 3 ? C.dw.p : C.du.p, C.dp.p, rho, dt, 0, 1.0, &local, false, true);
         NB_CK(cudaMemcpyAsync(u, C.du.p, C.du.bytes(), cudaMemcpyDeviceToHost, C.st));
         NB_CK(cudaMemcpyAsync(v, C.dv.p, C.dv.bytes(), cudaMemcpyDeviceToHost, C.st));

@@ -164,11 +164,7 @@ void nb_server::Slot(int dev)
             }
             else
             {
-                C.du.upload(r.u, C.FieldSizeU(), C.st);
-                C.dv.upload(r.v, C.FieldSizeV(), C.st);
-                if (C.dim == 3) C.dw.upload(r.w, C.FieldSizeW(), C.st);
-                C.dp.upload(r.p, C.Cells(), C.st);
-                if (r.p_prev) C.dpPrev.upload(r.p_prev, C.Cells(), C.st);
+                C.UploadFields(r.u, r.v, r.w, r.p, r.p_prev);
                 status = C.ProjectDevice(C.du.p, C.dv.p, C.dim == 3 ? C.dw.p : C.du.p, C.dp.p, r.rho, r.dt,
                                          r.needs_compat, r.tol, &res, true, true, r.p_prev ? C.dpPrev.p : nullptr,
                                          r.scheme, r.warm_start != 0);

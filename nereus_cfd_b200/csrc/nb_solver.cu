@@ -370,7 +370,7 @@ void Context::BuildHierarchy()
 // and takes 5.0 ms on this layout. A stretched grid's FP32 levels keep the cell-pair kernels.
 void Context::AssignSplit()
 {
-    const bool on = opt.pair_kernels == 2 && (!nonuniform || opt.precision == NB_PRECISION_FP64);
+    const bool on = opt.pair_kernels == 2 && !lean && (!nonuniform || opt.precision == NB_PRECISION_FP64);
     bool finer = true;
     for (size_t l = 0; l < L.size(); l++)
     {
@@ -572,6 +572,39 @@ void Context::AllocVectors()
         q32.release();
         x32.release();
     }
+}
+
+// This shape's arrays again in the grid layout (WithRoom). What they held is lost: between a layout and a solve only.
+void Context::GoLean()
+{
+    cudaGetLastError(); // the allocation's
+    const bool was = built;
+    built = false;
+    lean = true;
+    NB_CK(cudaStreamSynchronize(st));
+    for (auto &g : graphs) g.Release();
+    ReleaseSolveGraph();
+    solvesOnShape = 0;
+    L.clear();
+    for (auto *a : {&p32[0], &p32[1], &q32, &x32}) a->release();
+    for (auto *a : {&p64[0], &p64[1], &q64, &x64}) a->release();
+    arrays.Trim();
+    ArrayPoolScope pooled(&arrays);
+    BuildHierarchy();
+    AllocVectors();
+    NB_CK(cudaStreamSynchronize(st));
+    built = was;
+}
+
+void Context::UploadFields(const double *u, const double *v, const double *w, const double *p, const double *pPrev)
+{
+    WithRoom([&] {
+        du.upload(u, FieldSizeU(), st);
+        dv.upload(v, FieldSizeV(), st);
+        if (dim == 3) dw.upload(w, FieldSizeW(), st);
+        dp.upload(p, Cells(), st);
+        if (pPrev) dpPrev.upload(pPrev, Cells(), st);
+    });
 }
 
 // The solver's vectors as a layout starts with them. The kernels keep what is no unknown (solids, ring, the colour-split
@@ -882,7 +915,12 @@ void Context::SetLayout(int dim_, int Nx_, int Ny_, int Nz_, const uint8_t *type
             for (double x : gt[a])
                 if (!(x > 0.0) || !std::isfinite(x)) throw InputError("gap table entries must be positive");
         }
-        BuildHierarchy();
+        lean = false;
+        WithRoom([&] {
+            if (lean) return; // GoLean has built it
+            BuildHierarchy();
+            AllocVectors();
+        });
     }
     // the system size and the singular flag, counted on the device (the IDP numbering waits until it is asked for)
     LaunchCountUnknowns(L[0].view(), red, S_RES, st);
@@ -897,7 +935,7 @@ void Context::SetLayout(int dim_, int Nx_, int Ny_, int Nz_, const uint8_t *type
     }
     hostSlots[S_NUNK] = (double)n;
     NB_CK(cudaMemcpyAsync(slots.p + S_NUNK, hostSlots + S_NUNK, sizeof(double), cudaMemcpyHostToDevice, st));
-    AllocVectors();
+    if (shapeSame || rescale) AllocVectors();
     NB_CK(cudaStreamSynchronize(st));
     built = true;
 }
@@ -1728,6 +1766,11 @@ int Context::ProjectDevice(double *u, double *v, double *w, double *p, double rh
     const bool incr = scheme == NB_SCHEME_INCREMENTAL;
     if ((incr || warm) && !pPrev) throw InputError("the previous pressure is required");
     if (incr && !(solve && correct)) throw InputError("the incremental scheme runs the whole step");
+    if (incr)
+        WithRoom([&] {
+            pSave.alloc(Cells());
+            dq.alloc(Cells());
+        });
     std::memset(out, 0, sizeof(*out));
     out->n = n;
     out->singular = singular ? 1 : 0;
@@ -1754,8 +1797,6 @@ int Context::ProjectDevice(double *u, double *v, double *w, double *p, double rh
     if (incr)
     {
         // SolveIncremental: the known Dirichlet values are p_b(t^{n+1}) - p_b(t^n); p_b(t^{n+1}) is kept for the end
-        pSave.alloc(Cells());
-        dq.alloc(Cells());
         NB_CK(cudaMemcpyAsync(pSave.p, p, pSave.bytes(), cudaMemcpyDeviceToDevice, st));
         LaunchCellwise(v0, CELL_DELTA, const_cast<double *>(p), pPrev, dq.p, st);
         pKnown = dq.p;
@@ -1891,16 +1932,16 @@ void Context::BatchEnd(double *x, double *u, double *v, double *w, double *p, do
 int Context::SolveLaplacian(const double *f, double *xh, double tol, nb_result *out)
 {
     if (!built) throw InputError("set_layout has not been called");
-    EnsureIdp();
+    WithRoom([&] { EnsureIdp(); });
     std::memset(out, 0, sizeof(*out));
     out->n = n;
     out->singular = singular ? 1 : 0;
     out->levels = (int)L.size();
     out->max_div = -1.0;
     if (n == 0) return NB_BAD_INPUT; // SolveLaplacian returns false on an empty system
-    const LevelView v0 = L[0].view();
     DevArray<double> fc;
-    fc.upload(f, (size_t)n, st);
+    WithRoom([&] { fc.upload(f, (size_t)n, st); });
+    const LevelView v0 = L[0].view();
     b.zero(st);
     LaunchScatterVolume(v0, idp.p, fc.p, b.p, 1, st); // b = f * CellVolume (PressureSolver3D.cpp:360-369)
     NB_CK(cudaEventRecord(ev0, st));
@@ -1990,7 +2031,7 @@ void Context::EnsureIdp()
 void Context::GetIdp(int32_t *out)
 {
     if (!built) throw InputError("set_layout has not been called");
-    EnsureIdp();
+    WithRoom([&] { EnsureIdp(); });
     NB_CK(cudaMemcpyAsync(out, idp.p, sizeof(int32_t) * Cells(), cudaMemcpyDeviceToHost, st));
     NB_CK(cudaStreamSynchronize(st));
 }

@@ -72,8 +72,7 @@ struct ArrayPool
         {
             // memory the pool keeps but nothing uses goes back to the device, then once more
             cudaGetLastError();
-            cudaStreamSynchronize(st);
-            cudaMemPoolTrimTo(pool, 0);
+            Trim();
             e = cudaMallocFromPoolAsync(&p, bytes, pool, st);
         }
         if (e != cudaSuccess) throw CudaError("cudaMallocFromPoolAsync", e);
@@ -83,6 +82,12 @@ struct ArrayPool
         return p;
     }
     void Put(void *p) { cudaFreeAsync(p, st); }
+    // what the pool keeps and nothing uses goes back to the device
+    void Trim()
+    {
+        cudaStreamSynchronize(st);
+        cudaMemPoolTrimTo(pool, 0);
+    }
 };
 
 // the pool that DevArray allocations made on this thread draw on (set by a Context around its layout work)
@@ -368,6 +373,26 @@ struct Context
     size_t FieldSizeW() const { return dim == 3 ? (size_t)Nx * Ny * (Nz + 1) : 0; }
     size_t Cells() const { return (size_t)Nx * Ny * Nz; }
 
+    // Runs f, which takes device memory, before a solve's first launch. The colour-split layout takes 10 to 40 bytes a cell
+    // more than the grid layout (a correction vector in FP64, the padding of short rows, a stretched level's diagonals):
+    // where the device has no room for that, the shape changes to the grid layout's kernels and f runs again.
+    template <typename F> void WithRoom(F &&f)
+    {
+        try
+        {
+            f();
+            return;
+        }
+        catch (const CudaError &e)
+        {
+            if (e.code != cudaErrorMemoryAllocation || lean || opt.pair_kernels != 2 || dim != 3) throw;
+        }
+        GoLean();
+        f();
+    }
+    // the caller's host fields on the device (w is not read in 2D)
+    void UploadFields(const double *u, const double *v, const double *w, const double *p, const double *pPrev = nullptr);
+
   private:
     friend struct Batch;
     void BuildHierarchy();
@@ -377,6 +402,7 @@ struct Context
     void EnsureIdp();
     void AllocVectors();
     void ClearVectors();
+    void GoLean();
     double ReadSlot(int s);
     void ReadSlots(int s, int count);
     // Solve A x = b (b in this->b, grid layout); the solution ends in *xOut (xa or xb). Fills out->iters/rel_res.
@@ -421,6 +447,8 @@ struct Context
     bool PairLevel(int l) const { return opt.pair_kernels && L[l].du.p != nullptr; }
     // the solver's vectors of this level are colour-split and its V-cycle runs the split kernels
     bool Split(int l) const { return L[l].sRS != 0; }
+    // this shape runs on the grid layout's kernels although pair_kernels = 2 (WithRoom)
+    bool lean = false;
     // Levels of at most this many cells run their legs in one launch each: measured faster on 66^3 and below, slower on
     // 130^3 (nb_legs.cu)
     static constexpr long long kLegCells = 300000;

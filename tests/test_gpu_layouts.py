@@ -69,3 +69,57 @@ def test_2d_moved_labels_equal_fresh(nb, precision):
                                  ((0.62, 0.40), 1.0), ((0.62, 0.40), 2.5), ((0.30, 0.55), 2.5), ((0.30, 0.55), 2.5))):
         solve_both(reused, disc_channel(150, 130, at, 20 + n, L), precision)
     reused.DestroyPressureSolver()
+
+
+# (interior x, y, z), stretched; where the memory ends: at the layout, or at the step's copies of host fields
+@pytest.mark.parametrize("at", ["layout", "fields"])
+@pytest.mark.parametrize("n,stretched,precision", [((320, 160, 161), True, "fp64"), ((240, 240, 239), False, "fp64"),
+                                                   ((900, 1000, 9), False, "mixed")])
+def test_without_room_for_the_split_layout(nb, n, stretched, precision, at):
+    """A grid whose colour-split layout does not fit the device's free memory while the grid layout does, as it did before
+    the split layout was these grids' default: it is solved by the grid layout's kernels (those of pair_kernels = 1), bit
+    for bit."""
+    import torch
+
+    if stretched:
+        case = W.stretched_cylinder_3d(*n)
+    else:
+        h = 1.0 / min(n[:2])
+        g = W.uniform_grid(3, (0.0, n[0] * h, 0.0, n[1] * h, 0.0, n[2] * h), min(n[:2]))
+        case = W.Case("box", g, W.walls_scene(3, outlet_face=1), 3)
+    job = serving.job_from_case(case, tol=1e-6)
+
+    def free():
+        return torch.cuda.mem_get_info()[0]
+
+    def run(family, room=None):
+        """The step's fields, and the memory that the layout and the whole context take. room: the free bytes there are
+        for the layout, or for all of it."""
+        torch.cuda.empty_cache()
+        j, hog = copy.deepcopy(job), None
+        if room is not None:
+            hog = torch.empty(free() - room, dtype=torch.uint8, device="cuda")
+        start = free()
+        s = PressureSolver(precision, pair_kernels=family, max_iters=4, max_outer=1)
+        s.InitializePressureSolver(j.grid)
+        layout = start - free()
+        if at == "layout":
+            del hog
+            torch.cuda.empty_cache()
+        s.SolvePressure(j.grid, tol=j.tol)
+        whole = start - free()
+        s.DestroyPressureSolver()
+        return j.grid, layout, whole
+
+    run(2)  # loads the kernels' code
+    run(1)
+    expect, *lean = run(1)
+    _, *split = run(2)
+    q = 0 if at == "layout" else 1
+    assert split[q] - lean[q] > 64 << 20
+    try:
+        got, _, _ = run(2, (lean[q] + split[q]) // 2)
+    finally:
+        torch.cuda.empty_cache()  # the memory that was held back
+    for f in ("p", "u", "v", "w"):
+        assert np.array_equal(getattr(got, f), getattr(expect, f)), f
