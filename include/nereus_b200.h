@@ -76,8 +76,9 @@ typedef struct nb_options
     int pair_kernels;    /* kernels of 3D levels: 2 (default): the colour-split layout, red and black cells in separate
                             arrays, so that one colour's sweep moves half the bytes (uniform levels in both
                             precisions, stretched ones in FP64); 1: the mixed form's cell pairs in the grid layout
-                            (Nz even, uniform or stretched; also what 2 gives on its stretched levels); 0: the
-                            general per-cell kernels. 2D levels: 2 (with one or two sweeps): a launch per leg of the
+                            (Nz even, uniform or stretched; also what 2 gives on its stretched levels, and on a
+                            grid for whose colour-split layout the device has no room); 0: the general per-cell
+                            kernels. 2D levels: 2 (with one or two sweeps): a launch per leg of the
                             V-cycle; else the per-cell kernels */
     int tail_cells;      /* the coarse end runs in one thread block from the first level with at most this many
                             cells, or the coarsest level alone whatever its cells (and shared memory for all of

@@ -395,7 +395,8 @@ constexpr int kWarps = kBlock / 32;
 // every block of the launch has read before any block can be the last).
 // addSlot0 >= 0 (sums only): each total also adds out[addSlot0 + s], the totals an earlier launch left there.
 // GridReduceB: the same over the blocks bid = 0 .. nblk-1 of one reduction (a batched launch runs one reduction per
-// request, each over its own blocks and Reducer). True on the one thread that stored the totals.
+// request, each over its own blocks and Reducer). True on the last block's first thread, after the totals are stored for
+// it to read where NV is 1 (lane s stores total s).
 //
 // Its latency ends every launch of a CG iteration that sums (about 5 us of a 12 us half-sweep on a 130^3 level), so a lane
 // per value adds the warps' sums, one acquire-release addition to the counter orders the partials, and the totals to add

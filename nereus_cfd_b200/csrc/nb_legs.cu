@@ -16,8 +16,12 @@
 // would need a cell outside the region belongs to a cell no result depends on.
 //
 // Measured (B200): the 64^3 cavity's step (three such levels, 16 iterations) 1.77 -> 1.38 ms, two 128^3 FLIP steps (such
-// levels from 66^3 down) 15.5 -> 13.5 ms, 256^3 (the same levels) 6.0 -> 5.9 ms. On a 130^3 level the recomputation
-// costs more than the launches: with its legs fused too the two FLIP steps took 16.5 ms.
+// levels from 66^3 down) 15.5 -> 13.5 ms, 256^3 (the same levels) 6.0 -> 5.9 ms. By level size, a whole step with the
+// level's legs in launches of their operations / in one launch each (FP32, FP64; us): 34^3 994 / 845, 1035 / 902; 50^3
+// 1243 / 1051, 1171 / 1021; 66^3 1259 / 1101, 1324 / 1148; 74^3 1443 / 1308, 1541 / 1509; 82^3 1710 / 1560, 1652 / 1609;
+// 98^3 1737 / 1704, 1743 / 1894; 114^3 2034 / 2329, 2257 / 2810; 130^3 2053 / 2636, 2625 / 3559, where the recomputation
+// costs more than the launches. Elongated levels gain too (122 x 122 x 18: 3741 / 3137, 3392 / 2843; 18 x 18 x 1002:
+// 1325 / 1167, 2623 / 2450).
 #include "nb_quad.cuh"
 
 namespace nb

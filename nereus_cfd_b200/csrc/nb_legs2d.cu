@@ -14,7 +14,9 @@
 // moved the pressure by up to 3e-7 of itself (FP32 rounding, carried through a solve to 1e-8).
 //
 // Measured (B200): the 128^2 closed box's step in mixed precision to 1e-10 (13 iterations, two such levels) 1.03 -> 0.79 ms
-// with the ring replay in one launch.
+// with the ring replay in one launch. No line in size: a step around a disc to 1e-10 with the per-cell kernels / with the
+// legs (mixed, FP64; ms) 64^2 1.02 / 0.84, 0.91 / 0.74; 256^2 1.59 / 1.15, 1.51 / 1.13; 1024^2 4.86 / 3.42, 4.36 / 3.30;
+// 2048^2 14.1 / 10.3, 12.8 / 10.0; 3900^2 71.4 / 48.7, 56.7 / 41.0.
 #include "nb_kernels.h"
 
 namespace nb
@@ -119,7 +121,8 @@ __global__ void __launch_bounds__(256) k_build_2d(LevelView v, LevelView cv, dou
         for (int q = 1; q < 4; q++)
         {
             const int di = q & 1, dj = q >> 1;
-            if (cv.types[(long long)(I + di * si) * cv.sI + J + dj * sj] == SOLID) moved += 4u * (di ? 1u : 3u) * (dj ? 1u : 3u);
+            if (cv.types[(long long)(I + di * si) * cv.sI + J + dj * sj] == SOLID)
+                moved += 4u * (di ? 1u : 3u) * (dj ? 1u : 3u);
         }
     }
     dg[c] = (double)d;

@@ -1110,8 +1110,8 @@ void LaunchLinXR(long long cells, T *x, T *r, const T *p0, const T *p1, const T 
 {
     const long long quads = cells * (long long)sizeof(T) / 16, want = (quads + 255) / 256;
     NB_COUNT_LAUNCH();
-    LaunchPdl(k_lin_xr<T>, dim3((unsigned)(want < 1 ? 1 : std::min<long long>(want, kLinBlocks))), dim3(256), 0, st, cells, x, r, p0, p1, q, R, S, it, baseEven, baseOdd,
-              slotN, singular, slotPQ, slotRR, lc);
+    LaunchPdl(k_lin_xr<T>, dim3((unsigned)(want < 1 ? 1 : std::min<long long>(want, kLinBlocks))), dim3(256), 0, st,
+              cells, x, r, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, lc);
 }
 
 template <typename T>
@@ -1126,23 +1126,19 @@ void LaunchSplitLinXR(const LevelView &v, long long vecLen, T *x, T *r, const T 
     }
     // no more blocks than tiles: on a 66^3 level the last block had 1184 partial sums to add for 396 tiles
     NB_COUNT_LAUNCH();
-    LaunchPdl(k_lin_xr_tiles<T>, dim3((unsigned)std::min(2 * v.Ny * v.actTiles, kLinBlocks)), dim3(256), 0, st, v, x, r, p0, p1, q, R, S, it, baseEven, baseOdd,
-              slotN, singular, slotPQ, slotRR, lc);
+    LaunchPdl(k_lin_xr_tiles<T>, dim3((unsigned)std::min(2 * v.Ny * v.actTiles, kLinBlocks)), dim3(256), 0, st, v, x, r,
+              p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, slotRR, lc);
 }
 
-template void LaunchLinXR<double>(long long, double *, double *, const double *, const double *, const double *,
-                                  const Reducer &, const double *, int *, int, int, int, int, int, int, cudaStream_t,
-    const LoopCond &);
-template void LaunchLinXR<float>(long long, float *, float *, const float *, const float *, const float *,
-                                 const Reducer &, const double *, int *, int, int, int, int, int, int, cudaStream_t,
-    const LoopCond &);
-template void LaunchSplitLinXR<float>(const LevelView &, long long, float *, float *, const float *, const float *,
-                                      const float *, const Reducer &, const double *, int *, int, int, int, int, int,
-                                      int, cudaStream_t,
-    const LoopCond &);
-template void LaunchSplitLinXR<double>(const LevelView &, long long, double *, double *, const double *,
-                                       const double *, const double *, const Reducer &, const double *, int *, int,
-                                       int, int, int, int, int, cudaStream_t,
-    const LoopCond &);
+#define NB_INST(T)                                                                                                 \
+    template void LaunchLinXR<T>(long long, T *, T *, const T *, const T *, const T *, const Reducer &,            \
+                                 const double *, int *, int, int, int, int, int, int, cudaStream_t,                \
+                                 const LoopCond &);                                                                \
+    template void LaunchSplitLinXR<T>(const LevelView &, long long, T *, T *, const T *, const T *, const T *,     \
+                                      const Reducer &, const double *, int *, int, int, int, int, int, int,        \
+                                      cudaStream_t, const LoopCond &);
+NB_INST(float)
+NB_INST(double)
+#undef NB_INST
 
 } // namespace nb

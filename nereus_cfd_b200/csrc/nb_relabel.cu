@@ -18,12 +18,11 @@
 //      the pass left them. The result is the unique solution of that recurrence, which is what is computed here:
 //        k_relabel_fill: four cells a thread, read as words; a cell none of whose upper neighbours is FLUID can get at
 //          most as many FLUID neighbours as it has lower ones, too few, so most of the air is passed over by
-//          comparing words. Filled cells get the
-//          marker kFilled, which counts as FLUID for the cells above and not at all for the cells below (they read
-//          the label from before the pass). A filled cell has at most one uncounted neighbour, so at most one of its
-//          upper neighbours can continue a chain of fills: the thread walks up that chain at once. A cell still EMPTY
-//          that could yet be filled once its lower neighbours are (the count with every EMPTY interior lower
-//          neighbour taken as filled reaches the threshold) goes on a pending list.
+//          comparing words. Filled cells get the marker kFilled, which counts as FLUID for the cells above and not at
+//          all for the cells below (they read the label from before the pass). A filled cell has at most one uncounted
+//          neighbour, so at most one of its upper neighbours can continue a chain of fills: the thread walks up that
+//          chain at once. A cell still EMPTY that could yet be filled once its lower neighbours are (the count with
+//          every EMPTY interior lower neighbour taken as filled reaches the threshold) goes on a pending list.
 //        k_relabel_settle: one block iterates over the pending list until a pass fills nothing. Every fill is
 //          justified by neighbours that belong to the solution, and every cell of the solution not yet filled is on
 //          the list, so the fixed point is the solution; each pass but the last fills at least one cell, which bounds

@@ -449,8 +449,8 @@ struct Context
     bool Split(int l) const { return L[l].sRS != 0; }
     // this shape runs on the grid layout's kernels although pair_kernels = 2 (WithRoom)
     bool lean = false;
-    // Levels of at most this many cells run their legs in one launch each: measured faster on 66^3 and below, slower on
-    // 130^3 (nb_legs.cu)
+    // Levels of at most this many cells run their legs in one launch each: faster at every size up to it, and in both
+    // precisions up to 82^3; slower in FP64 from 98^3 and in FP32 from 114^3 (the table in nb_legs.cu)
     static constexpr long long kLegCells = 300000;
     bool Legs(int l) const
     {

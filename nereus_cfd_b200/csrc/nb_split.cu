@@ -4,8 +4,9 @@
 //
 // Colour-split layout. Cell (i, j, k) has colour c = (i + j + k) & 1 and sits at c*H + i*PS + j*RS + (k >> 1) of a
 // level vector: each colour is an Ny x Nx x RS array whose rows hold that colour's cells (RS = (Nz+1)/2 rounded up
-// to 4, the padding kept at zero; with Nz odd the rows of one colour hold a cell less, its element counts as padding). In row (i, j) the cell of colour c at element m is k = 2m + q with
-// q = (i + j + c) & 1, and its six neighbours all have the other colour:
+// to 4, the padding kept at zero; with Nz odd the rows of one colour hold a cell less, its element counts as padding).
+// In row (i, j) the cell of colour c at element m is k = 2m + q with q = (i + j + c) & 1, and its six neighbours all have
+// the other colour:
 //   (i +- 1, j, m), (i, j +- 1, m), (i, j, m) and (i, j, m + (q ? 1 : -1)).
 // A half-sweep of colour c therefore reads the other colour, r and the diagonal bytes of colour c, and writes
 // colour c: half of every array, where a cell-pair sweep reads and writes both colours.
@@ -292,9 +293,9 @@ __device__ __forceinline__ void SplitResidual(const LevelView &v, const uint8_t 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kPairThreads, sizeof(T) == 8 ? 3 : 4) k_split_residual(LevelView v, const uint8_t *__restrict__ du,
-                                                                 const T *__restrict__ r,
-                                                                 const T *__restrict__ e, T *__restrict__ res)
+__global__ void __launch_bounds__(kPairThreads, sizeof(T) == 8 ? 3 : 4)
+    k_split_residual(LevelView v, const uint8_t *__restrict__ du, const T *__restrict__ r, const T *__restrict__ e,
+                     T *__restrict__ res)
 {
     PdlWait();
     PdlTrigger();
@@ -923,7 +924,8 @@ void LaunchSplitPApply(const LevelView &v, const uint8_t *du, const T *z, T *p0,
                        int singular, int slotPQ, cudaStream_t st)
 {
     if constexpr (sizeof(T) == 8)
-        if (v.stretched) return LaunchStretchedPApply(v, du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, st);
+        if (v.stretched)
+            return LaunchStretchedPApply(v, du, z, p0, p1, q, R, S, it, baseEven, baseOdd, slotN, singular, slotPQ, st);
     NB_COUNT_LAUNCH();
     if (singular)
         LaunchPdl(k_split_papply<T, true>, SumGrid(R, QuadGrid<kQ<T>>(v, Occ<k_split_papply<T, true>>())), kPairThreads, 0,
@@ -1246,8 +1248,8 @@ __global__ void __launch_bounds__(kPairThreads, 3)
     const BatchLevel &L = lv[q * ls];
     const BatchReq &Q = rq[q];
     const bool odd = parity[q] & 1;
-    SplitRefine64<float, true>(L.v, L.du, Q.b, odd ? Q.xout : Q.xin, Q.x, odd ? Q.xin : Q.xout, L.r, Q.scale, Q.sfac, Q.red, slot,
-                  ThisBlk());
+    SplitRefine64<float, true>(L.v, L.du, Q.b, odd ? Q.xout : Q.xin, Q.x, odd ? Q.xin : Q.xout, L.r, Q.scale, Q.sfac,
+                               Q.red, slot, ThisBlk());
 }
 
 namespace

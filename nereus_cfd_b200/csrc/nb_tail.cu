@@ -131,7 +131,10 @@ template <typename T> __device__ __forceinline__ int ListLen(const SmemLevel<T> 
 
 // A phase runs over the whole block (kWarp false) or over warp 0 alone (kWarp true), and ends with the matching
 // barrier.
-template <bool kWarp> __device__ __forceinline__ int PhaseStart() { return kWarp ? (int)(threadIdx.x & 31) : (int)threadIdx.x; }
+template <bool kWarp> __device__ __forceinline__ int PhaseStart()
+{
+    return kWarp ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
+}
 template <bool kWarp> __device__ __forceinline__ int PhaseStride() { return kWarp ? 32 : (int)blockDim.x; }
 template <bool kWarp> __device__ __forceinline__ void PhaseSync()
 {
