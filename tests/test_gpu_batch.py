@@ -184,3 +184,32 @@ def test_skipping_idle_tiles_changes_nothing(nb, jobs):
         out2, res2 = batched(b, jobs[:3])
     for o, r, o2, r2 in zip(out, res, out2, res2):
         assert_same(o, r, o2, r2)
+
+
+def test_an_overflowed_request_leaves_nothing_behind(nb):
+    """A request whose solve overflows in FP32 (velocities of 1e60: NOT_CONVERGED, no finite pressure) changes neither the
+    other requests of its batch nor a later step in its slot: both the bits of a batch that never saw it."""
+    import torch
+
+    jobs = tank_jobs(3)
+    bad = copy.deepcopy(jobs)
+    for f in ("u", "v", "w"):
+        getattr(bad[1].grid, f)[:] *= 1e60
+    with serving.Batch(3) as fresh:
+        for q, j in enumerate(jobs):
+            fresh.set_layout(q, j.grid)
+        expect, rexp = batched(fresh, jobs)
+    with serving.Batch(3) as b:
+        for q, j in enumerate(jobs):
+            b.set_layout(q, j.grid)
+        for _ in range(2):
+            js = [serving.to_device(copy.deepcopy(j)) for j in bad]
+            res = b.project(js)
+            torch.cuda.synchronize()
+            got = [serving.fetch(j) for j in js]
+            assert res[1]["status"] == capi.NB_NOT_CONVERGED and not np.all(np.isfinite(got[1].grid.p))
+            for q in (0, 2):
+                assert_same(got[q], res[q], expect[q], rexp[q])
+            again, ragain = batched(b, jobs)
+            for q in range(3):
+                assert_same(again[q], ragain[q], expect[q], rexp[q])

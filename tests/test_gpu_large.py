@@ -11,6 +11,7 @@
     (oracle/_ref/ref_harness, AMGCL SA+SPAI0 CG, run on this host): relative residual <= 1e-8, pressure within 1e-6
     relative L2 of the reference's solve at 1e-12, and max |div u| within 10x of the reference's at 1e-8, driven the
     way tests/suite_pressure.cpp:104-141 drives the reference.
+* A 2D box of 4608^2 cells, whose sums run over more blocks than a solver keeps room for at least, against numpy's sums.
 """
 import os
 
